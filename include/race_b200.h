@@ -269,6 +269,17 @@ int race_b200_bucket_probs_streams(const void* x, const float* planes, void* pro
                                    int32_t n_bits, int32_t dtype_x, int32_t dtype_probs, void* stream);
 
 /*
+ * Gradient of x for race_b200_bucket_probs_streams (the derivative of src/race_baseline.py:41-44, which the reference
+ * leaves to autograd): d_probs [outer*heads, seq_len, L, 2^K] -> d_x in the layout of x [outer, seq_len, heads, d_k];
+ * all three tensors have one type.  Geometries: race_b200_bucket_probs_bwd_is_supported (d_k = 64, L = 4, K = 4 and
+ * d_k = 128, L = 8, K = 6, fp32 and bf16).
+ */
+int race_b200_bucket_probs_bwd_is_supported(int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype);
+int race_b200_bucket_probs_streams_bwd(const void* x, const float* planes, const void* d_probs, void* d_x,
+                                       int64_t outer, int64_t seq_len, int32_t heads, int32_t d_k,
+                                       int32_t n_tables, int32_t n_bits, int32_t dtype, void* stream);
+
+/*
  * Host-buffer causal forward: same arithmetic as race_b200_causal_fwd with every tensor in
  * HOST memory (pinned for full copy bandwidth).  Allocates device staging buffers, streams
  * the sequence through them in segments (copy-in, kernel and copy-out overlapped on three

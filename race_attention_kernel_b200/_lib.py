@@ -27,6 +27,7 @@ EXPORTS = [
     "race_b200_static_scratch_bytes", "race_b200_causal_fwd_static", "race_b200_decode_step",
     "race_b200_causal_fwd_global", "race_b200_causal_bwd_workspace_bytes", "race_b200_causal_bwd",
     "race_b200_causal_bwd_carry", "race_b200_selftest_bounded_wait", "race_b200_host_release",
+    "race_b200_bucket_probs_bwd_is_supported", "race_b200_bucket_probs_streams_bwd",
     "race_b200_qkv_is_supported", "race_b200_causal_fwd_qkv",
 ]
 
@@ -76,6 +77,10 @@ def lib() -> ctypes.CDLL:
     L.race_b200_bucket_probs.argtypes = [vp, vp, vp, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_bucket_probs_streams.restype = i32
     L.race_b200_bucket_probs_streams.argtypes = [vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, i32, vp]
+    L.race_b200_bucket_probs_bwd_is_supported.restype = i32
+    L.race_b200_bucket_probs_bwd_is_supported.argtypes = [i32, i32, i32, i32]
+    L.race_b200_bucket_probs_streams_bwd.restype = i32
+    L.race_b200_bucket_probs_streams_bwd.argtypes = [vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_causal_fwd_host.restype = i32
     L.race_b200_causal_fwd_host.argtypes = [vp, vp, vp, vp, vp, vp, shp, i64, i32, i32]
     L.race_b200_host_release.restype = i32

@@ -270,7 +270,7 @@ int race_b200_selftest_bounded_wait(const void* probs_q, const void* probs_k, co
 
 size_t race_b200_causal_bwd_workspace_bytes(const RaceShape* shape) {
     Dims dm;
-    if (check_shape(shape, &dm) != RACE_OK || !causal_bwd_supported(dm)) return 0;
+    if (check_shape(shape, &dm) != RACE_OK || !causal_bwd_supported(dm, shape->dtype)) return 0;
     return causal_bwd_workspace_bytes(dm, shape->dtype, causal_bwd_tile_tokens(dm, shape->dtype, sm_count()));
 }
 
@@ -288,7 +288,7 @@ int race_b200_causal_bwd_carry(const void* probs_q, const void* probs_k, const v
     Dims dm;
     int rc = check_shape(shape, &dm);
     if (rc != RACE_OK) return rc;
-    if (!causal_bwd_supported(dm)) return RACE_ERR_SHAPE;
+    if (!causal_bwd_supported(dm, shape->dtype)) return RACE_ERR_SHAPE;
     if (dm.N == 0) return RACE_OK;
     if (dm.T == 0) {   // no tokens: the state passes through, and so does its gradient
         if (!d_carry_in) return RACE_OK;
@@ -440,6 +440,23 @@ int race_b200_bucket_probs_streams(const void* x, const float* planes, void* pro
                                    int32_t n_bits, int32_t dtype_x, int32_t dtype_probs, void* stream) {
     return probs_entry(x, planes, probs, outer, seq_len, heads, d_k, n_tables, n_bits, dtype_x, dtype_probs,
                        stream);
+}
+
+int race_b200_bucket_probs_bwd_is_supported(int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype) {
+    return bucket_probs_bwd_supported(d_k, n_tables, n_bits, dtype) ? 1 : 0;
+}
+
+int race_b200_bucket_probs_streams_bwd(const void* x, const float* planes, const void* d_probs, void* d_x, int64_t outer,
+                                       int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables, int32_t n_bits,
+                                       int32_t dtype, void* stream) {
+    if (outer < 0 || seq_len < 0 || heads < 1 || !bucket_probs_bwd_supported(d_k, n_tables, n_bits, dtype))
+        return RACE_ERR_SHAPE;
+    const int64_t rows = outer * heads * seq_len;
+    if (rows == 0) return RACE_OK;
+    if (!x || !planes || !d_probs || !d_x) return RACE_ERR_NULL;
+    if (!aligned16(x) || !aligned16(planes) || !aligned16(d_probs) || !aligned16(d_x)) return RACE_ERR_ALIGN;
+    return (int)bucket_probs_bwd(x, planes, d_probs, d_x, rows, seq_len, heads, d_k, n_tables, n_bits, dtype,
+                                 (cudaStream_t)stream);
 }
 
 }  // extern "C"

@@ -9,7 +9,7 @@
 //   bwd_prefix_pass : walks a tile forwards with B on chip; per chunk of 32 tokens
 //                       X = dO B^T + tril(dO V^T) pK ;  writes dPQ, and W, g to scratch;
 //                       B += pK^T V ;  tile totals of (W (x) dO, g)
-//   tile_scan_suffix: exclusive suffix scan of those totals over the tiles of a stream
+//   causal_scan_tiles (reverse): exclusive suffix scan of those totals over the tiles of a stream
 //   bwd_suffix_pass : walks a tile backwards with SB on chip; per chunk
 //                       dPK = SA + V SB^T + triu(V dO^T) W ;  dV = pK SB + triu(pK W^T) dO ;
 //                       SB += W^T dO ;  SA += colsum(g)
@@ -299,38 +299,6 @@ bwd_prefix_pass(const Tin* __restrict__ pq, const Tin* __restrict__ pk, const Ti
 }
 
 // ------------------------------------------------------------------------------------------
-// exclusive suffix scan over the tiles of a stream, one thread per state float
-// ------------------------------------------------------------------------------------------
-// d_state (nullable): gradient reaching the state after the last token, the carry of the last tile;
-// d_carry (nullable): receives the sum over all tiles + d_state, the gradient of the carried-in state
-__global__ void __launch_bounds__(128)
-tile_scan_suffix(float* __restrict__ ws, int64_t tiles, int state_floats, const float* __restrict__ d_state,
-                 float* __restrict__ d_carry) {
-    constexpr int kInFlight = 16;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= state_floats) return;
-    float* p = ws + (int64_t)blockIdx.y * tiles * state_floats + i;
-    float run = d_state ? d_state[(int64_t)blockIdx.y * state_floats + i] : 0.f;
-    int64_t t = tiles;
-    for (; t >= kInFlight; t -= kInFlight) {
-        float x[kInFlight];
-#pragma unroll
-        for (int j = 0; j < kInFlight; ++j) x[j] = p[(t - 1 - j) * state_floats];
-#pragma unroll
-        for (int j = 0; j < kInFlight; ++j) {
-            p[(t - 1 - j) * state_floats] = run;
-            run += x[j];
-        }
-    }
-    for (; t > 0; --t) {
-        const float x = p[(t - 1) * state_floats];
-        p[(t - 1) * state_floats] = run;
-        run += x;
-    }
-    if (d_carry) d_carry[(int64_t)blockIdx.y * state_floats + i] = run;
-}
-
-// ------------------------------------------------------------------------------------------
 // suffix pass: dPK and dV
 // ------------------------------------------------------------------------------------------
 template <typename Tin, int SPT, int DV>
@@ -551,9 +519,9 @@ cudaError_t launch_bwd(const Tin* pq, const Tin* pk, const Tin* v, const Tin* do
                                              groups);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    dim3 sgrid((unsigned)((sf + 127) / 128), (unsigned)dm.N);
-    tile_scan_suffix<<<sgrid, 128, 0, stream>>>(ws_suffix, tiles, sf, d_state, d_carry);
-    err = cudaGetLastError();
+    // d_state (nullable): gradient reaching the state after the last token, the carry of the last tile; d_carry
+    // (nullable): the sum over all tiles + d_state, the gradient of the carried-in state
+    err = causal_scan_tiles(ws_suffix, d_state, d_carry, dm, tile_tokens, stream, /*write_prefix=*/true, /*reverse=*/true);
     if (err != cudaSuccess) return err;
     // the bucket groups of a tile form one thread-block cluster: they add their shares of dV through
     // distributed shared memory
@@ -593,8 +561,9 @@ cudaError_t dispatch_bwd(const void* pq, const void* pk, const void* v, const vo
 
 }  // namespace
 
-bool causal_bwd_supported(const Dims& dm) {
-    return simt_supported(dm) && dm.H == 1;   // S <= 64, or a multiple of 64 up to 512 (one cluster); d_k <= 128
+bool causal_bwd_supported(const Dims& dm, int dtype) {
+    // S <= 64, or a multiple of 64 up to 512 (one cluster); d_k <= 128; V, dO, dV with heads on the tensor kernels only
+    return simt_supported(dm) && (dm.H == 1 || causal_bwd_tensor_supported(dm, dtype));
 }
 
 int causal_bwd_tile_tokens(const Dims& dm, int dtype, int sm_count) {

@@ -19,6 +19,7 @@
 //                                              total the gradient of the carried-in B
 //     4. P  = raw_reverse(V, dO, W)            state = the transpose of pass 3's
 //     5. reverse scan of the chunk sums of g (carry: gradient of the final A), then dPK = P + running suffix sum
+// V, dO and dV may be in the layout [N / heads, T, heads, 64] (dm.H > 1).
 // P is written into the dPK buffer (same shape and type), so the scratch memory is W and g ([N, T, 64] fp32 each)
 // plus the block / chunk sums and the tile states of the passes.
 #include <algorithm>
@@ -196,7 +197,7 @@ BwdLayout bwd_layout(const Dims& dm, int tile_tokens) {
 }  // namespace
 
 bool causal_bwd_tensor_supported(const Dims& dm, int dtype) {
-    return dtype == RACE_DTYPE_F32 && dm.H == 1 && tensor_supported(dm, dtype);
+    return dtype == RACE_DTYPE_F32 && tensor_supported(dm, dtype);
 }
 
 int causal_bwd_tensor_tile_tokens(const Dims& dm, int sm_count) {
@@ -247,23 +248,23 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     bx.block_tokens = kBlk;
     bx.eps = dm.eps;
     RACE_CK(causal_raw_tensor(dout, v, pk, dpq, carry_in ? st_t : nullptr, nullptr, ws_tiles, dm, tile_tokens,
-                              /*reverse=*/false, stream, status, kPhaseAll, &bx));
+                              /*reverse=*/false, stream, status, kPhaseAll, &bx, dm.H, dm.H, 1, 1));
     bwd_block_sums<<<pw_grid, kPwThreads, 0, stream>>>(g, gsum, dm.T, nblk, total_blocks);
     RACE_CK(cudaGetLastError());
     // 3. dV = raw_reverse(pK, W, dO); state sum W^T dO: carry = gradient of the final B, total = gradient of carry_in's B.
     //    Pass 4 below has the roles of W and dO swapped, so its tile totals are the transposes of this pass's:
     //    the totals launch runs once and the second tile buffer gets the transposed states.
     RACE_CK(causal_raw_tensor(nullptr, w, dout, nullptr, nullptr, nullptr, ws_tiles, dm, tile_tokens, true, stream, status,
-                              kPhaseTotals));
+                              kPhaseTotals, nullptr, 1, 1, dm.H, 1));
     bwd_transpose_state<<<(unsigned)(dm.N * tiles), 256, 0, stream>>>(ws_tiles, ws_tiles2);
     RACE_CK(cudaGetLastError());
     RACE_CK(causal_raw_tensor(pk, w, dout, dv, d_state, d_carry ? d_carry : st_dv, ws_tiles, dm, tile_tokens,
-                              /*reverse=*/true, stream, status, kPhaseOutput));
+                              /*reverse=*/true, stream, status, kPhaseOutput, nullptr, 1, 1, dm.H, dm.H));
     // 4. P = raw_reverse(V, dO, W) into the dPK buffer; state = the transpose of pass 3's
     if (d_state) bwd_transpose_state<<<(unsigned)dm.N, 256, 0, stream>>>(d_state, st_t);
     RACE_CK(cudaGetLastError());
     RACE_CK(causal_raw_tensor(v, dout, w, dpk, d_state ? st_t : nullptr, nullptr, ws_tiles2, dm, tile_tokens,
-                              /*reverse=*/true, stream, status, kPhaseOutput));
+                              /*reverse=*/true, stream, status, kPhaseOutput, nullptr, dm.H, dm.H, 1, 1));
     // 5. dPK = P + suffix sums of g (carry: gradient of the final A; total: gradient of carry_in's A, which
     //    overwrites the A part that pass 3 left in d_carry)
     bwd_block_scan<<<(unsigned)dm.N, 64, 0, stream>>>(gsum, d_state, d_carry, nblk, 1);

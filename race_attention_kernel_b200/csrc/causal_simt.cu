@@ -128,7 +128,10 @@ tile_totals_simt(const Tin* __restrict__ pk, const Tin* __restrict__ v, float* _
 }
 
 // ------------------------------------------------------------------------------------------
-// K2: exclusive scan over tiles, one thread per state float, 32 loads in flight
+// K2: exclusive scan over tiles, one thread per state float, up to 32 loads in flight.  Bound by the read and the
+// write of the tile states: a batch that is not full is loaded under predicates, all of it before its first use (a
+// loop over the remaining tiles ran one dependent load and store at a time, because the store may alias the next
+// load: 16 tiles of 32 streams at S = 512, d_k = 128, 135 MB of states, took 0.67 ms).
 // ------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128)
 tile_scan(float* __restrict__ ws, const float* __restrict__ carry_in, float* __restrict__ state_out,
@@ -138,24 +141,19 @@ tile_scan(float* __restrict__ ws, const float* __restrict__ carry_in, float* __r
     if (i >= state_floats) return;
     const int64_t n = blockIdx.y;
     float run = carry_in ? carry_in[n * state_floats + i] : 0.f;
-    float* p = ws + n * tiles * state_floats + i;
     // reverse: exclusive SUFFIX sums -- slot t gets carry + the totals of the tiles after t (last tile first)
-    auto at = [&](int64_t t) { return (reverse ? tiles - 1 - t : t) * state_floats; };
-    int64_t t = 0;
-    for (; t + kInFlight <= tiles; t += kInFlight) {
+    float* p = ws + (n * tiles + (reverse ? tiles - 1 : 0)) * state_floats + i;
+    const int64_t step = reverse ? -state_floats : state_floats;
+    for (int64_t t = 0; t < tiles; t += kInFlight, p += kInFlight * step) {
+        const int cnt = (int)min((int64_t)kInFlight, tiles - t);
         float x[kInFlight];
 #pragma unroll
-        for (int j = 0; j < kInFlight; ++j) x[j] = p[at(t + j)];
+        for (int j = 0; j < kInFlight; ++j) x[j] = j < cnt ? p[j * step] : 0.f;
 #pragma unroll
         for (int j = 0; j < kInFlight; ++j) {
-            if (write_prefix) p[at(t + j)] = run;
+            if (write_prefix && j < cnt) p[j * step] = run;
             run += x[j];
         }
-    }
-    for (; t < tiles; ++t) {
-        const float x = p[at(t)];
-        if (write_prefix) p[at(t)] = run;
-        run += x;
     }
     if (state_out) state_out[n * state_floats + i] = run;
 }

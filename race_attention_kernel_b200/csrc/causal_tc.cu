@@ -230,13 +230,16 @@ __device__ __forceinline__ void out_phase_init_bars(const Ctx& cx, bool again, u
 // kModeRawX: the plain product with the epilogue of the first backward pass (BwdX in launch.h): after G . V the
 // issuer also runs the triangular running-sum product over the chunk's V operand into the accumulator that G has
 // left, and the worker warps turn X (the product) into dPQ, W and g where they would store it.
+struct Heads {   // head counts of the layouts [N/h, T, h, 64] of the four tensors of a pass (1: plain [N, T, 64])
+    int q, k, v, o;
+};
 constexpr int kModeBucket = 0, kModeGlobal = 1, kModeRaw = 2, kModeRawX = 3;
 template <int kMode, bool kReverse = false, bool kProj = false, bool kWorkerK = kProj>
 __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, const float* __restrict__ pq,
                                           const CUtensorMap* map_k, const CUtensorMap* map_v,
                                           float* __restrict__ out, const float* __restrict__ slice, int64_t T,
                                           const int64_t t_begin, const int64_t t_end, const int64_t n, float eps,
-                                          int heads, int withhold_chunk, const bool l2_last_use = false,
+                                          const Heads hd, int withhold_chunk, const bool l2_last_use = false,
                                           const uint32_t* ptab = nullptr, const BwdX* bx = nullptr) {
     constexpr bool kGlobal = kMode == kModeGlobal;
     constexpr bool kRaw = kMode == kModeRaw || kMode == kModeRawX;   // no running sum, no normalisation in the W stage
@@ -257,12 +260,11 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
         const int wg = warp >> 2, w = warp & 3;
         const int q = lane & 3, rbase = 16 * w + (lane >> 2);
         const uint32_t lane_base = (uint32_t)(32 * w) << 16;
-        // V and out are [N/heads, T, heads, D]: stream n = outer * heads + h (heads = 1: plain [N, T, D])
-        const int64_t orow_stride = (int64_t)heads * D;
-        float* out_n = out + ((n / heads) * T * heads + (n % heads)) * D;
-        // probabilities [N, T, S]; with kProj the rows of Q in the layout of V
-        const float* pq_n = kProj ? pq + ((n / heads) * T * heads + (n % heads)) * D : pq + n * T * S;
-        const int64_t pq_stride = kProj ? orow_stride : (int64_t)S;
+        // [N/h, T, h, D]: stream n = outer * h + head (h = 1: plain [N, T, D])
+        const int64_t orow_stride = (int64_t)hd.o * D;
+        float* out_n = out + ((n / hd.o) * T * hd.o + (n % hd.o)) * D;
+        const float* pq_n = pq + ((n / hd.q) * T * hd.q + (n % hd.q)) * D;
+        const int64_t pq_stride = (int64_t)hd.q * D;
         float v[32];
         uint32_t ohi[16], olo[16];   // operand limbs of W / masked G on their way to tensor memory
 
@@ -637,12 +639,11 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
                 const int tok = (int)chunk_tok0(c);
                 mbar_arrive_expect_tx(bar, kStageBytes);
                 if (l2_last_use) {
-                    tma_load_4d_hint(dst, map_k, bar, 0, tok, 0, (int)n, pol);
-                    tma_load_5d_hint(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads), pol);
+                    tma_load_5d_hint(dst, map_k, bar, 0, tok, 0, (int)(n % hd.k), (int)(n / hd.k), pol);
+                    tma_load_5d_hint(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % hd.v), (int)(n / hd.v), pol);
                 } else {
-                    if (kProj) tma_load_5d(dst, map_k, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads));
-                    else tma_load_4d(dst, map_k, bar, 0, tok, 0, (int)n);
-                    tma_load_5d(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads));
+                    tma_load_5d(dst, map_k, bar, 0, tok, 0, (int)(n % hd.k), (int)(n / hd.k));
+                    tma_load_5d(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % hd.v), (int)(n / hd.v));
                 }
                 issued = c + 1;
             }
@@ -752,7 +753,7 @@ template <int kMode, bool kReverse, bool kProj>
 __global__ void __launch_bounds__(kThreads, 1)
 causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, float* __restrict__ out,
-              const float* __restrict__ ws, int64_t T, int tile_tokens, float eps, int heads, int* status,
+              const float* __restrict__ ws, int64_t T, int tile_tokens, float eps, const Heads hd, int* status,
               long long wait_cycles, int withhold_chunk, const float* __restrict__ planes, const BwdX bwdx) {
     extern __shared__ uint8_t smem_raw[];
     Ctx cx;
@@ -784,7 +785,7 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     out_phase<kMode, kReverse, kProj, kWorkerK>(cx, tmem, pq, &map_k, &map_v, out, slice, T, t_begin, t_end, n, eps,
-                                                heads, (tile == 0 && n == 0) ? withhold_chunk : -1, false, ptab, &bwdx);
+                                                hd, (tile == 0 && n == 0) ? withhold_chunk : -1, false, ptab, &bwdx);
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -918,7 +919,7 @@ __device__ __forceinline__ void totals_phase_init_bars(const Ctx& cx, bool again
 template <bool kProj = false, typename TL = T1>
 __device__ __forceinline__ void totals_phase(const Ctx& cx, const uint32_t tmem, const CUtensorMap* map_k,
                                              const CUtensorMap* map_v, float* __restrict__ slice,
-                                             const int64_t t_begin, const int64_t t_end, const int64_t n, int heads,
+                                             const int64_t t_begin, const int64_t t_end, const int64_t n, const Heads hd,
                                              const bool l2_keep = false, const uint32_t* ptab = nullptr) {
     constexpr int kT1Groups = TL::kGroups, kT1Stages = TL::kStages, kT1ProducerWarp = TL::kProducerWarp,
                   kT1MmaWarp = TL::kMmaWarp, o1Stage = TL::oStage, o1Kt = TL::oKt, o1Vt = TL::oVt, o1Red = TL::oRed,
@@ -998,12 +999,11 @@ __device__ __forceinline__ void totals_phase(const Ctx& cx, const uint32_t tmem,
                 const int tok = (int)(t_begin + (int64_t)c * C);
                 mbar_arrive_expect_tx(bar, kT1StageBytes);
                 if (l2_keep) {
-                    tma_load_4d_hint(dst, map_k, bar, 0, tok, 0, (int)n, pol);
-                    tma_load_5d_hint(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads), pol);
+                    tma_load_5d_hint(dst, map_k, bar, 0, tok, 0, (int)(n % hd.k), (int)(n / hd.k), pol);
+                    tma_load_5d_hint(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % hd.v), (int)(n / hd.v), pol);
                 } else {
-                    if (kProj) tma_load_5d(dst, map_k, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads));
-                    else tma_load_4d(dst, map_k, bar, 0, tok, 0, (int)n);
-                    tma_load_5d(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads));
+                    tma_load_5d(dst, map_k, bar, 0, tok, 0, (int)(n % hd.k), (int)(n / hd.k));
+                    tma_load_5d(dst + kTileF32, map_v, bar, 0, tok, 0, (int)(n % hd.v), (int)(n / hd.v));
                 }
                 issued = c + 1;
                 RACE_PROF_LANE(12, tq);
@@ -1085,7 +1085,7 @@ template <bool kProj> using TotalsLayoutOf = std::conditional_t<kProj, T1P, T1>;
 template <bool kProj>
 __global__ void __launch_bounds__(TotalsLayoutOf<kProj>::kThreads, 1)
 tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-               float* __restrict__ ws, int64_t T, int tile_tokens, int heads, int* status,
+               float* __restrict__ ws, int64_t T, int tile_tokens, const Heads hd, int* status,
                const float* __restrict__ planes) {
     extern __shared__ uint8_t smem_raw[];
     Ctx cx;
@@ -1112,7 +1112,7 @@ tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    totals_phase<kProj, TL>(cx, tmem, &map_k, &map_v, slice, t_begin, t_end, n, heads, false, ptab);
+    totals_phase<kProj, TL>(cx, tmem, &map_k, &map_v, slice, t_begin, t_end, n, hd, false, ptab);
     tc_fence_before();
     __syncthreads();
     if (warp == TL::kMmaWarp) {
@@ -1223,7 +1223,8 @@ causal_fused_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         (void)tp;
         if (warp == 0) totals_phase_reinit_bars_warp(cxA, tid, !first);
         __syncthreads();
-        totals_phase(cxA, tmem, &map_k, &map_v, agg_n + tile * kSF, t_begin, t_end, n, a.heads, /*l2_keep=*/true);
+        totals_phase(cxA, tmem, &map_k, &map_v, agg_n + tile * kSF, t_begin, t_end, n, Heads{1, 1, a.heads, a.heads},
+                     /*l2_keep=*/true);
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
@@ -1314,7 +1315,7 @@ causal_fused_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant
 
         // ---- 3. outputs of the tile ---------------------------------------------------------------
         out_phase<kGlobal ? kModeGlobal : kModeBucket>(cxB, tmem, a.pq, &map_k, &map_v, a.out, a.cta_carry + (int64_t)blockIdx.x * kSF, a.T,
-                           t_begin, t_end, n, a.eps, a.heads, (tile == 0 && n == 0) ? a.withhold_chunk : -1,
+                           t_begin, t_end, n, a.eps, Heads{1, 1, a.heads, a.heads}, (tile == 0 && n == 0) ? a.withhold_chunk : -1,
                            /*l2_last_use=*/true);
         first = false;
         fence_proxy_async();
@@ -1368,19 +1369,6 @@ bool make_map_heads(CUtensorMap* map, const void* base, int64_t N, int64_t T, in
     cuuint32_t box[5] = {32, (cuuint32_t)C, (cuuint32_t)(width / 32), 1, 1};
     cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<void*>(base), dims, strides, box, estr,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// [N][T][width] fp32 viewed as (32 values, T tokens, width/32 column blocks, N streams); boxes as above
-bool make_map(CUtensorMap* map, const void* base, int64_t N, int64_t T, int width) {
-    auto fn = encode_fn();
-    if (!fn) return false;
-    cuuint64_t dims[4] = {32, (cuuint64_t)T, (cuuint64_t)(width / 32), (cuuint64_t)N};
-    cuuint64_t strides[3] = {(cuuint64_t)width * 4, 128, (cuuint64_t)T * width * 4};
-    cuuint32_t box[4] = {32, (cuuint32_t)C, (cuuint32_t)(width / 32), 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<void*>(base), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -1453,7 +1441,7 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
                                      const float* carry_in, float* state_out, void* ws, bool single_pass,
                                      const Dims& dm, int tile_tokens, cudaStream_t stream, int* status, int phases,
                                      int mode, bool reverse, long long wait_cycles, int withhold_chunk,
-                                     const float* planes = nullptr, const BwdX* bwdx = nullptr);
+                                     const Heads hd, const float* planes = nullptr, const BwdX* bwdx = nullptr);
 
 cudaError_t causal_fwd_tensor(const void* pq, const void* pk, const void* v, void* out,
                               const float* carry_in, float* state_out, void* ws, bool single_pass, const Dims& dm,
@@ -1463,7 +1451,8 @@ cudaError_t causal_fwd_tensor(const void* pq, const void* pk, const void* v, voi
         return causal_fwd_tensor_bf16(pq, pk, v, out, carry_in, state_out, ws, dm, tile_tokens, stream,
                                       status, phases, global_norm);
     return tensor_f32_launch(pq, pk, v, out, carry_in, state_out, ws, single_pass, dm, tile_tokens, stream, status,
-                             phases, global_norm ? kModeGlobal : kModeBucket, false, wait_cycles, withhold_chunk);
+                             phases, global_norm ? kModeGlobal : kModeBucket, false, wait_cycles, withhold_chunk,
+                             Heads{1, 1, dm.H, dm.H});
 }
 
 // The causal forward from Q, K, V and the hyperplanes (fp32, d_k = 64, L = 4, R = 16; Q, K, V and out in the layout
@@ -1478,7 +1467,7 @@ cudaError_t causal_fwd_qkv_tensor(const void* q, const void* k, const void* v, c
                                   cudaStream_t stream, int* status, int phases, bool global_norm) {
     if (!planes) return cudaErrorInvalidValue;
     return tensor_f32_launch(q, k, v, out, carry_in, state_out, ws, false, dm, tile_tokens, stream, status, phases,
-                             global_norm ? kModeGlobal : kModeBucket, false, 0, -1, planes);
+                             global_norm ? kModeGlobal : kModeBucket, false, 0, -1, Heads{dm.H, dm.H, dm.H, dm.H}, planes);
 }
 
 // The plain causal (or, with reverse, anti-causal) product out_t = sum_{j <= t} (q_t . k_j) v_j + q_t . carry over
@@ -1486,10 +1475,11 @@ cudaError_t causal_fwd_qkv_tensor(const void* q, const void* k, const void* v, c
 // everywhere: carry[s][c] = sum_j k_j[s] v_j[c] (the A part is carried along and ignored).
 cudaError_t causal_raw_tensor(const void* q, const void* k, const void* v, void* out, const float* carry_in,
                               float* state_out, void* ws, const Dims& dm, int tile_tokens, bool reverse,
-                              cudaStream_t stream, int* status, int phases, const BwdX* bwdx) {
-    if (bwdx && (reverse || dm.H != 1)) return cudaErrorInvalidValue;
+                              cudaStream_t stream, int* status, int phases, const BwdX* bwdx, int hq, int hk, int hv,
+                              int ho) {
+    if (bwdx && (reverse || ho != 1)) return cudaErrorInvalidValue;
     return tensor_f32_launch(q, k, v, out, carry_in, state_out, ws, false, dm, tile_tokens, stream, status, phases,
-                             bwdx ? kModeRawX : kModeRaw, reverse, 0, -1, nullptr, bwdx);
+                             bwdx ? kModeRawX : kModeRaw, reverse, 0, -1, Heads{hq, hk, hv, ho}, nullptr, bwdx);
 }
 
 // planes != nullptr: pq and pk are Q and K in the layout of V and the kernels form the probabilities (the
@@ -1498,7 +1488,7 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
                                      const float* carry_in, float* state_out, void* ws, bool single_pass,
                                      const Dims& dm, int tile_tokens, cudaStream_t stream, int* status, int phases,
                                      int mode, bool reverse, long long wait_cycles, int withhold_chunk,
-                                     const float* planes, const BwdX* bwdx) {
+                                     const Heads hd, const float* planes, const BwdX* bwdx) {
     const bool global_norm = mode == kModeGlobal;
     const bool proj = planes != nullptr;
     const bool raw = mode == kModeRaw || mode == kModeRawX;
@@ -1512,8 +1502,7 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
     cudaError_t err = cudaFuncSetAttribute(totals_kern, cudaFuncAttributeMaxDynamicSharedMemorySize, totals_smem);
     if (err != cudaSuccess) return err;
     CUtensorMap mk, mv;
-    if (!(proj ? make_map_heads(&mk, pk, dm.N, dm.T, dm.D, dm.H) : make_map(&mk, pk, dm.N, dm.T, dm.S)) ||
-        !make_map_heads(&mv, v, dm.N, dm.T, dm.D, dm.H))
+    if (!make_map_heads(&mk, pk, dm.N, dm.T, dm.D, hd.k) || !make_map_heads(&mv, v, dm.N, dm.T, dm.D, hd.v))
         return cudaErrorInvalidValue;
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
     const FusedLayout lay = fused_layout(dm, tile_tokens);
@@ -1552,7 +1541,7 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
     dim3 grid((unsigned)tiles, (unsigned)dm.N);
     // 1. tile totals (tensor cores)  2. exclusive scan over tiles  3. output pass
     if (phases & kPhaseTotals) {
-        totals_kern<<<grid, totals_threads, totals_smem, stream>>>(mk, mv, (float*)ws, dm.T, tile_tokens, dm.H, status,
+        totals_kern<<<grid, totals_threads, totals_smem, stream>>>(mk, mv, (float*)ws, dm.T, tile_tokens, hd, status,
                                                                 planes);
         err = cudaGetLastError();
         if (err != cudaSuccess) return err;
@@ -1574,7 +1563,7 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (err != cudaSuccess) return err;
     kern<<<grid, kThreads, kSmemBytes, stream>>>((const float*)pq, mk, mv, (float*)out, (const float*)ws, dm.T,
-                                                 tile_tokens, dm.eps, dm.H, status, wait_cycles, withhold_chunk, planes,
+                                                 tile_tokens, dm.eps, hd, status, wait_cycles, withhold_chunk, planes,
                                                  bwdx ? *bwdx : BwdX{});
     return cudaGetLastError();
 }

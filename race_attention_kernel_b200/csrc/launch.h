@@ -28,7 +28,7 @@ cudaError_t causal_scan_tiles(float* ws, const float* carry_in, float* state_out
 constexpr int kPhaseTotals = 1, kPhaseOutput = 2, kPhaseAll = 3;
 
 // ---- causal backward (causal_bwd_simt.cu): S <= 64, d_k <= 128 ---------------------------------
-bool causal_bwd_supported(const Dims& dm);
+bool causal_bwd_supported(const Dims& dm, int dtype);
 int causal_bwd_tile_tokens(const Dims& dm, int dtype, int sm_count);
 size_t causal_bwd_workspace_bytes(const Dims& dm, int dtype, int tile_tokens);
 // carry_in: state before the first token (nullable); d_state: gradient reaching the state after the last token
@@ -59,6 +59,11 @@ cudaError_t noncausal_token_grads_tensor(const void* pk, const void* v, const vo
 cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
                          int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream);
 
+// dx of the same (bucket_probs_bwd.cu): dprobs [outer*heads, T, L, 2^K] and x, dx [outer, T, heads, d], one type
+bool bucket_probs_bwd_supported(int d, int L, int K, int dtype);
+cudaError_t bucket_probs_bwd(const void* x, const float* planes, const void* dprobs, void* dx, int64_t rows, int64_t T,
+                             int heads, int d, int L, int K, int dtype, cudaStream_t stream);
+
 // ---- incremental step (decode.cu) -------------------------------------------------------------
 // a few new tokens per stream (dm.T <= decode_max_tokens()) against a running state; state_in may be
 // null (zeros) or equal state_out (in place)
@@ -82,7 +87,8 @@ cudaError_t causal_fwd_tensor(const void* pq, const void* pk, const void* v, voi
                               int withhold_chunk = -1);
 
 // out_t = sum_{j <= t} (q_t . k_j) v_j + q_t . carry (reverse: j >= t, carry = state of the tokens after the call)
-// on fp32 [N, T, 64] tensors with the three launches of the fp32 tensor forward, no normalisation
+// on fp32 [N, T, 64] tensors with the three launches of the fp32 tensor forward, no normalisation; hq, hk, hv, ho > 1:
+// that tensor is laid out [N / h, T, h, 64]
 // The causal forward from Q, K, V and the hyperplanes [16][64] on the fp32 tensor kernels (d_k = 64, L = 4, R = 16);
 // Q, K, V, out in the layout [N/heads, T, heads, 64]; workspace as for the three-launch form.
 bool tensor_qkv_supported(const Dims& dm, int dtype, int L, int R);
@@ -105,7 +111,8 @@ struct BwdX {
 };
 cudaError_t causal_raw_tensor(const void* q, const void* k, const void* v, void* out, const float* carry_in,
                               float* state_out, void* ws, const Dims& dm, int tile_tokens, bool reverse,
-                              cudaStream_t stream, int* status, int phases = kPhaseAll, const BwdX* bwdx = nullptr);
+                              cudaStream_t stream, int* status, int phases = kPhaseAll, const BwdX* bwdx = nullptr,
+                              int hq = 1, int hk = 1, int hv = 1, int ho = 1);
 
 // ---- causal backward on the tensor kernels (causal_bwd_tc.cu): fp32, S = 64, d_k = 64 ----------
 bool causal_bwd_tensor_supported(const Dims& dm, int dtype);

@@ -12,9 +12,9 @@ accepted and streamed through the device; there is no CPU compute path.
 
 Gradients: the reference module is differentiable through K, V and Q (plain autograd over
 src/race_baseline.py:41-51).  Here, when autograd is recording and an input requires a gradient,
-``forward`` forms the bucket probabilities with differentiable torch ops on the GPU (the producer
-kernel has no backward) and runs the prefix path through ``ops.race_causal`` -- the same forward
-kernels with the hand-written backward kernels.  Without gradients it is the pure kernel path.
+``forward`` is one autograd node over the kernels: the producer, the prefix forward, and for the gradients
+the causal backward and the backward of the producer.  Geometries the producer's backward does not cover form
+the bucket probabilities with differentiable torch ops and run the prefix path through ``ops.race_causal``.
 """
 from __future__ import annotations
 
@@ -24,6 +24,57 @@ import torch
 from torch import nn
 
 from . import ops
+
+
+class _CausalOperator(torch.autograd.Function):
+    """``BatchedACE.forward`` with gradients for K, V and Q ([M,B,T,H,d_k], contiguous, on the GPU; planes [L*K, d_k]).
+    Saved: the inputs and the two probability tensors; the backward recomputes the prefix states tile by tile."""
+
+    @staticmethod
+    def forward(ctx, Khf, Vhf, Qhf, planes, L, K, eps):
+        M, B, T, H, dk = Khf.shape
+        pK = ops.bucket_probs_streams(Khf, planes, L, K)
+        pQ = ops.bucket_probs_streams(Qhf, planes, L, K)
+        shape = (M * B * H, T, L, 1 << K, dk, Vhf.dtype)
+        V2 = None
+        if ops.is_supported(*shape, "auto", heads=H):
+            out = ops.race_causal_prefix(pQ, pK, Vhf, eps)
+        else:
+            V2 = _streams(Vhf)
+            out = _unstreams(ops.race_causal_prefix(pQ, pK, V2, eps), M, B, H)
+        ctx.bwd_heads = ops.causal_bwd_takes_heads(*shape, H)
+        if ctx.bwd_heads or V2 is None:
+            V2 = Vhf
+        ctx.save_for_backward(Khf, V2, Qhf, pK, pQ, planes)
+        ctx.dims, ctx.eps = (M, B, H, L, K), eps
+        return out
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_out):
+        Khf, V, Qhf, pK, pQ, planes = ctx.saved_tensors
+        M, B, H, L, K = ctx.dims
+        want_k, want_v, want_q = ctx.needs_input_grad[:3]
+        grad_out = grad_out.to(V.dtype)
+        if ctx.bwd_heads:
+            dpq, dpk, dV = ops.race_causal_backward(pQ, pK, V, grad_out, ctx.eps)
+        else:
+            V2 = V if V.dim() == 3 else _streams(V)
+            dpq, dpk, dV = ops.race_causal_backward(pQ, pK, V2, _streams(grad_out), ctx.eps)
+            dV = _unstreams(dV, M, B, H)
+        dK = ops.bucket_probs_streams_bwd(Khf, planes, dpk, L, K) if want_k else None
+        dQ = ops.bucket_probs_streams_bwd(Qhf, planes, dpq, L, K) if want_q else None
+        return dK, dV if want_v else None, dQ, None, None, None, None
+
+
+def _streams(x: torch.Tensor) -> torch.Tensor:
+    """[M,B,T,H,d_k] -> [M*B*H, T, d_k] (src/race_baseline.py:35-40)."""
+    M, B, T, H, dk = x.shape
+    return x.permute(0, 1, 3, 2, 4).contiguous().view(M * B * H, T, dk)
+
+
+def _unstreams(x2: torch.Tensor, M: int, B: int, H: int) -> torch.Tensor:
+    return x2.view(M, B, H, *x2.shape[1:]).permute(0, 1, 3, 2, 4)
 
 
 class BatchedACE(nn.Module):
@@ -45,8 +96,7 @@ class BatchedACE(nn.Module):
         self.fuse_producer = True
 
     def _streams(self, x: torch.Tensor) -> torch.Tensor:
-        M, B, T, H, dk = x.shape
-        return x.permute(0, 1, 3, 2, 4).contiguous().view(M * B * H, T, dk)
+        return _streams(x)
 
     def bucket_probs(self, x2: torch.Tensor) -> torch.Tensor:
         """[N,T,d_k] -> [N,T,L,R] with this module's planes."""
@@ -65,6 +115,11 @@ class BatchedACE(nn.Module):
     def _forward_autograd(self, Khf, Vhf, Qhf):
         M, B, T, H, dk = Khf.shape
         dev = self.planes_T.device if self.planes_T.is_cuda else torch.device("cuda", torch.cuda.current_device())
+        if (ops.bucket_probs_bwd_is_supported(dk, self.L, self.K, Khf.dtype)
+                and not (self.planes_T.requires_grad or self.protos_T.requires_grad)):
+            planes = self.planes_T.T.contiguous().float().to(dev)
+            out = _CausalOperator.apply(*(t.to(dev).contiguous() for t in (Khf, Vhf, Qhf)), planes, self.L, self.K, self.eps)
+            return out if Khf.is_cuda else out.cpu()
         K2, V2, Q2 = (self._streams(t.to(dev)) for t in (Khf, Vhf, Qhf))
         out2 = ops.race_causal(self._probs_autograd(Q2), self._probs_autograd(K2), V2, self.eps)
         out = out2.view(M, B, H, T, dk).permute(0, 1, 3, 2, 4)

@@ -401,6 +401,30 @@ def bucket_probs_streams(x: torch.Tensor, planes: torch.Tensor, L: int, K: int,
     return probs
 
 
+def bucket_probs_bwd_is_supported(dk: int, L: int, K: int, dtype=torch.float32) -> bool:
+    return dtype in _DTYPES and bool(_lib.lib().race_b200_bucket_probs_bwd_is_supported(dk, L, K, _DTYPES[dtype]))
+
+
+def bucket_probs_streams_bwd(x: torch.Tensor, planes: torch.Tensor, d_probs: torch.Tensor, L: int, K: int) -> torch.Tensor:
+    """Gradient of ``bucket_probs_streams(x, planes, L, K)`` in x for the gradient ``d_probs`` [M*B*H, T, L, 2**K] of
+    its result (geometries: ``bucket_probs_bwd_is_supported``)."""
+    if not x.is_cuda or x.dtype not in _DTYPES or not x.is_contiguous() or x.dim() != 5:
+        raise RuntimeError("x must be a contiguous fp32/bf16 CUDA tensor [M,B,T,H,d_k]")
+    M, B, T, H, dk = x.shape
+    if (d_probs.shape != (M * B * H, T, L, 1 << K) or d_probs.dtype != x.dtype or d_probs.device != x.device
+            or not d_probs.is_contiguous()):
+        raise RuntimeError("d_probs must be a contiguous [M*B*H, T, L, 2**K] tensor of x's type on its device")
+    planes = planes.to(device=x.device, dtype=torch.float32).contiguous()
+    if planes.shape != (L * K, dk):
+        raise RuntimeError(f"planes must be [L*K, d_k] = [{L * K}, {dk}]")
+    with torch.cuda.device(x.device):
+        dx = torch.empty_like(x)
+        rc = _lib.lib().race_b200_bucket_probs_streams_bwd(_ptr(x), _ptr(planes), _ptr(d_probs), _ptr(dx), M * B, T, H,
+                                                           dk, L, K, _DTYPES[x.dtype], _stream())
+    _lib.check(rc, "race_b200_bucket_probs_streams_bwd")
+    return dx
+
+
 class _RaceCausal(torch.autograd.Function):
     """The causal forward (``race_causal_prefix``) with the hand-written backward kernels.  Only the
     three inputs are saved: the backward recomputes the prefix states tile by tile."""
@@ -423,6 +447,14 @@ class _RaceCausal(torch.autograd.Function):
         return (dpq if g[0] else None, dpk if g[1] else None, dv if g[2] else None, None)
 
 
+def causal_bwd_takes_heads(N, T, L, R, dk, dtype, heads: int) -> bool:
+    """Whether ``race_causal_backward`` reads V and grad_out and writes dV as [N/heads, T, heads, d_k]."""
+    if dtype not in _DTYPES or heads < 1 or N == 0 or T == 0:
+        return False
+    sh = make_shape(N, T, L, R, dk, dtype, 1e-6, heads)
+    return _lib.lib().race_b200_causal_bwd_workspace_bytes(ctypes.byref(sh)) > 0
+
+
 def race_causal_backward(probsQ, probsK, V, grad_out, eps: float = 1e-6, *, carry_in=None, grad_state=None,
                          return_grad_carry: bool = False):
     """(d probsQ, d probsK, d V) of ``race_causal_prefix(probsQ, probsK, V, eps)`` for the output
@@ -431,16 +463,17 @@ def race_causal_backward(probsQ, probsK, V, grad_out, eps: float = 1e-6, *, carr
 
     For one chunk of a longer sequence: ``carry_in`` is the packed state the forward was given,
     ``grad_state`` the gradient reaching the packed state it returned, and ``return_grad_carry=True``
-    appends the gradient of ``carry_in`` to the result."""
+    appends the gradient of ``carry_in`` to the result.
+
+    V and ``grad_out`` may also be in the operator's layout [M,B,T,H,d_k] where ``causal_bwd_takes_heads`` says so;
+    dV then has it too."""
     N, T, L, R, dk = _check_inputs(probsQ, probsK, V)
-    if V.dim() != 3:
-        raise RuntimeError("race_causal_backward takes V as [N,T,d_k]")
     if grad_out.shape != V.shape or not grad_out.is_cuda:
         raise RuntimeError("grad_out must be a CUDA tensor shaped like V")
     # autograd may hand over an expanded (stride-0) gradient: the kernels need dense rows
     grad_out = grad_out.to(V.dtype).contiguous()
     L_ = _lib.lib()
-    sh = make_shape(N, T, L, R, dk, V.dtype, eps)
+    sh = make_shape(N, T, L, R, dk, V.dtype, eps, _heads(V))
     with torch.cuda.device(V.device):
         dpq, dpk, dv = torch.empty_like(probsQ), torch.empty_like(probsK), torch.empty_like(V)
         ws_bytes = L_.race_b200_causal_bwd_workspace_bytes(ctypes.byref(sh))

@@ -1,0 +1,72 @@
+"""Gradients on the GPU: the backward of the producer and the operator under autograd at the geometries that run on the
+kernels alone, against torch.autograd through the restated forward (src/race_baseline.py:41-51) in fp64."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import race_oracle as ro
+
+pytestmark = pytest.mark.gpu
+
+# fp32: three-limb projections, two-limb products elsewhere (2^-17 per factor); bf16: the outputs' own rounding (2^-9)
+# and that of the probabilities and their gradients, each of which enters a result once
+TOL = {torch.float32: 3e-5, torch.bfloat16: 1e-2}
+GEOMETRIES = [(64, 4, 4, torch.float32), (64, 4, 4, torch.bfloat16), (128, 6, 8, torch.bfloat16)]   # d_k, K, L, type
+
+
+def _probs64(x, planes, L, K):
+    """[M,B,T,H,d_k] fp64 -> [N,T,L,R] (src/race_baseline.py:35-44)."""
+    M, B, T, H, dk = x.shape
+    corners = torch.tensor([[2.0 * ((r >> (K - 1 - k)) & 1) - 1 for r in range(1 << K)] for k in range(K)],
+                           dtype=torch.float64, device=x.device)
+    x2 = x.permute(0, 1, 3, 2, 4).reshape(M * B * H, T, dk)
+    proj = (x2 @ planes.double().T).view(M * B * H, T, L, K)
+    return torch.softmax(proj.tanh() / dk ** 0.5 @ corners, -1)
+
+
+def _leaf(x):
+    return x.detach().double().requires_grad_(True)
+
+
+@pytest.mark.parametrize("dk,K,L,dt", GEOMETRIES + [(128, 6, 8, torch.float32)])
+@pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 37, 3), (1, 1003, 4)])
+def test_producer_backward(dk, K, L, dt, B, T, H):
+    import race_attention_kernel_b200.ops as ops
+    g = torch.Generator(device="cuda").manual_seed(T + dk)
+    x = torch.randn(1, B, T, H, dk, device="cuda", generator=g).to(dt)
+    planes = torch.randn(L * K, dk, device="cuda", generator=g)
+    dp = torch.randn(B * H, T, L, 1 << K, device="cuda", generator=g).to(dt)
+    got = ops.bucket_probs_streams_bwd(x, planes, dp, L, K)
+    x64 = _leaf(x)
+    (ref,) = torch.autograd.grad(_probs64(x64, planes, L, K), x64, dp.double())
+    # nothing but the result is rounded here: 2^-9 for bf16
+    assert ro.rel_l2(got, ref) <= (2e-5 if dt == torch.float32 else 4e-3)
+
+
+@pytest.mark.parametrize("dk,K,L,dt", GEOMETRIES)
+@pytest.mark.parametrize("B,T,H", [(1, 1, 2), (2, 127, 3), (1, 128, 2), (1, 129, 1), (1, 2500, 2)])
+def test_operator_gradients(dk, K, L, dt, B, T, H):
+    """Edges of the 64- and 128-token chunks, one token, several state tiles."""
+    import race_attention_kernel_b200 as rk
+    torch.manual_seed(T)
+    ace = rk.BatchedACE(dk, K, L, 1).cuda()
+    Kh, Vh, Qh, dO = (torch.randn(1, B, T, H, dk, device="cuda").to(dt) for _ in range(4))
+    for t in (Kh, Vh, Qh):
+        t.requires_grad_(True)
+    out = ace(Kh, Vh, Qh)
+    got = (out, *torch.autograd.grad(out, (Kh, Vh, Qh), dO))
+    k, v, q = _leaf(Kh), _leaf(Vh), _leaf(Qh)
+    planes = ace.planes_T.T
+    pK, pQ = _probs64(k, planes, L, K).flatten(2), _probs64(q, planes, L, K).flatten(2)
+    v2 = v.permute(0, 1, 3, 2, 4).reshape(B * H, T, dk)
+    o = torch.tril((pQ / (pK.cumsum(1) + ace.eps)) @ pK.transpose(1, 2)) @ v2
+    o = o.view(1, B, H, T, dk).permute(0, 1, 3, 2, 4)
+    ref = (o, *torch.autograd.grad(o, (k, v, q), dO.double()))
+    for name, a, b in zip(("out", "dK", "dV", "dQ"), got, ref):
+        assert a.shape == b.shape and a.dtype == dt
+        if name == "dK" and T == 1:
+            # the two terms of the gradient of pK cancel to O(eps): only their size (2^-8 of which bf16 leaves) is bound
+            assert float(a.double().abs().max()) <= {torch.float32: 1e-3, torch.bfloat16: 0.5}[dt]
+            continue
+        assert ro.rel_l2(a, b) <= TOL[dt], (name, ro.rel_l2(a, b))
