@@ -210,6 +210,15 @@ int race_b200_causal_bwd_carry(const void* probs_q, const void* probs_k, const v
                                const RaceShape* shape, void* stream, int* status);
 
 /*
+ * race_b200_causal_bwd_carry with v, d_out and d_v in the operator's layout [n_streams/heads, seq_len, heads, d_k] when
+ * shape->heads > 1 (fp32 with L*R = 64, d_k = 64; race_b200_causal_bwd_workspace_bytes is 0 where it is not built).
+ */
+int race_b200_causal_bwd_heads(const void* probs_q, const void* probs_k, const void* v, const void* d_out,
+                               const float* carry_in, const float* d_state_out, void* d_probs_q, void* d_probs_k,
+                               void* d_v, float* d_carry_in, void* workspace, size_t workspace_bytes,
+                               const RaceShape* shape, void* stream, int* status);
+
+/*
  * Incremental (decode) step: race_b200_causal_fwd for a few NEW tokens per stream (seq_len <= 64,
  * typically 1) against a running state kept in device memory between calls, i.e. chunked_forward's
  * state update (src/race_chunked.py:54-63) with a chunk of seq_len tokens, costing one read and one
@@ -222,6 +231,17 @@ int race_b200_causal_bwd_carry(const void* probs_q, const void* probs_k, const v
  */
 int race_b200_decode_step(const void* probs_q, const void* probs_k, const void* v, void* out,
                           const float* state_in, float* state_out, const RaceShape* shape, void* stream);
+
+/*
+ * The incremental step of the operator in one launch: race_b200_bucket_probs_streams for the new tokens of K and Q and
+ * race_b200_decode_step.  k, v, q, out [n_streams/heads, seq_len, heads, d_k] (shape->heads as for the forward), planes
+ * [L*n_planes, d_k] fp32; the probabilities are formed in fp32 and never written.  Geometries (fp32 and bf16):
+ * d_k = 64, L = 4, n_planes = 4 and d_k = 128, L = 8, n_planes = 6, as race_b200_decode_qkv_is_supported says.
+ */
+int race_b200_decode_qkv_is_supported(const RaceShape* shape, int n_planes);
+int race_b200_decode_step_qkv(const void* k, const void* v, const void* q, const float* planes, void* out,
+                              const float* state_in, float* state_out, const RaceShape* shape, int n_planes,
+                              void* stream);
 
 /*
  * Non-causal per-bucket forward (upstream scaling/benchmark_time.py:155-162 as quoted in the
@@ -267,6 +287,14 @@ int race_b200_bucket_probs(const void* x, const float* planes, void* probs, int6
 int race_b200_bucket_probs_streams(const void* x, const float* planes, void* probs, int64_t outer,
                                    int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables,
                                    int32_t n_bits, int32_t dtype_x, int32_t dtype_probs, void* stream);
+
+/*
+ * race_b200_bucket_probs_streams with projections of fp32 accuracy for fp32 rows (three 16-bit limbs instead of two),
+ * x and probs of one type: the forward of a training step, where errors of the probabilities grow in the gradients.
+ */
+int race_b200_bucket_probs_streams_exact(const void* x, const float* planes, void* probs, int64_t outer,
+                                         int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables,
+                                         int32_t n_bits, int32_t dtype, void* stream);
 
 /*
  * Gradient of x for race_b200_bucket_probs_streams (the derivative of src/race_baseline.py:41-44, which the reference

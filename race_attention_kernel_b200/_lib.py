@@ -26,7 +26,8 @@ EXPORTS = [
     "race_b200_bucket_probs", "race_b200_bucket_probs_streams", "race_b200_causal_fwd_host",
     "race_b200_static_scratch_bytes", "race_b200_causal_fwd_static", "race_b200_decode_step",
     "race_b200_causal_fwd_global", "race_b200_causal_bwd_workspace_bytes", "race_b200_causal_bwd",
-    "race_b200_causal_bwd_carry", "race_b200_selftest_bounded_wait", "race_b200_host_release",
+    "race_b200_causal_bwd_carry", "race_b200_causal_bwd_heads", "race_b200_selftest_bounded_wait", "race_b200_host_release",
+    "race_b200_bucket_probs_streams_exact", "race_b200_decode_qkv_is_supported", "race_b200_decode_step_qkv",
     "race_b200_bucket_probs_bwd_is_supported", "race_b200_bucket_probs_streams_bwd",
     "race_b200_qkv_is_supported", "race_b200_causal_fwd_qkv",
 ]
@@ -77,6 +78,8 @@ def lib() -> ctypes.CDLL:
     L.race_b200_bucket_probs.argtypes = [vp, vp, vp, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_bucket_probs_streams.restype = i32
     L.race_b200_bucket_probs_streams.argtypes = [vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, i32, vp]
+    L.race_b200_bucket_probs_streams_exact.restype = i32
+    L.race_b200_bucket_probs_streams_exact.argtypes = [vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_bucket_probs_bwd_is_supported.restype = i32
     L.race_b200_bucket_probs_bwd_is_supported.argtypes = [i32, i32, i32, i32]
     L.race_b200_bucket_probs_streams_bwd.restype = i32
@@ -103,9 +106,27 @@ def lib() -> ctypes.CDLL:
     L.race_b200_causal_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, sz, shp, vp, vp]
     L.race_b200_causal_bwd_carry.restype = i32
     L.race_b200_causal_bwd_carry.argtypes = [vp] * 10 + [vp, sz, shp, vp, vp]
+    L.race_b200_causal_bwd_heads.restype = i32
+    L.race_b200_causal_bwd_heads.argtypes = L.race_b200_causal_bwd_carry.argtypes
     L.race_b200_decode_step.restype = i32
     L.race_b200_decode_step.argtypes = [vp, vp, vp, vp, vp, vp, shp, vp]
+    L.race_b200_decode_qkv_is_supported.restype = i32
+    L.race_b200_decode_qkv_is_supported.argtypes = [shp, i32]
+    L.race_b200_decode_step_qkv.restype = i32
+    L.race_b200_decode_step_qkv.argtypes = [vp, vp, vp, vp, vp, vp, vp, shp, i32, vp]
     return L
+
+
+@functools.cache
+def native():
+    """The C++ host path of the hot calls (``csrc/torch_entry.cpp``); like the library it has no fallback."""
+    lib()
+    try:
+        from . import _native
+    except ImportError as e:
+        raise RuntimeError(f"{HERE}/_native.so cannot be loaded ({e}): build it with "
+                           "`python -m race_attention_kernel_b200.build`") from e
+    return _native
 
 
 def check(code: int, what: str) -> None:

@@ -1,4 +1,5 @@
-"""Build the C-ABI shared library ``lib/librace_b200.so`` from ``csrc/*.cu`` with nvcc.
+"""Build the C-ABI shared library ``lib/librace_b200.so`` from ``csrc/*.cu`` with nvcc, and the torch host path
+``_native.so`` (``csrc/torch_entry.cpp``, a CPython module that calls the library) with g++.
 
     python -m race_attention_kernel_b200.build [--force] [--verbose]
 
@@ -17,6 +18,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 OBJDIR = os.path.join(HERE, "build")
 LIB_PATH = os.path.join(LIBDIR, "librace_b200.so")
+NATIVE_PATH = os.path.join(HERE, "_native.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -40,6 +42,30 @@ def _newest_header() -> float:
             if f.endswith((".h", ".cuh")):
                 t = max(t, os.path.getmtime(os.path.join(d, f)))
     return t
+
+
+def build_native(force: bool = False) -> str:
+    import sysconfig
+
+    src = os.path.join(CSRC, "torch_entry.cpp")
+    header = os.path.join(INCLUDE, "race_b200.h")
+    if (not force and os.path.exists(NATIVE_PATH)
+            and os.path.getmtime(NATIVE_PATH) >= max(os.path.getmtime(src), os.path.getmtime(header))):
+        return NATIVE_PATH
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           "-I", INCLUDE, "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include/torch/csrc/api/include"),
+           "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include"), src, "-o", NATIVE_PATH,
+           "-L", LIBDIR, "-lrace_b200", "-Wl,-rpath,$ORIGIN/lib", "-L", os.path.join(root, "lib"),
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python", "-L", os.path.join(cuda, "lib64"), "-lcudart"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("g++ failed for torch_entry.cpp")
+    return NATIVE_PATH
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -79,6 +105,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    build_native(force)
     return LIB_PATH
 
 

@@ -286,6 +286,18 @@ int race_b200_causal_bwd_carry(const void* probs_q, const void* probs_k, const v
                                void* d_v, float* d_carry_in, void* workspace, size_t workspace_bytes,
                                const RaceShape* shape, void* stream, int* status) {
     Dims dm;
+    const int rc = check_shape(shape, &dm);
+    if (rc != RACE_OK) return rc;
+    if (dm.H > 1) return RACE_ERR_SHAPE;
+    return race_b200_causal_bwd_heads(probs_q, probs_k, v, d_out, carry_in, d_state_out, d_probs_q, d_probs_k, d_v,
+                                      d_carry_in, workspace, workspace_bytes, shape, stream, status);
+}
+
+int race_b200_causal_bwd_heads(const void* probs_q, const void* probs_k, const void* v, const void* d_out,
+                               const float* carry_in, const float* d_state_out, void* d_probs_q, void* d_probs_k,
+                               void* d_v, float* d_carry_in, void* workspace, size_t workspace_bytes,
+                               const RaceShape* shape, void* stream, int* status) {
+    Dims dm;
     int rc = check_shape(shape, &dm);
     if (rc != RACE_OK) return rc;
     if (!causal_bwd_supported(dm, shape->dtype)) return RACE_ERR_SHAPE;
@@ -327,6 +339,35 @@ int race_b200_decode_step(const void* probs_q, const void* probs_k, const void* 
         !aligned16(state_out))
         return RACE_ERR_ALIGN;
     return (int)decode_step_launch(probs_q, probs_k, v, out, state_in, state_out, dm, shape->dtype, st);
+}
+
+int race_b200_decode_qkv_is_supported(const RaceShape* shape, int n_planes) {
+    Dims dm;
+    if (check_shape(shape, &dm) != RACE_OK || shape->n_buckets != (1 << n_planes)) return 0;
+    return decode_qkv_supported(dm.N, dm.T, dm.D, shape->n_tables, n_planes, shape->dtype) ? 1 : 0;
+}
+
+int race_b200_decode_step_qkv(const void* k, const void* v, const void* q, const float* planes, void* out,
+                              const float* state_in, float* state_out, const RaceShape* shape, int n_planes,
+                              void* stream) {
+    Dims dm;
+    int rc = check_shape(shape, &dm);
+    if (rc != RACE_OK) return rc;
+    if (!race_b200_decode_qkv_is_supported(shape, n_planes)) return RACE_ERR_SHAPE;
+    if (!state_out) return RACE_ERR_NULL;
+    if (dm.N == 0) return RACE_OK;
+    if (dm.T == 0) {
+        const size_t sf = (size_t)dm.N * state_floats_per_stream(dm.S, dm.D) * sizeof(float);
+        if (state_in == state_out) return RACE_OK;
+        return (int)(state_in ? cudaMemcpyAsync(state_out, state_in, sf, cudaMemcpyDeviceToDevice, (cudaStream_t)stream)
+                              : cudaMemsetAsync(state_out, 0, sf, (cudaStream_t)stream));
+    }
+    if (!k || !v || !q || !planes || !out) return RACE_ERR_NULL;
+    if (!aligned16(k) || !aligned16(v) || !aligned16(q) || !aligned16(planes) || !aligned16(out) ||
+        !aligned16(state_in) || !aligned16(state_out))
+        return RACE_ERR_ALIGN;
+    return (int)decode_step_qkv_launch(k, v, q, planes, out, state_in, state_out, dm.N, (int)dm.T, dm.H, dm.D,
+                                       shape->dtype, dm.eps, (cudaStream_t)stream);
 }
 
 namespace {
@@ -413,7 +454,7 @@ int race_b200_noncausal_bwd(const void* probs_q, const void* probs_k, const void
 namespace {
 int probs_entry(const void* x, const float* planes, void* probs, int64_t outer, int64_t seq_len, int32_t heads,
                 int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype_x, int32_t dtype_probs,
-                void* stream) {
+                void* stream, bool exact = false) {
     if (outer < 0 || seq_len < 0 || heads < 1 || d_k < 4 || d_k > 256 || (d_k & (d_k - 1)) || n_tables <= 0 ||
         n_bits < 1 || n_bits > 6 || n_tables * n_bits > 64)
         return RACE_ERR_SHAPE;
@@ -425,7 +466,7 @@ int probs_entry(const void* x, const float* planes, void* probs, int64_t outer, 
     if (!x || !planes || !probs) return RACE_ERR_NULL;
     if (!aligned16(x) || !aligned16(planes) || !aligned16(probs)) return RACE_ERR_ALIGN;
     return (int)bucket_probs(x, planes, probs, rows, seq_len, heads, d_k, n_tables, n_bits, dtype_x, dtype_probs,
-                             (cudaStream_t)stream);
+                             (cudaStream_t)stream, exact);
 }
 }  // namespace
 
@@ -440,6 +481,12 @@ int race_b200_bucket_probs_streams(const void* x, const float* planes, void* pro
                                    int32_t n_bits, int32_t dtype_x, int32_t dtype_probs, void* stream) {
     return probs_entry(x, planes, probs, outer, seq_len, heads, d_k, n_tables, n_bits, dtype_x, dtype_probs,
                        stream);
+}
+
+int race_b200_bucket_probs_streams_exact(const void* x, const float* planes, void* probs, int64_t outer,
+                                         int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables,
+                                         int32_t n_bits, int32_t dtype, void* stream) {
+    return probs_entry(x, planes, probs, outer, seq_len, heads, d_k, n_tables, n_bits, dtype, dtype, stream, true);
 }
 
 int race_b200_bucket_probs_bwd_is_supported(int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype) {

@@ -283,8 +283,10 @@ __device__ __forceinline__ void pack8(const float* v, uint4& w) {
     w.z = *reinterpret_cast<uint32_t*>(&c); w.w = *reinterpret_cast<uint32_t*>(&d);
 }
 
-template <int D, int L, int K, typename Tx, typename Tp>
-__global__ void __launch_bounds__(kWideThreads, (sizeof(Tx) == 4 ? 3 : 4))
+// kExact (fp32 rows): three limbs of rows and planes in six products, the accuracy of an fp32 product, for the forward
+// of a training step: the gradients of the probabilities nearly cancel over a table, which magnifies the 2^-17 of two.
+template <int D, int L, int K, typename Tx, typename Tp, bool kExact>
+__global__ void __launch_bounds__(kWideThreads, (sizeof(Tx) == 4 && D > 64 ? 3 : 4))
 bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes, Tp* __restrict__ probs,
                       int64_t rows, int64_t T, int heads) {
     using W = WideProbs<D, L, K>;
@@ -294,11 +296,12 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
     uint4* tab = reinterpret_cast<uint4*>(wide_smem);          // [(nt NJ + j) 32 + lane] = {b0 hi, b1 hi, b0 lo, b1 lo}
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     // staging: PB bytes per (row, table); a flush covers 8 rows x kTPF tables = 8 KB, i.e. kPPF passes over tb
-    // (tables of 32 bytes, R = 16 in bf16, go straight to memory: a quad's four tables are one 128-byte row)
+    // (tables of 32 or 64 bytes, R = 16, go straight to memory: a quad's four tables are one row)
     constexpr int PB = R * (int)sizeof(Tp), kTPF = W::kStageBytes / (8 * PB), kPPF = kTPF / 4;
-    constexpr bool kDirect = PB == 32;
+    constexpr bool kDirect = PB < 128;
     static_assert(kDirect || (kPPF >= 1 && TPL % kPPF == 0 && PB % 128 == 0), "staging geometry");
-    uint8_t* stage = wide_smem + W::kTabBytes + (threadIdx.x >> 5) * W::kStageBytes;
+    uint2* tab3 = reinterpret_cast<uint2*>(wide_smem + W::kTabBytes);   // kExact: the third limbs {b0, b1}
+    uint8_t* stage = wide_smem + W::kTabBytes + (kExact ? W::kTabBytes / 2 : 0) + (threadIdx.x >> 5) * W::kStageBytes;
     auto swz = [](int off) {   // 16-byte piece (off >> 4) & 7 of 128-byte block b = off >> 7, XOR (b / 8 + 2 (b % 8)) % 8
         const int b = off >> 7;
         return (b << 7) | (((((off >> 4) & 7) ^ ((b >> 3) + 2 * (b & 7))) & 7) << 4);
@@ -314,6 +317,7 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
         split_pair(v.x, v.y, w.x, w.z);
         split_pair(v.z, v.w, w.y, w.w);
         tab[i] = w;
+        if (kExact) tab3[i] = make_uint2(rest_pair(v.x, v.y, w.x, w.z), rest_pair(v.z, v.w, w.y, w.w));
     }
     __syncthreads();
     const float inv_scale = rsqrtf((float)D);
@@ -343,7 +347,7 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
 #pragma unroll
         for (int m = 0; m < D / 32; ++m) {
             // the lane's eight features [32 m + 8 t, +8) of both rows: words {k-step 2m: a0|a2, k-step 2m+1: a0|a2}
-            uint32_t hi[2][4], lo[2][4];
+            uint32_t hi[2][4], lo[2][4], rest[2][4];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 if (kX32) {
@@ -356,6 +360,12 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
                     split_pair(v0.z, v0.w, hi[h][1], lo[h][1]);
                     split_pair(v1.x, v1.y, hi[h][2], lo[h][2]);
                     split_pair(v1.z, v1.w, hi[h][3], lo[h][3]);
+                    if (kExact) {
+                        rest[h][0] = rest_pair(v0.x, v0.y, hi[h][0], lo[h][0]);
+                        rest[h][1] = rest_pair(v0.z, v0.w, hi[h][1], lo[h][1]);
+                        rest[h][2] = rest_pair(v1.x, v1.y, hi[h][2], lo[h][2]);
+                        rest[h][3] = rest_pair(v1.z, v1.w, hi[h][3], lo[h][3]);
+                    }
                 } else {
                     uint4 v = make_uint4(0u, 0u, 0u, 0u);
                     if (live[h]) v = __ldcs(reinterpret_cast<const uint4*>(src[h] + 32 * m));
@@ -376,6 +386,13 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
                     mma_bf16_16816(acc[0][nt], ahi, b.x, b.y);
                     mma_bf16_16816(acc[1][nt], ahi, b.z, b.w);
                     if (kX32) mma_bf16_16816(acc[2][nt], alo, b.x, b.y);
+                    if (kExact) {
+                        const uint2 r = tab3[(nt * NJ + j) * 32 + lane];
+                        const uint32_t ar[4] = {rest[0][2 * jj], rest[1][2 * jj], rest[0][2 * jj + 1], rest[1][2 * jj + 1]};
+                        mma_bf16_16816(acc[2][nt], ar, b.x, b.y);
+                        mma_bf16_16816(acc[1][nt], ahi, r.x, r.y);
+                        mma_bf16_16816(acc[2][nt], alo, b.z, b.w);
+                    }
                 }
             }
         }
@@ -415,11 +432,18 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
                 if constexpr (kDirect) {
                     if (live[h]) {
                         uint8_t* dst = reinterpret_cast<uint8_t*>(probs) + ((r0 + g + 8 * h) * L + TPL * t + tb) * (int64_t)PB;
+                        if constexpr (sizeof(Tp) == 4) {
 #pragma unroll
-                        for (int i = 0; i < R; i += 8) {
-                            uint4 w;
-                            pack8(vals + i, w);
-                            __stcs(reinterpret_cast<uint4*>(dst + 2 * i), w);
+                            for (int i = 0; i < R; i += 4)
+                                __stcs(reinterpret_cast<float4*>(dst + 4 * i),
+                                       make_float4(vals[i], vals[i + 1], vals[i + 2], vals[i + 3]));
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < R; i += 8) {
+                                uint4 w;
+                                pack8(vals + i, w);
+                                __stcs(reinterpret_cast<uint4*>(dst + 2 * i), w);
+                            }
                         }
                     }
                     continue;
@@ -461,12 +485,12 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
     }
 }
 
-template <int D, int L, int K, typename Tx, typename Tp>
+template <int D, int L, int K, typename Tx, typename Tp, bool kExact = false>
 cudaError_t launch_probs_wide(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
                               cudaStream_t stream) {
-    auto kern = bucket_probs_mma_wide<D, L, K, Tx, Tp>;
-    constexpr int smem = WideProbs<D, L, K>::kTabBytes +
-                         ((int)sizeof(Tp) << K == 32 ? 0 : (kWideThreads / 32) * WideProbs<D, L, K>::kStageBytes);
+    auto kern = bucket_probs_mma_wide<D, L, K, Tx, Tp, kExact>;
+    constexpr int smem = WideProbs<D, L, K>::kTabBytes + (kExact ? WideProbs<D, L, K>::kTabBytes / 2 : 0) +
+                         ((int)sizeof(Tp) << K < 128 ? 0 : (kWideThreads / 32) * WideProbs<D, L, K>::kStageBytes);
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return err;
     int dev = 0, sms = 148;
@@ -519,7 +543,13 @@ cudaError_t launch_probs(const void* x, const float* planes, void* probs, int64_
 }  // namespace
 
 cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
-                         int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream) {
+                         int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream, bool exact) {
+    if (exact && dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32) {
+        if (d == 64 && L == 4 && K == 4)
+            return launch_probs_wide<64, 4, 4, float, float, true>(x, planes, probs, rows, T, heads, stream);
+        if (d == 128 && L == 8 && K == 6)
+            return launch_probs_wide<128, 8, 6, float, float, true>(x, planes, probs, rows, T, heads, stream);
+    }
     if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32 && d == 64 && L == 4 && K == 4) {
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -38,13 +38,6 @@ struct BwdProbs {
     static __device__ __forceinline__ int plane(int t, int s) { return (TPL * t + s / K) * K + s % K; }
 };
 
-// the third limb: what hi + lo of split_pair leave of (a, b)
-__device__ __forceinline__ uint32_t rest_pair(float a, float b, uint32_t hi, uint32_t lo) {
-    __nv_bfloat162 r = __floats2bfloat162_rn((a - __uint_as_float(hi << 16)) - __uint_as_float(lo << 16),
-                                             (b - __uint_as_float(hi & 0xffff0000u)) - __uint_as_float(lo & 0xffff0000u));
-    return *reinterpret_cast<uint32_t*>(&r);
-}
-
 // gradient of the probabilities of one (row, table): R consecutive values
 template <int R>
 __device__ __forceinline__ void load_dp(const float* p, float (&v)[R]) {

@@ -55,9 +55,10 @@ cudaError_t noncausal_token_grads_tensor(const void* pk, const void* v, const vo
                                          int dtype, int sm_count, cudaStream_t stream);
 
 // ---- bucket-probability producer (bucket_probs.cu) --------------------------------------------
+// exact: fp32 accuracy of the projections (training) at the tensor-core geometries
 // x [outer, T, heads, d] -> probs [outer*heads, T, L, 2^K]; rows = outer*heads*T (heads = 1: plain rows)
 cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
-                         int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream);
+                         int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream, bool exact = false);
 
 // dx of the same (bucket_probs_bwd.cu): dprobs [outer*heads, T, L, 2^K] and x, dx [outer, T, heads, d], one type
 bool bucket_probs_bwd_supported(int d, int L, int K, int dtype);
@@ -70,6 +71,13 @@ cudaError_t bucket_probs_bwd(const void* x, const float* planes, const void* dpr
 int decode_max_tokens();
 cudaError_t decode_step_launch(const void* pq, const void* pk, const void* v, void* out, const float* state_in,
                                float* state_out, const Dims& dm, int dtype, cudaStream_t stream);
+
+// the same from K, V, Q [N/heads, T, heads, d] and the hyperplanes (decode_qkv.cu): d = 64, L = 4, K = 4 and d = 128,
+// L = 8, K = 6
+bool decode_qkv_supported(int64_t N, int64_t T, int d, int L, int K, int dtype);
+cudaError_t decode_step_qkv_launch(const void* k, const void* v, const void* q, const float* planes, void* out,
+                                   const float* state_in, float* state_out, int64_t N, int T, int heads, int d,
+                                   int dtype, float eps, cudaStream_t stream);
 
 // ---- tcgen05 tensor-core causal path (causal_tc.cu) ------------------------------------------
 bool tensor_supported(const Dims& dm, int dtype);

@@ -34,6 +34,12 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t& hi, uint3
     __nv_bfloat162 l = __floats2bfloat162_rn(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
     lo = *reinterpret_cast<uint32_t*>(&l);
 }
+// the third limb: what hi + lo of split_pair leave of (a, b)
+__device__ __forceinline__ uint32_t rest_pair(float a, float b, uint32_t hi, uint32_t lo) {
+    __nv_bfloat162 r = __floats2bfloat162_rn((a - __uint_as_float(hi << 16)) - __uint_as_float(lo << 16),
+                                             (b - __uint_as_float(hi & 0xffff0000u)) - __uint_as_float(lo & 0xffff0000u));
+    return *reinterpret_cast<uint32_t*>(&r);
+}
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
                  "{%0, %1, %2, %3};"

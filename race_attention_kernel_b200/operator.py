@@ -23,7 +23,7 @@ import itertools
 import torch
 from torch import nn
 
-from . import ops
+from . import _lib, ops
 
 
 class _CausalOperator(torch.autograd.Function):
@@ -33,8 +33,8 @@ class _CausalOperator(torch.autograd.Function):
     @staticmethod
     def forward(ctx, Khf, Vhf, Qhf, planes, L, K, eps):
         M, B, T, H, dk = Khf.shape
-        pK = ops.bucket_probs_streams(Khf, planes, L, K)
-        pQ = ops.bucket_probs_streams(Qhf, planes, L, K)
+        pK = ops.bucket_probs_streams(Khf, planes, L, K, exact=True)
+        pQ = ops.bucket_probs_streams(Qhf, planes, L, K, exact=True)
         shape = (M * B * H, T, L, 1 << K, dk, Vhf.dtype)
         V2 = None
         if ops.is_supported(*shape, "auto", heads=H):
@@ -126,12 +126,21 @@ class BatchedACE(nn.Module):
         return out if Khf.is_cuda else out.cpu()
 
     def forward(self, Khf, Vhf, Qhf, *, carry_in=None, return_state=False):
+        grad = torch.is_grad_enabled() and (Khf.requires_grad or Vhf.requires_grad or Qhf.requires_grad)
+        if not grad and self.variant == "auto" and Khf.is_cuda:
+            # the plain call in C++ (None: something about the arguments needs the general path below)
+            if isinstance(carry_in, (tuple, list)):
+                carry_in = ops.pack_state(*carry_in)
+            res = _lib.native().forward(self.planes_T, Khf, Vhf, Qhf, self.L, self.K, self.eps, carry_in, bool(return_state),
+                                        bool(self.fuse_producer), ops._status_ptr(Khf.get_device()))
+            if res is not None:
+                return res
         if not (Khf.shape == Vhf.shape == Qhf.shape) or Khf.dim() != 5:
             raise RuntimeError("expected K, V, Q of identical shape [M,B,T,H,d_k]")
         M, B, T, H, dk = Khf.shape
         if dk != self.d_k:
             raise RuntimeError(f"d_k mismatch: module {self.d_k}, input {dk}")
-        if torch.is_grad_enabled() and (Khf.requires_grad or Vhf.requires_grad or Qhf.requires_grad):
+        if grad:
             if carry_in is not None or return_state:
                 raise RuntimeError("carry_in / return_state are inference-only; chain ops.race_causal_chunk "
                                    "for differentiable chunked sequences")
@@ -178,13 +187,20 @@ class BatchedACE(nn.Module):
             out = out.cpu()
         return (out, res[1], res[2]) if return_state else out
 
-    @torch.no_grad()
     def step(self, Khf, Vhf, Qhf, state: torch.Tensor):
         """Token-by-token generation: outputs for the ``t`` <= 64 NEW tokens ``[M,B,t,H,d_k]`` given the
         packed running state ``[M*B*H, S*(d_k+1)]`` of everything before them (``torch.zeros`` or
         ``ops.pack_state(A, B)`` of a ``forward(..., return_state=True)`` prefill); ``state`` is advanced
         in place.  Equals continuing the reference's chunked evaluation (src/race_chunked.py:54-63) by a
         chunk of ``t`` tokens."""
+        if Khf.is_cuda:   # one launch where the geometry has it (None: the general path below)
+            out = _lib.native().step(self.planes_T, Khf, Vhf, Qhf, state, self.L, self.K, self.eps)
+            if out is not None:
+                return out
+        with torch.no_grad():
+            return self._step(Khf, Vhf, Qhf, state)
+
+    def _step(self, Khf, Vhf, Qhf, state: torch.Tensor):
         if not (Khf.shape == Vhf.shape == Qhf.shape) or Khf.dim() != 5:
             raise RuntimeError("expected K, V, Q of identical shape [M,B,t,H,d_k]")
         M, B, T, H, dk = Khf.shape

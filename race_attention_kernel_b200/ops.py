@@ -37,6 +37,17 @@ def _status_word(device: torch.device) -> torch.Tensor:
     return _STATUS[idx]
 
 
+_STATUS_PTR: dict[int, int] = {}
+
+
+def _status_ptr(index: int) -> int:
+    """Address of the status word of CUDA device ``index``."""
+    p = _STATUS_PTR.get(index)
+    if p is None:
+        p = _STATUS_PTR[index] = _status_word(torch.device("cuda", index)).data_ptr()
+    return p
+
+
 def prepare(device=None) -> None:
     """Create the per-device status word now.  Callers that must not allocate later (stream capture,
     ``race_causal_prefix_static``) call this once per device at start-up; without it the static wrapper
@@ -162,6 +173,15 @@ def race_causal_prefix(probsQ, probsK, V, eps: float = 1e-6, *, carry_in=None,
     tcgen05 kernels for fp32 S = 64, d_k = 64 and for bf16 S = 64, else on the CUDA-core kernels; states and
     carries are the same quantities in both forms.
     """
+    if (variant == "auto" and normalization == "bucket" and not tile_tokens and out is None and totals_workspace is None
+            and isinstance(V, torch.Tensor) and V.is_cuda):
+        # the plain call in C++ (None: something about the arguments needs the general path below)
+        if isinstance(carry_in, (tuple, list)):
+            carry_in = pack_state(*carry_in)
+        res = _lib.native().causal_prefix(probsQ, probsK, V, float(eps), carry_in, bool(return_state),
+                                          _status_ptr(V.get_device()))
+        if res is not None:
+            return res
     N, T, L, R, dk = _check_inputs(probsQ, probsK, V)
     if variant not in _lib.VARIANTS:
         raise RuntimeError(f"unknown variant {variant!r}")
@@ -381,11 +401,12 @@ def bucket_probs(x: torch.Tensor, planes: torch.Tensor, L: int, K: int,
 
 
 def bucket_probs_streams(x: torch.Tensor, planes: torch.Tensor, L: int, K: int,
-                         out_dtype: torch.dtype | None = None) -> torch.Tensor:
+                         out_dtype: torch.dtype | None = None, *, exact: bool = False) -> torch.Tensor:
     """x [M, B, T, H, d_k] (the operator's layout) -> probs [M*B*H, T, L, 2**K]: the stream flattening
     of src/race_baseline.py:35-40 fused into the producer of :41-44; no flattened copy of x is made.
 
-    planes: fp32 [L*K, d_k] row-major (``planes_T.T``)."""
+    planes: fp32 [L*K, d_k] row-major (``planes_T.T``).  exact: projections of fp32 accuracy for fp32 rows (the
+    forward of a training step)."""
     if not x.is_cuda or x.dtype not in _DTYPES or not x.is_contiguous() or x.dim() != 5:
         raise RuntimeError("x must be a contiguous fp32/bf16 CUDA tensor [M,B,T,H,d_k]")
     M, B, T, H, dk = x.shape
@@ -395,8 +416,12 @@ def bucket_probs_streams(x: torch.Tensor, planes: torch.Tensor, L: int, K: int,
     out_dtype = out_dtype or x.dtype
     with torch.cuda.device(x.device):
         probs = torch.empty(M * B * H, T, L, 1 << K, dtype=out_dtype, device=x.device)
-        rc = _lib.lib().race_b200_bucket_probs_streams(_ptr(x), _ptr(planes), _ptr(probs), M * B, T, H, dk,
-                                                       L, K, _DTYPES[x.dtype], _DTYPES[out_dtype], _stream())
+        if exact and out_dtype == x.dtype:
+            rc = _lib.lib().race_b200_bucket_probs_streams_exact(_ptr(x), _ptr(planes), _ptr(probs), M * B, T, H, dk, L,
+                                                                 K, _DTYPES[x.dtype], _stream())
+        else:
+            rc = _lib.lib().race_b200_bucket_probs_streams(_ptr(x), _ptr(planes), _ptr(probs), M * B, T, H, dk,
+                                                           L, K, _DTYPES[x.dtype], _DTYPES[out_dtype], _stream())
     _lib.check(rc, "race_b200_bucket_probs_streams")
     return probs
 
@@ -483,7 +508,7 @@ def race_causal_backward(probsQ, probsK, V, grad_out, eps: float = 1e-6, *, carr
                                    or st.numel() != N * L * R * (dk + 1)):
                 raise RuntimeError("carry_in / grad_state must be contiguous fp32 CUDA states of N*S*(d_k+1) floats")
         dcarry = torch.empty(N, L * R * (dk + 1), dtype=torch.float32, device=V.device) if return_grad_carry else None
-        rc = L_.race_b200_causal_bwd_carry(_ptr(probsQ), _ptr(probsK), _ptr(V), _ptr(grad_out), _ptr(carry_in),
+        rc = L_.race_b200_causal_bwd_heads(_ptr(probsQ), _ptr(probsK), _ptr(V), _ptr(grad_out), _ptr(carry_in),
                                            _ptr(grad_state), _ptr(dpq), _ptr(dpk), _ptr(dv), _ptr(dcarry), _ptr(ws),
                                            ws_bytes, ctypes.byref(sh), _stream(), _ptr(_status_word(V.device)))
     _lib.check(rc, "race_b200_causal_bwd_carry")

@@ -65,8 +65,10 @@ def test_operator_gradients(dk, K, L, dt, B, T, H):
     ref = (o, *torch.autograd.grad(o, (k, v, q), dO.double()))
     for name, a, b in zip(("out", "dK", "dV", "dQ"), got, ref):
         assert a.shape == b.shape and a.dtype == dt
-        if name == "dK" and T == 1:
-            # the two terms of the gradient of pK cancel to O(eps): only their size (2^-8 of which bf16 leaves) is bound
+        if name in ("dK", "dQ") and T == 1:
+            # with one token the output does not depend on the probabilities (pQ_1 B_1 / A_1 = pQ_1 (x) V_1 summed over
+            # a softmax): both gradients cancel to O(eps).  What is left are rounding errors of terms of size
+            # |V . dO| <= 40, 2^-17 of them in fp32 and 2^-9 in bf16, through a Jacobian below 1.
             assert float(a.double().abs().max()) <= {torch.float32: 1e-3, torch.bfloat16: 0.5}[dt]
             continue
         assert ro.rel_l2(a, b) <= TOL[dt], (name, ro.rel_l2(a, b))
