@@ -210,8 +210,18 @@ int race_b200_causal_bwd_carry(const void* probs_q, const void* probs_k, const v
                                const RaceShape* shape, void* stream, int* status);
 
 /*
+ * race_b200_causal_fwd on the tensor kernels with v and out in the operator's layout [n_streams/heads, seq_len, heads,
+ * d_k]: every geometry race_b200_is_supported grants that layout, and bf16 with L*R = 64 as well.
+ * race_b200_causal_heads_workspace_bytes: the workspace it needs, 0 where it is not built (or nothing is to do).
+ */
+size_t race_b200_causal_heads_workspace_bytes(const RaceShape* shape);
+int race_b200_causal_fwd_heads(const void* probs_q, const void* probs_k, const void* v, void* out,
+                               const float* carry_in, float* state_out, void* workspace, size_t workspace_bytes,
+                               const RaceShape* shape, void* stream, int* status);
+
+/*
  * race_b200_causal_bwd_carry with v, d_out and d_v in the operator's layout [n_streams/heads, seq_len, heads, d_k] when
- * shape->heads > 1 (fp32 with L*R = 64, d_k = 64; race_b200_causal_bwd_workspace_bytes is 0 where it is not built).
+ * shape->heads > 1 (fp32 with L*R = 64, d_k = 64; bf16 with L*R 64, 128, 256 or 512, d_k 64 or 128; race_b200_causal_bwd_workspace_bytes is 0 where it is not built).
  */
 int race_b200_causal_bwd_heads(const void* probs_q, const void* probs_k, const void* v, const void* d_out,
                                const float* carry_in, const float* d_state_out, void* d_probs_q, void* d_probs_k,

@@ -27,7 +27,7 @@ EXPORTS = [
     "race_b200_static_scratch_bytes", "race_b200_causal_fwd_static", "race_b200_decode_step",
     "race_b200_causal_fwd_global", "race_b200_causal_bwd_workspace_bytes", "race_b200_causal_bwd",
     "race_b200_causal_bwd_carry", "race_b200_causal_bwd_heads", "race_b200_selftest_bounded_wait", "race_b200_host_release",
-    "race_b200_bucket_probs_streams_exact", "race_b200_decode_qkv_is_supported", "race_b200_decode_step_qkv",
+    "race_b200_causal_heads_workspace_bytes", "race_b200_causal_fwd_heads", "race_b200_bucket_probs_streams_exact", "race_b200_decode_qkv_is_supported", "race_b200_decode_step_qkv",
     "race_b200_bucket_probs_bwd_is_supported", "race_b200_bucket_probs_streams_bwd",
     "race_b200_qkv_is_supported", "race_b200_causal_fwd_qkv",
 ]
@@ -110,6 +110,10 @@ def lib() -> ctypes.CDLL:
     L.race_b200_causal_bwd_heads.argtypes = L.race_b200_causal_bwd_carry.argtypes
     L.race_b200_decode_step.restype = i32
     L.race_b200_decode_step.argtypes = [vp, vp, vp, vp, vp, vp, shp, vp]
+    L.race_b200_causal_heads_workspace_bytes.restype = sz
+    L.race_b200_causal_heads_workspace_bytes.argtypes = [shp]
+    L.race_b200_causal_fwd_heads.restype = i32
+    L.race_b200_causal_fwd_heads.argtypes = [vp, vp, vp, vp, vp, vp, vp, sz, shp, vp, vp]
     L.race_b200_decode_qkv_is_supported.restype = i32
     L.race_b200_decode_qkv_is_supported.argtypes = [shp, i32]
     L.race_b200_decode_step_qkv.restype = i32

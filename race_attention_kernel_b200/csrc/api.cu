@@ -134,17 +134,22 @@ size_t race_b200_causal_workspace_bytes(const RaceShape* shape, int tile_tokens,
     return workspace_bytes_for(dm, shape->dtype, var, tile);
 }
 
+static bool causal_heads_supported(const Dims& dm, int dtype) {
+    return tensor_supported(dm, dtype) || (dtype == RACE_DTYPE_BF16 && tensor_bf16_heads_supported(dm));
+}
+
 static int causal_entry(const void* probs_q, const void* probs_k, const void* v, void* out,
                         const float* carry_in, float* state_out, void* workspace,
                         size_t workspace_bytes, const RaceShape* shape, int tile_tokens,
                         int variant, void* stream, int* status, int phases, bool global_norm = false,
-                        long long wait_cycles = 0, int withhold_chunk = -1) {
+                        long long wait_cycles = 0, int withhold_chunk = -1, bool heads_entry = false) {
     Dims dm;
     int rc = check_shape(shape, &dm);
     if (rc != RACE_OK) return rc;
     const int var = resolve_variant(dm, shape->dtype, variant);
     if (var != RACE_VARIANT_SIMT && var != RACE_VARIANT_TENSOR && !is_single_pass(var)) return RACE_ERR_VARIANT;
-    if (!variant_supported(dm, shape->dtype, var)) return var == variant ? RACE_ERR_VARIANT : RACE_ERR_SHAPE;
+    if (heads_entry ? !causal_heads_supported(dm, shape->dtype) : !variant_supported(dm, shape->dtype, var))
+        return var == variant ? RACE_ERR_VARIANT : RACE_ERR_SHAPE;
     // the global-normalisation form runs on the CUDA-core kernels and on the fp32 tensor kernels
     // the global-normalisation form: CUDA-core kernels, fp32 tensor kernels, bf16 tensor kernels with one bucket group
     if (global_norm && family(var) == RACE_VARIANT_TENSOR && shape->dtype != RACE_DTYPE_F32 && dm.S != 64)
@@ -189,6 +194,19 @@ int race_b200_causal_fwd(const void* probs_q, const void* probs_k, const void* v
                          int variant, void* stream, int* status) {
     return causal_entry(probs_q, probs_k, v, out, carry_in, state_out, workspace, workspace_bytes,
                         shape, tile_tokens, variant, stream, status, kPhaseAll);
+}
+
+size_t race_b200_causal_heads_workspace_bytes(const RaceShape* shape) {
+    Dims dm;
+    if (check_shape(shape, &dm) != RACE_OK || !causal_heads_supported(dm, shape->dtype)) return 0;
+    return workspace_bytes_for(dm, shape->dtype, RACE_VARIANT_TENSOR, pick_tile(dm, shape->dtype, RACE_VARIANT_TENSOR));
+}
+
+int race_b200_causal_fwd_heads(const void* probs_q, const void* probs_k, const void* v, void* out,
+                               const float* carry_in, float* state_out, void* workspace, size_t workspace_bytes,
+                               const RaceShape* shape, void* stream, int* status) {
+    return causal_entry(probs_q, probs_k, v, out, carry_in, state_out, workspace, workspace_bytes, shape, 0,
+                        RACE_VARIANT_TENSOR, stream, status, kPhaseAll, false, 0, -1, /*heads_entry=*/true);
 }
 
 int race_b200_tile_totals(const void* probs_k, const void* v, float* totals, void* workspace,

@@ -1375,6 +1375,8 @@ bool make_map_heads(CUtensorMap* map, const void* base, int64_t N, int64_t T, in
 
 }  // namespace
 
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() { return encode_fn(); }
+
 bool tensor_supported(const Dims& dm, int dtype) {
     // the shape test alone decides: a missing driver entry point surfaces as an error at launch
     if (dtype == RACE_DTYPE_BF16) return tensor_bf16_supported(dm);

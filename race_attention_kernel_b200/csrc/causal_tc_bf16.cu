@@ -105,7 +105,7 @@ template <int D, bool kGlobal>
 __global__ void __launch_bounds__(kThreads, 1)
 causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
-                   const float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, float eps,
+                   const float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, float eps, int heads,
                    int* status) {
     using Ly = Lay<D>;
     constexpr int DH = D / 64;   // 64-column halves of a [64][D] accumulator
@@ -187,7 +187,9 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
         const int q = lane & 3, rbase = 16 * w + (lane >> 2);
         const uint32_t lane_base = (uint32_t)(32 * w) << 16;
         uint8_t* wt = cx.sm + Ly::oWt + wg * Ly::kTileP;
-        __nv_bfloat16* out_n = out + n * T * D;
+        // heads > 1: V and out are laid out [N / heads][T][heads][D] (map_v is the 5-D map of that layout)
+        __nv_bfloat16* out_n = out + ((n / heads) * T * heads + n % heads) * D;
+        const int64_t out_stride = (int64_t)heads * D;
         const uint8_t* pq_tile = cx.sm + Ly::oPq + wg * Ly::kTileP;
         float v[32];
         uint32_t ov[16];   // W / masked G pairs on their way to tensor memory (d_k = 64)
@@ -314,7 +316,7 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 for (int h = 0; h < 2; ++h) {
                     const int row = rbase + 8 * h;
                     if (row < valid) {
-                        __nv_bfloat16* orow = out_n + (tok0 + row) * D + dh * 64 + 2 * q;
+                        __nv_bfloat16* orow = out_n + (tok0 + row) * out_stride + dh * 64 + 2 * q;
                         const float sc = kGlobal ? (den[h] != 0.f ? 1.f / den[h] : 0.f) : 1.f;
 #pragma unroll
                         for (int x = 0; x < 8; ++x)
@@ -428,7 +430,9 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
                 const int tok = (int)(t_begin + (int64_t)c * C);
                 mbar_arrive_expect_tx(bar, Ly::kStage);
                 tma_load_4d(dst, &map_k, bar, 0, tok, g, (int)n);
-                tma_load_4d(dst + Ly::kTileP, &map_v, bar, 0, tok, 0, (int)n);   // one box: all D / 64 column blocks
+                // one box: all D / 64 column blocks
+                if (heads > 1) tma_load_5d(dst + Ly::kTileP, &map_v, bar, 0, tok, 0, (int)(n % heads), (int)(n / heads));
+                else tma_load_4d(dst + Ly::kTileP, &map_v, bar, 0, tok, 0, (int)n);
                 issued = c + 1;
                 // pQ of the chunk into the slot of its worker group (c & 1), once the group has taken chunk c - 2
                 if (c >= 2 && !wait_bar(cx, bPqEmpty + st, ((c >> 1) - 1) & 1, 302)) break;
@@ -1223,42 +1227,6 @@ enum BarW4 {
 };
 static_assert(w4NumBars <= LayW4<64, 2, 3>::kNumBars, "barrier array of the wide kernel");
 
-__device__ __forceinline__ constexpr uint32_t idesc_mn(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-// 32 lanes x 32 columns of fp32: thread t of the warp <-> lane (lane of taddr) + t, register j <-> column + j
-__device__ __forceinline__ void tmem_ld_rows32(uint32_t taddr, float (&v)[32]) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_st_rows32(uint32_t taddr, const float (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
-        ::"r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
-          "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
-          "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
-          "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])),
-          "r"(__float_as_uint(v[16])), "r"(__float_as_uint(v[17])), "r"(__float_as_uint(v[18])), "r"(__float_as_uint(v[19])),
-          "r"(__float_as_uint(v[20])), "r"(__float_as_uint(v[21])), "r"(__float_as_uint(v[22])), "r"(__float_as_uint(v[23])),
-          "r"(__float_as_uint(v[24])), "r"(__float_as_uint(v[25])), "r"(__float_as_uint(v[26])), "r"(__float_as_uint(v[27])),
-          "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31])),
-          "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
 // 16 lanes x 16 columns of packed bf16 pairs (half of tmem_st_pairs: 32 K-values per row).  No wait inside.
 __device__ __forceinline__ void tmem_st_pairs4(uint32_t taddr, const uint32_t (&r)[8]) {
     asm volatile(
@@ -1901,25 +1869,12 @@ tile_totals4_tc_bf16(const __grid_constant__ CUtensorMap map_k4, const __grid_co
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn_bf16() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (fn) return fn;
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-        p = nullptr;
-    if (!p) cudaGetLastError();
-    fn = (PFN_cuTensorMapEncodeTiled_v12000)p;
-    return fn;
-}
-
 // [N][T][width] bf16 viewed as (64 values, T tokens, width/64 column blocks, N streams); one box =
 // `blocks` adjacent column blocks of 64 values x 64 tokens (128-byte rows, 128B swizzle), which land as consecutive
 // 8 KB tiles: one TMA instruction instead of `blocks` (an elected thread needs about 0.3 k clk for each); tokens past
 // T read as zero
 bool make_map_bf16(CUtensorMap* map, const void* base, int64_t N, int64_t T, int width, int blocks = 1, int heads = 1) {
-    auto fn = encode_fn_bf16();
+    auto fn = tensor_map_encoder();
     if (!fn) return false;
     if (heads > 1) {   // [N / heads][T][heads][width]: (64 values, T tokens, column blocks, heads, outer)
         cuuint64_t dims5[5] = {64, (cuuint64_t)T, (cuuint64_t)(width / 64), (cuuint64_t)heads, (cuuint64_t)(N / heads)};
@@ -1943,7 +1898,7 @@ bool make_map_bf16(CUtensorMap* map, const void* base, int64_t N, int64_t T, int
 // V [N][T][width] bf16 viewed as (ds values, T tokens, width/ds column blocks, N streams); one box =
 // ds values x 64 tokens (rows of 2 ds bytes, no swizzle); tokens past T read as zero
 bool make_map_bf16_slice(CUtensorMap* map, const void* base, int64_t N, int64_t T, int width, int ds, int heads = 1) {
-    auto fn = encode_fn_bf16();
+    auto fn = tensor_map_encoder();
     if (!fn) return false;
     if (heads > 1) {   // [N / heads][T][heads][width]
         cuuint64_t dims5[5] = {(cuuint64_t)ds, (cuuint64_t)T, (cuuint64_t)(width / ds), (cuuint64_t)heads,
@@ -1971,7 +1926,7 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
                         int* status, int phases, bool global_norm) {
     const int G = dm.S / SG;
     if (global_norm && G > 1) return cudaErrorInvalidValue;   // the one-group kernel has the global form
-    if (dm.H > 1 && G < 4) return cudaErrorInvalidValue;      // the heads layout of V / out: the wide kernel below
+    if (dm.H > 1 && G == 2 && phases != kPhaseTotals) return cudaErrorInvalidValue;   // its output kernel takes [N, T, D]
     // two bucket groups per totals CTA where there are at least two (they share the V tile)
     const int GP = G >= 2 ? 2 : 1;
     auto k1 = GP == 2 ? tile_totals_tc_bf16<D, 2> : tile_totals_tc_bf16<D, 1>;
@@ -2046,11 +2001,17 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
     CUtensorMap mq1;
     if (!make_map_bf16(&mq1, pq, dm.N, dm.T, dm.S)) return cudaErrorInvalidValue;
     k3<<<grid, kThreads, Lay<D>::kSmem, stream>>>(mq1, mk, mv, (__nv_bfloat16*)out,
-                                                  (const float*)ws, dm.T, dm.S, G, tile_tokens, dm.eps, status);
+                                                  (const float*)ws, dm.T, dm.S, G, tile_tokens, dm.eps, dm.H, status);
     return cudaGetLastError();
 }
 
 }  // namespace
+
+bool tensor_bf16_heads_supported(const Dims& dm) {
+    Dims flat = dm;
+    flat.H = 1;
+    return tensor_bf16_supported(flat) && dm.S != 2 * SG && dm.N % dm.H == 0;
+}
 
 bool tensor_bf16_supported(const Dims& dm) {
     const int G = dm.S / SG;

@@ -5,7 +5,12 @@
 
 #include "common.cuh"
 
+#include <cudaTypedefs.h>
+
 namespace race {
+
+// the driver's tensor-map encoder (causal_tc.cu); null if it cannot be looked up
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
 // ---- CUDA-core causal path (causal_simt.cu) -------------------------------------------------
 int simt_groups(int S);
@@ -130,8 +135,18 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
                               const float* d_state, void* dpq, void* dpk, void* dv, float* d_carry, void* ws,
                               const Dims& dm, int tile_tokens, cudaStream_t stream, int* status);
 
+// bf16, S = 64, 128, 256 or 512, d_k 64 or 128 (causal_bwd_bf16_tc.cu); v, dout, dv with dm.H heads
+bool causal_bwd_bf16_supported(const Dims& dm);
+int causal_bwd_bf16_tile_tokens(const Dims& dm, int sm_count);
+size_t causal_bwd_bf16_workspace_bytes(const Dims& dm, int tile_tokens);
+cudaError_t causal_bwd_bf16(const void* pq, const void* pk, const void* v, const void* dout, const float* carry_in,
+                            const float* d_state, void* dpq, void* dpk, void* dv, float* d_carry, void* ws,
+                            const Dims& dm, int tile_tokens, cudaStream_t stream, int* status);
+
 // bf16 tensor path (causal_tc_bf16.cu): S a multiple of 64 (1, 2, 4 or 8 bucket groups), d_k 64 or 128
 bool tensor_bf16_supported(const Dims& dm);
+// ... with V / out in the layout [N/H, T, H, D] also for one bucket group (race_b200_causal_fwd_heads)
+bool tensor_bf16_heads_supported(const Dims& dm);
 cudaError_t causal_fwd_tensor_bf16(const void* pq, const void* pk, const void* v, void* out,
                                    const float* carry_in, float* state_out, void* ws, const Dims& dm,
                                    int tile_tokens, cudaStream_t stream, int* status, int phases,

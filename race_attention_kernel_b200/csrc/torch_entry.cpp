@@ -12,6 +12,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdlib>
@@ -126,7 +128,9 @@ PyObject* forward_impl(PyObject* const* args, Py_ssize_t nargs) {
         (carry && !state_ok(*carry, *k, N * L * R * (dk + 1))))
         return none();
     const bool qkv = fuse && race_b200_qkv_is_supported(&sh, (int)P);
-    if (!qkv && !race_b200_is_supported(&sh, RACE_VARIANT_AUTO)) return none();
+    const size_t wb = qkv ? race_b200_causal_workspace_bytes(&sh, 0, RACE_VARIANT_TENSOR)
+                          : race_b200_causal_heads_workspace_bytes(&sh);
+    if (!qkv && !wb) return none();
     int* status = (int*)PyLong_AsVoidPtr(args[10]);
     c10::cuda::CUDAGuard guard(k->device());
     void* stream = c10::cuda::getCurrentCUDAStream().stream();
@@ -135,7 +139,6 @@ PyObject* forward_impl(PyObject* const* args, Py_ssize_t nargs) {
     at::Tensor state = want_state ? floats({N, L * R * (dk + 1)}, *k) : at::Tensor();
     const float* carry_p = carry ? carry->const_data_ptr<float>() : nullptr;
     float* state_p = want_state ? state.data_ptr<float>() : nullptr;
-    const size_t wb = race_b200_causal_workspace_bytes(&sh, 0, qkv ? RACE_VARIANT_TENSOR : RACE_VARIANT_AUTO);
     at::Tensor ws = bytes(wb, *k);
     if (qkv) {
         check(race_b200_causal_fwd_qkv(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), planes.const_data_ptr<float>(),
@@ -149,9 +152,9 @@ PyObject* forward_impl(PyObject* const* args, Py_ssize_t nargs) {
             check(race_b200_bucket_probs_streams(src[i]->const_data_ptr(), planes.const_data_ptr<float>(), dst[i]->data_ptr(), MB, T,
                                                  (int32_t)H, (int32_t)dk, (int32_t)L, (int32_t)P, sh.dtype, sh.dtype, stream),
                   "race_b200_bucket_probs_streams");
-        check(race_b200_causal_fwd(pq.const_data_ptr(), pk.const_data_ptr(), v->const_data_ptr(), out.data_ptr(), carry_p, state_p,
-                                   ws.data_ptr(), wb, &sh, 0, RACE_VARIANT_AUTO, stream, status),
-              "race_b200_causal_fwd");
+        check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), v->const_data_ptr(), out.data_ptr(), carry_p,
+                                         state_p, ws.data_ptr(), wb, &sh, stream, status),
+              "race_b200_causal_fwd_heads");
     }
     raise_on_wait(status, "BatchedACE.forward");
     return result(out, state, N, L, R, dk);
@@ -186,6 +189,104 @@ PyObject* prefix_impl(PyObject* const* args, Py_ssize_t nargs) {
     return result(out, state, N, L, R, dk);
 }
 
+// The operator with gradients for K, V and Q as one autograd node: producers, prefix forward; causal backward, producer
+// backward.  Saved are the inputs and the two probability tensors.
+struct TrainOp : torch::autograd::Function<TrainOp> {
+    static RaceShape shape(const at::Tensor& k, int64_t L, int64_t P, double eps) {
+        return RaceShape{k.size(0) * k.size(1) * k.size(3), k.size(2), (int32_t)L, (int32_t)(1 << P), (int32_t)k.size(4),
+                         dtype_of(k), (float)eps, (int32_t)k.size(3)};
+    }
+
+    static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& k, const at::Tensor& v,
+                              const at::Tensor& q, const at::Tensor& planes, int64_t L, int64_t P, double eps, int64_t status) {
+        c10::cuda::CUDAGuard guard(k.device());
+        void* stream = c10::cuda::getCurrentCUDAStream().stream();
+        const RaceShape sh = shape(k, L, P, eps);
+        at::Tensor pk = at::empty({sh.n_streams, sh.seq_len, L, 1ll << P}, k.options()), pq = at::empty_like(pk);
+        const at::Tensor* src[2] = {&k, &q};
+        at::Tensor* dst[2] = {&pk, &pq};
+        for (int i = 0; i < 2; ++i)
+            check(race_b200_bucket_probs_streams_exact(src[i]->const_data_ptr(), planes.const_data_ptr<float>(), dst[i]->data_ptr(),
+                                                       k.size(0) * k.size(1), sh.seq_len, sh.heads, sh.head_dim, (int32_t)L,
+                                                       (int32_t)P, sh.dtype, stream),
+                  "race_b200_bucket_probs_streams_exact");
+        at::Tensor out = at::empty(v.sizes(), v.options());
+        const size_t wb = race_b200_causal_heads_workspace_bytes(&sh);
+        at::Tensor ws = bytes(wb, k);
+        check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), v.const_data_ptr(), out.data_ptr(), nullptr,
+                                         nullptr, ws.data_ptr(), wb, &sh, stream, (int*)status),
+              "race_b200_causal_fwd_heads");
+        raise_on_wait((int*)status, "BatchedACE.forward");
+        ctx->save_for_backward({k, v, q, planes, pk, pq});
+        ctx->saved_data["dims"] = std::vector<int64_t>{L, P, status};
+        ctx->saved_data["eps"] = eps;
+        return out;
+    }
+
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const at::Tensor &k = saved[0], &v = saved[1], &q = saved[2], &planes = saved[3], &pk = saved[4], &pq = saved[5];
+        const auto dims = ctx->saved_data["dims"].toIntVector();
+        const int64_t L = dims[0], P = dims[1];
+        int* status = (int*)dims[2];
+        torch::autograd::variable_list res(8);
+        {
+            at::AutoGradMode no_grad(false);
+            c10::cuda::CUDAGuard guard(k.device());
+            void* stream = c10::cuda::getCurrentCUDAStream().stream();
+            const RaceShape sh = shape(k, L, P, ctx->saved_data["eps"].toDouble());
+            const at::Tensor g = grads[0].to(v.scalar_type()).contiguous();   // may come expanded (stride 0)
+            at::Tensor dpq = at::empty_like(pq), dpk = at::empty_like(pk), dv = at::empty(v.sizes(), v.options());
+            const size_t wb = race_b200_causal_bwd_workspace_bytes(&sh);
+            at::Tensor ws = bytes(wb, k);
+            check(race_b200_causal_bwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), v.const_data_ptr(), g.const_data_ptr(), nullptr,
+                                             nullptr, dpq.data_ptr(), dpk.data_ptr(), dv.data_ptr(), nullptr, ws.data_ptr(), wb,
+                                             &sh, stream, status),
+                  "race_b200_causal_bwd_heads");
+            const at::Tensor* x[2] = {&k, &q};
+            const at::Tensor* dp[2] = {&dpk, &dpq};
+            for (int i = 0; i < 2; ++i) {
+                if (!ctx->needs_input_grad(i ? 2 : 0)) continue;
+                at::Tensor dx = at::empty(x[i]->sizes(), x[i]->options());
+                check(race_b200_bucket_probs_streams_bwd(x[i]->const_data_ptr(), planes.const_data_ptr<float>(), dp[i]->const_data_ptr(),
+                                                         dx.data_ptr(), k.size(0) * k.size(1), sh.seq_len, sh.heads, sh.head_dim,
+                                                         (int32_t)L, (int32_t)P, sh.dtype, stream),
+                      "race_b200_bucket_probs_streams_bwd");
+                res[i ? 2 : 0] = dx;
+            }
+            if (ctx->needs_input_grad(1)) res[1] = dv;
+            raise_on_wait(status, "BatchedACE backward");
+        }
+        if (at::GradMode::is_enabled()) {   // the backward has no derivative of its own
+            torch::autograd::variable_list first{res[0], res[1], res[2]};
+            auto err = std::make_shared<torch::autograd::DelayedError>(
+                "trying to differentiate twice a function that was marked with @once_differentiable", 3);
+            for (auto& t : first)
+                if (t.defined()) t.requires_grad_(true);
+            first = (*err)(std::move(first));
+            for (int i = 0; i < 3; ++i) res[i] = first[i];
+        }
+        return res;
+    }
+};
+
+// train_forward(planes_T, K, V, Q, L, n_planes, eps, status pointer) -> out | None
+PyObject* train_impl(PyObject* const* args, Py_ssize_t nargs) {
+    if (nargs != 8) throw Fail("train_forward takes 8 arguments");
+    const at::Tensor *pt = tensor_of(args[0]), *k = tensor_of(args[1]), *v = tensor_of(args[2]), *q = tensor_of(args[3]);
+    if (!pt || pt->requires_grad() || !k || !v || !q || k->dim() != 5 || !plain(*k) || !like(*v, *k) || !like(*q, *k)) return none();
+    const int64_t L = PyLong_AsLongLong(args[4]), P = PyLong_AsLongLong(args[5]);
+    if (L < 1 || P < 1 || P > 12 || k->numel() == 0) return none();
+    const double eps = PyFloat_AsDouble(args[6]);
+    const RaceShape sh = TrainOp::shape(*k, L, P, eps);
+    if (pt->dim() != 2 || pt->size(0) != sh.head_dim || pt->size(1) != L * P ||
+        !race_b200_bucket_probs_bwd_is_supported(sh.head_dim, (int32_t)L, (int32_t)P, sh.dtype) ||
+        !race_b200_causal_heads_workspace_bytes(&sh) || !race_b200_causal_bwd_workspace_bytes(&sh))
+        return none();
+    const int64_t status = (int64_t)PyLong_AsVoidPtr(args[7]);
+    return THPVariable_Wrap(TrainOp::apply(*k, *v, *q, planes_rows(*pt, *k), L, P, eps, status));
+}
+
 template <PyObject* (*kImpl)(PyObject* const*, Py_ssize_t)>
 PyObject* guarded(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     try {
@@ -213,6 +314,7 @@ PyObject* guarded(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 PyMethodDef kMethods[] = {
     {"step", (PyCFunction)(void (*)(void))guarded<step_impl>, METH_FASTCALL, nullptr},
     {"forward", (PyCFunction)(void (*)(void))guarded<forward_impl>, METH_FASTCALL, nullptr},
+    {"train_forward", (PyCFunction)(void (*)(void))guarded<train_impl>, METH_FASTCALL, nullptr},
     {"causal_prefix", (PyCFunction)(void (*)(void))guarded<prefix_impl>, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

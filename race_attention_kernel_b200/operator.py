@@ -13,7 +13,7 @@ accepted and streamed through the device; there is no CPU compute path.
 Gradients: the reference module is differentiable through K, V and Q (plain autograd over
 src/race_baseline.py:41-51).  Here, when autograd is recording and an input requires a gradient,
 ``forward`` is one autograd node over the kernels: the producer, the prefix forward, and for the gradients
-the causal backward and the backward of the producer.  Geometries the producer's backward does not cover form
+the causal backward and the backward of the producer (in C++ where every kernel takes the operator's layout).  Geometries the producer's backward does not cover form
 the bucket probabilities with differentiable torch ops and run the prefix path through ``ops.race_causal``.
 """
 from __future__ import annotations
@@ -144,6 +144,11 @@ class BatchedACE(nn.Module):
             if carry_in is not None or return_state:
                 raise RuntimeError("carry_in / return_state are inference-only; chain ops.race_causal_chunk "
                                    "for differentiable chunked sequences")
+            if Khf.is_cuda and not self.protos_T.requires_grad:
+                out = _lib.native().train_forward(self.planes_T, Khf, Vhf, Qhf, self.L, self.K, self.eps,
+                                                  ops._status_ptr(Khf.get_device()))
+                if out is not None:
+                    return out
             if Khf.dtype not in (torch.float32, torch.bfloat16):
                 raise RuntimeError("fp32 or bf16 inputs only")
             return self._forward_autograd(Khf, Vhf, Qhf)
