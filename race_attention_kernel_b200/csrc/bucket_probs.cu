@@ -210,6 +210,8 @@ bucket_probs_mma_d64_l4k4(const float* __restrict__ x, const float* __restrict__
                           int64_t rows, int64_t T, int heads) {
     constexpr int D = 64, R = 16, LR = 64;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    chain_release();
+    chain_wait();
     PlaneFrags pf;
     load_plane_frags(planes, lane, pf);
     const float inv_scale = rsqrtf((float)D);
@@ -302,6 +304,8 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
     static_assert(kDirect || (kPPF >= 1 && TPL % kPPF == 0 && PB % 128 == 0), "staging geometry");
     uint2* tab3 = reinterpret_cast<uint2*>(wide_smem + W::kTabBytes);   // kExact: the third limbs {b0, b1}
     uint8_t* stage = wide_smem + W::kTabBytes + (kExact ? W::kTabBytes / 2 : 0) + (threadIdx.x >> 5) * W::kStageBytes;
+    chain_release();
+    chain_wait();
     auto swz = [](int off) {   // 16-byte piece (off >> 4) & 7 of 128-byte block b = off >> 7, XOR (b / 8 + 2 (b % 8)) % 8
         const int b = off >> 7;
         return (b << 7) | (((((off >> 4) & 7) ^ ((b >> 3) + 2 * (b & 7))) & 7) << 4);
@@ -497,8 +501,7 @@ cudaError_t launch_probs_wide(const void* x, const float* planes, void* probs, i
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int64_t want = (rows + 63) / 64;   // 64 rows per CTA and pass
     const unsigned blocks = (unsigned)std::min<int64_t>(want, (int64_t)(sms > 0 ? sms : 148) * 12);
-    kern<<<blocks, kWideThreads, smem, stream>>>((const Tx*)x, planes, (Tp*)probs, rows, T, heads);
-    return cudaGetLastError();
+    return launch_chain(chain_launches(rows, L << K), kern, blocks, kWideThreads, smem, stream, (const Tx*)x, planes, (Tp*)probs, rows, T, heads);
 }
 
 template <typename Tx, typename Tp, int K>
@@ -555,9 +558,8 @@ cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int64_t want = (rows + 63) / 64;   // 64 rows per CTA and pass
         const unsigned blocks = (unsigned)std::min<int64_t>(want, (int64_t)(sms > 0 ? sms : 148) * 16);
-        bucket_probs_mma_d64_l4k4<<<blocks, kFastThreads, 0, stream>>>((const float*)x, planes, (float*)probs, rows, T,
-                                                                       heads);
-        return cudaGetLastError();
+        return launch_chain(chain_launches(rows, 64), bucket_probs_mma_d64_l4k4, blocks, kFastThreads, 0, stream, (const float*)x, planes, (float*)probs,
+                            rows, T, heads);
     }
     // the small geometry with bf16 rows: its tables need no staging (48 streams of 5003 tokens: 51 us on the general
     // kernel, which runs sixteen dot products per row on the CUDA cores)

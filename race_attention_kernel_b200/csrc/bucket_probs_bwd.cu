@@ -73,6 +73,8 @@ bucket_probs_bwd_mma(const Tx* __restrict__ x, const float* __restrict__ planes,
     uint4* tab2 = tab1 + W::kTab1;                             // [(nb KS + j) 32 + lane]
     uint2* tab1r = reinterpret_cast<uint2*>(tab2 + W::kTab2);   // fp32 rows: third limbs {b0, b1} of tab1
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    chain_release();
+    chain_wait();
     for (int i = threadIdx.x; i < W::kTab1; i += kBwdThreads) {
         const int ln = i & 31, f = i >> 5, j = f % NJ, nt = f / NJ;
         const int fg = ln >> 2, ft = ln & 3;
@@ -271,8 +273,8 @@ cudaError_t launch_probs_bwd(const void* x, const float* planes, const void* dpr
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // the plane tables are built once per CTA: the resident CTAs walk the rows
     const unsigned blocks = (unsigned)std::min<int64_t>((rows + 63) / 64, (int64_t)(sms > 0 ? sms : 148) * BwdProbs<D, L, K>::kCtas);
-    kern<<<blocks, kBwdThreads, smem, stream>>>((const Tx*)x, planes, (const Tp*)dprobs, (Tx*)dx, rows, T, heads);
-    return cudaGetLastError();
+    return launch_chain(chain_launches(rows, L << K), kern, blocks, kBwdThreads, smem, stream, (const Tx*)x, planes, (const Tp*)dprobs, (Tx*)dx, rows, T,
+                        heads);
 }
 
 }  // namespace

@@ -17,8 +17,8 @@
 // Precision is that of fp32 arithmetic on the bf16 inputs up to 2^-17: inputs are exact one-limb operands, everything
 // computed (W, the masked products, the states, g) is split into hi + lo bf16 limbs, accumulators are fp32.
 //
-// Why this shape of kernel.  On CUDA cores the two passes took 3.3 of 3.4 ms of ... (S = 64) and 9.0 of 9.8 ms (S = 512)
-// of a training step.  Chunks of 128 tokens and blocks of 128 buckets make every product 128 x 128 x 128 (full M, N of
+// Why this shape of kernel.  On CUDA cores the two passes took 1.31 of the 1.73 ms of a training step at S = 64 (96
+// streams of 4096 tokens) and 9.05 of 9.79 ms at S = 512, d_k = 128 (32 streams of 4096).  Chunks of 128 tokens and blocks of 128 buckets make every product 128 x 128 x 128 (full M, N of
 // the tensor core; M = 64 runs at half rate), an accumulator row is a thread's token, and TMA writes the operand tiles
 // as the tensor core reads them (128-byte swizzle, both majors), so the only data the warps move are the computed
 // limbs.  Shared memory (224 KB at 128 x 128) holds one chunk: a chunk's chain of products is serial, and what bounds
@@ -35,9 +35,12 @@ namespace race {
 namespace {
 
 constexpr int C = 128;              // tokens per chunk
-constexpr int kThreads = 16 * 32;   // 8 worker warps, 4 state warps, one group with the TMA and MMA warps
-constexpr int kTmaWarp = 12, kMmaWarp = 13;
-constexpr uint32_t tG = 256;        // tensor-memory columns: states [0, 256), masked products [256, 384), results [384, 512)
+// 8 warps on the bucket side (W, dPQ / dPK), 8 on the token x token products (masks, sums of g, dV), 4 on the state, and
+// one group with the TMA and MMA warps
+constexpr int kThreads = 24 * 32;
+constexpr int kStateWarp = 16, kTmaWarp = 20, kMmaWarp = 21;
+constexpr int kRegsP = 104, kRegsG = 72, kRegsS = 64, kRegsM = 64;   // 8, 8, 4, 4 warps: exactly the 768 x 80 of the launch
+constexpr uint32_t tG = 256;        // tensor-memory columns of the token x token products
 
 __device__ __forceinline__ float2 unpack2(uint32_t u) {
     return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
@@ -60,17 +63,19 @@ struct Lay {
     static constexpr int oB = oWlo + (kSuffix ? kP : 0);                     // [hi | lo][SB rows][D]
     static constexpr int kB = SB * D * 2;
     static constexpr int oCar = oB + 2 * kB;                                 // [2][SB] fp32 running A / later g
-    static constexpr int oTot = oCar + 2 * SB * 4;                           // [SB] fp32 totals of g (prefix pass)
+    static constexpr int oTot = oCar + 2 * SB * 4;                           // [SB] prefix: totals of g; suffix: A before the chunk
     static constexpr int oBars = oTot + SB * 4;
-    static constexpr int kNumBars = 20;
+    static constexpr int kNumBars = 24;
     static constexpr int oMisc = oBars + kNumBars * 8;
     static constexpr int kSmem = oMisc + 16 + 1024;
     static_assert(kSmem <= 227 * 1024, "shared memory of the backward");
 };
+// A wait on a barrier never lags it by two phases: every party that waits on one also has to arrive somewhere before the
+// next phase of that barrier can complete.
 enum Bar {
     bFull = 0,      // [2] dO, V, pK of the stage have landed
     bFullQ = 2,     // [2] pQ
-    bTri = 4,       // the triangular matrix of the chunk is in the G columns, every result of the chunk before is read (8)
+    bTri = 4,       // triangular matrix of the chunk in the G columns; prefix: the sums of g of the chunk before are read (8)
     bA = 5,         // running sums of pK inside the chunk
     bG = 6,         // first token x token product
     bSt = 7,        // state updated with the chunk
@@ -78,11 +83,15 @@ enum Bar {
     bBt = 9,        // operand tiles of the state before the chunk written, accumulator read (4)
     bW = 10,        // W limbs written, running sums read (8)
     bGm = 11,       // masked first product written (8)
-    bX = 12,        // prefix: X complete.  suffix: second token x token product complete
-    bXg = 13,       // prefix: X read, g limbs written (8).  suffix: masked second product written (8)
-    bEnd = 14,      // every product of the chunk has run
-    bEmpty = 15,    // [2] ... of the chunk in the stage
-    bDrain = 17
+    bX = 12,        // bucket-side result (X / P) complete
+    bXg = 13,       // prefix: X read, g limbs written, upper triangle written (16)
+    bH = 14,        // suffix: second token x token product.  prefix: totals updated, W no longer read
+    bHm = 15,       // suffix: masked second product written (8)
+    bPf = 16,       // suffix: P read (8)
+    bVf = 17,       // suffix: dV read (8)
+    bEnd = 18,      // every product of the chunk has run
+    bEmpty = 19,    // [2] ... of the chunk in the stage
+    bDrain = 21
 };
 
 struct Args {
@@ -123,11 +132,12 @@ __device__ __forceinline__ Setup begin(const Args& a) {
     s.t_begin = s.tile * a.tile_tokens;
     s.t_end = min(a.T, s.t_begin + (int64_t)a.tile_tokens);
     s.nch = (int)((s.t_end - s.t_begin + C - 1) / C);
+    chain_release();
     if (threadIdx.x == 0) {
         *s.cx.abort_flag = 0;
         for (int i = 0; i < Ly::kNumBars; ++i) {
-            const uint32_t cnt = (i == bTri || i == bW || i == bGm || i == bXg) ? 8u : i == bBt ? 4u : 1u;
-            mbar_init(s.cx.bar(i), cnt);
+            constexpr uint32_t kEight = (1u << bTri) | (1u << bW) | (1u << bGm) | (1u << bHm) | (1u << bPf) | (1u << bVf);
+            mbar_init(s.cx.bar(i), (kEight >> i) & 1u ? 8u : i == bXg ? 16u : i == bBt ? 4u : 1u);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -140,6 +150,7 @@ __device__ __forceinline__ Setup begin(const Args& a) {
     __syncthreads();
     tc_fence_after();
     s.tmem = *reinterpret_cast<volatile uint32_t*>(s.cx.sm + Ly::oMisc);
+    chain_wait();
     return s;
 }
 __device__ __forceinline__ void finish(uint32_t tmem) {
@@ -149,6 +160,11 @@ __device__ __forceinline__ void finish(uint32_t tmem) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
+}
+// the lanes of a warp have written operands or read accumulators: one arrival
+__device__ __forceinline__ void arrive_warp(const Ctx& cx, int bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(cx.bar(bar));
 }
 
 // TMA producer (one lane): dO, V, pK, pQ of the c-th chunk that is processed
@@ -191,13 +207,13 @@ struct StateRow {
 };
 template <int SB>
 __device__ __forceinline__ void store_state_limbs(uint8_t* hi_tile, int lo_off, const StateRow<SB>& r, int col,
-                                                  const float (&v)[32]) {
-    uint32_t hi[16], lo[16];
+                                                  const float (&v)[16]) {
+    uint32_t hi[8], lo[8];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) split2(v[2 * i], v[2 * i + 1], hi[i], lo[i]);
+    for (int i = 0; i < 8; ++i) split2t(v[2 * i], v[2 * i + 1], hi[i], lo[i]);
     if (r.live) {
-        sw_store_row<SB, 16>(hi_tile, r.row, col, hi);
-        sw_store_row<SB, 16>(hi_tile + lo_off, r.row, col, lo);
+        sw_store_row<SB, 8>(hi_tile, r.row, col, hi);
+        sw_store_row<SB, 8>(hi_tile + lo_off, r.row, col, lo);
     }
 }
 
@@ -206,63 +222,73 @@ template <int SB, int D, typename Ly>
 __device__ __forceinline__ void load_state(const Setup& s, const Args& a, int w, int lane) {
     const StateRow<SB> r(w, lane);
     const float* src = a.ws + (s.n * s.tiles + s.tile) * (int64_t)(a.S * (D + 1)) + (int64_t)(s.g0 + r.row) * D;
+#pragma unroll 1
+    for (int cb = 0; cb < D; cb += 16) {
+        float v[16];
 #pragma unroll
-    for (int cb = 0; cb < D; cb += 32) {
-        float v[32];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
+        for (int i = 0; i < 16; i += 4) {
             const float4 x = r.live ? __ldg(reinterpret_cast<const float4*>(src + cb + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
             v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
         }
-        tmem_st_rows32(((uint32_t)(32 * w) << 16) + s.tmem + cb, v);
+        tmem_st_words16(((uint32_t)(32 * w) << 16) + s.tmem + cb, reinterpret_cast<const uint32_t(&)[16]>(v));
         store_state_limbs<SB>(s.cx.sm + Ly::oB, Ly::kB, r, cb, v);
     }
+    tmem_wait_st();
     fence_proxy_async();
     tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(s.cx.bar(bBt));
+    arrive_warp(s.cx, bBt);
 }
 // after every chunk but the last: updated accumulator -> operand tiles
 template <int SB, int D, typename Ly>
 __device__ __forceinline__ void carry_state(const Setup& s, int w, int lane) {
-    const StateRow<SB> r(w, lane);
+    StateRow<SB> r(w, lane);
     bool ok = true;
     for (int c = 1; c < s.nch && ok; ++c) {
+        asm volatile("" : "+r"(r.row));   // (addresses per chunk, not kept in registers this group does not have)
+        RACE_TRACE(2, c, 0);
         if (!(ok = wait_bar_warp(s.cx, bSt, (uint32_t)((c - 1) & 1), 201))) break;
         if (!(ok = wait_bar_warp(s.cx, bXb, (uint32_t)((c - 1) & 1), 202))) break;
+        RACE_TRACE(2, c, 1);
         tc_fence_after();
 #pragma unroll
-        for (int cb = 0; cb < D; cb += 32) {
-            float v[32];
-            tmem_ld_rows32(((uint32_t)(32 * w) << 16) + s.tmem + cb, v);
+        for (int cb = 0; cb < D; cb += 16) {
+            float v[16];
+            tmem_ld_rows16(((uint32_t)(32 * w) << 16) + s.tmem + cb, v);
             store_state_limbs<SB>(s.cx.sm + Ly::oB, Ly::kB, r, cb, v);
         }
         fence_proxy_async();
         tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(s.cx.bar(bBt));
+        arrive_warp(s.cx, bBt);
+        RACE_TRACE(2, c, 2);
     }
 }
 
 // the 64 columns [64 wg, +64) of a token x token product: mask (kUpper: column >= row stays), split, and write the limbs
-// over the columns just read (hi in the first 32, lo in the second)
+// over the 32 columns they came from (16 words of hi, 16 of lo).  32-column blocks outside the triangle are only zeroed.
 template <bool kUpper>
 __device__ __forceinline__ void mask_product(uint32_t tm_lane, int row, int wg) {
-    uint32_t hi[32], lo[32];
 #pragma unroll
     for (int hb = 0; hb < 2; ++hb) {
-        float v[32];
-        tmem_ld_rows32(tm_lane + tG + 64 * wg + 32 * hb, v);
+        const int col0 = 64 * wg + 32 * hb;
+        uint32_t hi[16], lo[16];
+        if (kUpper ? col0 + 31 < (row & ~31) : col0 > (row | 31)) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int col = 64 * wg + 32 * hb + 2 * i;
-            const float x = (kUpper ? col >= row : col <= row) ? v[2 * i] : 0.f;
-            const float y = (kUpper ? col + 1 >= row : col + 1 <= row) ? v[2 * i + 1] : 0.f;
-            split2(x, y, hi[16 * hb + i], lo[16 * hb + i]);
+            for (int i = 0; i < 16; ++i) hi[i] = lo[i] = 0u;
+        } else {
+            float v[32];
+            tmem_ld_rows32(tm_lane + tG + col0, v);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const int col = col0 + 2 * i;
+                const float x = (kUpper ? col >= row : col <= row) ? v[2 * i] : 0.f;
+                const float y = (kUpper ? col + 1 >= row : col + 1 <= row) ? v[2 * i + 1] : 0.f;
+                split2t(x, y, hi[i], lo[i]);
+            }
         }
+        tmem_st_words16(tm_lane + tG + col0, hi);
+        tmem_st_words16(tm_lane + tG + col0 + 16, lo);
     }
-    tmem_st_words32(tm_lane + tG + 64 * wg, hi);
-    tmem_st_words32(tm_lane + tG + 64 * wg + 32, lo);
+    tmem_wait_st();
     tc_fence_before();
 }
 template <bool kUpper>
@@ -271,6 +297,16 @@ __device__ __forceinline__ void write_tri(uint32_t tm_lane, int row, int wg) {
     tri_words<kUpper>(row, wg, tr);
     tmem_st_words32(tm_lane + tG + 32 * wg, tr);
     tc_fence_before();
+}
+__device__ __forceinline__ void store_row16(float* dst, const float (&v)[16]) {
+    st_global_32b(dst, reinterpret_cast<const uint32_t(&)[8]>(v[0]));
+    st_global_32b(dst + 8, reinterpret_cast<const uint32_t(&)[8]>(v[8]));
+}
+__device__ __forceinline__ void store_row16(__nv_bfloat16* dst, const float (&v)[16]) {
+    uint32_t d[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d[i] = pack2(v[2 * i], v[2 * i + 1]);
+    st_global_32b(dst, d);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -287,22 +323,15 @@ bwd_prefix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
     float* car = reinterpret_cast<float*>(cx.sm + Ly::oCar);
     float* tot = reinterpret_cast<float*>(cx.sm + Ly::oTot);
     const int64_t sf = (int64_t)a.S * (D + 1);
+    const int wg = (warp >> 2) & 1, w = warp & 3, row = 32 * w + lane;
+    const uint32_t tm_lane = s.tmem + ((uint32_t)(32 * w) << 16);
+    const int col0 = HC * wg;                        // first bucket column of this thread inside the block
 
-    if (warp >= 12) regs_dec<72>();
     if (warp < 8) {
-        regs_inc<168>();
-        const int wg = warp >> 2, w = warp & 3, row = 32 * w + lane;
-        const uint32_t tm_lane = s.tmem + ((uint32_t)(32 * w) << 16);
-        const int col0 = HC * wg;                    // first bucket column of this thread inside the block
+        regs_inc<kRegsP>();
         const float* slice_a = a.ws + (s.n * s.tiles + s.tile) * sf + (int64_t)a.S * D + s.g0;
-        if (row < HC) {
-            car[col0 + row] = slice_a[col0 + row];
-            tot[col0 + row] = 0.f;
-        }
+        if (row < HC) car[col0 + row] = slice_a[col0 + row];
         asm volatile("bar.sync 5, 256;" ::: "memory");
-        write_tri<false>(tm_lane, row, wg);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(cx.bar(bTri));
         const int64_t nchunk = (a.T + C - 1) / C;
         bool ok = true;
         for (int c = 0; c < s.nch && ok; ++c) {
@@ -312,31 +341,30 @@ bwd_prefix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
             const int64_t tok = s.t_begin + (int64_t)c * C + row;
             const bool live = tok < s.t_end;
             // ---- running A, W = pQ / (A + eps) -> limbs over pQ and over V ---------------------------------
-            if (!(ok = wait_bar_warp(cx, bTri, ph, 101))) break;   // every worker has finished the chunk before
+            // every warp of the group has published / read the running A of the chunk before
+            if (c > 0 && !(ok = wait_bar_warp(cx, bXg, ph ^ 1, 101))) break;
             if (row < HC)
                 a.achunk[(s.n * nchunk + s.t_begin / C + c) * a.S + s.g0 + col0 + row] = car[(c & 1) * SB + col0 + row];
             if (!(ok = wait_bar_warp(cx, bFullQ + st, (uint32_t)((c / Ly::kStages) & 1), 102))) break;
+            RACE_TRACE(wg, c, 0);
             if (!(ok = wait_bar_warp(cx, bA, ph, 103))) break;
+            RACE_TRACE(wg, c, 1);
             tc_fence_after();
             float inv[HC];
-            uint32_t pq[HC / 2];
 #pragma unroll
-            for (int cb = 0; cb < HC; cb += 32) {
-                float v[32];
-                tmem_ld_rows32(tm_lane + tX + col0 + cb, v);
+            for (int cb = 0; cb < HC; cb += 16) {
+                float v[16];
+                tmem_ld_rows16(tm_lane + tX + col0 + cb, v);
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
+                for (int i = 0; i < 16; i += 4) {
                     const float4 c4 = *reinterpret_cast<const float4*>(car + (c & 1) * SB + col0 + cb + i);
                     v[i] += c4.x; v[i + 1] += c4.y; v[i + 2] += c4.z; v[i + 3] += c4.w;
-                }
-                if (row == C - 1) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4)
+                    if (row == C - 1)
                         *reinterpret_cast<float4*>(car + ((c + 1) & 1) * SB + col0 + cb + i) =
                             make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
                 }
 #pragma unroll
-                for (int i = 0; i < 32; ++i) inv[cb + i] = __fdividef(1.f, v[i] + a.eps);
+                for (int i = 0; i < 16; ++i) inv[cb + i] = __fdividef(1.f, v[i] + a.eps);
             }
             if (!(ok = wait_bar_warp(cx, bSt, ph, 104))) break;   // V has been read: its slot takes the low limbs
 #pragma unroll
@@ -347,127 +375,153 @@ bwd_prefix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
                 uint32_t hi[4], lo[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    pq[4 * p + i] = qq[i];
                     const float2 q2 = unpack2(qq[i]);
-                    split2(q2.x * inv[8 * p + 2 * i], q2.y * inv[8 * p + 2 * i + 1], hi[i], lo[i]);
+                    split2t(q2.x * inv[8 * p + 2 * i], q2.y * inv[8 * p + 2 * i + 1], hi[i], lo[i]);
                 }
                 *reinterpret_cast<uint4*>(stage + Ly::oQ + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                 *reinterpret_cast<uint4*>(stage + Ly::oV + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
             fence_proxy_async();
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bW));
-            // ---- causal mask of dO V^T --------------------------------------------------------------------
-            if (!(ok = wait_bar_warp(cx, bG, ph, 105))) break;
-            tc_fence_after();
-            mask_product<false>(tm_lane, row, wg);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bGm));
-            // ---- X -> dPQ, g limbs over W ---------------------------------------------------------------------
+            arrive_warp(cx, bW);
+            RACE_TRACE(wg, c, 2);
+            // ---- X -> dPQ, g = -dPQ W -> limbs over W ----------------------------------------------------------
             if (!(ok = wait_bar_warp(cx, bX, ph, 106))) break;
+            RACE_TRACE(wg, c, 3);
             tc_fence_after();
             __nv_bfloat16* dst = a.dp + (s.n * a.T + tok) * a.S + s.g0 + col0;
 #pragma unroll
-            for (int cb = 0; cb < HC; cb += 32) {
-                float v[32];
-                tmem_ld_rows32(tm_lane + tX + col0 + cb, v);
-                uint32_t hi[16], lo[16], d[16];
+            for (int cb = 0; cb < HC; cb += 16) {     // inv <- dPQ
+                float v[16];
+                tmem_ld_rows16(tm_lane + tX + col0 + cb, v);
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    const float i0 = inv[cb + 2 * i], i1 = inv[cb + 2 * i + 1];
-                    const float2 q2 = unpack2(pq[cb / 2 + i]);
-                    const float d0 = v[2 * i] * i0, d1 = v[2 * i + 1] * i1;
-                    d[i] = pack2(d0, d1);
-                    split2(-d0 * (q2.x * i0), -d1 * (q2.y * i1), hi[i], lo[i]);
-                }
-                sw_store_row<C, 16>(stage + Ly::oQ, row, col0 + cb, hi);
-                sw_store_row<C, 16>(stage + Ly::oV, row, col0 + cb, lo);
-                if (live) {
-                    st_global_32b(dst + cb, reinterpret_cast<const uint32_t(&)[8]>(d[0]));
-                    st_global_32b(dst + cb + 16, reinterpret_cast<const uint32_t(&)[8]>(d[8]));
-                }
+                for (int i = 0; i < 16; ++i) inv[cb + i] = v[i] *= inv[cb + i];
+                if (live) store_row16(dst + cb, v);
             }
-            write_tri<true>(tm_lane, row, wg);
+            if (!(ok = wait_bar_warp(cx, bH, ph, 107))) break;    // the totals have read W
+            RACE_TRACE(wg, c, 4);
+#pragma unroll
+            for (int p = 0; p < HC / 8; ++p) {
+                const uint32_t off = sw_piece<C>(row, col0 + 8 * p);
+                const uint4 h4 = *reinterpret_cast<const uint4*>(stage + Ly::oQ + off);
+                const uint4 l4 = *reinterpret_cast<const uint4*>(stage + Ly::oV + off);
+                const uint32_t hh[4] = {h4.x, h4.y, h4.z, h4.w}, ll[4] = {l4.x, l4.y, l4.z, l4.w};
+                uint32_t hi[4], lo[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 wh = unpack2(hh[i]), wl = unpack2(ll[i]);
+                    split2t(-inv[8 * p + 2 * i] * (wh.x + wl.x), -inv[8 * p + 2 * i + 1] * (wh.y + wl.y), hi[i], lo[i]);
+                }
+                *reinterpret_cast<uint4*>(stage + Ly::oQ + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                *reinterpret_cast<uint4*>(stage + Ly::oV + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
             fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bXg));
+            tc_fence_before();
+            arrive_warp(cx, bXg);
+            RACE_TRACE(wg, c, 5);
+        }
+    } else if (warp < kStateWarp) {
+        regs_dec<kRegsG>();
+        if (row < HC) tot[col0 + row] = 0.f;
+        asm volatile("bar.sync 6, 256;" ::: "memory");
+        write_tri<false>(tm_lane, row, wg);
+        arrive_warp(cx, bTri);
+        bool ok = true;
+        for (int c = 0; c < s.nch && ok; ++c) {
+            const uint32_t ph = (uint32_t)(c & 1);
+            const int64_t tok = s.t_begin + (int64_t)c * C + row;
+            const bool live = tok < s.t_end;
+            // ---- causal mask of dO V^T --------------------------------------------------------------------
+            if (!(ok = wait_bar_warp(cx, bG, ph, 105))) break;
+            RACE_TRACE(3, c, 0);
+            tc_fence_after();
+            mask_product<false>(tm_lane, row, wg);
+            arrive_warp(cx, bGm);
+            RACE_TRACE(3, c, 1);
+            if (!(ok = wait_bar_warp(cx, bX, ph, 106))) break;
+            tc_fence_after();
+            write_tri<true>(tm_lane, row, wg);
+            arrive_warp(cx, bXg);
             // ---- suffix sums of g inside the chunk ------------------------------------------------------------
             if (!(ok = wait_bar_warp(cx, bEnd, ph, 107))) break;
+            RACE_TRACE(3, c, 2);
             tc_fence_after();
+            write_tri<false>(tm_lane, row, wg);
             float* gdst = a.gs + (s.n * a.T + tok) * a.S + s.g0 + col0;
 #pragma unroll
-            for (int cb = 0; cb < HC; cb += 32) {
-                float v[32];
-                tmem_ld_rows32(tm_lane + tX + col0 + cb, v);
-                if (live) {
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8)
-                        st_global_32b(gdst + cb + i, reinterpret_cast<const uint32_t(&)[8]>(v[i]));
-                }
+            for (int cb = 0; cb < HC; cb += 16) {
+                float v[16];
+                tmem_ld_rows16(tm_lane + tX + col0 + cb, v);
+                if (live) store_row16(gdst + cb, v);
                 if (row == 0) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
+                    for (int i = 0; i < 16; i += 4) {
                         float4* t4 = reinterpret_cast<float4*>(tot + col0 + cb + i);
                         const float4 x = *t4;
                         *t4 = make_float4(x.x + v[i], x.y + v[i + 1], x.z + v[i + 2], x.w + v[i + 3]);
                     }
                 }
             }
-            write_tri<false>(tm_lane, row, wg);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bTri));
+            tc_fence_before();
+            arrive_warp(cx, bTri);
+            RACE_TRACE(3, c, 3);
         }
-    } else if (warp < 12) {
-        regs_dec<96>();
-        load_state<SB, D, Ly>(s, a, warp & 3, lane);
-        carry_state<SB, D, Ly>(s, warp & 3, lane);
-    } else if (warp == kTmaWarp) {
-        if (lane == 0) produce<Ly>(s, a, &map_do, &map_v, &map_k, &map_q, false);
-    } else if (warp == kMmaWarp) {
-        const uint32_t tm = __shfl_sync(0xffffffffu, s.tmem, 0), smb = __shfl_sync(0xffffffffu, cx.sm_u32, 0);
-        constexpr uint32_t iTS = idesc_mn(C, SB), iTT = idesc_mn(C, C), iSD = idesc_mn(SB, D);
-        if (elect_one()) {
-            bool ok = true;
-            for (int c = 0; c < s.nch && ok; ++c) {
-                const uint32_t ph = (uint32_t)(c & 1);
-                const int st = c % Ly::kStages;
-                const uint32_t base = smb + st * Ly::kStage;
-                const uint32_t sDO = base + Ly::oDO, sV = base + Ly::oV, sK = base + Ly::oK, sQ = base + Ly::oQ;
-                if (!(ok = wait_bar(cx, bTri, ph, 401))) break;
-                if (!(ok = wait_bar(cx, bFull + st, (uint32_t)((c / Ly::kStages) & 1), 402))) break;
-                tc_fence_after();
-                mma_sw_ta<true, 8, true, C>(tm + tX, tm + tG, sK, iTS);                      // A_loc = tril . pK
-                mma_commit(cx.bar(bA));
-                mma_sw<true, D / 16, false, C, false, C>(tm + tG, sDO, sV, iTT);             // G = dO . V^T (over tril)
-                mma_commit(cx.bar(bG));
-                if (!(ok = wait_bar(cx, bBt, ph, 403))) break;
-                tc_fence_after();
-                mma_sw<false, 8, true, C, true, C>(tm, sK, sV, iSD);                         // B += pK^T . V
-                mma_commit(cx.bar(bSt));
-                if (!(ok = wait_bar(cx, bW, ph, 404))) break;
-                tc_fence_after();
-                mma_sw<true, D / 16, false, C, false, SB>(tm + tX, sDO, smb + Ly::oB, iTS);  // X = dO . B^T
-                mma_sw<false, D / 16, false, C, false, SB>(tm + tX, sDO, smb + Ly::oB + Ly::kB, iTS);
-                mma_commit(cx.bar(bXb));
-                if (c == 0) mma_sw<true, 8, true, C, true, C>(tm + tTot, sQ, sDO, iSD);      // totals += W^T . dO
-                else mma_sw<false, 8, true, C, true, C>(tm + tTot, sQ, sDO, iSD);
-                mma_sw<false, 8, true, C, true, C>(tm + tTot, sV, sDO, iSD);
-                if (!(ok = wait_bar(cx, bGm, ph, 405))) break;
-                tc_fence_after();
-                mma_sw_ta<false, 8, true, C, true>(tm + tX, tm + tG, sK, iTS);               // X += tril(G) . pK
-                mma_sw_ta<false, 8, true, C, true>(tm + tX, tm + tG + 32, sK, iTS);
-                mma_commit(cx.bar(bX));
-                if (!(ok = wait_bar(cx, bXg, ph, 406))) break;
-                tc_fence_after();
-                mma_sw_ta<true, 8, true, C>(tm + tX, tm + tG, sQ, iTS);                      // GS = triu . g
-                mma_sw_ta<false, 8, true, C>(tm + tX, tm + tG, sV, iTS);
-                mma_commit(cx.bar(bEnd));
-                mma_commit(cx.bar(bEmpty + st));
+    } else if (warp < kTmaWarp) {
+        regs_dec<kRegsS>();
+        load_state<SB, D, Ly>(s, a, w, lane);
+        carry_state<SB, D, Ly>(s, w, lane);
+    } else {
+        regs_dec<kRegsM>();
+        if (warp == kTmaWarp && lane == 0) produce<Ly>(s, a, &map_do, &map_v, &map_k, &map_q, false);
+        if (warp == kMmaWarp) {
+            const uint32_t tm0 = __shfl_sync(0xffffffffu, s.tmem, 0), smb0 = __shfl_sync(0xffffffffu, cx.sm_u32, 0);
+            constexpr uint32_t iTS = idesc_mn(C, SB), iTT = idesc_mn(C, C), iSD = idesc_mn(SB, D);
+            if (elect_one()) {
+                bool ok = true;
+                for (int c = 0; c < s.nch && ok; ++c) {
+                    const uint32_t ph = (uint32_t)(c & 1);
+                    const int st = c % Ly::kStages;
+                    // opaque per chunk: the descriptors are one addition each; kept across chunks they would be spilled
+                    uint32_t tm = tm0, smb = smb0;
+                    asm volatile("" : "+r"(tm), "+r"(smb));
+                    const uint32_t base = smb + st * Ly::kStage;
+                    const uint32_t sDO = base + Ly::oDO, sV = base + Ly::oV, sK = base + Ly::oK, sQ = base + Ly::oQ;
+                    if (!(ok = wait_bar(cx, bTri, ph, 401))) break;
+                    if (!(ok = wait_bar(cx, bFull + st, (uint32_t)((c / Ly::kStages) & 1), 402))) break;
+                    tc_fence_after();
+                    mma_sw_ta<true, 8, true, C>(tm + tX, tm + tG, sK, iTS);                      // A_loc = tril . pK
+                    mma_commit(cx.bar(bA));
+                    mma_sw<true, D / 16, false, C, false, C>(tm + tG, sDO, sV, iTT);             // G = dO . V^T (over tril)
+                    mma_commit(cx.bar(bG));
+                    if (!(ok = wait_bar(cx, bBt, ph, 403))) break;
+                    tc_fence_after();
+                    mma_sw<false, 8, true, C, true, C>(tm, sK, sV, iSD);                         // B += pK^T . V
+                    mma_commit(cx.bar(bSt));
+                    if (!(ok = wait_bar(cx, bW, ph, 404))) break;
+                    tc_fence_after();
+                    mma_sw<true, D / 16, false, C, false, SB>(tm + tX, sDO, smb + Ly::oB, iTS);  // X = dO . B^T
+                    mma_sw<false, D / 16, false, C, false, SB>(tm + tX, sDO, smb + Ly::oB + Ly::kB, iTS);
+                    mma_commit(cx.bar(bXb));
+                    if (!(ok = wait_bar(cx, bGm, ph, 405))) break;
+                    tc_fence_after();
+                    mma_sw_ta<false, 8, true, C, true>(tm + tX, tm + tG, sK, iTS);               // X += tril(G) . pK
+                    mma_sw_ta<false, 8, true, C, true>(tm + tX, tm + tG + 16, sK, iTS);
+                    mma_commit(cx.bar(bX));
+                    if (c == 0) mma_sw<true, 8, true, C, true, C>(tm + tTot, sQ, sDO, iSD);      // totals += W^T . dO
+                    else mma_sw<false, 8, true, C, true, C>(tm + tTot, sQ, sDO, iSD);
+                    mma_sw<false, 8, true, C, true, C>(tm + tTot, sV, sDO, iSD);
+                    mma_commit(cx.bar(bH));
+                    if (!(ok = wait_bar(cx, bXg, ph, 406))) break;
+                    tc_fence_after();
+                    mma_sw_ta<true, 8, true, C>(tm + tX, tm + tG, sQ, iTS);                      // GS = triu . g
+                    mma_sw_ta<false, 8, true, C>(tm + tX, tm + tG, sV, iTS);
+                    mma_commit(cx.bar(bEnd));
+                    mma_commit(cx.bar(bEmpty + st));
+                }
+                mma_commit(cx.bar(bDrain));
+                const long long t0 = clock64();
+                while (!mbar_try_wait(cx.bar(bDrain), 0) && clock64() - t0 < cx.limit) {}
             }
-            mma_commit(cx.bar(bDrain));
-            const long long t0 = clock64();
-            while (!mbar_try_wait(cx.bar(bDrain), 0) && clock64() - t0 < cx.limit) {}
         }
     }
     tc_fence_before();
@@ -475,21 +529,17 @@ bwd_prefix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
     tc_fence_after();
     // totals of the tile
     float* slice = a.ws_out + (s.n * s.tiles + s.tile) * sf;
-    if (warp >= 8 && warp < 12) {
-        const int w = warp & 3;
+    if (warp < 4) {
         const StateRow<SB> r(w, lane);
         float* dst = slice + (int64_t)(s.g0 + r.row) * D;
 #pragma unroll
-        for (int cb = 0; cb < D; cb += 32) {
-            float v[32];
-            tmem_ld_rows32(((uint32_t)(32 * w) << 16) + s.tmem + tTot + cb, v);
-            if (r.live) {
-#pragma unroll
-                for (int i = 0; i < 32; i += 8) st_global_32b(dst + cb + i, reinterpret_cast<const uint32_t(&)[8]>(v[i]));
-            }
+        for (int cb = 0; cb < D; cb += 16) {
+            float v[16];
+            tmem_ld_rows16(tm_lane + tTot + cb, v);
+            if (r.live) store_row16(dst + cb, v);
         }
-    } else if (tid < SB) {
-        slice[(int64_t)a.S * D + s.g0 + tid] = tot[tid];
+    } else if (tid >= 256 && tid < 256 + SB) {
+        slice[(int64_t)a.S * D + s.g0 + tid - 256] = tot[tid - 256];
     }
     finish(s.tmem);
 }
@@ -506,22 +556,24 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
     const Ctx& cx = s.cx;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float* car = reinterpret_cast<float*>(cx.sm + Ly::oCar);
+    float* sac = reinterpret_cast<float*>(cx.sm + Ly::oTot);
     const int64_t sf = (int64_t)a.S * (D + 1);
+    const int wg = (warp >> 2) & 1, w = warp & 3, row = 32 * w + lane;
+    const uint32_t tm_lane = s.tmem + ((uint32_t)(32 * w) << 16);
+    const int col0 = HC * wg;
 
-    if (warp >= 12) regs_dec<72>();
     if (warp < 8) {
-        regs_inc<168>();
-        const int wg = warp >> 2, w = warp & 3, row = 32 * w + lane;
-        const uint32_t tm_lane = s.tmem + ((uint32_t)(32 * w) << 16);
-        const int col0 = HC * wg;
+        regs_inc<kRegsP>();
         const float* slice_a = a.ws + (s.n * s.tiles + s.tile) * sf + (int64_t)a.S * D + s.g0;
-        if (row < HC) car[col0 + row] = slice_a[col0 + row];
-        asm volatile("bar.sync 5, 256;" ::: "memory");
-        write_tri<false>(tm_lane, row, wg);
-        __syncwarp();
-        if (lane == 0) mbar_arrive(cx.bar(bTri));
         const int64_t nchunk = (a.T + C - 1) / C;
-        const bool shares = a.S > SB;
+        // running A before chunk cc, read a chunk ahead by the thread of column col0 + row
+        const float* ac = a.achunk + (s.n * nchunk + s.t_begin / C) * a.S + s.g0 + col0 + row;
+        if (row < HC) {
+            car[col0 + row] = slice_a[col0 + row];
+            sac[col0 + row] = ac[(int64_t)(s.nch - 1) * a.S];
+        }
+        asm volatile("bar.sync 5, 256;" ::: "memory");
+        arrive_warp(cx, bPf);
         bool ok = true;
         for (int c = 0; c < s.nch && ok; ++c) {
             const uint32_t ph = (uint32_t)(c & 1);
@@ -530,23 +582,25 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
             const int64_t tok = s.t_begin + (int64_t)cc * C + row;
             const bool live = tok < s.t_end;
             // ---- W limbs over pQ and in a slot of its own ----------------------------------------------------
-            if (!(ok = wait_bar_warp(cx, bTri, ph, 101))) break;   // every worker has finished the chunk before
-            const float* ac = a.achunk + (s.n * nchunk + s.t_begin / C + cc) * a.S + s.g0 + col0;
+            if (!(ok = wait_bar_warp(cx, bPf, ph, 101))) break;   // the group has finished the chunk before
+            const float next_a = (row < HC && cc > 0) ? ac[(int64_t)(cc - 1) * a.S] : 0.f;
             if (!(ok = wait_bar_warp(cx, bFullQ + st, (uint32_t)((c / Ly::kStages) & 1), 102))) break;
+            RACE_TRACE(wg, c, 0);
             if (!(ok = wait_bar_warp(cx, bA, ph, 103))) break;
+            RACE_TRACE(wg, c, 1);
             tc_fence_after();
 #pragma unroll
-            for (int cb = 0; cb < HC; cb += 32) {
-                float v[32];
-                tmem_ld_rows32(tm_lane + tP + col0 + cb, v);
+            for (int cb = 0; cb < HC; cb += 16) {
+                float v[16];
+                tmem_ld_rows16(tm_lane + tP + col0 + cb, v);
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
-                    const float4 c4 = __ldg(reinterpret_cast<const float4*>(ac + cb + i));
+                for (int i = 0; i < 16; i += 4) {
+                    const float4 c4 = *reinterpret_cast<const float4*>(sac + col0 + cb + i);
                     v[i] = __fdividef(1.f, v[i] + c4.x + a.eps); v[i + 1] = __fdividef(1.f, v[i + 1] + c4.y + a.eps);
                     v[i + 2] = __fdividef(1.f, v[i + 2] + c4.z + a.eps); v[i + 3] = __fdividef(1.f, v[i + 3] + c4.w + a.eps);
                 }
 #pragma unroll
-                for (int p = 0; p < 4; ++p) {
+                for (int p = 0; p < 2; ++p) {
                     const uint32_t off = sw_piece<C>(row, col0 + cb + 8 * p);
                     const uint4 q4 = *reinterpret_cast<const uint4*>(stage + Ly::oQ + off);
                     const uint32_t qq[4] = {q4.x, q4.y, q4.z, q4.w};
@@ -554,7 +608,7 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const float2 q2 = unpack2(qq[i]);
-                        split2(q2.x * v[8 * p + 2 * i], q2.y * v[8 * p + 2 * i + 1], hi[i], lo[i]);
+                        split2t(q2.x * v[8 * p + 2 * i], q2.y * v[8 * p + 2 * i + 1], hi[i], lo[i]);
                     }
                     *reinterpret_cast<uint4*>(stage + Ly::oQ + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
                     *reinterpret_cast<uint4*>(cx.sm + Ly::oWlo + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -562,129 +616,145 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
             }
             fence_proxy_async();
             tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bW));
-            // ---- mask of V dO^T, then of pK W^T -------------------------------------------------------------
-            if (!(ok = wait_bar_warp(cx, bG, ph, 105))) break;
-            tc_fence_after();
-            mask_product<true>(tm_lane, row, wg);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bGm));
-            // sums of g of this chunk, requested while the products run
-            float gsv[HC];
+            arrive_warp(cx, bW);
+            RACE_TRACE(wg, c, 2);
+            // ---- dPK = P + sums of g (requested while the products run) -------------------------------------------
             const float* gsrc = a.gs + (s.n * a.T + tok) * a.S + s.g0 + col0;
+            float gsv[HC];
 #pragma unroll
             for (int i = 0; i < HC; i += 4) {
                 const float4 x = live ? __ldcs(reinterpret_cast<const float4*>(gsrc + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 gsv[i] = x.x; gsv[i + 1] = x.y; gsv[i + 2] = x.z; gsv[i + 3] = x.w;
             }
             if (!(ok = wait_bar_warp(cx, bX, ph, 106))) break;
+            RACE_TRACE(wg, c, 3);
             tc_fence_after();
-            mask_product<true>(tm_lane, row, wg);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bXg));
-            // ---- dPK = P + sums of g ------------------------------------------------------------------------------
             __nv_bfloat16* dst = a.dp + (s.n * a.T + tok) * a.S + s.g0 + col0;
 #pragma unroll
-            for (int cb = 0; cb < HC; cb += 32) {
-                float v[32];
-                tmem_ld_rows32(tm_lane + tP + col0 + cb, v);
+            for (int cb = 0; cb < HC; cb += 16) {
+                float v[16];
+                tmem_ld_rows16(tm_lane + tP + col0 + cb, v);
 #pragma unroll
-                for (int i = 0; i < 32; i += 4) {
+                for (int i = 0; i < 16; i += 4) {
                     const float4 c4 = *reinterpret_cast<const float4*>(car + (c & 1) * SB + col0 + cb + i);
                     const float4 g4 = make_float4(gsv[cb + i] + c4.x, gsv[cb + i + 1] + c4.y, gsv[cb + i + 2] + c4.z,
                                                   gsv[cb + i + 3] + c4.w);
                     if (row == 0) *reinterpret_cast<float4*>(car + ((c + 1) & 1) * SB + col0 + cb + i) = g4;
                     v[i] += g4.x; v[i + 1] += g4.y; v[i + 2] += g4.z; v[i + 3] += g4.w;
                 }
-                uint32_t d[16];
-#pragma unroll
-                for (int i = 0; i < 16; ++i) d[i] = pack2(v[2 * i], v[2 * i + 1]);
-                if (live) {
-                    st_global_32b(dst + cb, reinterpret_cast<const uint32_t(&)[8]>(d[0]));
-                    st_global_32b(dst + cb + 16, reinterpret_cast<const uint32_t(&)[8]>(d[8]));
-                }
+                if (live) store_row16(dst + cb, v);
             }
+            if (row < HC) sac[col0 + row] = next_a;   // every warp has formed its W: the products are done
+            tc_fence_before();
+            arrive_warp(cx, bPf);
+            RACE_TRACE(wg, c, 4);
+        }
+    } else if (warp < kStateWarp) {
+        regs_dec<kRegsG>();
+        write_tri<false>(tm_lane, row, wg);
+        arrive_warp(cx, bTri);
+        arrive_warp(cx, bVf);
+        const bool shares = a.S > SB;
+        bool ok = true;
+        for (int c = 0; c < s.nch && ok; ++c) {
+            const uint32_t ph = (uint32_t)(c & 1);
+            const int64_t tok = s.t_begin + (int64_t)(s.nch - 1 - c) * C + row;
+            const bool live = tok < s.t_end;
+            // ---- masks of V dO^T and of pK W^T ---------------------------------------------------------------
+            if (!(ok = wait_bar_warp(cx, bG, ph, 105))) break;
+            RACE_TRACE(3, c, 0);
+            tc_fence_after();
+            mask_product<true>(tm_lane, row, wg);
+            arrive_warp(cx, bGm);
+            RACE_TRACE(3, c, 1);
+            if (!(ok = wait_bar_warp(cx, bH, ph, 108))) break;
+            RACE_TRACE(3, c, 2);
+            tc_fence_after();
+            mask_product<true>(tm_lane, row, wg);
+            arrive_warp(cx, bHm);
+            RACE_TRACE(3, c, 3);
             // ---- dV ---------------------------------------------------------------------------------------------------
             if (!(ok = wait_bar_warp(cx, bEnd, ph, 107))) break;
+            RACE_TRACE(3, c, 4);
             tc_fence_after();
-#pragma unroll
-            for (int cb = 0; cb < HD; cb += 32) {
-                float v[32];
-                tmem_ld_rows32(tm_lane + tV + HD * wg + cb, v);
-                if (!live) continue;
-                if (shares) {
-                    float* o = (float*)a.dv + (((int64_t)s.block * gridDim.y + s.n) * a.T + tok) * D + HD * wg + cb;
-#pragma unroll
-                    for (int i = 0; i < 32; i += 8) st_global_32b(o + i, reinterpret_cast<const uint32_t(&)[8]>(v[i]));
-                } else {
-                    __nv_bfloat16* o = (__nv_bfloat16*)a.dv +
-                                       (((s.n / a.heads) * a.T + tok) * a.heads + s.n % a.heads) * D + HD * wg + cb;
-                    uint32_t d[16];
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) d[i] = pack2(v[2 * i], v[2 * i + 1]);
-                    st_global_32b(o, reinterpret_cast<const uint32_t(&)[8]>(d[0]));
-                    st_global_32b(o + 16, reinterpret_cast<const uint32_t(&)[8]>(d[8]));
-                }
-            }
             write_tri<false>(tm_lane, row, wg);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cx.bar(bTri));
-        }
-    } else if (warp < 12) {
-        regs_dec<96>();
-        load_state<SB, D, Ly>(s, a, warp & 3, lane);
-        carry_state<SB, D, Ly>(s, warp & 3, lane);
-    } else if (warp == kTmaWarp) {
-        if (lane == 0) produce<Ly>(s, a, &map_do, &map_v, &map_k, &map_q, true);
-    } else if (warp == kMmaWarp) {
-        const uint32_t tm = __shfl_sync(0xffffffffu, s.tmem, 0), smb = __shfl_sync(0xffffffffu, cx.sm_u32, 0);
-        constexpr uint32_t iTS = idesc_mn(C, SB), iTT = idesc_mn(C, C), iTD = idesc_mn(C, D), iSD = idesc_mn(SB, D);
-        const uint32_t sBh = smb + Ly::oB, sBl = sBh + Ly::kB, sWl = smb + Ly::oWlo;
-        if (elect_one()) {
-            bool ok = true;
-            for (int c = 0; c < s.nch && ok; ++c) {
-                const uint32_t ph = (uint32_t)(c & 1);
-                const int st = c % Ly::kStages;
-                const uint32_t base = smb + st * Ly::kStage;
-                const uint32_t sDO = base + Ly::oDO, sV = base + Ly::oV, sK = base + Ly::oK, sWh = base + Ly::oQ;
-                if (!(ok = wait_bar(cx, bTri, ph, 401))) break;
-                if (!(ok = wait_bar(cx, bFull + st, (uint32_t)((c / Ly::kStages) & 1), 402))) break;
-                tc_fence_after();
-                mma_sw_ta<true, 8, true, C>(tm + tP, tm + tG, sK, iTS);                  // A_loc = tril . pK
-                mma_commit(cx.bar(bA));
-                mma_sw<true, D / 16, false, C, false, C>(tm + tG, sV, sDO, iTT);         // V . dO^T (over tril)
-                mma_commit(cx.bar(bG));
-                if (!(ok = wait_bar(cx, bBt, ph, 403))) break;
-                tc_fence_after();
-                mma_sw<true, SB / 16, false, C, true, SB>(tm + tV, sK, sBh, iTD);        // dV = pK . SB
-                mma_sw<false, SB / 16, false, C, true, SB>(tm + tV, sK, sBl, iTD);
-                if (!(ok = wait_bar(cx, bW, ph, 404))) break;
-                tc_fence_after();
-                mma_sw<true, D / 16, false, C, false, SB>(tm + tP, sV, sBh, iTS);        // P = V . SB^T
-                mma_sw<false, D / 16, false, C, false, SB>(tm + tP, sV, sBl, iTS);
-                mma_commit(cx.bar(bXb));
-                mma_sw<false, 8, true, C, true, C>(tm, sWh, sDO, iSD);                   // SB += W^T . dO
-                mma_sw<false, 8, true, C, true, C>(tm, sWl, sDO, iSD);
-                mma_commit(cx.bar(bSt));
-                if (!(ok = wait_bar(cx, bGm, ph, 405))) break;
-                tc_fence_after();
-                mma_sw_ta<false, 8, true, C, true>(tm + tP, tm + tG, sWh, iTS);          // P += triu(V dO^T) . W
-                mma_sw_ta<false, 8, true, C, true>(tm + tP, tm + tG, sWl, iTS);
-                mma_sw_ta<false, 8, true, C, true>(tm + tP, tm + tG + 32, sWh, iTS);
-                mma_sw<true, SB / 16, false, C, false, C>(tm + tG, sK, sWh, iTT);        // pK . W^T
-                mma_sw<false, SB / 16, false, C, false, C>(tm + tG, sK, sWl, iTT);
-                mma_commit(cx.bar(bX));
-                if (!(ok = wait_bar(cx, bXg, ph, 406))) break;
-                tc_fence_after();
-                mma_sw_ta<false, 8, true, C, true>(tm + tV, tm + tG, sDO, iTD);          // dV += triu(pK W^T) . dO
-                mma_sw_ta<false, 8, true, C, true>(tm + tV, tm + tG + 32, sDO, iTD);
-                mma_commit(cx.bar(bEnd));
-                mma_commit(cx.bar(bEmpty + st));
+            arrive_warp(cx, bTri);
+            const int64_t srow = ((int64_t)s.block * gridDim.y + s.n) * a.T + tok;
+            const int64_t orow = ((s.n / a.heads) * a.T + tok) * a.heads + s.n % a.heads;
+#pragma unroll
+            for (int cb = 0; cb < HD; cb += 16) {
+                float v[16];
+                tmem_ld_rows16(tm_lane + tV + HD * wg + cb, v);
+                if (!live) continue;
+                if (shares) store_row16((float*)a.dv + srow * D + HD * wg + cb, v);
+                else store_row16((__nv_bfloat16*)a.dv + orow * D + HD * wg + cb, v);
             }
-            mma_commit(cx.bar(bDrain));
-            const long long t0 = clock64();
-            while (!mbar_try_wait(cx.bar(bDrain), 0) && clock64() - t0 < cx.limit) {}
+            tc_fence_before();
+            arrive_warp(cx, bVf);
+            RACE_TRACE(3, c, 5);
+        }
+    } else if (warp < kTmaWarp) {
+        regs_dec<kRegsS>();
+        load_state<SB, D, Ly>(s, a, w, lane);
+        carry_state<SB, D, Ly>(s, w, lane);
+    } else {
+        regs_dec<kRegsM>();
+        if (warp == kTmaWarp && lane == 0) produce<Ly>(s, a, &map_do, &map_v, &map_k, &map_q, true);
+        if (warp == kMmaWarp) {
+            const uint32_t tm0 = __shfl_sync(0xffffffffu, s.tmem, 0), smb0 = __shfl_sync(0xffffffffu, cx.sm_u32, 0);
+            constexpr uint32_t iTS = idesc_mn(C, SB), iTT = idesc_mn(C, C), iTD = idesc_mn(C, D), iSD = idesc_mn(SB, D);
+            if (elect_one()) {
+                bool ok = true;
+                for (int c = 0; c < s.nch && ok; ++c) {
+                    const uint32_t ph = (uint32_t)(c & 1);
+                    const int st = c % Ly::kStages;
+                    // opaque per chunk: the descriptors are one addition each; kept across chunks they would be spilled
+                    uint32_t tm = tm0, smb = smb0;
+                    asm volatile("" : "+r"(tm), "+r"(smb));
+                    const uint32_t base = smb + st * Ly::kStage;
+                    const uint32_t sDO = base + Ly::oDO, sV = base + Ly::oV, sK = base + Ly::oK, sWh = base + Ly::oQ;
+                    const uint32_t sBh = smb + Ly::oB, sBl = sBh + Ly::kB, sWl = smb + Ly::oWlo;
+                    if (!(ok = wait_bar(cx, bTri, ph, 401))) break;
+                    if (!(ok = wait_bar(cx, bPf, ph, 407))) break;
+                    if (!(ok = wait_bar(cx, bFull + st, (uint32_t)((c / Ly::kStages) & 1), 402))) break;
+                    tc_fence_after();
+                    mma_sw_ta<true, 8, true, C>(tm + tP, tm + tG, sK, iTS);                  // A_loc = tril . pK
+                    mma_commit(cx.bar(bA));
+                    mma_sw<true, D / 16, false, C, false, C>(tm + tG, sV, sDO, iTT);         // V . dO^T (over tril)
+                    mma_commit(cx.bar(bG));
+                    if (!(ok = wait_bar(cx, bBt, ph, 403))) break;
+                    if (!(ok = wait_bar(cx, bVf, ph, 408))) break;
+                    tc_fence_after();
+                    mma_sw<true, SB / 16, false, C, true, SB>(tm + tV, sK, sBh, iTD);        // dV = pK . SB
+                    mma_sw<false, SB / 16, false, C, true, SB>(tm + tV, sK, sBl, iTD);
+                    if (!(ok = wait_bar(cx, bW, ph, 404))) break;
+                    tc_fence_after();
+                    mma_sw<true, D / 16, false, C, false, SB>(tm + tP, sV, sBh, iTS);        // P = V . SB^T
+                    mma_sw<false, D / 16, false, C, false, SB>(tm + tP, sV, sBl, iTS);
+                    mma_commit(cx.bar(bXb));
+                    if (!(ok = wait_bar(cx, bGm, ph, 405))) break;
+                    tc_fence_after();
+                    mma_sw_ta<false, 8, true, C, true>(tm + tP, tm + tG, sWh, iTS);          // P += triu(V dO^T) . W
+                    mma_sw_ta<false, 8, true, C, true>(tm + tP, tm + tG, sWl, iTS);
+                    mma_sw_ta<false, 8, true, C, true>(tm + tP, tm + tG + 16, sWh, iTS);
+                    mma_commit(cx.bar(bX));
+                    mma_sw<true, SB / 16, false, C, false, C>(tm + tG, sK, sWh, iTT);        // pK . W^T
+                    mma_sw<false, SB / 16, false, C, false, C>(tm + tG, sK, sWl, iTT);
+                    mma_commit(cx.bar(bH));
+                    mma_sw<false, 8, true, C, true, C>(tm, sWh, sDO, iSD);                   // SB += W^T . dO
+                    mma_sw<false, 8, true, C, true, C>(tm, sWl, sDO, iSD);
+                    mma_commit(cx.bar(bSt));
+                    if (!(ok = wait_bar(cx, bHm, ph, 406))) break;
+                    tc_fence_after();
+                    mma_sw_ta<false, 8, true, C, true>(tm + tV, tm + tG, sDO, iTD);          // dV += triu(pK W^T) . dO
+                    mma_sw_ta<false, 8, true, C, true>(tm + tV, tm + tG + 16, sDO, iTD);
+                    mma_commit(cx.bar(bEnd));
+                    mma_commit(cx.bar(bEmpty + st));
+                }
+                mma_commit(cx.bar(bDrain));
+                const long long t0 = clock64();
+                while (!mbar_try_wait(cx.bar(bDrain), 0) && clock64() - t0 < cx.limit) {}
+            }
         }
     }
     finish(s.tmem);
@@ -694,6 +764,8 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
 __global__ void __launch_bounds__(256)
 bwd_dv_sum(const float* __restrict__ shares, __nv_bfloat16* __restrict__ dv, int64_t rows, int64_t T, int heads, int D,
            int blocks) {
+    chain_release();
+    chain_wait();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int per = D / 8;
     if (i >= rows * per) return;
@@ -784,20 +856,17 @@ cudaError_t launch(const void* pq, const void* pk, const void* v, const void* do
     a.eps = dm.eps;
     a.status = status;
     const dim3 grid((unsigned)(tiles * blocks), (unsigned)dm.N);
-    k1<<<grid, kThreads, smem1, stream>>>(mdo, mv, mk, mq, a);
-    err = cudaGetLastError();
+    err = launch_chain(chain_launches(dm), k1, grid, kThreads, smem1, stream, mdo, mv, mk, mq, a);
     if (err == cudaSuccess) err = causal_scan_tiles(wsf, d_state, d_carry, dm, tile, stream, true, /*reverse=*/true);
     if (err != cudaSuccess) return err;
     a.ws = wsf;
     a.dp = (__nv_bfloat16*)dpk;
     a.dv = blocks > 1 ? (void*)(base + l.shares) : dv;
-    k2<<<grid, kThreads, smem2, stream>>>(mdo, mv, mk, mq, a);
-    err = cudaGetLastError();
+    err = launch_chain(chain_launches(dm), k2, grid, kThreads, smem2, stream, mdo, mv, mk, mq, a);
     if (err != cudaSuccess || blocks == 1) return err;
     const int64_t rows = dm.N * dm.T;
-    bwd_dv_sum<<<(unsigned)((rows * (D / 8) + 255) / 256), 256, 0, stream>>>((const float*)(base + l.shares),
-                                                                             (__nv_bfloat16*)dv, rows, dm.T, dm.H, D, blocks);
-    return cudaGetLastError();
+    return launch_chain(chain_launches(dm), bwd_dv_sum, (unsigned)((rows * (D / 8) + 255) / 256), 256, 0, stream, (const float*)(base + l.shares),
+                        (__nv_bfloat16*)dv, rows, dm.T, dm.H, D, blocks);
 }
 
 }  // namespace

@@ -40,6 +40,8 @@ inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // sums[n][b][c] = sum over the tokens of block b of x[n][t][c]
 __global__ void __launch_bounds__(kPwThreads)
 bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, int64_t T, int64_t nblk, int64_t total_blocks) {
+    chain_release();
+    chain_wait();
     const int64_t gb = (int64_t)blockIdx.x * (kPwThreads / 64) + (threadIdx.x >> 6);
     if (gb >= total_blocks) return;
     const int c = threadIdx.x & 63;
@@ -64,6 +66,8 @@ bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, int64_t T,
 __global__ void __launch_bounds__(64)
 bwd_block_scan(float* __restrict__ sums, const float* __restrict__ carry_state, float* __restrict__ total_state,
                int64_t nblk, int reverse) {
+    chain_release();
+    chain_wait();
     const int c = threadIdx.x;
     const int64_t n = blockIdx.x;
     float run = carry_state ? carry_state[n * kSF + S * D + c] : 0.f;
@@ -93,6 +97,8 @@ bwd_block_scan(float* __restrict__ sums, const float* __restrict__ carry_state, 
 __global__ void __launch_bounds__(kPwThreads)
 bwd_block_chunk_sums(const float* __restrict__ x, float* __restrict__ sums, float* __restrict__ chunk, int64_t T,
                      int64_t nblk, int64_t nchunk, int64_t total_blocks) {
+    chain_release();
+    chain_wait();
     const int64_t gb = (int64_t)blockIdx.x * (kPwThreads / 64) + (threadIdx.x >> 6);
     if (gb >= total_blocks) return;
     const int c = threadIdx.x & 63;
@@ -125,6 +131,8 @@ bwd_block_chunk_sums(const float* __restrict__ x, float* __restrict__ sums, floa
 __global__ void __launch_bounds__(kPwThreads)
 bwd_pointwise_rev(const float* __restrict__ g, float* __restrict__ pdpk, const float* __restrict__ gsuffix, int64_t T,
                   int64_t nblk, int64_t total_blocks) {
+    chain_release();
+    chain_wait();
     const int64_t gb = (int64_t)blockIdx.x * (kPwThreads / 64) + (threadIdx.x >> 6);
     if (gb >= total_blocks) return;
     const int c = threadIdx.x & 63;
@@ -155,6 +163,8 @@ bwd_pointwise_rev(const float* __restrict__ g, float* __restrict__ pdpk, const f
 __global__ void __launch_bounds__(256)
 bwd_transpose_state(const float* __restrict__ src, float* __restrict__ dst) {
     __shared__ float tile[64][65];
+    chain_release();
+    chain_wait();
     const int64_t n = blockIdx.x;
     const float* s = src + n * kSF;
     float* d = dst + n * kSF;
@@ -229,14 +239,11 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     // 1. sums of pK: per block (then scanned, carry included) and inside the block up to every chunk start
     float* achunk = (float*)(base + l.achunk);
     const int64_t nchunk = (dm.T + 63) / 64;
-    bwd_block_chunk_sums<<<pw_grid, kPwThreads, 0, stream>>>((const float*)pk, asum, achunk, dm.T, nblk, nchunk,
-                                                             total_blocks);
-    RACE_CK(cudaGetLastError());
-    bwd_block_scan<<<(unsigned)dm.N, 64, 0, stream>>>(asum, carry_in, nullptr, nblk, 0);
-    RACE_CK(cudaGetLastError());
+    RACE_CK(launch_chain(chain_launches(dm), bwd_block_chunk_sums, pw_grid, kPwThreads, 0, stream, (const float*)pk, asum, achunk, dm.T, nblk,
+                         nchunk, total_blocks));
+    RACE_CK(launch_chain(chain_launches(dm), bwd_block_scan, (unsigned)dm.N, 64, 0, stream, asum, carry_in, nullptr, nblk, 0));
     // 2. X = raw(dO, V, pK), the state of the pass is B^T; its epilogue writes dPQ, W and g.  Then the block sums of g.
-    if (carry_in) bwd_transpose_state<<<(unsigned)dm.N, 256, 0, stream>>>(carry_in, st_t);
-    RACE_CK(cudaGetLastError());
+    if (carry_in) RACE_CK(launch_chain(chain_launches(dm), bwd_transpose_state, (unsigned)dm.N, 256, 0, stream, carry_in, st_t));
     BwdX bx;
     bx.pq_true = (const float*)pq;
     bx.ablock = asum;
@@ -249,28 +256,24 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     bx.eps = dm.eps;
     RACE_CK(causal_raw_tensor(dout, v, pk, dpq, carry_in ? st_t : nullptr, nullptr, ws_tiles, dm, tile_tokens,
                               /*reverse=*/false, stream, status, kPhaseAll, &bx, dm.H, dm.H, 1, 1));
-    bwd_block_sums<<<pw_grid, kPwThreads, 0, stream>>>(g, gsum, dm.T, nblk, total_blocks);
-    RACE_CK(cudaGetLastError());
+    RACE_CK(launch_chain(chain_launches(dm), bwd_block_sums, pw_grid, kPwThreads, 0, stream, (const float*)g, gsum, dm.T, nblk, total_blocks));
     // 3. dV = raw_reverse(pK, W, dO); state sum W^T dO: carry = gradient of the final B, total = gradient of carry_in's B.
     //    Pass 4 below has the roles of W and dO swapped, so its tile totals are the transposes of this pass's:
     //    the totals launch runs once and the second tile buffer gets the transposed states.
     RACE_CK(causal_raw_tensor(nullptr, w, dout, nullptr, nullptr, nullptr, ws_tiles, dm, tile_tokens, true, stream, status,
                               kPhaseTotals, nullptr, 1, 1, dm.H, 1));
-    bwd_transpose_state<<<(unsigned)(dm.N * tiles), 256, 0, stream>>>(ws_tiles, ws_tiles2);
-    RACE_CK(cudaGetLastError());
+    RACE_CK(launch_chain(chain_launches(dm), bwd_transpose_state, (unsigned)(dm.N * tiles), 256, 0, stream, (const float*)ws_tiles, ws_tiles2));
     RACE_CK(causal_raw_tensor(pk, w, dout, dv, d_state, d_carry ? d_carry : st_dv, ws_tiles, dm, tile_tokens,
                               /*reverse=*/true, stream, status, kPhaseOutput, nullptr, 1, 1, dm.H, dm.H));
     // 4. P = raw_reverse(V, dO, W) into the dPK buffer; state = the transpose of pass 3's
-    if (d_state) bwd_transpose_state<<<(unsigned)dm.N, 256, 0, stream>>>(d_state, st_t);
-    RACE_CK(cudaGetLastError());
+    if (d_state) RACE_CK(launch_chain(chain_launches(dm), bwd_transpose_state, (unsigned)dm.N, 256, 0, stream, d_state, st_t));
     RACE_CK(causal_raw_tensor(v, dout, w, dpk, d_state ? st_t : nullptr, nullptr, ws_tiles2, dm, tile_tokens,
                               /*reverse=*/true, stream, status, kPhaseOutput, nullptr, dm.H, dm.H, 1, 1));
     // 5. dPK = P + suffix sums of g (carry: gradient of the final A; total: gradient of carry_in's A, which
     //    overwrites the A part that pass 3 left in d_carry)
-    bwd_block_scan<<<(unsigned)dm.N, 64, 0, stream>>>(gsum, d_state, d_carry, nblk, 1);
-    RACE_CK(cudaGetLastError());
-    bwd_pointwise_rev<<<pw_grid, kPwThreads, 0, stream>>>(g, (float*)dpk, gsum, dm.T, nblk, total_blocks);
-    return cudaGetLastError();
+    RACE_CK(launch_chain(chain_launches(dm), bwd_block_scan, (unsigned)dm.N, 64, 0, stream, gsum, d_state, d_carry, nblk, 1));
+    return launch_chain(chain_launches(dm), bwd_pointwise_rev, pw_grid, kPwThreads, 0, stream, (const float*)g, (float*)dpk, (const float*)gsum,
+                        dm.T, nblk, total_blocks);
 }
 
 }  // namespace race

@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(128)
 tile_scan(float* __restrict__ ws, const float* __restrict__ carry_in, float* __restrict__ state_out,
           int64_t tiles, int state_floats, int write_prefix, int reverse) {
     constexpr int kInFlight = 32;
+    chain_release();
+    chain_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= state_floats) return;
     const int64_t n = blockIdx.y;
@@ -415,8 +417,7 @@ cudaError_t launch_simt(const Tin* pq, const Tin* pk, const Tin* v, Tin* out, co
     }
 
     dim3 sgrid((unsigned)((sf + 127) / 128), (unsigned)dm.N);
-    tile_scan<<<sgrid, 128, 0, stream>>>(ws, carry_in, state_out, tiles, sf, totals_only ? 0 : 1, 0);
-    err = cudaGetLastError();
+    err = launch_chain(chain_launches(dm), tile_scan, sgrid, 128, 0, stream, ws, carry_in, state_out, tiles, sf, totals_only ? 0 : 1, 0);
     if (err != cudaSuccess || totals_only || skip_output) return err;
 
     const size_t smem3 = (size_t)(groups > 1 ? Ly::floats_cluster : Ly::floats_single) * sizeof(float);
@@ -467,8 +468,8 @@ cudaError_t causal_scan_tiles(float* ws, const float* carry_in, float* state_out
     if (tiles == 1 && !carry_in && !write_prefix && state_out)   // one tile per stream: its totals are the state
         return cudaMemcpyAsync(state_out, ws, (size_t)dm.N * sf * sizeof(float), cudaMemcpyDeviceToDevice, stream);
     dim3 sgrid((unsigned)((sf + 127) / 128), (unsigned)dm.N);
-    tile_scan<<<sgrid, 128, 0, stream>>>(ws, carry_in, state_out, tiles, sf, write_prefix ? 1 : 0, reverse ? 1 : 0);
-    return cudaGetLastError();
+    return launch_chain(chain_launches(dm), tile_scan, sgrid, 128, 0, stream, ws, carry_in, state_out, tiles, sf, write_prefix ? 1 : 0,
+                        reverse ? 1 : 0);
 }
 
 int simt_groups(int S) { return S <= kGroupBuckets ? 1 : (S + kGroupBuckets - 1) / kGroupBuckets; }

@@ -772,11 +772,13 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
     // The worker groups write their own pK tile only where forming the probabilities makes that tile expensive: with
     // probabilities in, leaving it to the converter group measured 3 % faster.
     constexpr bool kWorkerK = kProj;
+    chain_release();
     if (tid == 0) {
         *cx.abort_flag = 0;
         out_phase_init_bars(cx, false, kWorkerK ? 8u : 4u);
     }
     uint32_t* ptab = reinterpret_cast<uint32_t*>(cx.sm + oPlaneTab);
+    // (ahead of chain_wait: the planes are never the result of a chained launch)
     if (kProj) build_plane_tab(planes, ptab, tid, kThreads);
     if (warp == kMmaWarp) tmem_alloc(cx.sm_u32 + oMisc, kTmemCols);
     fence_proxy_async();
@@ -784,6 +786,7 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
     out_phase<kMode, kReverse, kProj, kWorkerK>(cx, tmem, pq, &map_k, &map_v, out, slice, T, t_begin, t_end, n, eps,
                                                 hd, (tile == 0 && n == 0) ? withhold_chunk : -1, false, ptab, &bwdx);
     tc_fence_before();
@@ -1101,6 +1104,7 @@ tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     const int64_t t_begin = tile * tile_tokens;
     const int64_t t_end = min(T, t_begin + (int64_t)tile_tokens);
     float* slice = ws + (n * tiles + tile) * (int64_t)(S * (D + 1));
+    chain_release();
     if (tid == 0) {
         *cx.abort_flag = 0;
         totals_phase_init_bars<TL>(cx, false);
@@ -1112,6 +1116,7 @@ tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
     totals_phase<kProj, TL>(cx, tmem, &map_k, &map_v, slice, t_begin, t_end, n, hd, false, ptab);
     tc_fence_before();
     __syncthreads();
@@ -1397,11 +1402,12 @@ int tensor_single_pass_tile_tokens(const Dims& dm, int sm_count) {
 }
 
 int tensor_default_tile_tokens(const Dims& dm, int, int sm_count) {
-    // One CTA per SM (and per bucket group) at a time: the CTAs run in waves of sm_count, so the tile
+    // One CTA per SM at a time: the CTAs run in waves of sm_count, so the tile
     // length (a multiple of the chunk, at most 2048 tokens) is chosen to fill the last wave:
     // cost = waves x (tokens per tile + the set-up of a CTA, about one and a half chunks).  For long
     // sequences this stays at 2048; for shorter ones it avoids a mostly empty last wave.
-    const int64_t groups = dm.S > 64 ? dm.S / 64 : 1;
+    // CTAs of the output pass per (stream, tile): slices of the head dimension when there are several bucket groups
+    const int64_t groups = dm.S > 128 ? dm.D / 64 : dm.S > 64 ? dm.D / 32 : 1;
     const int64_t sms = sm_count > 0 ? sm_count : 148;
     int best = 2048;
     double best_cost = 1e300;
@@ -1543,9 +1549,8 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
     dim3 grid((unsigned)tiles, (unsigned)dm.N);
     // 1. tile totals (tensor cores)  2. exclusive scan over tiles  3. output pass
     if (phases & kPhaseTotals) {
-        totals_kern<<<grid, totals_threads, totals_smem, stream>>>(mk, mv, (float*)ws, dm.T, tile_tokens, hd, status,
-                                                                planes);
-        err = cudaGetLastError();
+        err = launch_chain(chain_launches(dm), totals_kern, grid, totals_threads, totals_smem, stream, mk, mv, (float*)ws, dm.T, tile_tokens, hd,
+                           status, planes);
         if (err != cudaSuccess) return err;
     }
     if (!(phases & kPhaseOutput)) {
@@ -1564,10 +1569,8 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
                                           : causal_out_tc<kModeBucket, false, false>);
     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (err != cudaSuccess) return err;
-    kern<<<grid, kThreads, kSmemBytes, stream>>>((const float*)pq, mk, mv, (float*)out, (const float*)ws, dm.T,
-                                                 tile_tokens, dm.eps, hd, status, wait_cycles, withhold_chunk, planes,
-                                                 bwdx ? *bwdx : BwdX{});
-    return cudaGetLastError();
+    return launch_chain(chain_launches(dm), kern, grid, kThreads, kSmemBytes, stream, (const float*)pq, mk, mv, (float*)out, (const float*)ws,
+                        dm.T, tile_tokens, dm.eps, hd, status, wait_cycles, withhold_chunk, planes, bwdx ? *bwdx : BwdX{});
 }
 
 #ifdef RACE_FUSED_PROF

@@ -117,6 +117,7 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
     cx.abort_flag = reinterpret_cast<volatile int*>(cx.sm + Ly::oMisc + 4);
     cx.status = status;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(cx.sm + Ly::oMisc);
+    chain_release();
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = (int)(blockIdx.x % (unsigned)G);          // bucket group = rank in the cluster
@@ -172,6 +173,7 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
     const uint32_t tmB = tmem;                                                   // [0, D)
     auto tmAG = [&](int wg) { return tmem + D + wg * (64 + D); };                // A_loc, then G
     auto tmO = [&](int wg) { return tmem + D + wg * (64 + D) + 64; };            // O
@@ -550,6 +552,7 @@ tile_totals_tc_bf16(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     cx.abort_flag = reinterpret_cast<volatile int*>(cx.sm + Ly::oMisc + 4);
     cx.status = status;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(cx.sm + Ly::oMisc);
+    chain_release();
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int GC = G / GP;                                   // CTAs per (stream, tile)
@@ -584,6 +587,7 @@ tile_totals_tc_bf16(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
 
     if (warp < 8) {
         const int wg = warp >> 2, wtid = tid & 127;
@@ -778,6 +782,7 @@ causal_out_wide_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_con
     cx.abort_flag = reinterpret_cast<volatile int*>(cx.sm + Ly::oMisc + 4);
     cx.status = status;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(cx.sm + Ly::oMisc);
+    chain_release();
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int NS = D / DS;                                   // slices of the head dimension
@@ -835,6 +840,7 @@ causal_out_wide_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_con
         }
         *reinterpret_cast<uint4*>(cx.sm + Ly::oTril + off_w<64>(t, jg * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+    chain_wait();
     for (int i = tid; i < G * 64; i += kWThreads)   // running A of every group: the carry-in
         reinterpret_cast<float*>(cx.sm + Ly::oAcar)[i] = slice[(int64_t)S * D + i];
     fence_proxy_async();
@@ -1249,6 +1255,7 @@ causal_out_wide4_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_co
     cx.abort_flag = reinterpret_cast<volatile int*>(cx.sm + Ly::oMisc + 4);
     cx.status = status;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(cx.sm + Ly::oMisc);
+    chain_release();
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int NS = D / DSX;                                  // slices of the head dimension
@@ -1308,6 +1315,7 @@ causal_out_wide4_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_co
         }
         *reinterpret_cast<uint4*>(cx.sm + Ly::oTril + off_w<64>(t, jg * 8)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
+    chain_wait();
     for (int i = tid; i < G * 64; i += Ly::kThreads)   // running A of every group: the carry-in
         reinterpret_cast<float*>(cx.sm + Ly::oAcar)[i] = slice[(int64_t)S * D + i];
     fence_proxy_async();
@@ -1721,6 +1729,7 @@ tile_totals4_tc_bf16(const __grid_constant__ CUtensorMap map_k4, const __grid_co
     cx.abort_flag = reinterpret_cast<volatile int*>(cx.sm + Ly::oMisc + 4);
     cx.status = status;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(cx.sm + Ly::oMisc);
+    chain_release();
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int GC = G / 4;                                    // CTAs per (stream, tile)
@@ -1761,6 +1770,7 @@ tile_totals4_tc_bf16(const __grid_constant__ CUtensorMap map_k4, const __grid_co
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    chain_wait();
 
     if (warp < 8) {
         const int wg = warp >> 2, wtid = tid & 127;
@@ -1950,13 +1960,12 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
         err = cudaFuncSetAttribute(k4, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay4<D>::kSmem);
         if (err != cudaSuccess) return err;
         dim3 grid4((unsigned)(tiles * (G / 4)), (unsigned)dm.N);
-        k4<<<grid4, kT1Threads, Lay4<D>::kSmem, stream>>>(mk4, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H, status);
-        err = cudaGetLastError();
+        err = launch_chain(chain_launches(dm), k4, grid4, kT1Threads, Lay4<D>::kSmem, stream, mk4, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H,
+                           status);
         if (err != cudaSuccess) return err;
     } else if (phases & kPhaseTotals) {
         dim3 grid1((unsigned)(tiles * (G / GP)), (unsigned)dm.N);
-        k1<<<grid1, kT1Threads, k1_smem, stream>>>(mk2, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H, status);
-        err = cudaGetLastError();
+        err = launch_chain(chain_launches(dm), k1, grid1, kT1Threads, k1_smem, stream, mk2, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H, status);
         if (err != cudaSuccess) return err;
     }
     if (!(phases & kPhaseOutput)) {
@@ -1980,10 +1989,8 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
             err = cudaFuncSetAttribute(kw, cudaFuncAttributeMaxDynamicSharedMemorySize, LyW::kSmem);
             if (err != cudaSuccess) return err;
             dim3 wgrid4((unsigned)(tiles * (D / ds)), (unsigned)dm.N);
-            kw<<<wgrid4, LyW::kThreads, LyW::kSmem, stream>>>(
-                mq, mk2, mvs, (__nv_bfloat16*)out, (const float*)ws, dm.T, dm.S, D, G, tile_tokens,
-                dm.eps, dm.H, status);
-            return cudaGetLastError();
+            return launch_chain(chain_launches(dm), kw, wgrid4, LyW::kThreads, LyW::kSmem, stream, mq, mk2, mvs, (__nv_bfloat16*)out,
+                                (const float*)ws, dm.T, dm.S, D, G, tile_tokens, dm.eps, dm.H, status);
         }
         if (!make_map_bf16_slice(&mvs, v, dm.N, dm.T, dm.D, DS)) return cudaErrorInvalidValue;
         dim3 wgrid((unsigned)(tiles * (D / DS)), (unsigned)dm.N);
@@ -1991,18 +1998,15 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
         if (err != cudaSuccess) return err;
         CUtensorMap mq2;
         if (!make_map_bf16(&mq2, pq, dm.N, dm.T, dm.S)) return cudaErrorInvalidValue;
-        causal_out_wide_bf16<<<wgrid, kWThreads, LayW::kSmem, stream>>>(
-            mq2, mk, mvs, (__nv_bfloat16*)out, (const float*)ws, dm.T, dm.S, D, G, tile_tokens,
-            dm.eps, status);
-        return cudaGetLastError();
+        return launch_chain(chain_launches(dm), causal_out_wide_bf16, wgrid, kWThreads, LayW::kSmem, stream, mq2, mk, mvs, (__nv_bfloat16*)out,
+                            (const float*)ws, dm.T, dm.S, D, G, tile_tokens, dm.eps, status);
     }
     err = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay<D>::kSmem);
     if (err != cudaSuccess) return err;
     CUtensorMap mq1;
     if (!make_map_bf16(&mq1, pq, dm.N, dm.T, dm.S)) return cudaErrorInvalidValue;
-    k3<<<grid, kThreads, Lay<D>::kSmem, stream>>>(mq1, mk, mv, (__nv_bfloat16*)out,
-                                                  (const float*)ws, dm.T, dm.S, G, tile_tokens, dm.eps, dm.H, status);
-    return cudaGetLastError();
+    return launch_chain(chain_launches(dm), k3, grid, kThreads, Lay<D>::kSmem, stream, mq1, mk, mv, (__nv_bfloat16*)out, (const float*)ws, dm.T,
+                        dm.S, G, tile_tokens, dm.eps, dm.H, status);
 }
 
 }  // namespace

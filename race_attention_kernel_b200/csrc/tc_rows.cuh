@@ -37,9 +37,8 @@ __device__ __forceinline__ void mma_sw(uint32_t d, uint32_t a_addr, uint32_t b_a
         else mma_issue<true>(d, ad, bd, id);
     }
 }
-// the same with A in tensor memory (packed bf16 pairs, 8 columns per k-step).  kLimbs: A is one limb of a 128 x 128 matrix
-// written by two warp groups, each over the 64 columns it read: k-steps 0-3 at a_tmem, 4-7 at a_tmem + 64 (and the other
-// limb 32 columns further)
+// the same with A in tensor memory (packed bf16 pairs, 8 columns per k-step).  kLimbs: A is one limb of a 128 x 128
+// matrix that was written over the fp32 columns it came from, 32 columns at a time: [16 words of hi | 16 words of lo]
 template <bool kZero, int kSteps, bool kBMn, int kBRows, bool kLimbs = false>
 __device__ __forceinline__ void mma_sw_ta(uint32_t d, uint32_t a_tmem, uint32_t b_addr, uint32_t idesc) {
     const uint32_t b = sw_lo<kBMn, kBRows>(b_addr);
@@ -47,7 +46,7 @@ __device__ __forceinline__ void mma_sw_ta(uint32_t d, uint32_t a_tmem, uint32_t 
 #pragma unroll
     for (int k = 0; k < kSteps; ++k) {
         const uint64_t bd = desc64(kHiSw, b + sw_step<kBMn, kBRows>(k));
-        const uint32_t at = a_tmem + (kLimbs ? 64 * (k >> 2) + 8 * (k & 3) : 8 * k);
+        const uint32_t at = a_tmem + (kLimbs ? 32 * (k >> 1) + 8 * (k & 1) : 8 * k);
         if (kZero && k == 0) mma_issue_ta<false>(d, at, bd, id);
         else mma_issue_ta<true>(d, at, bd, id);
     }
@@ -65,7 +64,41 @@ __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.a
 template <int kRegs>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegs)); }
 
-// 32 packed words of the warp's lanes <-> 32 columns; the loads and stores wait for completion
+// hi + lo limbs of a pair: hi is the upper half of the fp32 word (exact remainder), lo its remainder rounded to bf16;
+// |error| <= 2^-16 |x|.  One conversion instead of two per pair: that instruction runs at a quarter of the ALU rate and
+// is what a stage of limb splitting is bound by.
+__device__ __forceinline__ void split2t(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+    hi = __byte_perm(ua, ub, 0x7632);
+    const float2 r = __fadd2_rn(make_float2(a, b), make_float2(-__uint_as_float(ua & 0xffff0000u), -__uint_as_float(ub & 0xffff0000u)));
+    __nv_bfloat162 l = __floats2bfloat162_rn(r.x, r.y);
+    lo = *reinterpret_cast<uint32_t*>(&l);
+}
+
+// 32 lanes x 16 columns
+__device__ __forceinline__ void tmem_ld_rows16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr) : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// ... and words; no wait inside (tmem_wait_st)
+__device__ __forceinline__ void tmem_st_words16(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
+        ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+          "r"(taddr) : "memory");
+}
+
+// 32 packed words of the warp's lanes <-> 32 columns; waits for completion
 __device__ __forceinline__ void tmem_st_words32(uint32_t taddr, const uint32_t (&r)[32]) {
     tmem_st_rows32(taddr, reinterpret_cast<const float(&)[32]>(r));
 }
