@@ -416,8 +416,10 @@ int race_b200_noncausal_fwd(const void* probs_q, const void* probs_k, const void
     if (!aligned16(probs_q) || !aligned16(probs_k) || !aligned16(v) || !aligned16(out) ||
         !aligned16(totals) || !aligned16(workspace))
         return RACE_ERR_ALIGN;
-    rc = race_b200_tile_totals(probs_k, v, totals, workspace, workspace_bytes, shape,
-                               noncausal_totals_tile(shape, dm), RACE_VARIANT_AUTO, stream, nullptr);
+    const int tile = noncausal_totals_tile(shape, dm);
+    const bool direct = tile >= dm.T;   // one tile per stream: its totals are the state, no workspace between them
+    rc = race_b200_tile_totals(probs_k, v, totals, direct ? (void*)totals : workspace,
+                               direct ? sf * sizeof(float) : workspace_bytes, shape, tile, RACE_VARIANT_AUTO, stream, nullptr);
     if (rc != RACE_OK) return rc;
     if (noncausal_tensor_supported(dm, shape->dtype))
         return (int)noncausal_query_tensor(probs_q, totals, out, dm, shape->dtype, sm_count(), st);
@@ -457,14 +459,16 @@ int race_b200_noncausal_bwd(const void* probs_q, const void* probs_k, const void
     float* dE_state = (float*)((char*)workspace + ((tile_ws + 255) / 256 * 256));
     float* grads = (float*)((char*)dE_state + sfb);
     // dE = pQ^T dO : the tile-totals pass with (pQ, dO) in the roles of (pK, V)
-    rc = race_b200_tile_totals(probs_q, d_out, dE_state, ws_tiles, tile_ws, shape,
-                               noncausal_totals_tile(shape, dm), RACE_VARIANT_AUTO, stream, nullptr);
+    const int tile = noncausal_totals_tile(shape, dm);
+    const bool direct = tile >= dm.T;   // as in the forward
+    rc = race_b200_tile_totals(probs_q, d_out, dE_state, direct ? dE_state : ws_tiles, direct ? sfb : tile_ws, shape, tile,
+                               RACE_VARIANT_AUTO, stream, nullptr);
     if (rc != RACE_OK) return rc;
+    if (noncausal_tensor_supported(dm, shape->dtype))   // derives the gradients of the state from dE by itself
+        return (int)noncausal_token_grads_tensor(probs_k, v, d_out, totals, dE_state, d_probs_q, d_probs_k, d_v,
+                                                 dm, shape->dtype, sm_count(), st);
     cudaError_t e = noncausal_state_grads(totals, dE_state, grads, dm, st);
     if (e != cudaSuccess) return (int)e;
-    if (noncausal_tensor_supported(dm, shape->dtype))
-        return (int)noncausal_token_grads_tensor(probs_k, v, d_out, totals, grads, d_probs_q, d_probs_k, d_v,
-                                                 dm, shape->dtype, sm_count(), st);
     return (int)noncausal_token_grads(probs_k, v, d_out, totals, grads, d_probs_q, d_probs_k, d_v, dm,
                                       shape->dtype, sm_count(), st);
 }

@@ -466,7 +466,7 @@ cudaError_t causal_scan_tiles(float* ws, const float* carry_in, float* state_out
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
     const int sf = state_floats_per_stream(dm.S, dm.D);
     if (tiles == 1 && !carry_in && !write_prefix && state_out)   // one tile per stream: its totals are the state
-        return cudaMemcpyAsync(state_out, ws, (size_t)dm.N * sf * sizeof(float), cudaMemcpyDeviceToDevice, stream);
+        return ws == state_out ? cudaSuccess : cudaMemcpyAsync(state_out, ws, (size_t)dm.N * sf * sizeof(float), cudaMemcpyDeviceToDevice, stream);
     dim3 sgrid((unsigned)((sf + 127) / 128), (unsigned)dm.N);
     return launch_chain(chain_launches(dm), tile_scan, sgrid, 128, 0, stream, ws, carry_in, state_out, tiles, sf, write_prefix ? 1 : 0,
                         reverse ? 1 : 0);

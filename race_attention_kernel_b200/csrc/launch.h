@@ -78,8 +78,9 @@ cudaError_t noncausal_token_grads(const void* pk, const void* v, const void* dou
 bool noncausal_tensor_supported(const Dims& dm, int dtype);
 cudaError_t noncausal_query_tensor(const void* pq, const float* totals, void* out, const Dims& dm, int dtype,
                                    int sm_count, cudaStream_t stream);
+// de_state: the totals pass over (pQ, dO) in state layout
 cudaError_t noncausal_token_grads_tensor(const void* pk, const void* v, const void* dout, const float* totals,
-                                         const float* grads, void* dpq, void* dpk, void* dv, const Dims& dm,
+                                         const float* de_state, void* dpq, void* dpk, void* dv, const Dims& dm,
                                          int dtype, int sm_count, cudaStream_t stream);
 
 // ---- bucket-probability producer (bucket_probs.cu) --------------------------------------------

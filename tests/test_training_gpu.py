@@ -72,3 +72,24 @@ def test_operator_gradients(dk, K, L, dt, B, T, H):
             assert float(a.double().abs().max()) <= {torch.float32: 1e-3, torch.bfloat16: 0.5}[dt]
             continue
         assert ro.rel_l2(a, b) <= TOL[dt], (name, ro.rel_l2(a, b))
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,T", [(1, 1), (2, 127), (3, 128), (40, 300), (300, 130), (2, 20000)])
+def test_noncausal_shares(N, T, dt):
+    """The non-causal token kernel deals the 128-token chunks of all streams out to the SMs in equal shares: one chunk,
+    remainders, fewer and more chunks than SMs, shares that begin and end inside a stream."""
+    import race_attention_kernel_b200.ops as ops
+    g = torch.Generator(device="cuda").manual_seed(T)
+    pq, pk = (torch.softmax(torch.randn(N, T, 4, 16, device="cuda", generator=g), -1).to(dt).requires_grad_(True)
+              for _ in range(2))
+    v, dO = (torch.randn(N, T, 64, device="cuda", generator=g).to(dt) for _ in range(2))
+    v.requires_grad_(True)
+    out = ops.race_noncausal(pq, pk, v)
+    got = (out, *torch.autograd.grad(out, (pq, pk, v), dO))
+    a, b, c = (_leaf(t) for t in (pq, pk, v))
+    o = a.flatten(2) @ ((b.flatten(2).transpose(1, 2) @ c) / (b.flatten(2).sum(1).unsqueeze(-1) + 1e-6))
+    for name, x, y in zip(("out", "dPQ", "dPK", "dV"), got, (o, *torch.autograd.grad(o, (a, b, c), dO.double()))):
+        if name == "dPK" and T == 1:
+            continue    # cancels to O(eps): only rounding errors are left
+        assert ro.rel_l2(x, y) <= (2e-5 if dt == torch.float32 else 4e-3), (name, ro.rel_l2(x, y))
