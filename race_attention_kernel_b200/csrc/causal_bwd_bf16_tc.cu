@@ -835,7 +835,7 @@ cudaError_t launch(const void* pq, const void* pk, const void* v, const void* do
     if (err != cudaSuccess) return err;
     // state before every tile: the forward's totals and scan
     err = causal_fwd_tensor(nullptr, pk, v, nullptr, nullptr, nullptr, wp, false, dm, RACE_DTYPE_BF16, tile, stream, status,
-                            kPhaseTotals);
+                            kPhaseTotals | kPhasePrefixOnly);
     if (err == cudaSuccess) err = causal_scan_tiles(wp, carry_in, nullptr, dm, tile, stream, true);
     if (err != cudaSuccess) return err;
     CUtensorMap mdo, mv, mk, mq;

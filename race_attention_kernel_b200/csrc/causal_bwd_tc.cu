@@ -175,7 +175,7 @@ bwd_transpose_state(const float* __restrict__ src, float* __restrict__ dst) {
 }
 
 struct BwdLayout {
-    size_t tiles, tiles2, w, g, asum, gsum, achunk, st0, st1, total;
+    size_t tiles, tiles2, w, g, asum, gsum, achunk, st0, total;
 };
 BwdLayout bwd_layout(const Dims& dm, int tile_tokens) {
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
@@ -193,8 +193,7 @@ BwdLayout bwd_layout(const Dims& dm, int tile_tokens) {
     l.gsum = l.asum + blk;
     l.achunk = l.gsum + blk;
     l.st0 = l.achunk + align256((size_t)dm.N * ((dm.T + 63) / 64) * 64 * sizeof(float));
-    l.st1 = l.st0 + st;
-    l.total = l.st1 + st;
+    l.total = l.st0 + st;
     return l;
 }
 
@@ -231,7 +230,6 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     float* gsum = (float*)(base + l.gsum);
     float* ws_tiles2 = (float*)(base + l.tiles2);
     float* st_t = (float*)(base + l.st0);      // a transposed carry
-    float* st_dv = (float*)(base + l.st1);     // final state of pass 3 when the caller does not want it
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
     const int64_t nblk = (dm.T + kBlk - 1) / kBlk, total_blocks = dm.N * nblk;
     const unsigned pw_grid = (unsigned)((total_blocks + kPwThreads / 64 - 1) / (kPwThreads / 64));
@@ -261,9 +259,9 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     //    Pass 4 below has the roles of W and dO swapped, so its tile totals are the transposes of this pass's:
     //    the totals launch runs once and the second tile buffer gets the transposed states.
     RACE_CK(causal_raw_tensor(nullptr, w, dout, nullptr, nullptr, nullptr, ws_tiles, dm, tile_tokens, true, stream, status,
-                              kPhaseTotals, nullptr, 1, 1, dm.H, 1));
+                              d_carry ? kPhaseTotals : kPhaseTotals | kPhasePrefixOnly, nullptr, 1, 1, dm.H, 1));
     RACE_CK(launch_chain(chain_launches(dm), bwd_transpose_state, (unsigned)(dm.N * tiles), 256, 0, stream, (const float*)ws_tiles, ws_tiles2));
-    RACE_CK(causal_raw_tensor(pk, w, dout, dv, d_state, d_carry ? d_carry : st_dv, ws_tiles, dm, tile_tokens,
+    RACE_CK(causal_raw_tensor(pk, w, dout, dv, d_state, d_carry, ws_tiles, dm, tile_tokens,
                               /*reverse=*/true, stream, status, kPhaseOutput, nullptr, 1, 1, dm.H, dm.H));
     // 4. P = raw_reverse(V, dO, W) into the dPK buffer; state = the transpose of pass 3's
     if (d_state) RACE_CK(launch_chain(chain_launches(dm), bwd_transpose_state, (unsigned)dm.N, 256, 0, stream, d_state, st_t));

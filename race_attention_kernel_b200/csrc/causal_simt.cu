@@ -146,11 +146,12 @@ tile_scan(float* __restrict__ ws, const float* __restrict__ carry_in, float* __r
     // reverse: exclusive SUFFIX sums -- slot t gets carry + the totals of the tiles after t (last tile first)
     float* p = ws + (n * tiles + (reverse ? tiles - 1 : 0)) * state_floats + i;
     const int64_t step = reverse ? -state_floats : state_floats;
+    const int64_t have = state_out ? tiles : tiles - 1;   // without a final state the last tile's totals are not formed
     for (int64_t t = 0; t < tiles; t += kInFlight, p += kInFlight * step) {
         const int cnt = (int)min((int64_t)kInFlight, tiles - t);
         float x[kInFlight];
 #pragma unroll
-        for (int j = 0; j < kInFlight; ++j) x[j] = j < cnt ? p[j * step] : 0.f;
+        for (int j = 0; j < kInFlight; ++j) x[j] = t + j < have ? p[j * step] : 0.f;
 #pragma unroll
         for (int j = 0; j < kInFlight; ++j) {
             if (write_prefix && j < cnt) p[j * step] = run;

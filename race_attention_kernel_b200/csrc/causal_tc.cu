@@ -48,6 +48,7 @@ constexpr uint32_t kTmemCols = 512;
 constexpr int kTileF32 = C * 64 * 4;        // one staged fp32 tile: 64 tokens x 64 values
 constexpr int kStageBytes = 2 * kTileF32;   // pK | V  (pQ goes global -> registers)
 constexpr int kOpTile = C * 64 * 2;         // one bf16 operand tile (8 KB)
+constexpr int kSF = S * (D + 1);                  // floats of one state
 constexpr int oStage = 0;                               // [2][kStageBytes]
 constexpr int oKt = oStage + 2 * kStageBytes;           // [2 wg][2 buffers][hi|lo]
 constexpr int oVt = oKt + 8 * kOpTile;
@@ -225,6 +226,8 @@ __device__ __forceinline__ void out_phase_init_bars(const Ctx& cx, bool again, u
 // src/race_baseline.py:41-44): `pq` is Q and map_k covers K, both in the layout of V ([N/heads, T, heads, 64]); the
 // worker warps turn their rows of Q into probabilities in the accumulator-fragment layout, the converter group turns
 // the staged K tile into the pK operand tiles; ptab = the plane fragments in shared memory (build_plane_tab).
+// carry_smem: the B part of the carry has been formed in shared memory (fold_prefix; the A part in the first buffer of
+// the running A) by the twelve worker and converter warps.
 // kWorkerK: the pK operand tile of a chunk is written by the warps of the chunk's own worker group (at the start of
 // their work on the chunk) instead of the converter group, which then only converts V and copies the running B.
 // kModeRawX: the plain product with the epilogue of the first backward pass (BwdX in launch.h): after G . V the
@@ -240,7 +243,8 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
                                           float* __restrict__ out, const float* __restrict__ slice, int64_t T,
                                           const int64_t t_begin, const int64_t t_end, const int64_t n, float eps,
                                           const Heads hd, int withhold_chunk, const bool l2_last_use = false,
-                                          const uint32_t* ptab = nullptr, const BwdX* bx = nullptr) {
+                                          const uint32_t* ptab = nullptr, const BwdX* bx = nullptr,
+                                          const float* carry_smem = nullptr) {
     constexpr bool kGlobal = kMode == kModeGlobal;
     constexpr bool kRaw = kMode == kModeRaw || kMode == kModeRawX;   // no running sum, no normalisation in the W stage
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -545,8 +549,9 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
         for (int x = 0; x < 8; ++x)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float2 b2 = __ldcg(reinterpret_cast<const float2*>(
-                    slice + (rbase + 8 * h) * D + 8 * x + 2 * q));
+                const int off = (rbase + 8 * h) * D + 8 * x + 2 * q;
+                const float2 b2 = carry_smem ? *reinterpret_cast<const float2*>(carry_smem + off)
+                                             : __ldcg(reinterpret_cast<const float2*>(slice + off));
                 v[4 * x + 2 * h] = b2.x; v[4 * x + 2 * h + 1] = b2.y;
             }
         {   // tril[t][j] = (j <= t), exact in bf16, as an A operand in tensor memory
@@ -562,7 +567,7 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
         }
         tmem_st64(lane_base + tmB, v);   // waits for both stores
         tc_fence_before();
-        if (warp == 8) {
+        if (warp == 8 && !carry_smem) {   // (folded: the A part is there already)
             float* ac = reinterpret_cast<float*>(cx.sm + oAcar);
             ac[lane] = __ldcg(slice + S * D + lane);
             ac[lane + 32] = __ldcg(slice + S * D + lane + 32);
@@ -754,7 +759,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, float* __restrict__ out,
               const float* __restrict__ ws, int64_t T, int tile_tokens, float eps, const Heads hd, int* status,
-              long long wait_cycles, int withhold_chunk, const float* __restrict__ planes, const BwdX bwdx) {
+              long long wait_cycles, int withhold_chunk, const float* __restrict__ planes, const BwdX bwdx,
+              const CarryFold cf) {
     extern __shared__ uint8_t smem_raw[];
     Ctx cx;
     cx.sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -787,8 +793,21 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     chain_wait();
+    // the prefix lands in the second state operand buffer, which the converter group writes first after chunk 0, and
+    // the TMA and MMA warps are ahead with chunk 0 meanwhile
+    float* carry_smem = cf.fold ? reinterpret_cast<float*>(cx.sm + oBt + 2 * kOpTile) : nullptr;
+    if (cf.fold && warp < 12) {
+        static_assert(S * D * 4 == 2 * kOpTile, "the carry fills one state operand buffer");
+        const bool last = kReverse ? tile == 0 : tile == tiles - 1;
+        fold_prefix<12 * 32>(ws + (n * tiles + (kReverse ? tiles - 1 : 0)) * kSF, kReverse ? -kSF : kSF,
+                             (int)(kReverse ? tiles - 1 - tile : tile), cf.carry_in ? cf.carry_in + n * kSF : nullptr,
+                             last && cf.state_out ? cf.state_out + n * kSF : nullptr, carry_smem,
+                             reinterpret_cast<float*>(cx.sm + oAcar), S * D, kSF, tid);
+        asm volatile("bar.sync 1, 384;" ::: "memory");
+    }
     out_phase<kMode, kReverse, kProj, kWorkerK>(cx, tmem, pq, &map_k, &map_v, out, slice, T, t_begin, t_end, n, eps,
-                                                hd, (tile == 0 && n == 0) ? withhold_chunk : -1, false, ptab, &bwdx);
+                                                hd, (tile == 0 && n == 0) ? withhold_chunk : -1, false, ptab, &bwdx,
+                                                carry_smem);
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -1089,7 +1108,7 @@ template <bool kProj>
 __global__ void __launch_bounds__(TotalsLayoutOf<kProj>::kThreads, 1)
 tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                float* __restrict__ ws, int64_t T, int tile_tokens, const Heads hd, int* status,
-               const float* __restrict__ planes) {
+               const float* __restrict__ planes, int64_t tiles, int tile0) {
     extern __shared__ uint8_t smem_raw[];
     Ctx cx;
     cx.sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -1100,7 +1119,7 @@ tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     cx.status = status;
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(cx.sm + TL::oMisc);
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int64_t tiles = gridDim.x, tile = blockIdx.x, n = blockIdx.y;
+    const int64_t tile = tile0 + blockIdx.x, n = blockIdx.y;
     const int64_t t_begin = tile * tile_tokens;
     const int64_t t_end = min(T, t_begin + (int64_t)tile_tokens);
     float* slice = ws + (n * tiles + tile) * (int64_t)(S * (D + 1));
@@ -1141,7 +1160,6 @@ tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
 // Every spin is bounded (cx.limit): a flag that never comes raises the status word and the CTA
 // stops taking tickets; nothing is in flight at that point.
 // ------------------------------------------------------------------------------------------------
-constexpr int kSF = S * (D + 1);                  // floats of one state
 constexpr int kFusedMaxGrid = 160;                // per-CTA carry slots in the workspace
 constexpr int kLookbackDepth = 24;                // tiles whose totals a look-back adds at most
 constexpr int oFusedMisc = (oMisc > o1Misc ? oMisc : o1Misc) + 16;   // tmem base, abort, ticket, j
@@ -1548,9 +1566,12 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
     }
     dim3 grid((unsigned)tiles, (unsigned)dm.N);
     // 1. tile totals (tensor cores)  2. exclusive scan over tiles  3. output pass
-    if (phases & kPhaseTotals) {
-        err = launch_chain(chain_launches(dm), totals_kern, grid, totals_threads, totals_smem, stream, mk, mv, (float*)ws, dm.T, tile_tokens, hd,
-                           status, planes);
+    // (the totals of the last tile -- reverse: the first -- only enter the final state)
+    const bool all_tiles = state_out || !(phases & (kPhaseOutput | kPhasePrefixOnly));
+    const int64_t tiles_run = all_tiles ? tiles : tiles - 1;
+    if ((phases & kPhaseTotals) && tiles_run > 0) {
+        err = launch_chain(chain_launches(dm), totals_kern, dim3((unsigned)tiles_run, (unsigned)dm.N), totals_threads, totals_smem, stream, mk, mv,
+                           (float*)ws, dm.T, tile_tokens, hd, status, planes, tiles, reverse && !all_tiles ? 1 : 0);
         if (err != cudaSuccess) return err;
     }
     if (!(phases & kPhaseOutput)) {
@@ -1559,8 +1580,11 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
         if (!state_out) return cudaSuccess;
         return causal_scan_tiles((float*)ws, carry_in, state_out, dm, tile_tokens, stream, /*write_prefix=*/false);
     }
-    err = causal_scan_tiles((float*)ws, carry_in, state_out, dm, tile_tokens, stream, /*write_prefix=*/true, reverse);
-    if (err != cudaSuccess) return err;
+    CarryFold cf{carry_in, state_out, fold_carry(dm.N, tiles, kSF, carry_in, state_out) ? 1 : 0};
+    if (!cf.fold) {
+        err = causal_scan_tiles((float*)ws, carry_in, state_out, dm, tile_tokens, stream, /*write_prefix=*/true, reverse);
+        if (err != cudaSuccess) return err;
+    }
     auto kern = mode == kModeRawX ? causal_out_tc<kModeRawX, false, false>
                 : mode == kModeRaw
                     ? (reverse ? causal_out_tc<kModeRaw, true, false> : causal_out_tc<kModeRaw, false, false>)
@@ -1570,7 +1594,7 @@ static cudaError_t tensor_f32_launch(const void* pq, const void* pk, const void*
     err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     if (err != cudaSuccess) return err;
     return launch_chain(chain_launches(dm), kern, grid, kThreads, kSmemBytes, stream, (const float*)pq, mk, mv, (float*)out, (const float*)ws,
-                        dm.T, tile_tokens, dm.eps, hd, status, wait_cycles, withhold_chunk, planes, bwdx ? *bwdx : BwdX{});
+                        dm.T, tile_tokens, dm.eps, hd, status, wait_cycles, withhold_chunk, planes, bwdx ? *bwdx : BwdX{}, cf);
 }
 
 #ifdef RACE_FUSED_PROF

@@ -40,7 +40,8 @@ struct Lay {
     static constexpr int oTril = oBt + 2 * kTileV;
     static constexpr int oAcar = oTril + kTileP;        // [2][64] fp32
     static constexpr int oPq = (oAcar + 2 * 64 * 4 + 1023) / 1024 * 1024;   // [2 wg][kTileP] pQ of the group's next chunk
-    static constexpr int oBars = oPq + 2 * kTileP;
+    static constexpr int oCarry = oPq + 2 * kTileP;     // [64][D] fp32: the folded carry
+    static constexpr int oBars = oCarry + SG * D * 4;
     static constexpr int kNumBars = 36;
     static constexpr int oMisc = oBars + kNumBars * 8;
     static constexpr int kSmem = oMisc + 16 + 1024;
@@ -106,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
                    const float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, float eps, int heads,
-                   int* status) {
+                   int* status, const CarryFold cf) {
     using Ly = Lay<D>;
     constexpr int DH = D / 64;   // 64-column halves of a [64][D] accumulator
     extern __shared__ uint8_t smem_raw[];
@@ -174,6 +175,15 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     chain_wait();
+    const float* carry_smem = cf.fold ? reinterpret_cast<const float*>(cx.sm + Ly::oCarry) : nullptr;
+    if (cf.fold && warp < 12) {   // (one bucket group)
+        constexpr int kState = SG * (D + 1);
+        fold_prefix<12 * 32>(ws + n * tiles * kState, kState, (int)tile, cf.carry_in ? cf.carry_in + n * kState : nullptr,
+                             cf.state_out && tile == tiles - 1 ? cf.state_out + n * kState : nullptr,
+                             reinterpret_cast<float*>(cx.sm + Ly::oCarry), reinterpret_cast<float*>(cx.sm + Ly::oAcar),
+                             SG * D, kState, tid);
+        asm volatile("bar.sync 1, 384;" ::: "memory");
+    }
     const uint32_t tmB = tmem;                                                   // [0, D)
     auto tmAG = [&](int wg) { return tmem + D + wg * (64 + D); };                // A_loc, then G
     auto tmO = [&](int wg) { return tmem + D + wg * (64 + D) + 64; };            // O
@@ -361,14 +371,14 @@ causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_const
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const float2 b2 = *reinterpret_cast<const float2*>(
-                        sliceB + (rbase + 8 * h) * D + dh * 64 + 8 * x + 2 * q);
+                        (carry_smem ? carry_smem : sliceB) + (rbase + 8 * h) * D + dh * 64 + 8 * x + 2 * q);
                     v[4 * x + 2 * h] = b2.x; v[4 * x + 2 * h + 1] = b2.y;
                 }
             tmem_st64(lane_base + tmB + dh * 64, v);
             write_bt(0, dh);
         }
         tc_fence_before();
-        if (warp == 8) {
+        if (warp == 8 && !carry_smem) {
             float* ac = reinterpret_cast<float*>(cx.sm + Ly::oAcar);
             ac[lane] = sliceA[lane];
             ac[lane + 32] = sliceA[lane + 32];
@@ -540,7 +550,7 @@ enum Bar1B { b1Full = 0, b1Empty = 4, b1KvReady = 8, b1KvFree = 10, b1Done = 12 
 template <int D, int GP>
 __global__ void __launch_bounds__(kT1Threads, 1)
 tile_totals_tc_bf16(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                    float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, int heads, int* status) {
+                    float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, int heads, int64_t tiles, int* status) {
     using Ly = Lay1<D, GP>;
     constexpr int DH = D / 64;
     static_assert(GP * D <= 512, "one accumulator per group");
@@ -557,7 +567,7 @@ tile_totals_tc_bf16(const __grid_constant__ CUtensorMap map_k, const __grid_cons
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int GC = G / GP;                                   // CTAs per (stream, tile)
     const int g = (int)(blockIdx.x % (unsigned)GC) * GP;     // first bucket group of this CTA
-    const int64_t tiles = gridDim.x / GC, tile = blockIdx.x / GC, n = blockIdx.y;
+    const int64_t tile = blockIdx.x / GC, n = blockIdx.y;
     const int64_t t_begin = tile * tile_tokens;
     const int64_t t_end = min(T, t_begin + (int64_t)tile_tokens);
     const int nch = (int)((t_end - t_begin + C - 1) / C);
@@ -1718,7 +1728,7 @@ static_assert(Lay4<128>::kSmem <= 227 * 1024 && Lay4<64>::kSmem <= 227 * 1024, "
 template <int D>
 __global__ void __launch_bounds__(kT1Threads, 1)
 tile_totals4_tc_bf16(const __grid_constant__ CUtensorMap map_k4, const __grid_constant__ CUtensorMap map_v,
-                     float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, int heads, int* status) {
+                     float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, int heads, int64_t tiles, int* status) {
     using Ly = Lay4<D>;
     constexpr int DX = Ly::DX;
     extern __shared__ uint8_t smem_raw[];
@@ -1734,7 +1744,7 @@ tile_totals4_tc_bf16(const __grid_constant__ CUtensorMap map_k4, const __grid_co
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int GC = G / 4;                                    // CTAs per (stream, tile)
     const int g = (int)(blockIdx.x % (unsigned)GC) * 4;      // first bucket group of this CTA
-    const int64_t tiles = gridDim.x / GC, tile = blockIdx.x / GC, n = blockIdx.y;
+    const int64_t tile = blockIdx.x / GC, n = blockIdx.y;
     const int64_t t_begin = tile * tile_tokens;
     const int64_t t_end = min(T, t_begin + (int64_t)tile_tokens);
     const int nch = (int)((t_end - t_begin + C - 1) / C);
@@ -1952,28 +1962,35 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
         return cudaErrorInvalidValue;
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
     dim3 grid((unsigned)(tiles * G), (unsigned)dm.N);
-    if ((phases & kPhaseTotals) && G >= 4) {
+    // (the totals of the last tile only enter the final state)
+    const int64_t tiles_run = state_out || !(phases & (kPhaseOutput | kPhasePrefixOnly)) ? tiles : tiles - 1;
+    if ((phases & kPhaseTotals) && tiles_run > 0 && G >= 4) {
         // four bucket groups per CTA, pair-stacked accumulators, column sums by the tensor core
         CUtensorMap mk4;
         if (!make_map_bf16(&mk4, pk, dm.N, dm.T, dm.S, 4)) return cudaErrorInvalidValue;
         auto k4 = tile_totals4_tc_bf16<D>;
         err = cudaFuncSetAttribute(k4, cudaFuncAttributeMaxDynamicSharedMemorySize, Lay4<D>::kSmem);
         if (err != cudaSuccess) return err;
-        dim3 grid4((unsigned)(tiles * (G / 4)), (unsigned)dm.N);
+        dim3 grid4((unsigned)(tiles_run * (G / 4)), (unsigned)dm.N);
         err = launch_chain(chain_launches(dm), k4, grid4, kT1Threads, Lay4<D>::kSmem, stream, mk4, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H,
-                           status);
+                           tiles, status);
         if (err != cudaSuccess) return err;
-    } else if (phases & kPhaseTotals) {
-        dim3 grid1((unsigned)(tiles * (G / GP)), (unsigned)dm.N);
-        err = launch_chain(chain_launches(dm), k1, grid1, kT1Threads, k1_smem, stream, mk2, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H, status);
+    } else if ((phases & kPhaseTotals) && tiles_run > 0) {
+        dim3 grid1((unsigned)(tiles_run * (G / GP)), (unsigned)dm.N);
+        err = launch_chain(chain_launches(dm), k1, grid1, kT1Threads, k1_smem, stream, mk2, mv, (float*)ws, dm.T, dm.S, G, tile_tokens, dm.H, tiles,
+                           status);
         if (err != cudaSuccess) return err;
     }
     if (!(phases & kPhaseOutput)) {
         if (!state_out) return cudaSuccess;   // the caller wants the per-tile totals alone
         return causal_scan_tiles((float*)ws, carry_in, state_out, dm, tile_tokens, stream, false);
     }
-    err = causal_scan_tiles((float*)ws, carry_in, state_out, dm, tile_tokens, stream, true);
-    if (err != cudaSuccess) return err;
+    const CarryFold cf{carry_in, state_out,
+                       G == 1 && fold_carry(dm.N, tiles, state_floats_per_stream(dm.S, dm.D), carry_in, state_out) ? 1 : 0};
+    if (!cf.fold) {
+        err = causal_scan_tiles((float*)ws, carry_in, state_out, dm, tile_tokens, stream, true);
+        if (err != cudaSuccess) return err;
+    }
     if (G > 1) {
         // all bucket groups in one CTA, the head dimension in slices
         CUtensorMap mvs;
@@ -2006,7 +2023,7 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
     CUtensorMap mq1;
     if (!make_map_bf16(&mq1, pq, dm.N, dm.T, dm.S)) return cudaErrorInvalidValue;
     return launch_chain(chain_launches(dm), k3, grid, kThreads, Lay<D>::kSmem, stream, mq1, mk, mv, (__nv_bfloat16*)out, (const float*)ws, dm.T,
-                        dm.S, G, tile_tokens, dm.eps, dm.H, status);
+                        dm.S, G, tile_tokens, dm.eps, dm.H, status, cf);
 }
 
 }  // namespace

@@ -32,6 +32,63 @@ __host__ __device__ inline int state_floats_per_stream(int S, int D) { return S 
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// The state a tile starts from, formed by the output kernel itself (fold): carry_in + the totals of the tiles before it,
+// added tile by tile in the order tile_scan adds them, so both routes give the same bits.  Not folded: the slot of the
+// tile already holds that prefix (tile_scan).  The CTA of the last tile also writes the state after the sequence.
+struct CarryFold {
+    const float* carry_in;    // [N][state] or null (zeros)
+    float* state_out;         // [N][state] or null
+    int fold;
+};
+
+// Threads 0 .. NT-1 of the CTA: prefix of `cnt` tiles at p, p + step, ... (4 floats per thread and column, up to three
+// columns and six tiles in flight: the loads are L2 latencies, a column at a time they were a chain of them).
+// b_floats: floats of the B part, which goes to sb; the A part goes to sa.
+template <int NT>
+__device__ __forceinline__ void fold_prefix(const float* p, int64_t step, int cnt, const float* carry, float* state_out,
+                                            float* sb, float* sa, int b_floats, int state_floats, int tid) {
+    constexpr int kCols = 3, kTiles = 6;
+    for (int base = 4 * tid; base < state_floats; base += 4 * NT * kCols) {
+        float4 run[kCols];
+#pragma unroll
+        for (int u = 0; u < kCols; ++u) {
+            const int i = base + 4 * NT * u;
+            run[u] = carry && i < state_floats ? __ldcg(reinterpret_cast<const float4*>(carry + i))
+                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (int t = 0; t < cnt; t += kTiles) {
+            float4 x[kTiles][kCols];
+#pragma unroll
+            for (int j = 0; j < kTiles; ++j)
+#pragma unroll
+                for (int u = 0; u < kCols; ++u) {
+                    const int i = base + 4 * NT * u;
+                    x[j][u] = t + j < cnt && i < state_floats
+                                  ? __ldcg(reinterpret_cast<const float4*>(p + (t + j) * step + i))
+                                  : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+            for (int j = 0; j < kTiles; ++j)
+                if (t + j < cnt)
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u) {
+                        run[u].x += x[j][u].x; run[u].y += x[j][u].y; run[u].z += x[j][u].z; run[u].w += x[j][u].w;
+                    }
+        }
+#pragma unroll
+        for (int u = 0; u < kCols; ++u) {
+            const int i = base + 4 * NT * u;
+            if (i >= state_floats) continue;
+            *reinterpret_cast<float4*>(i < b_floats ? sb + i : sa + (i - b_floats)) = run[u];
+            if (state_out) {
+                const float4 x = __ldcg(reinterpret_cast<const float4*>(p + cnt * step + i));
+                *reinterpret_cast<float4*>(state_out + i) =
+                    make_float4(run[u].x + x.x, run[u].y + x.y, run[u].z + x.z, run[u].w + x.w);
+            }
+        }
+    }
+}
+
 // ---- element access: 4 consecutive elements as float4 -------------------------------------
 __device__ __forceinline__ float4 load4(const float* p) {
     return *reinterpret_cast<const float4*>(p);

@@ -52,8 +52,23 @@ cudaError_t causal_fwd_simt(const void* pq, const void* pk, const void* v, void*
 cudaError_t causal_scan_tiles(float* ws, const float* carry_in, float* state_out, const Dims& dm,
                               int tile_tokens, cudaStream_t stream, bool write_prefix = true, bool reverse = false);
 
-// which passes of a causal forward to run: totals (per-tile sums into ws) and/or scan + outputs
-constexpr int kPhaseTotals = 1, kPhaseOutput = 2, kPhaseAll = 3;
+// which passes of a causal forward to run: totals (per-tile sums into ws) and/or scan + outputs.  kPhasePrefixOnly, with
+// kPhaseTotals alone: the caller uses the totals for the prefixes of the tiles only, so the last tile's are not formed
+// (with kPhaseAll that follows from state_out == null).
+constexpr int kPhaseTotals = 1, kPhaseOutput = 2, kPhaseAll = 3, kPhasePrefixOnly = 4;
+
+// Whether the output kernel forms the state before each tile itself (CarryFold) instead of a tile_scan launch between
+// the two.  A launch costs 3 to 5 us in the chain of a small call; folding reads every tile's predecessors again, about
+// tiles^2 / 2 states per stream, from lines of L2 that many CTAs ask for at once: fp32 with 8 streams, 13 tiles (777
+// tokens) 17.8 -> 16.1 us, 16 tiles (4096 tokens) 28.4 -> 28.6; hence the line at N tiles^2 = 10 per SM.  One or two
+// tiles: always less than the scan reads and writes (bf16, 48 streams of three tiles: 100 -> 93 us).
+// A state written over the carry it came from would be read by other tiles' CTAs after the write: scan then.
+inline bool fold_carry(int64_t N, int64_t tiles, int64_t state_floats, const float* carry_in, const float* state_out) {
+    if (tiles > 1 && carry_in && state_out && carry_in < state_out + N * state_floats &&
+        state_out < carry_in + N * state_floats)
+        return false;
+    return tiles <= 2 || (tiles <= 32 && N * tiles * tiles <= 10 * 148);
+}
 
 // ---- causal backward (causal_bwd_simt.cu): S <= 64, d_k <= 128 ---------------------------------
 bool causal_bwd_supported(const Dims& dm, int dtype);
