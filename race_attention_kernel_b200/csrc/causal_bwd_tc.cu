@@ -32,33 +32,72 @@ namespace {
 
 constexpr int S = 64, D = 64;
 constexpr int kSF = S * (D + 1);
-constexpr int kBlk = 512;          // tokens per block of the streaming kernels (one thread per block and column)
-constexpr int kPwThreads = 256;    // 4 blocks x 64 columns per CTA
+constexpr int kBlk = 512;          // tokens per block of the streaming kernels
+constexpr int kPwThreads = 256;    // one CTA per block
 
 inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// sums[n][b][c] = sum over the tokens of block b of x[n][t][c]
+// sums[n][b][c] = sum over the tokens of block b of x[n][t][c]; kChunks: also chunk[n][j][c] = the sum of x over the
+// tokens of chunk j's block that precede chunk j (64-token chunks; a block is kBlk / 64 of them).
+// Bound by the read of x.  A CTA per block, 16-byte loads: 16 threads per row, 16 rows at a time, eight loads of a thread
+// in flight, partial sums added through shared memory.  (One thread per block and column read 4 bytes at a time along
+// a chain of 512 tokens: 32 streams of 16384 tokens, 134 MB, took 39 us.)
+template <bool kChunks>
 __global__ void __launch_bounds__(kPwThreads)
-bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, int64_t T, int64_t nblk, int64_t total_blocks) {
+bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, float* __restrict__ chunk, int64_t T, int64_t nblk,
+               int64_t nchunk) {
+    constexpr int kCh = kBlk / 64, kSums = kChunks ? kCh : 1, kWarps = kPwThreads / 32;
+    __shared__ __align__(16) float red[kWarps][kSums][64];
+    __shared__ float tot[kSums][64];
     chain_release();
     chain_wait();
-    const int64_t gb = (int64_t)blockIdx.x * (kPwThreads / 64) + (threadIdx.x >> 6);
-    if (gb >= total_blocks) return;
-    const int c = threadIdx.x & 63;
-    const int64_t n = gb / nblk, b = gb - n * nblk;
-    const int64_t t0 = b * kBlk, t1 = min(T, t0 + (int64_t)kBlk);
-    const float* p = x + (n * T + t0) * 64 + c;
-    float acc = 0.f;
-    int64_t t = t0;
-    for (; t + 8 <= t1; t += 8, p += 8 * 64) {
-        float v[8];
+    const int64_t gb = blockIdx.x, n = gb / nblk, b = gb - n * nblk;
+    const int64_t t0 = b * kBlk;
+    const int len = (int)min(T - t0, (int64_t)kBlk);
+    const int tid = threadIdx.x, c4 = tid & 15, slot = tid >> 4;
+    const float4* p = reinterpret_cast<const float4*>(x + (n * T + t0) * 64) + c4;
+    float4 acc[kSums];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) v[u] = __ldg(p + u * 64);
+    for (int j = 0; j < kSums; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) acc += v[u];
+    for (int j = 0; j < kCh; j += 2) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int t = 64 * j + 16 * u + slot;
+            v[u] = t < len ? __ldg(p + t * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            float4& s = acc[kChunks ? j + u / 4 : 0];
+            s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w;
+        }
     }
-    for (; t < t1; ++t, p += 64) acc += __ldg(p);
-    sums[gb * 64 + c] = acc;
+#pragma unroll
+    for (int j = 0; j < kSums; ++j) {
+        acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, 16);
+        acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, 16);
+        acc[j].z += __shfl_xor_sync(0xffffffffu, acc[j].z, 16);
+        acc[j].w += __shfl_xor_sync(0xffffffffu, acc[j].w, 16);
+        if ((tid & 31) < 16) *reinterpret_cast<float4*>(&red[tid >> 5][j][4 * c4]) = acc[j];
+    }
+    __syncthreads();
+    for (int i = tid; i < kSums * 64; i += kPwThreads) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) s += red[w][i >> 6][i & 63];
+        tot[i >> 6][i & 63] = s;
+    }
+    __syncthreads();
+    if (tid < 64) {
+        float run = 0.f;
+#pragma unroll
+        for (int j = 0; j < kSums; ++j) {
+            if (kChunks && 64 * j < len) chunk[(n * nchunk + t0 / 64 + j) * 64 + tid] = run;
+            run += tot[j][tid];
+        }
+        sums[gb * 64 + tid] = run;
+    }
 }
 
 // in-place exclusive scan over the blocks of a stream (reverse: suffix sums, last block first); carry is the A part
@@ -92,70 +131,54 @@ bwd_block_scan(float* __restrict__ sums, const float* __restrict__ carry_state, 
     if (total_state) total_state[n * kSF + S * D + c] = run;
 }
 
-// sums[n][b][c] as bwd_block_sums, and chunk[n][j][c] = the sum of x over the tokens of chunk j's block that precede
-// chunk j (64-token chunks; a block is kBlk / 64 of them)
-__global__ void __launch_bounds__(kPwThreads)
-bwd_block_chunk_sums(const float* __restrict__ x, float* __restrict__ sums, float* __restrict__ chunk, int64_t T,
-                     int64_t nblk, int64_t nchunk, int64_t total_blocks) {
-    chain_release();
-    chain_wait();
-    const int64_t gb = (int64_t)blockIdx.x * (kPwThreads / 64) + (threadIdx.x >> 6);
-    if (gb >= total_blocks) return;
-    const int c = threadIdx.x & 63;
-    const int64_t n = gb / nblk, b = gb - n * nblk;
-    const int64_t t0 = b * kBlk, t1 = min(T, t0 + (int64_t)kBlk);
-    const float* p = x + (n * T + t0) * 64 + c;
-    float* cp = chunk + (n * nchunk + t0 / 64) * 64 + c;
-    float acc = 0.f;
-    for (int64_t t = t0; t < t1; t += 64, cp += 64) {
-        *cp = acc;
-        const int cnt = (int)min((int64_t)64, t1 - t);
-        if (cnt == 64) {
-#pragma unroll
-            for (int u8 = 0; u8 < 8; ++u8) {
-                float v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = __ldg(p + (u8 * 8 + u) * 64);
-#pragma unroll
-                for (int u = 0; u < 8; ++u) acc += v[u];
-            }
-        } else {
-            for (int u = 0; u < cnt; ++u) acc += __ldg(p + u * 64);
-        }
-        p += 64 * 64;
-    }
-    sums[gb * 64 + c] = acc;
-}
-
-// reverse streaming kernel: dPK_j = P_j + suffix[block] + sum_{t >= j, t in block} g_t (P in pdpk on entry)
+// reverse streaming kernel: dPK_j = P_j + suffix[block] + sum_{t >= j, t in block} g_t (P in pdpk on entry).
+// Bound by two reads and a write of [N, T, 64].  A CTA per block walks it from its end in pieces of 128 tokens: 16 threads
+// (4 columns each) per token, eight consecutive tokens per thread, so that sixteen 16-byte loads of a thread are in
+// flight; the sums of the threads behind it come through shared memory.  (One thread per block and column, 4 bytes and
+// four tokens at a time: 32 streams of 16384 tokens, 403 MB, took 103 us.)
 __global__ void __launch_bounds__(kPwThreads)
 bwd_pointwise_rev(const float* __restrict__ g, float* __restrict__ pdpk, const float* __restrict__ gsuffix, int64_t T,
-                  int64_t nblk, int64_t total_blocks) {
+                  int64_t nblk) {
+    constexpr int kOwn = 8, kSlots = kPwThreads / 16, kPiece = kOwn * kSlots;
+    __shared__ float4 part[2][kSlots][16];
     chain_release();
     chain_wait();
-    const int64_t gb = (int64_t)blockIdx.x * (kPwThreads / 64) + (threadIdx.x >> 6);
-    if (gb >= total_blocks) return;
-    const int c = threadIdx.x & 63;
-    const int64_t n = gb / nblk, b = gb - n * nblk;
-    const int64_t t0 = b * kBlk, t1 = min(T, t0 + (int64_t)kBlk);
-    float sa = gsuffix[gb * 64 + c];
-    for (int64_t t = t1; t > t0; t -= 4) {
-        const int cnt = (int)min((int64_t)4, t - t0);
-        float g4[4], p4[4];
+    const int64_t gb = blockIdx.x, n = gb / nblk, b = gb - n * nblk;
+    const int64_t t0 = b * kBlk;
+    const int len = (int)min(T - t0, (int64_t)kBlk);
+    const int c4 = threadIdx.x & 15, slot = threadIdx.x >> 4;
+    const int64_t row0 = (n * T + t0) * 16 + c4;
+    const float4* gp = reinterpret_cast<const float4*>(g) + row0;
+    float4* pp = reinterpret_cast<float4*>(pdpk) + row0;
+    auto add = [](float4& a, const float4& x) { a.x += x.x; a.y += x.y; a.z += x.z; a.w += x.w; };
+    float4 carry = reinterpret_cast<const float4*>(gsuffix)[gb * 16 + c4];
+    for (int s = (len - 1) / kPiece; s >= 0; --s) {
+        const int t = s * kPiece + slot * kOwn;
+        float4 gv[kOwn], pv[kOwn];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (u < cnt) {
-                const int64_t off = (n * T + (t - 1 - u)) * 64 + c;
-                g4[u] = __ldcs(g + off);
-                p4[u] = pdpk[off];
-            }
+        for (int u = 0; u < kOwn; ++u) {
+            const bool live = t + u < len;
+            gv[u] = live ? __ldcs(gp + (t + u) * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+            pv[u] = live ? pp[(t + u) * 16] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (u < cnt) {
-                const int64_t off = (n * T + (t - 1 - u)) * 64 + c;
-                sa += g4[u];
-                pdpk[off] = p4[u] + sa;
-            }
+        for (int u = kOwn - 1; u >= 0; --u) add(own, gv[u]);
+        part[s & 1][slot][c4] = own;
+        __syncthreads();   // (the buffer of the piece before last was read before everyone came here)
+        float4 run = carry;
+#pragma unroll
+        for (int k = kSlots - 1; k >= 0; --k) {
+            const float4 x = part[s & 1][k][c4];
+            if (k > slot) add(run, x);
+            add(carry, x);
+        }
+#pragma unroll
+        for (int u = kOwn - 1; u >= 0; --u) {
+            add(run, gv[u]);
+            add(pv[u], run);
+            if (t + u < len) pp[(t + u) * 16] = pv[u];
+        }
     }
 }
 
@@ -231,14 +254,14 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     float* ws_tiles2 = (float*)(base + l.tiles2);
     float* st_t = (float*)(base + l.st0);      // a transposed carry
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
-    const int64_t nblk = (dm.T + kBlk - 1) / kBlk, total_blocks = dm.N * nblk;
-    const unsigned pw_grid = (unsigned)((total_blocks + kPwThreads / 64 - 1) / (kPwThreads / 64));
+    const int64_t nblk = (dm.T + kBlk - 1) / kBlk;
+    const unsigned pw_grid = (unsigned)(dm.N * nblk);
 
     // 1. sums of pK: per block (then scanned, carry included) and inside the block up to every chunk start
     float* achunk = (float*)(base + l.achunk);
     const int64_t nchunk = (dm.T + 63) / 64;
-    RACE_CK(launch_chain(chain_launches(dm), bwd_block_chunk_sums, pw_grid, kPwThreads, 0, stream, (const float*)pk, asum, achunk, dm.T, nblk,
-                         nchunk, total_blocks));
+    RACE_CK(launch_chain(chain_launches(dm), bwd_block_sums<true>, pw_grid, kPwThreads, 0, stream, (const float*)pk, asum, achunk, dm.T, nblk,
+                         nchunk));
     RACE_CK(launch_chain(chain_launches(dm), bwd_block_scan, (unsigned)dm.N, 64, 0, stream, asum, carry_in, nullptr, nblk, 0));
     // 2. X = raw(dO, V, pK), the state of the pass is B^T; its epilogue writes dPQ, W and g.  Then the block sums of g.
     if (carry_in) RACE_CK(launch_chain(chain_launches(dm), bwd_transpose_state, (unsigned)dm.N, 256, 0, stream, carry_in, st_t));
@@ -254,7 +277,7 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     bx.eps = dm.eps;
     RACE_CK(causal_raw_tensor(dout, v, pk, dpq, carry_in ? st_t : nullptr, nullptr, ws_tiles, dm, tile_tokens,
                               /*reverse=*/false, stream, status, kPhaseAll, &bx, dm.H, dm.H, 1, 1));
-    RACE_CK(launch_chain(chain_launches(dm), bwd_block_sums, pw_grid, kPwThreads, 0, stream, (const float*)g, gsum, dm.T, nblk, total_blocks));
+    RACE_CK(launch_chain(chain_launches(dm), bwd_block_sums<false>, pw_grid, kPwThreads, 0, stream, (const float*)g, gsum, nullptr, dm.T, nblk, nchunk));
     // 3. dV = raw_reverse(pK, W, dO); state sum W^T dO: carry = gradient of the final B, total = gradient of carry_in's B.
     //    Pass 4 below has the roles of W and dO swapped, so its tile totals are the transposes of this pass's:
     //    the totals launch runs once and the second tile buffer gets the transposed states.
@@ -271,7 +294,7 @@ cudaError_t causal_bwd_tensor(const void* pq, const void* pk, const void* v, con
     //    overwrites the A part that pass 3 left in d_carry)
     RACE_CK(launch_chain(chain_launches(dm), bwd_block_scan, (unsigned)dm.N, 64, 0, stream, gsum, d_state, d_carry, nblk, 1));
     return launch_chain(chain_launches(dm), bwd_pointwise_rev, pw_grid, kPwThreads, 0, stream, (const float*)g, (float*)dpk, (const float*)gsum,
-                        dm.T, nblk, total_blocks);
+                        dm.T, nblk);
 }
 
 }  // namespace race
