@@ -128,37 +128,57 @@ tile_totals_simt(const Tin* __restrict__ pk, const Tin* __restrict__ v, float* _
 }
 
 // ------------------------------------------------------------------------------------------
-// K2: exclusive scan over tiles, one thread per state float, up to 32 loads in flight.  Bound by the read and the
-// write of the tile states: a batch that is not full is loaded under predicates, all of it before its first use (a
-// loop over the remaining tiles ran one dependent load and store at a time, because the store may alias the next
-// load: 16 tiles of 32 streams at S = 512, d_k = 128, 135 MB of states, took 0.67 ms).
+// K2: exclusive scan over tiles.  Bound by the read and the write of the tile states: a batch that is not full is
+// loaded under predicates, all of it before its first use (a loop over the remaining tiles ran one dependent load and
+// store at a time, because the store may alias the next load: 16 tiles of 32 streams at S = 512, d_k = 128, 135 MB of
+// states, took 0.67 ms).
+// Many tiles: one thread per float, 32 loads in flight.  Up to eight: four floats per thread and one batch of eight;
+// with 32 predicated iterations for two or three tiles the scan was bound by instructions.
 // ------------------------------------------------------------------------------------------
+template <int V> struct ScanVec;
+template <> struct ScanVec<1> { using T = float; };
+template <> struct ScanVec<4> { using T = float4; };
+__device__ __forceinline__ void scan_add(float& a, float b) { a += b; }
+__device__ __forceinline__ void scan_add(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+constexpr int kScanShort = 8;   // tiles
+
+template <int V, int kInFlight>
 __global__ void __launch_bounds__(128)
 tile_scan(float* __restrict__ ws, const float* __restrict__ carry_in, float* __restrict__ state_out,
           int64_t tiles, int state_floats, int write_prefix, int reverse) {
-    constexpr int kInFlight = 32;
+    using Vec = typename ScanVec<V>::T;
     chain_release();
     chain_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) * V;
     if (i >= state_floats) return;
     const int64_t n = blockIdx.y;
-    float run = carry_in ? carry_in[n * state_floats + i] : 0.f;
+    Vec run = carry_in ? *reinterpret_cast<const Vec*>(carry_in + n * state_floats + i) : Vec{};
     // reverse: exclusive SUFFIX sums -- slot t gets carry + the totals of the tiles after t (last tile first)
     float* p = ws + (n * tiles + (reverse ? tiles - 1 : 0)) * state_floats + i;
     const int64_t step = reverse ? -state_floats : state_floats;
-    const int64_t have = state_out ? tiles : tiles - 1;   // without a final state the last tile's totals are not formed
     for (int64_t t = 0; t < tiles; t += kInFlight, p += kInFlight * step) {
         const int cnt = (int)min((int64_t)kInFlight, tiles - t);
-        float x[kInFlight];
+        // without a final state the last tile's totals are not formed
+        const int have = cnt - (!state_out && t + cnt == tiles ? 1 : 0);
+        Vec x[kInFlight];
 #pragma unroll
-        for (int j = 0; j < kInFlight; ++j) x[j] = t + j < have ? p[j * step] : 0.f;
+        for (int j = 0; j < kInFlight; ++j) x[j] = j < have ? *reinterpret_cast<const Vec*>(p + j * step) : Vec{};
 #pragma unroll
         for (int j = 0; j < kInFlight; ++j) {
-            if (write_prefix && j < cnt) p[j * step] = run;
-            run += x[j];
+            if (write_prefix && j < cnt) *reinterpret_cast<Vec*>(p + j * step) = run;
+            scan_add(run, x[j]);
         }
     }
-    if (state_out) state_out[n * state_floats + i] = run;
+    if (state_out) *reinterpret_cast<Vec*>(state_out + n * state_floats + i) = run;
+}
+
+cudaError_t launch_scan(float* ws, const float* carry_in, float* state_out, const Dims& dm, int64_t tiles, int sf,
+                        bool write_prefix, bool reverse, cudaStream_t stream) {
+    const bool vec = tiles <= kScanShort && sf % 4 == 0;
+    const int per_block = vec ? 4 * 128 : 128;
+    return launch_chain(chain_launches(dm), vec ? tile_scan<4, kScanShort> : tile_scan<1, 32>,
+                        dim3((unsigned)((sf + per_block - 1) / per_block), (unsigned)dm.N), 128, 0, stream, ws, carry_in,
+                        state_out, tiles, sf, write_prefix ? 1 : 0, reverse ? 1 : 0);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -417,8 +437,7 @@ cudaError_t launch_simt(const Tin* pq, const Tin* pk, const Tin* v, Tin* out, co
         if (err != cudaSuccess) return err;
     }
 
-    dim3 sgrid((unsigned)((sf + 127) / 128), (unsigned)dm.N);
-    err = launch_chain(chain_launches(dm), tile_scan, sgrid, 128, 0, stream, ws, carry_in, state_out, tiles, sf, totals_only ? 0 : 1, 0);
+    err = launch_scan(ws, carry_in, state_out, dm, tiles, sf, !totals_only, false, stream);
     if (err != cudaSuccess || totals_only || skip_output) return err;
 
     const size_t smem3 = (size_t)(groups > 1 ? Ly::floats_cluster : Ly::floats_single) * sizeof(float);
@@ -468,9 +487,7 @@ cudaError_t causal_scan_tiles(float* ws, const float* carry_in, float* state_out
     const int sf = state_floats_per_stream(dm.S, dm.D);
     if (tiles == 1 && !carry_in && !write_prefix && state_out)   // one tile per stream: its totals are the state
         return ws == state_out ? cudaSuccess : cudaMemcpyAsync(state_out, ws, (size_t)dm.N * sf * sizeof(float), cudaMemcpyDeviceToDevice, stream);
-    dim3 sgrid((unsigned)((sf + 127) / 128), (unsigned)dm.N);
-    return launch_chain(chain_launches(dm), tile_scan, sgrid, 128, 0, stream, ws, carry_in, state_out, tiles, sf, write_prefix ? 1 : 0,
-                        reverse ? 1 : 0);
+    return launch_scan(ws, carry_in, state_out, dm, tiles, sf, write_prefix, reverse, stream);
 }
 
 int simt_groups(int S) { return S <= kGroupBuckets ? 1 : (S + kGroupBuckets - 1) / kGroupBuckets; }
