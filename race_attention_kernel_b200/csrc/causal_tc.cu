@@ -1419,20 +1419,24 @@ int tensor_single_pass_tile_tokens(const Dims& dm, int sm_count) {
     return (int)(tile < C ? C : (tile > 1024 ? 1024 : tile));
 }
 
-int tensor_default_tile_tokens(const Dims& dm, int, int sm_count) {
-    // One CTA per SM at a time: the CTAs run in waves of sm_count, so the tile
-    // length (a multiple of the chunk, at most 2048 tokens) is chosen to fill the last wave:
-    // cost = waves x (tokens per tile + the set-up of a CTA, about one and a half chunks).  For long
-    // sequences this stays at 2048; for shorter ones it avoids a mostly empty last wave.
+int tensor_default_tile_tokens(const Dims& dm, int dtype, int sm_count) {
+    // One CTA per SM at a time: the CTAs of the output pass run in waves of sm_count, so the tile length (a multiple of
+    // the chunk) is chosen to fill the last wave, against the totals pass, which covers every tile but the last of a
+    // stream: cost = waves x (tokens per tile + the set-up of a CTA, about one and a half chunks) + 0.4 x the totals'
+    // tokens per SM (a token costs the totals kernels 0.36 to 0.43 of what it costs the output kernels; they are bound by
+    // memory, not by waves).  So many short streams get one tile each and no totals at all.  At most 2048 tokens in
+    // fp32, where a longer tile would add more terms into one accumulator, and 4096 in bf16.
     // CTAs of the output pass per (stream, tile): slices of the head dimension when there are several bucket groups
     const int64_t groups = dm.S > 128 ? dm.D / 64 : dm.S > 64 ? dm.D / 32 : 1;
     const int64_t sms = sm_count > 0 ? sm_count : 148;
+    const int longest = dtype == RACE_DTYPE_BF16 ? 4096 : 2048;
     int best = 2048;
     double best_cost = 1e300;
-    for (int tile = 2048; tile >= C; tile -= C) {
-        const int64_t ctas = dm.N * groups * ((dm.T + tile - 1) / tile);
+    for (int tile = longest; tile >= C; tile -= C) {
+        const int64_t tiles = (dm.T + tile - 1) / tile, ctas = dm.N * groups * tiles;
         const int64_t waves = (ctas + sms - 1) / sms;
-        const double cost = (double)waves * (tile + 96.0);
+        const int64_t len = std::min<int64_t>(tile, (dm.T + C - 1) / C * C);
+        const double cost = (double)waves * (len + 96.0) + 0.4 * (double)(dm.N * groups * (tiles - 1) * len) / sms;
         if (cost < best_cost * 0.999) { best_cost = cost; best = tile; }
         if (ctas > 64 * sms) break;   // many waves already: shorter tiles only add state traffic
     }
