@@ -1430,17 +1430,23 @@ int tensor_default_tile_tokens(const Dims& dm, int dtype, int sm_count) {
     const int64_t groups = dm.S > 128 ? dm.D / 64 : dm.S > 64 ? dm.D / 32 : 1;
     const int64_t sms = sm_count > 0 ? sm_count : 148;
     const int longest = dtype == RACE_DTYPE_BF16 ? 4096 : 2048;
-    int best = 2048;
-    double best_cost = 1e300;
+    int best = 2048, waves_only = 2048;
+    double best_cost = 1e300, best_waves = 1e300;
     for (int tile = longest; tile >= C; tile -= C) {
         const int64_t tiles = (dm.T + tile - 1) / tile, ctas = dm.N * groups * tiles;
         const int64_t waves = (ctas + sms - 1) / sms;
         const int64_t len = std::min<int64_t>(tile, (dm.T + C - 1) / C * C);
         const double cost = (double)waves * (len + 96.0) + 0.4 * (double)(dm.N * groups * (tiles - 1) * len) / sms;
         if (cost < best_cost * 0.999) { best_cost = cost; best = tile; }
+        if (tile <= 2048 && waves * (tile + 96.0) < best_waves * 0.999) {
+            best_waves = waves * (tile + 96.0);
+            waves_only = tile;
+        }
         if (ctas > 64 * sms) break;   // many waves already: shorter tiles only add state traffic
     }
-    return best;
+    // not shorter than what the waves alone ask for: near a tie the totals' term would take up to 1.7 times the tiles,
+    // and the workspace (bounded in the allocation-free entry) with them, for a part in a thousand of the time
+    return std::max(best, waves_only);
 }
 
 // fp32 single-pass kernel: [totals of every tile | inclusive prefix of every tile | carry slot per CTA | flags, ticket]

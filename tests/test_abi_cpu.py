@@ -107,6 +107,29 @@ def test_workspace_and_tile_selection():
     assert short.value == 32   # a short sequence gets the smallest tile
 
 
+def test_tile_length_leaves_the_workspace_where_the_waves_alone_put_it():
+    """148 SMs: the totals' share in the rule may lengthen a tile, never shorten it (a call that fits the built-in scratch
+    array keeps fitting)."""
+    L = _lib.lib()
+
+    def waves_only(N, T):
+        best, cost = 2048, 1e300
+        for tile in range(2048, 0, -64):
+            ctas = N * -(-T // tile)
+            c = -(-ctas // 148) * (tile + 96.0)
+            if c < cost * 0.999:
+                best, cost = tile, c
+            if ctas > 64 * 148:
+                break
+        return best
+
+    for N, T in [(23, 59823), (15, 56336), (118, 46883), (512, 2000), (96, 4096), (8, 777), (1, 100), (300, 64)]:
+        tile = ctypes.c_int(0)
+        for dtype in (0, 1):
+            assert L.race_b200_select_tile_tokens(ctypes.byref(_shape(N=N, T=T, dtype=dtype)), 2, ctypes.byref(tile)) == 0
+            assert tile.value >= waves_only(N, T)
+
+
 def test_python_binding_rejects_cpu_tensors():
     import torch
 
