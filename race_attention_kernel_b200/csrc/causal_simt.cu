@@ -132,15 +132,16 @@ tile_totals_simt(const Tin* __restrict__ pk, const Tin* __restrict__ v, float* _
 // loaded under predicates, all of it before its first use (a loop over the remaining tiles ran one dependent load and
 // store at a time, because the store may alias the next load: 16 tiles of 32 streams at S = 512, d_k = 128, 135 MB of
 // states, took 0.67 ms).
-// Many tiles: one thread per float, 32 loads in flight.  Up to eight: four floats per thread and one batch of eight;
-// with 32 predicated iterations for two or three tiles the scan was bound by instructions.
+// Many tiles: one thread per float, 32 loads in flight.  Up to 16: four floats per thread, all tiles in one batch; with 32
+// predicated iterations for two or three tiles the scan was bound by instructions.  32 streams at S = 512, d_k = 128:
+// two tiles 23 -> 7 us, 16 tiles 40 -> 28 us; 96 streams at S = 64, d_k = 64, three tiles: 12 -> 3.7 us.
 // ------------------------------------------------------------------------------------------
 template <int V> struct ScanVec;
 template <> struct ScanVec<1> { using T = float; };
 template <> struct ScanVec<4> { using T = float4; };
 __device__ __forceinline__ void scan_add(float& a, float b) { a += b; }
 __device__ __forceinline__ void scan_add(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
-constexpr int kScanShort = 8;   // tiles
+constexpr int kScanShort = 16;   // tiles
 
 template <int V, int kInFlight>
 __global__ void __launch_bounds__(128)

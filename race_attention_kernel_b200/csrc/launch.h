@@ -60,14 +60,15 @@ constexpr int kPhaseTotals = 1, kPhaseOutput = 2, kPhaseAll = 3, kPhasePrefixOnl
 // Whether the output kernel forms the state before each tile itself (CarryFold) instead of a tile_scan launch between
 // the two.  A launch costs 3 to 5 us in the chain of a small call; folding reads every tile's predecessors again, about
 // tiles^2 / 2 states per stream, from lines of L2 that many CTAs ask for at once: fp32 with 8 streams, 13 tiles (777
-// tokens) 17.8 -> 16.1 us, 16 tiles (4096 tokens) 28.4 -> 28.6; hence the line at N tiles^2 = 10 per SM.  One or two
+// tokens) 17.8 -> 16.1 us, 16 tiles (4096 tokens) equal,
+// and bf16 with 8 streams, 16 tiles (1000 tokens) 24.9 -> 22.1; hence the line at N tiles^2 = 14 per SM.  One or two
 // tiles: always less than the scan reads and writes (bf16, 48 streams of three tiles: 100 -> 93 us).
 // A state written over the carry it came from would be read by other tiles' CTAs after the write: scan then.
 inline bool fold_carry(int64_t N, int64_t tiles, int64_t state_floats, const float* carry_in, const float* state_out) {
     if (tiles > 1 && carry_in && state_out && carry_in < state_out + N * state_floats &&
         state_out < carry_in + N * state_floats)
         return false;
-    return tiles <= 2 || (tiles <= 32 && N * tiles * tiles <= 10 * 148);
+    return tiles <= 2 || (tiles <= 32 && N * tiles * tiles <= 14 * 148);
 }
 
 // ---- causal backward (causal_bwd_simt.cu): S <= 64, d_k <= 128 ---------------------------------
