@@ -318,6 +318,18 @@ int race_b200_bucket_probs_streams_bwd(const void* x, const float* planes, const
                                        int32_t n_tables, int32_t n_bits, int32_t dtype, void* stream);
 
 /*
+ * The two calls above for two tensors of one shape (K and Q of an operator call) in one launch, where the geometry has a
+ * kernel that takes two; exact: as race_b200_bucket_probs_streams_exact.
+ */
+int race_b200_bucket_probs_streams_pair(const void* x0, const void* x1, const float* planes, void* probs0, void* probs1,
+                                        int64_t outer, int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables,
+                                        int32_t n_bits, int32_t dtype, int32_t exact, void* stream);
+int race_b200_bucket_probs_streams_bwd_pair(const void* x0, const void* x1, const float* planes, const void* d_probs0,
+                                            const void* d_probs1, void* d_x0, void* d_x1, int64_t outer, int64_t seq_len,
+                                            int32_t heads, int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype,
+                                            void* stream);
+
+/*
  * Host-buffer causal forward: same arithmetic as race_b200_causal_fwd with every tensor in
  * HOST memory (pinned for full copy bandwidth).  Allocates device staging buffers, streams
  * the sequence through them in segments (copy-in, kernel and copy-out overlapped on three

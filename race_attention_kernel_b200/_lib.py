@@ -29,6 +29,7 @@ EXPORTS = [
     "race_b200_causal_bwd_carry", "race_b200_causal_bwd_heads", "race_b200_selftest_bounded_wait", "race_b200_host_release",
     "race_b200_causal_heads_workspace_bytes", "race_b200_causal_fwd_heads", "race_b200_bucket_probs_streams_exact", "race_b200_decode_qkv_is_supported", "race_b200_decode_step_qkv",
     "race_b200_bucket_probs_bwd_is_supported", "race_b200_bucket_probs_streams_bwd",
+    "race_b200_bucket_probs_streams_pair", "race_b200_bucket_probs_streams_bwd_pair",
     "race_b200_qkv_is_supported", "race_b200_causal_fwd_qkv",
 ]
 
@@ -82,6 +83,10 @@ def lib() -> ctypes.CDLL:
     L.race_b200_bucket_probs_streams_exact.argtypes = [vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_bucket_probs_bwd_is_supported.restype = i32
     L.race_b200_bucket_probs_bwd_is_supported.argtypes = [i32, i32, i32, i32]
+    L.race_b200_bucket_probs_streams_pair.restype = i32
+    L.race_b200_bucket_probs_streams_pair.argtypes = [vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, i32, vp]
+    L.race_b200_bucket_probs_streams_bwd_pair.restype = i32
+    L.race_b200_bucket_probs_streams_bwd_pair.argtypes = [vp, vp, vp, vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_bucket_probs_streams_bwd.restype = i32
     L.race_b200_bucket_probs_streams_bwd.argtypes = [vp, vp, vp, vp, i64, i64, i32, i32, i32, i32, i32, vp]
     L.race_b200_causal_fwd_host.restype = i32

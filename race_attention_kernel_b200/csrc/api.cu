@@ -476,7 +476,7 @@ int race_b200_noncausal_bwd(const void* probs_q, const void* probs_k, const void
 namespace {
 int probs_entry(const void* x, const float* planes, void* probs, int64_t outer, int64_t seq_len, int32_t heads,
                 int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype_x, int32_t dtype_probs,
-                void* stream, bool exact = false) {
+                void* stream, bool exact = false, const void* x1 = nullptr, void* probs1 = nullptr) {
     if (outer < 0 || seq_len < 0 || heads < 1 || d_k < 4 || d_k > 256 || (d_k & (d_k - 1)) || n_tables <= 0 ||
         n_bits < 1 || n_bits > 6 || n_tables * n_bits > 64)
         return RACE_ERR_SHAPE;
@@ -486,8 +486,8 @@ int probs_entry(const void* x, const float* planes, void* probs, int64_t outer, 
     const int64_t rows = outer * heads * seq_len;
     if (rows == 0) return RACE_OK;
     if (!x || !planes || !probs) return RACE_ERR_NULL;
-    if (!aligned16(x) || !aligned16(planes) || !aligned16(probs)) return RACE_ERR_ALIGN;
-    return (int)bucket_probs(x, planes, probs, rows, seq_len, heads, d_k, n_tables, n_bits, dtype_x, dtype_probs,
+    if (!aligned16(x) || !aligned16(planes) || !aligned16(probs) || !aligned16(x1) || !aligned16(probs1)) return RACE_ERR_ALIGN;
+    return (int)bucket_probs(x, x1, planes, probs, probs1, rows, seq_len, heads, d_k, n_tables, n_bits, dtype_x, dtype_probs,
                              (cudaStream_t)stream, exact);
 }
 }  // namespace
@@ -511,21 +511,47 @@ int race_b200_bucket_probs_streams_exact(const void* x, const float* planes, voi
     return probs_entry(x, planes, probs, outer, seq_len, heads, d_k, n_tables, n_bits, dtype, dtype, stream, true);
 }
 
+int race_b200_bucket_probs_streams_pair(const void* x0, const void* x1, const float* planes, void* probs0, void* probs1,
+                                        int64_t outer, int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables,
+                                        int32_t n_bits, int32_t dtype, int32_t exact, void* stream) {
+    if (outer > 0 && heads > 0 && seq_len > 0 && (!x1 || !probs1)) return RACE_ERR_NULL;
+    return probs_entry(x0, planes, probs0, outer, seq_len, heads, d_k, n_tables, n_bits, dtype, dtype, stream, exact != 0, x1,
+                       probs1);
+}
+
 int race_b200_bucket_probs_bwd_is_supported(int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype) {
     return bucket_probs_bwd_supported(d_k, n_tables, n_bits, dtype) ? 1 : 0;
+}
+
+static int probs_bwd_entry(const void* x, const void* x1, const float* planes, const void* d_probs, const void* d_probs1,
+                           void* d_x, void* d_x1, int64_t outer, int64_t seq_len, int32_t heads, int32_t d_k,
+                           int32_t n_tables, int32_t n_bits, int32_t dtype, void* stream) {
+    if (outer < 0 || seq_len < 0 || heads < 1 || !bucket_probs_bwd_supported(d_k, n_tables, n_bits, dtype))
+        return RACE_ERR_SHAPE;
+    const int64_t rows = outer * heads * seq_len;
+    if (rows == 0) return RACE_OK;
+    if (!x || !planes || !d_probs || !d_x || (x1 && (!d_probs1 || !d_x1))) return RACE_ERR_NULL;
+    if (!aligned16(x) || !aligned16(planes) || !aligned16(d_probs) || !aligned16(d_x) || !aligned16(x1) ||
+        !aligned16(d_probs1) || !aligned16(d_x1))
+        return RACE_ERR_ALIGN;
+    return (int)bucket_probs_bwd(x, x1, planes, d_probs, d_probs1, d_x, d_x1, rows, seq_len, heads, d_k, n_tables, n_bits, dtype,
+                                 (cudaStream_t)stream);
 }
 
 int race_b200_bucket_probs_streams_bwd(const void* x, const float* planes, const void* d_probs, void* d_x, int64_t outer,
                                        int64_t seq_len, int32_t heads, int32_t d_k, int32_t n_tables, int32_t n_bits,
                                        int32_t dtype, void* stream) {
-    if (outer < 0 || seq_len < 0 || heads < 1 || !bucket_probs_bwd_supported(d_k, n_tables, n_bits, dtype))
-        return RACE_ERR_SHAPE;
-    const int64_t rows = outer * heads * seq_len;
-    if (rows == 0) return RACE_OK;
-    if (!x || !planes || !d_probs || !d_x) return RACE_ERR_NULL;
-    if (!aligned16(x) || !aligned16(planes) || !aligned16(d_probs) || !aligned16(d_x)) return RACE_ERR_ALIGN;
-    return (int)bucket_probs_bwd(x, planes, d_probs, d_x, rows, seq_len, heads, d_k, n_tables, n_bits, dtype,
-                                 (cudaStream_t)stream);
+    return probs_bwd_entry(x, nullptr, planes, d_probs, nullptr, d_x, nullptr, outer, seq_len, heads, d_k, n_tables, n_bits,
+                           dtype, stream);
+}
+
+int race_b200_bucket_probs_streams_bwd_pair(const void* x0, const void* x1, const float* planes, const void* d_probs0,
+                                            const void* d_probs1, void* d_x0, void* d_x1, int64_t outer, int64_t seq_len,
+                                            int32_t heads, int32_t d_k, int32_t n_tables, int32_t n_bits, int32_t dtype,
+                                            void* stream) {
+    if (outer > 0 && heads > 0 && seq_len > 0 && !x1) return RACE_ERR_NULL;
+    return probs_bwd_entry(x0, x1, planes, d_probs0, d_probs1, d_x0, d_x1, outer, seq_len, heads, d_k, n_tables, n_bits, dtype,
+                           stream);
 }
 
 }  // extern "C"

@@ -289,8 +289,10 @@ __device__ __forceinline__ void pack8(const float* v, uint4& w) {
 // of a training step: the gradients of the probabilities nearly cancel over a table, which magnifies the 2^-17 of two.
 template <int D, int L, int K, typename Tx, typename Tp, bool kExact>
 __global__ void __launch_bounds__(kWideThreads, (sizeof(Tx) == 4 && D > 64 ? 3 : 4))
-bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes, Tp* __restrict__ probs,
-                      int64_t rows, int64_t T, int heads) {
+bucket_probs_mma_wide(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const float* __restrict__ planes,
+                      Tp* __restrict__ probs0, Tp* __restrict__ probs1, int64_t rows, int64_t T, int heads) {
+    const Tx* __restrict__ x = blockIdx.y ? x1 : x0;   // two tensors (K and Q): one launch, the halves of its grid
+    Tp* __restrict__ probs = blockIdx.y ? probs1 : probs0;
     using W = WideProbs<D, L, K>;
     constexpr int NT = W::NT, NJ = W::NJ, R = W::R, TPL = W::TPL;
     constexpr bool kX32 = sizeof(Tx) == 4;
@@ -489,19 +491,27 @@ bucket_probs_mma_wide(const Tx* __restrict__ x, const float* __restrict__ planes
     }
 }
 
+// x1, probs1: null, or a second tensor of the same shape
 template <int D, int L, int K, typename Tx, typename Tp, bool kExact = false>
-cudaError_t launch_probs_wide(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
-                              cudaStream_t stream) {
+cudaError_t launch_probs_wide(const void* x, const void* x1, const float* planes, void* probs, void* probs1, int64_t rows,
+                              int64_t T, int heads, cudaStream_t stream) {
     auto kern = bucket_probs_mma_wide<D, L, K, Tx, Tp, kExact>;
     constexpr int smem = WideProbs<D, L, K>::kTabBytes + (kExact ? WideProbs<D, L, K>::kTabBytes / 2 : 0) +
                          ((int)sizeof(Tp) << K < 128 ? 0 : (kWideThreads / 32) * WideProbs<D, L, K>::kStageBytes);
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return err;
-    int dev = 0, sms = 148;
+    int dev = 0, sms = 148, per_sm = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWideThreads, smem);
+    if (err != cudaSuccess) return err;
     const int64_t want = (rows + 63) / 64;   // 64 rows per CTA and pass
-    const unsigned blocks = (unsigned)std::min<int64_t>(want, (int64_t)(sms > 0 ? sms : 148) * 12);
-    return launch_chain(chain_launches(rows, L << K), kern, blocks, kWideThreads, smem, stream, (const Tx*)x, planes, (Tp*)probs, rows, T, heads);
+    // The CTAs that are resident together walk the rows: each builds the plane tables once (twelve per SM built them up to
+    // three times over).  K and Q in one launch share its tail.  bf16, two tensors: d_k = 128, 131072 rows 101 -> 79 us;
+    // d_k = 64, 393216 rows 47 -> 41 us.
+    const int64_t resident = (int64_t)std::max(sms, 1) * std::max(per_sm, 1) / (x1 ? 2 : 1);
+    const dim3 grid((unsigned)std::min<int64_t>(want, std::max<int64_t>(resident, 1)), x1 ? 2 : 1);
+    return launch_chain(chain_launches(rows, L << K), kern, grid, kWideThreads, smem, stream, (const Tx*)x, (const Tx*)x1, planes,
+                        (Tp*)probs, (Tp*)probs1, rows, T, heads);
 }
 
 template <typename Tx, typename Tp, int K>
@@ -545,13 +555,32 @@ cudaError_t launch_probs(const void* x, const float* planes, void* probs, int64_
 
 }  // namespace
 
-cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
-                         int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream, bool exact) {
+cudaError_t bucket_probs(const void* x, const void* x1, const float* planes, void* probs, void* probs1, int64_t rows,
+                         int64_t T, int heads, int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream, bool exact) {
     if (exact && dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32) {
         if (d == 64 && L == 4 && K == 4)
-            return launch_probs_wide<64, 4, 4, float, float, true>(x, planes, probs, rows, T, heads, stream);
+            return launch_probs_wide<64, 4, 4, float, float, true>(x, x1, planes, probs, probs1, rows, T, heads, stream);
         if (d == 128 && L == 8 && K == 6)
-            return launch_probs_wide<128, 8, 6, float, float, true>(x, planes, probs, rows, T, heads, stream);
+            return launch_probs_wide<128, 8, 6, float, float, true>(x, x1, planes, probs, probs1, rows, T, heads, stream);
+    }
+    // the small geometry with bf16 rows: its tables need no staging (48 streams of 5003 tokens: 51 us on the general
+    // kernel, which runs sixteen dot products per row on the CUDA cores)
+    if (d == 64 && L == 4 && K == 4 && dtype_x == RACE_DTYPE_BF16 && dtype_probs == RACE_DTYPE_BF16)
+        return launch_probs_wide<64, 4, 4, __nv_bfloat16, __nv_bfloat16>(x, x1, planes, probs, probs1, rows, T, heads, stream);
+    if (d == 128 && L == 8 && K == 6) {
+        if (dtype_x == RACE_DTYPE_BF16 && dtype_probs == RACE_DTYPE_BF16)
+            return launch_probs_wide<128, 8, 6, __nv_bfloat16, __nv_bfloat16>(x, x1, planes, probs, probs1, rows, T, heads, stream);
+        if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32)
+            return launch_probs_wide<128, 8, 6, float, float>(x, x1, planes, probs, probs1, rows, T, heads, stream);
+        if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_BF16)
+            return launch_probs_wide<128, 8, 6, float, __nv_bfloat16>(x, x1, planes, probs, probs1, rows, T, heads, stream);
+        if (dtype_x == RACE_DTYPE_BF16 && dtype_probs == RACE_DTYPE_F32)
+            return launch_probs_wide<128, 8, 6, __nv_bfloat16, float>(x, x1, planes, probs, probs1, rows, T, heads, stream);
+    }
+    if (x1) {   // the kernels below take one tensor
+        const cudaError_t err = bucket_probs(x1, nullptr, planes, probs1, nullptr, rows, T, heads, d, L, K, dtype_x, dtype_probs,
+                                             stream, exact);
+        if (err != cudaSuccess) return err;
     }
     if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32 && d == 64 && L == 4 && K == 4) {
         int dev = 0, sms = 148;
@@ -560,20 +589,6 @@ cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_
         const unsigned blocks = (unsigned)std::min<int64_t>(want, (int64_t)(sms > 0 ? sms : 148) * 16);
         return launch_chain(chain_launches(rows, 64), bucket_probs_mma_d64_l4k4, blocks, kFastThreads, 0, stream, (const float*)x, planes, (float*)probs,
                             rows, T, heads);
-    }
-    // the small geometry with bf16 rows: its tables need no staging (48 streams of 5003 tokens: 51 us on the general
-    // kernel, which runs sixteen dot products per row on the CUDA cores)
-    if (d == 64 && L == 4 && K == 4 && dtype_x == RACE_DTYPE_BF16 && dtype_probs == RACE_DTYPE_BF16)
-        return launch_probs_wide<64, 4, 4, __nv_bfloat16, __nv_bfloat16>(x, planes, probs, rows, T, heads, stream);
-    if (d == 128 && L == 8 && K == 6) {
-        if (dtype_x == RACE_DTYPE_BF16 && dtype_probs == RACE_DTYPE_BF16)
-            return launch_probs_wide<128, 8, 6, __nv_bfloat16, __nv_bfloat16>(x, planes, probs, rows, T, heads, stream);
-        if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32)
-            return launch_probs_wide<128, 8, 6, float, float>(x, planes, probs, rows, T, heads, stream);
-        if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_BF16)
-            return launch_probs_wide<128, 8, 6, float, __nv_bfloat16>(x, planes, probs, rows, T, heads, stream);
-        if (dtype_x == RACE_DTYPE_BF16 && dtype_probs == RACE_DTYPE_F32)
-            return launch_probs_wide<128, 8, 6, __nv_bfloat16, float>(x, planes, probs, rows, T, heads, stream);
     }
     if (dtype_x == RACE_DTYPE_F32 && dtype_probs == RACE_DTYPE_F32)
         return launch_probs<float, float>(x, planes, probs, rows, T, heads, d, L, K, stream);

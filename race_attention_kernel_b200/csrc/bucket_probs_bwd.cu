@@ -63,8 +63,12 @@ __device__ __forceinline__ void load_dp(const __nv_bfloat16* p, float (&v)[R]) {
 
 template <int D, int L, int K, typename Tx, typename Tp>
 __global__ void __launch_bounds__(kBwdThreads, BwdProbs<D, L, K>::kCtas)
-bucket_probs_bwd_mma(const Tx* __restrict__ x, const float* __restrict__ planes, const Tp* __restrict__ dprobs,
-                     Tx* __restrict__ dx, int64_t rows, int64_t T, int heads) {
+bucket_probs_bwd_mma(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const float* __restrict__ planes,
+                     const Tp* __restrict__ dprobs0, const Tp* __restrict__ dprobs1, Tx* __restrict__ dx0,
+                     Tx* __restrict__ dx1, int64_t rows, int64_t T, int heads) {
+    const Tx* __restrict__ x = blockIdx.y ? x1 : x0;   // two tensors (K and Q): one launch, the halves of its grid
+    const Tp* __restrict__ dprobs = blockIdx.y ? dprobs1 : dprobs0;
+    Tx* __restrict__ dx = blockIdx.y ? dx1 : dx0;
     using W = BwdProbs<D, L, K>;
     constexpr int NT = W::NT, NJ = W::NJ, R = W::R, TPL = W::TPL, KS = W::KS;
     constexpr bool kX32 = sizeof(Tx) == 4;
@@ -263,8 +267,8 @@ bucket_probs_bwd_mma(const Tx* __restrict__ x, const float* __restrict__ planes,
 }
 
 template <int D, int L, int K, typename Tx, typename Tp>
-cudaError_t launch_probs_bwd(const void* x, const float* planes, const void* dprobs, void* dx, int64_t rows, int64_t T,
-                             int heads, cudaStream_t stream) {
+cudaError_t launch_probs_bwd(const void* x, const void* x1, const float* planes, const void* dprobs, const void* dprobs1,
+                             void* dx, void* dx1, int64_t rows, int64_t T, int heads, cudaStream_t stream) {
     auto kern = bucket_probs_bwd_mma<D, L, K, Tx, Tp>;
     constexpr int smem = BwdProbs<D, L, K>::smem_bytes(sizeof(Tx) == 4);
     cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -272,9 +276,10 @@ cudaError_t launch_probs_bwd(const void* x, const float* planes, const void* dpr
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // the plane tables are built once per CTA: the resident CTAs walk the rows
-    const unsigned blocks = (unsigned)std::min<int64_t>((rows + 63) / 64, (int64_t)(sms > 0 ? sms : 148) * BwdProbs<D, L, K>::kCtas);
-    return launch_chain(chain_launches(rows, L << K), kern, blocks, kBwdThreads, smem, stream, (const Tx*)x, planes, (const Tp*)dprobs, (Tx*)dx, rows, T,
-                        heads);
+    const int64_t resident = (int64_t)(sms > 0 ? sms : 148) * BwdProbs<D, L, K>::kCtas / (x1 ? 2 : 1);
+    const dim3 grid((unsigned)std::min<int64_t>((rows + 63) / 64, std::max<int64_t>(resident, 1)), x1 ? 2 : 1);
+    return launch_chain(chain_launches(rows, L << K), kern, grid, kBwdThreads, smem, stream, (const Tx*)x, (const Tx*)x1, planes,
+                        (const Tp*)dprobs, (const Tp*)dprobs1, (Tx*)dx, (Tx*)dx1, rows, T, heads);
 }
 
 }  // namespace
@@ -284,17 +289,18 @@ bool bucket_probs_bwd_supported(int d, int L, int K, int dtype) {
            ((d == 64 && L == 4 && K == 4) || (d == 128 && L == 8 && K == 6));
 }
 
-cudaError_t bucket_probs_bwd(const void* x, const float* planes, const void* dprobs, void* dx, int64_t rows, int64_t T,
-                             int heads, int d, int L, int K, int dtype, cudaStream_t stream) {
+cudaError_t bucket_probs_bwd(const void* x, const void* x1, const float* planes, const void* dprobs, const void* dprobs1,
+                             void* dx, void* dx1, int64_t rows, int64_t T, int heads, int d, int L, int K, int dtype,
+                             cudaStream_t stream) {
     if (!bucket_probs_bwd_supported(d, L, K, dtype)) return cudaErrorInvalidValue;
     using b16 = __nv_bfloat16;
     if (d == 64)
         return dtype == RACE_DTYPE_F32
-                   ? launch_probs_bwd<64, 4, 4, float, float>(x, planes, dprobs, dx, rows, T, heads, stream)
-                   : launch_probs_bwd<64, 4, 4, b16, b16>(x, planes, dprobs, dx, rows, T, heads, stream);
+                   ? launch_probs_bwd<64, 4, 4, float, float>(x, x1, planes, dprobs, dprobs1, dx, dx1, rows, T, heads, stream)
+                   : launch_probs_bwd<64, 4, 4, b16, b16>(x, x1, planes, dprobs, dprobs1, dx, dx1, rows, T, heads, stream);
     return dtype == RACE_DTYPE_F32
-               ? launch_probs_bwd<128, 8, 6, float, float>(x, planes, dprobs, dx, rows, T, heads, stream)
-               : launch_probs_bwd<128, 8, 6, b16, b16>(x, planes, dprobs, dx, rows, T, heads, stream);
+               ? launch_probs_bwd<128, 8, 6, float, float>(x, x1, planes, dprobs, dprobs1, dx, dx1, rows, T, heads, stream)
+               : launch_probs_bwd<128, 8, 6, b16, b16>(x, x1, planes, dprobs, dprobs1, dx, dx1, rows, T, heads, stream);
 }
 
 }  // namespace race

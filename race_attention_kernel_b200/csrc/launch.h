@@ -102,13 +102,15 @@ cudaError_t noncausal_token_grads_tensor(const void* pk, const void* v, const vo
 // ---- bucket-probability producer (bucket_probs.cu) --------------------------------------------
 // exact: fp32 accuracy of the projections (training) at the tensor-core geometries
 // x [outer, T, heads, d] -> probs [outer*heads, T, L, 2^K]; rows = outer*heads*T (heads = 1: plain rows)
-cudaError_t bucket_probs(const void* x, const float* planes, void* probs, int64_t rows, int64_t T, int heads,
-                         int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream, bool exact = false);
+// x1, probs1: null, or a second tensor of the same shape, in the same launch where the geometry's kernel takes two
+cudaError_t bucket_probs(const void* x, const void* x1, const float* planes, void* probs, void* probs1, int64_t rows,
+                         int64_t T, int heads, int d, int L, int K, int dtype_x, int dtype_probs, cudaStream_t stream, bool exact = false);
 
 // dx of the same (bucket_probs_bwd.cu): dprobs [outer*heads, T, L, 2^K] and x, dx [outer, T, heads, d], one type
 bool bucket_probs_bwd_supported(int d, int L, int K, int dtype);
-cudaError_t bucket_probs_bwd(const void* x, const float* planes, const void* dprobs, void* dx, int64_t rows, int64_t T,
-                             int heads, int d, int L, int K, int dtype, cudaStream_t stream);
+cudaError_t bucket_probs_bwd(const void* x, const void* x1, const float* planes, const void* dprobs, const void* dprobs1,
+                             void* dx, void* dx1, int64_t rows, int64_t T, int heads, int d, int L, int K, int dtype,
+                             cudaStream_t stream);
 
 // ---- incremental step (decode.cu) -------------------------------------------------------------
 // a few new tokens per stream (dm.T <= decode_max_tokens()) against a running state; state_in may be

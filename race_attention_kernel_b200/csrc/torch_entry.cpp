@@ -146,12 +146,10 @@ PyObject* forward_impl(PyObject* const* args, Py_ssize_t nargs) {
               "race_b200_causal_fwd_qkv");
     } else {
         at::Tensor pk = at::empty({N, T, L, R}, k->options()), pq = at::empty({N, T, L, R}, k->options());
-        const at::Tensor* src[2] = {k, q};
-        at::Tensor* dst[2] = {&pk, &pq};
-        for (int i = 0; i < 2; ++i)
-            check(race_b200_bucket_probs_streams(src[i]->const_data_ptr(), planes.const_data_ptr<float>(), dst[i]->data_ptr(), MB, T,
-                                                 (int32_t)H, (int32_t)dk, (int32_t)L, (int32_t)P, sh.dtype, sh.dtype, stream),
-                  "race_b200_bucket_probs_streams");
+        check(race_b200_bucket_probs_streams_pair(k->const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
+                                                  pk.data_ptr(), pq.data_ptr(), MB, T, (int32_t)H, (int32_t)dk, (int32_t)L,
+                                                  (int32_t)P, sh.dtype, 0, stream),
+              "race_b200_bucket_probs_streams_pair");
         check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), v->const_data_ptr(), out.data_ptr(), carry_p,
                                          state_p, ws.data_ptr(), wb, &sh, stream, status),
               "race_b200_causal_fwd_heads");
@@ -203,13 +201,10 @@ struct TrainOp : torch::autograd::Function<TrainOp> {
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
         const RaceShape sh = shape(k, L, P, eps);
         at::Tensor pk = at::empty({sh.n_streams, sh.seq_len, L, 1ll << P}, k.options()), pq = at::empty_like(pk);
-        const at::Tensor* src[2] = {&k, &q};
-        at::Tensor* dst[2] = {&pk, &pq};
-        for (int i = 0; i < 2; ++i)
-            check(race_b200_bucket_probs_streams_exact(src[i]->const_data_ptr(), planes.const_data_ptr<float>(), dst[i]->data_ptr(),
-                                                       k.size(0) * k.size(1), sh.seq_len, sh.heads, sh.head_dim, (int32_t)L,
-                                                       (int32_t)P, sh.dtype, stream),
-                  "race_b200_bucket_probs_streams_exact");
+        check(race_b200_bucket_probs_streams_pair(k.const_data_ptr(), q.const_data_ptr(), planes.const_data_ptr<float>(),
+                                                  pk.data_ptr(), pq.data_ptr(), k.size(0) * k.size(1), sh.seq_len, sh.heads,
+                                                  sh.head_dim, (int32_t)L, (int32_t)P, sh.dtype, 1, stream),
+              "race_b200_bucket_probs_streams_pair");
         at::Tensor out = at::empty(v.sizes(), v.options());
         const size_t wb = race_b200_causal_heads_workspace_bytes(&sh);
         at::Tensor ws = bytes(wb, k);
@@ -243,16 +238,24 @@ struct TrainOp : torch::autograd::Function<TrainOp> {
                                              nullptr, dpq.data_ptr(), dpk.data_ptr(), dv.data_ptr(), nullptr, ws.data_ptr(), wb,
                                              &sh, stream, status),
                   "race_b200_causal_bwd_heads");
+            const int64_t MB = k.size(0) * k.size(1);
             const at::Tensor* x[2] = {&k, &q};
             const at::Tensor* dp[2] = {&dpk, &dpq};
-            for (int i = 0; i < 2; ++i) {
-                if (!ctx->needs_input_grad(i ? 2 : 0)) continue;
-                at::Tensor dx = at::empty(x[i]->sizes(), x[i]->options());
-                check(race_b200_bucket_probs_streams_bwd(x[i]->const_data_ptr(), planes.const_data_ptr<float>(), dp[i]->const_data_ptr(),
-                                                         dx.data_ptr(), k.size(0) * k.size(1), sh.seq_len, sh.heads, sh.head_dim,
-                                                         (int32_t)L, (int32_t)P, sh.dtype, stream),
-                      "race_b200_bucket_probs_streams_bwd");
-                res[i ? 2 : 0] = dx;
+            for (int i = 0; i < 2; ++i)
+                if (ctx->needs_input_grad(i ? 2 : 0)) res[i ? 2 : 0] = at::empty(x[i]->sizes(), x[i]->options());
+            if (res[0].defined() && res[2].defined()) {
+                check(race_b200_bucket_probs_streams_bwd_pair(k.const_data_ptr(), q.const_data_ptr(), planes.const_data_ptr<float>(),
+                                                              dpk.const_data_ptr(), dpq.const_data_ptr(), res[0].data_ptr(),
+                                                              res[2].data_ptr(), MB, sh.seq_len, sh.heads, sh.head_dim,
+                                                              (int32_t)L, (int32_t)P, sh.dtype, stream),
+                      "race_b200_bucket_probs_streams_bwd_pair");
+            } else {
+                for (int i = 0; i < 2; ++i)
+                    if (res[i ? 2 : 0].defined())
+                        check(race_b200_bucket_probs_streams_bwd(x[i]->const_data_ptr(), planes.const_data_ptr<float>(),
+                                                                 dp[i]->const_data_ptr(), res[i ? 2 : 0].data_ptr(), MB, sh.seq_len,
+                                                                 sh.heads, sh.head_dim, (int32_t)L, (int32_t)P, sh.dtype, stream),
+                              "race_b200_bucket_probs_streams_bwd");
             }
             if (ctx->needs_input_grad(1)) res[1] = dv;
             raise_on_wait(status, "BatchedACE backward");

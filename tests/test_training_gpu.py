@@ -44,6 +44,32 @@ def test_producer_backward(dk, K, L, dt, B, T, H):
     assert ro.rel_l2(got, ref) <= (2e-5 if dt == torch.float32 else 4e-3)
 
 
+@pytest.mark.parametrize("dk,K,L,dt", GEOMETRIES + [(128, 6, 8, torch.float32), (32, 3, 4, torch.float32)])
+@pytest.mark.parametrize("B,T,H", [(1, 1, 1), (2, 37, 3), (3, 1003, 16)])
+def test_two_tensors_in_one_launch(dk, K, L, dt, B, T, H):
+    """The pair entries give the bits of the single ones (the last geometry has no kernel for two tensors)."""
+    import race_attention_kernel_b200.ops as ops
+    from race_attention_kernel_b200 import _lib
+    g = torch.Generator(device="cuda").manual_seed(T + dk)
+    x = [torch.randn(1, B, T, H, dk, device="cuda", generator=g).to(dt) for _ in range(2)]
+    planes = torch.randn(L * K, dk, device="cuda", generator=g)
+    dims = (B, T, H, dk, L, K, ops._DTYPES[dt])
+    for exact in (0, 1):
+        p = [torch.empty(B * H, T, L, 1 << K, device="cuda", dtype=dt) for _ in range(2)]
+        assert _lib.lib().race_b200_bucket_probs_streams_pair(
+            *map(ops._ptr, x), ops._ptr(planes), *map(ops._ptr, p), *dims, exact, ops._stream()) == 0
+        for a, b in zip(x, p):
+            assert torch.equal(b, ops.bucket_probs_streams(a, planes, L, K, exact=bool(exact)))
+    if not ops.bucket_probs_bwd_is_supported(dk, L, K, dt):
+        return
+    dp = [torch.randn_like(t) for t in p]
+    dx = [torch.empty_like(t) for t in x]
+    assert _lib.lib().race_b200_bucket_probs_streams_bwd_pair(
+        *map(ops._ptr, x), ops._ptr(planes), *map(ops._ptr, dp), *map(ops._ptr, dx), *dims, ops._stream()) == 0
+    for a, b, c in zip(x, dp, dx):
+        assert torch.equal(c, ops.bucket_probs_streams_bwd(a, planes, b, L, K))
+
+
 @pytest.mark.parametrize("dk,K,L,dt", GEOMETRIES)
 @pytest.mark.parametrize("B,T,H", [(1, 1, 2), (2, 127, 3), (1, 128, 2), (1, 129, 1), (1, 2500, 2)])
 def test_operator_gradients(dk, K, L, dt, B, T, H):
