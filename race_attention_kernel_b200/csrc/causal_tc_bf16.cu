@@ -1946,7 +1946,7 @@ cudaError_t launch_bf16(const void* pq, const void* pk, const void* v, void* out
                         int* status, int phases, bool global_norm) {
     const int G = dm.S / SG;
     if (global_norm && G > 1) return cudaErrorInvalidValue;   // the one-group kernel has the global form
-    if (dm.H > 1 && G == 2 && phases != kPhaseTotals) return cudaErrorInvalidValue;   // its output kernel takes [N, T, D]
+    if (dm.H > 1 && G == 2 && (phases & kPhaseOutput)) return cudaErrorInvalidValue;   // its output kernel takes [N, T, D]
     // two bucket groups per totals CTA where there are at least two (they share the V tile)
     const int GP = G >= 2 ? 2 : 1;
     auto k1 = GP == 2 ? tile_totals_tc_bf16<D, 2> : tile_totals_tc_bf16<D, 1>;

@@ -1,0 +1,33 @@
+"""The bf16 causal backward at every geometry race_b200_causal_bwd_heads grants (S = 64, 128, 256, 512; d_k = 64, 128)."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+GEOMETRIES = [(L, R, dk) for L, R in ((4, 16), (2, 64), (4, 64), (8, 64)) for dk in (64, 128)]
+
+
+def _inputs(N, T, L, R, dk, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    pq, pk = (torch.softmax(torch.randn(N, T, L, R, device="cuda", generator=g), -1).bfloat16() for _ in range(2))
+    v, dO = (torch.randn(N, T, dk, device="cuda", generator=g).bfloat16() for _ in range(2))
+    return pq, pk, v, dO
+
+
+@pytest.mark.parametrize("L,R,dk", GEOMETRIES)
+@pytest.mark.parametrize("B,H,T", [(1, 2, 300), (2, 3, 129)])
+def test_operator_layout_has_the_bits_of_the_flat_one(L, R, dk, B, H, T):
+    import race_attention_kernel_b200.ops as ops
+    N = B * H
+    pq, pk, v, dO = _inputs(N, T, L, R, dk, seed=T + dk)
+    assert ops.causal_bwd_takes_heads(N, T, L, R, dk, torch.bfloat16, H)
+
+    def operator_layout(x):
+        return x.view(1, B, H, T, dk).permute(0, 1, 3, 2, 4).contiguous()
+
+    flat = ops.race_causal_backward(pq, pk, v, dO)
+    heads = ops.race_causal_backward(pq, pk, operator_layout(v), operator_layout(dO))
+    assert torch.equal(heads[0], flat[0]) and torch.equal(heads[1], flat[1])
+    assert torch.equal(heads[2], operator_layout(flat[2]))
