@@ -784,8 +784,6 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
         out_phase_init_bars(cx, false, kWorkerK ? 8u : 4u);
     }
     uint32_t* ptab = reinterpret_cast<uint32_t*>(cx.sm + oPlaneTab);
-    // (ahead of chain_wait: the planes are never the result of a chained launch)
-    if (kProj) build_plane_tab(planes, ptab, tid, kThreads);
     if (warp == kMmaWarp) tmem_alloc(cx.sm_u32 + oMisc, kTmemCols);
     fence_proxy_async();
     tc_fence_before();
@@ -793,9 +791,12 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     chain_wait();
-    // the prefix lands in the second state operand buffer, which the converter group writes first after chunk 0, and
-    // the TMA and MMA warps are ahead with chunk 0 meanwhile
+    // What the worker and converter warps start from, while the TMA warp is ahead with chunk 0.  The plane table is built
+    // by the two MMA warps, which have nothing to do yet, beside the prefix (built by all warps before that, it put its
+    // load latency in front of everything: 8 streams of 4096 tokens 28.7 -> 30.4 us).  The prefix lands in the second
+    // state operand buffer, which the converter group writes first after chunk 0.
     float* carry_smem = cf.fold ? reinterpret_cast<float*>(cx.sm + oBt + 2 * kOpTile) : nullptr;
+    if (kProj && warp > kProducerWarp) build_plane_tab(planes, ptab, tid - kMmaWarp * 32, 64);
     if (cf.fold && warp < 12) {
         static_assert(S * D * 4 == 2 * kOpTile, "the carry fills one state operand buffer");
         const bool last = kReverse ? tile == 0 : tile == tiles - 1;
@@ -803,6 +804,10 @@ causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap 
                              (int)(kReverse ? tiles - 1 - tile : tile), cf.carry_in ? cf.carry_in + n * kSF : nullptr,
                              last && cf.state_out ? cf.state_out + n * kSF : nullptr, carry_smem,
                              reinterpret_cast<float*>(cx.sm + oAcar), S * D, kSF, tid);
+    }
+    if (kProj) {
+        if (warp != kProducerWarp) asm volatile("bar.sync 1, 448;" ::: "memory");
+    } else if (cf.fold && warp < 12) {
         asm volatile("bar.sync 1, 384;" ::: "memory");
     }
     out_phase<kMode, kReverse, kProj, kWorkerK>(cx, tmem, pq, &map_k, &map_v, out, slice, T, t_begin, t_end, n, eps,
@@ -1129,13 +1134,16 @@ tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         totals_phase_init_bars<TL>(cx, false);
     }
     uint32_t* ptab = reinterpret_cast<uint32_t*>(cx.sm + TL::oPlaneTab);
-    if (kProj) build_plane_tab(planes, ptab, tid, TL::kThreads);
     if (warp == TL::kMmaWarp) tmem_alloc(cx.sm_u32 + TL::oMisc, 64u);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     chain_wait();
+    if (kProj && warp < 4 * TL::kGroups) {   // the converter warps, while the first copies are on their way
+        build_plane_tab(planes, ptab, tid, 128 * TL::kGroups);
+        asm volatile("bar.sync 1, %0;" ::"n"(128 * TL::kGroups) : "memory");
+    }
     totals_phase<kProj, TL>(cx, tmem, &map_k, &map_v, slice, t_begin, t_end, n, hd, false, ptab);
     tc_fence_before();
     __syncthreads();
