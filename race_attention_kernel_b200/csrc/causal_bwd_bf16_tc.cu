@@ -104,6 +104,7 @@ struct Args {
     int64_t T;
     int S, heads, tile_tokens;
     float eps;
+    bool sectors;            // dp and a bf16 dv begin on a 32-byte boundary
     int* status;
 };
 
@@ -298,15 +299,23 @@ __device__ __forceinline__ void write_tri(uint32_t tm_lane, int row, int wg) {
     tmem_st_words32(tm_lane + tG + 32 * wg, tr);
     tc_fence_before();
 }
+// fp32 rows lie in the workspace (256-byte aligned): 32-byte stores.  bf16 rows lie in the caller's tensors, which only
+// promise 16 bytes: a sector at a time where they happen to begin on one (sectors), else in two halves (96 streams of 4096
+// tokens, S = 64, d_k = 64, a training step: 508 us against 520).
 __device__ __forceinline__ void store_row16(float* dst, const float (&v)[16]) {
     st_global_32b(dst, reinterpret_cast<const uint32_t(&)[8]>(v[0]));
     st_global_32b(dst + 8, reinterpret_cast<const uint32_t(&)[8]>(v[8]));
 }
-__device__ __forceinline__ void store_row16(__nv_bfloat16* dst, const float (&v)[16]) {
+__device__ __forceinline__ void store_row16(__nv_bfloat16* dst, const float (&v)[16], bool sectors) {
     uint32_t d[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) d[i] = pack2(v[2 * i], v[2 * i + 1]);
-    st_global_32b(dst, d);
+    if (sectors) {
+        st_global_32b(dst, d);
+    } else {
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(d[0], d[1], d[2], d[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(d[4], d[5], d[6], d[7]);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -396,7 +405,7 @@ bwd_prefix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
                 tmem_ld_rows16(tm_lane + tX + col0 + cb, v);
 #pragma unroll
                 for (int i = 0; i < 16; ++i) inv[cb + i] = v[i] *= inv[cb + i];
-                if (live) store_row16(dst + cb, v);
+                if (live) store_row16(dst + cb, v, a.sectors);
             }
             if (!(ok = wait_bar_warp(cx, bH, ph, 107))) break;    // the totals have read W
             RACE_TRACE(wg, c, 4);
@@ -642,7 +651,7 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
                     if (row == 0) *reinterpret_cast<float4*>(car + ((c + 1) & 1) * SB + col0 + cb + i) = g4;
                     v[i] += g4.x; v[i + 1] += g4.y; v[i + 2] += g4.z; v[i + 3] += g4.w;
                 }
-                if (live) store_row16(dst + cb, v);
+                if (live) store_row16(dst + cb, v, a.sectors);
             }
             if (row < HC) sac[col0 + row] = next_a;   // every warp has formed its W: the products are done
             tc_fence_before();
@@ -687,7 +696,7 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
                 tmem_ld_rows16(tm_lane + tV + HD * wg + cb, v);
                 if (!live) continue;
                 if (shares) store_row16((float*)a.dv + srow * D + HD * wg + cb, v);
-                else store_row16((__nv_bfloat16*)a.dv + orow * D + HD * wg + cb, v);
+                else store_row16((__nv_bfloat16*)a.dv + orow * D + HD * wg + cb, v, a.sectors);
             }
             tc_fence_before();
             arrive_warp(cx, bVf);
@@ -855,6 +864,8 @@ cudaError_t launch(const void* pq, const void* pk, const void* v, const void* do
     a.tile_tokens = tile;
     a.eps = dm.eps;
     a.status = status;
+    auto on_sector = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; };
+    a.sectors = on_sector(dpq);
     const dim3 grid((unsigned)(tiles * blocks), (unsigned)dm.N);
     err = launch_chain(chain_launches(dm), k1, grid, kThreads, smem1, stream, mdo, mv, mk, mq, a);
     if (err == cudaSuccess) err = causal_scan_tiles(wsf, d_state, d_carry, dm, tile, stream, true, /*reverse=*/true);
@@ -862,6 +873,7 @@ cudaError_t launch(const void* pq, const void* pk, const void* v, const void* do
     a.ws = wsf;
     a.dp = (__nv_bfloat16*)dpk;
     a.dv = blocks > 1 ? (void*)(base + l.shares) : dv;
+    a.sectors = on_sector(dpk) && on_sector(a.dv);
     err = launch_chain(chain_launches(dm), k2, grid, kThreads, smem2, stream, mdo, mv, mk, mq, a);
     if (err != cudaSuccess || blocks == 1) return err;
     const int64_t rows = dm.N * dm.T;

@@ -31,3 +31,25 @@ def test_operator_layout_has_the_bits_of_the_flat_one(L, R, dk, B, H, T):
     heads = ops.race_causal_backward(pq, pk, operator_layout(v), operator_layout(dO))
     assert torch.equal(heads[0], flat[0]) and torch.equal(heads[1], flat[1])
     assert torch.equal(heads[2], operator_layout(flat[2]))
+
+
+@pytest.mark.parametrize("L,R,dk", [(4, 16, 64), (4, 16, 128), (2, 64, 64), (8, 64, 128)])
+def test_outputs_that_begin_between_two_sectors(L, R, dk):
+    """The ABI promises to take any 16-byte boundary; outputs carved out of one buffer often begin on an odd one."""
+    import ctypes
+
+    import race_attention_kernel_b200.ops as ops
+    from race_attention_kernel_b200 import _lib
+    N, T = 3, 200
+    pq, pk, v, dO = _inputs(N, T, L, R, dk, seed=7)
+    want = ops.race_causal_backward(pq, pk, v, dO)
+    got = [torch.empty(t.numel() + 8, device="cuda", dtype=t.dtype)[8:].view_as(t) for t in want]
+    assert all(t.data_ptr() % 32 == 16 for t in got)
+    sh = ops.make_shape(N, T, L, R, dk, torch.bfloat16, 1e-6)
+    n = _lib.lib().race_b200_causal_bwd_workspace_bytes(ctypes.byref(sh))
+    ws = torch.empty(n, dtype=torch.uint8, device="cuda")
+    rc = _lib.lib().race_b200_causal_bwd(*map(ops._ptr, (pq, pk, v, dO)), *map(ops._ptr, got), ops._ptr(ws), n,
+                                         ctypes.byref(sh), ops._stream(), None)
+    assert rc == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
