@@ -169,8 +169,11 @@ cudaError_t launch_step(const void* k, const void* v, const void* q, const float
                         cudaStream_t stream) {
     const size_t smem = Geo::G > 1 ? (size_t)Geo::G * T * Geo::D * sizeof(float) : 0;
     auto kern = decode_step_qkv<Geo, Tin>;
-    if (smem > 32 * 1024) {
-        cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (Geo::G > 1) {
+        // the attribute belongs to the process: always the most any call needs, or two threads with steps of different
+        // lengths take it from each other between setting it and launching
+        cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               Geo::G * decode_max_tokens() * Geo::D * (int)sizeof(float));
         if (err != cudaSuccess) return err;
     }
     cudaLaunchConfig_t cfg = {};

@@ -32,3 +32,33 @@ def test_planes_written_by_the_kernel_before(T):
         ace.planes_T = planes.T.contiguous()
         with torch.no_grad():
             assert torch.equal(ace(*x), want)
+
+
+def test_steps_of_different_lengths_from_two_threads():
+    """The wide step's shared memory grows with the number of new tokens; the limit is an attribute of the process."""
+    import ctypes
+    import threading
+
+    import race_attention_kernel_b200.ops as ops
+    from race_attention_kernel_b200 import _lib
+    ace = _ace(128, 6, 8)
+    planes = ace.planes_T.T.contiguous()
+    codes = {}
+
+    def steps(T):
+        x = _inputs(1, T, 2, 128, torch.bfloat16, n=4)
+        state = torch.zeros(2, 512 * 129, device="cuda")
+        sh = ops.make_shape(2, T, 8, 64, 128, torch.bfloat16, 1e-6, 2)
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        codes[T] = {_lib.lib().race_b200_decode_step_qkv(*map(ops._ptr, x[:3]), ops._ptr(planes), ops._ptr(x[3]),
+                                                         ops._ptr(state), ops._ptr(state), ctypes.byref(sh), 6,
+                                                         ctypes.c_void_p(stream.cuda_stream)) for _ in range(3000)}
+        stream.synchronize()
+
+    threads = [threading.Thread(target=steps, args=(T,)) for T in (64, 20)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert codes == {64: {0}, 20: {0}}
