@@ -206,7 +206,7 @@ bucket_probs_kernel(const Tx* __restrict__ x, const float* __restrict__ planes, 
 // ------------------------------------------------------------------------------------------------
 constexpr int kFastThreads = 128;
 __global__ void __launch_bounds__(kFastThreads, 4)
-bucket_probs_mma_d64_l4k4(const float* __restrict__ x, const float* __restrict__ planes, float* __restrict__ probs,
+bucket_probs_mma_d64_l4k4(const float* x, const float* planes, float* __restrict__ probs,
                           int64_t rows, int64_t T, int heads) {
     constexpr int D = 64, R = 16, LR = 64;
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -233,7 +233,7 @@ bucket_probs_mma_d64_l4k4(const float* __restrict__ x, const float* __restrict__
             const float* src = x + ((mb * T + tok) * heads + hd) * D + 2 * t;
 #pragma unroll
             for (int u = 0; u < 8; ++u)
-                raw[2 * u + h] = live[h] ? __ldcs(reinterpret_cast<const float2*>(src + 8 * u)) : make_float2(0.f, 0.f);
+                raw[2 * u + h] = live[h] ? ld_chain<kLdOnce>(reinterpret_cast<const float2*>(src + 8 * u)) : make_float2(0.f, 0.f);
         }
         float c[2][4];
         project_rows(raw, pf, c);
@@ -289,9 +289,9 @@ __device__ __forceinline__ void pack8(const float* v, uint4& w) {
 // of a training step: the gradients of the probabilities nearly cancel over a table, which magnifies the 2^-17 of two.
 template <int D, int L, int K, typename Tx, typename Tp, bool kExact>
 __global__ void __launch_bounds__(kWideThreads, (sizeof(Tx) == 4 && D > 64 ? 3 : 4))
-bucket_probs_mma_wide(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const float* __restrict__ planes,
+bucket_probs_mma_wide(const Tx* x0, const Tx* x1, const float* planes,
                       Tp* __restrict__ probs0, Tp* __restrict__ probs1, int64_t rows, int64_t T, int heads) {
-    const Tx* __restrict__ x = blockIdx.y ? x1 : x0;   // two tensors (K and Q): one launch, the halves of its grid
+    const Tx* x = blockIdx.y ? x1 : x0;   // two tensors (K and Q): one launch, the halves of its grid
     Tp* __restrict__ probs = blockIdx.y ? probs1 : probs0;
     using W = WideProbs<D, L, K>;
     constexpr int NT = W::NT, NJ = W::NJ, R = W::R, TPL = W::TPL;
@@ -318,7 +318,7 @@ bucket_probs_mma_wide(const Tx* __restrict__ x0, const Tx* __restrict__ x1, cons
         const int slot = 2 * nt + (fg & 1), owner = fg >> 1;   // column 8 nt + 2 owner + e
         const int plane = (TPL * owner + slot / K) * K + slot % K;
         const float* src = planes + (int64_t)plane * D + 32 * (j >> 1) + 8 * ft + 4 * (j & 1);
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+        const float4 v = ld_chain(reinterpret_cast<const float4*>(src));
         uint4 w;
         split_pair(v.x, v.y, w.x, w.z);
         split_pair(v.z, v.w, w.y, w.w);
@@ -359,8 +359,8 @@ bucket_probs_mma_wide(const Tx* __restrict__ x0, const Tx* __restrict__ x1, cons
                 if (kX32) {
                     float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
                     if (live[h]) {
-                        v0 = __ldcs(reinterpret_cast<const float4*>(src[h] + 32 * m));
-                        v1 = __ldcs(reinterpret_cast<const float4*>(src[h] + 32 * m) + 1);
+                        v0 = ld_chain<kLdOnce>(reinterpret_cast<const float4*>(src[h] + 32 * m));
+                        v1 = ld_chain<kLdOnce>(reinterpret_cast<const float4*>(src[h] + 32 * m) + 1);
                     }
                     split_pair(v0.x, v0.y, hi[h][0], lo[h][0]);
                     split_pair(v0.z, v0.w, hi[h][1], lo[h][1]);
@@ -374,7 +374,7 @@ bucket_probs_mma_wide(const Tx* __restrict__ x0, const Tx* __restrict__ x1, cons
                     }
                 } else {
                     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (live[h]) v = __ldcs(reinterpret_cast<const uint4*>(src[h] + 32 * m));
+                    if (live[h]) v = ld_chain<kLdOnce>(reinterpret_cast<const uint4*>(src[h] + 32 * m));
                     hi[h][0] = v.x; hi[h][1] = v.y; hi[h][2] = v.z; hi[h][3] = v.w;
                 }
             }

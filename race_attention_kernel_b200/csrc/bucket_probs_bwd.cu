@@ -43,7 +43,7 @@ template <int R>
 __device__ __forceinline__ void load_dp(const float* p, float (&v)[R]) {
 #pragma unroll
     for (int i = 0; i < R; i += 4) {
-        const float4 x = __ldg(reinterpret_cast<const float4*>(p + i));
+        const float4 x = ld_chain(reinterpret_cast<const float4*>(p + i));
         v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
     }
 }
@@ -51,7 +51,7 @@ template <int R>
 __device__ __forceinline__ void load_dp(const __nv_bfloat16* p, float (&v)[R]) {
 #pragma unroll
     for (int i = 0; i < R; i += 8) {
-        const uint4 x = __ldg(reinterpret_cast<const uint4*>(p + i));
+        const uint4 x = ld_chain(reinterpret_cast<const uint4*>(p + i));
         const uint32_t w[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -63,11 +63,11 @@ __device__ __forceinline__ void load_dp(const __nv_bfloat16* p, float (&v)[R]) {
 
 template <int D, int L, int K, typename Tx, typename Tp>
 __global__ void __launch_bounds__(kBwdThreads, BwdProbs<D, L, K>::kCtas)
-bucket_probs_bwd_mma(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const float* __restrict__ planes,
-                     const Tp* __restrict__ dprobs0, const Tp* __restrict__ dprobs1, Tx* __restrict__ dx0,
+bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
+                     const Tp* dprobs0, const Tp* dprobs1, Tx* __restrict__ dx0,
                      Tx* __restrict__ dx1, int64_t rows, int64_t T, int heads) {
-    const Tx* __restrict__ x = blockIdx.y ? x1 : x0;   // two tensors (K and Q): one launch, the halves of its grid
-    const Tp* __restrict__ dprobs = blockIdx.y ? dprobs1 : dprobs0;
+    const Tx* x = blockIdx.y ? x1 : x0;   // two tensors (K and Q): one launch, the halves of its grid
+    const Tp* dprobs = blockIdx.y ? dprobs1 : dprobs0;
     Tx* __restrict__ dx = blockIdx.y ? dx1 : dx0;
     using W = BwdProbs<D, L, K>;
     constexpr int NT = W::NT, NJ = W::NJ, R = W::R, TPL = W::TPL, KS = W::KS;
@@ -83,7 +83,7 @@ bucket_probs_bwd_mma(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const
         const int ln = i & 31, f = i >> 5, j = f % NJ, nt = f / NJ;
         const int fg = ln >> 2, ft = ln & 3;
         const float* src = planes + (int64_t)W::plane(fg >> 1, 2 * nt + (fg & 1)) * D + 32 * (j >> 1) + 8 * ft + 4 * (j & 1);
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src));
+        const float4 v = ld_chain(reinterpret_cast<const float4*>(src));
         uint4 w;
         split_pair(v.x, v.y, w.x, w.z);
         split_pair(v.z, v.w, w.y, w.w);
@@ -96,7 +96,7 @@ bucket_probs_bwd_mma(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const
         const int feat = 32 * (nb >> 2) + 8 * (fg >> 1) + 2 * (nb & 3) + (fg & 1);   // column fg of block nb
         float v[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = __ldg(planes + (int64_t)W::plane(ft, 4 * j + e) * D + feat);
+        for (int e = 0; e < 4; ++e) v[e] = ld_chain(planes + (int64_t)W::plane(ft, 4 * j + e) * D + feat);
         uint4 w;
         split_pair(v[0], v[1], w.x, w.z);
         split_pair(v[2], v[3], w.y, w.w);
@@ -133,8 +133,8 @@ bucket_probs_bwd_mma(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const
                 if constexpr (kX32) {
                     float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0;
                     if (live[h]) {
-                        v0 = __ldcs(reinterpret_cast<const float4*>(x + off[h] + 32 * m));
-                        v1 = __ldcs(reinterpret_cast<const float4*>(x + off[h] + 32 * m) + 1);
+                        v0 = ld_chain<kLdOnce>(reinterpret_cast<const float4*>(x + off[h] + 32 * m));
+                        v1 = ld_chain<kLdOnce>(reinterpret_cast<const float4*>(x + off[h] + 32 * m) + 1);
                     }
                     split_pair(v0.x, v0.y, hi[h][0], lo[h][0]);
                     split_pair(v0.z, v0.w, hi[h][1], lo[h][1]);
@@ -146,7 +146,7 @@ bucket_probs_bwd_mma(const Tx* __restrict__ x0, const Tx* __restrict__ x1, const
                     rest[h][3] = rest_pair(v1.z, v1.w, hi[h][3], lo[h][3]);
                 } else {
                     uint4 v = make_uint4(0u, 0u, 0u, 0u);
-                    if (live[h]) v = __ldcs(reinterpret_cast<const uint4*>(x + off[h] + 32 * m));
+                    if (live[h]) v = ld_chain<kLdOnce>(reinterpret_cast<const uint4*>(x + off[h] + 32 * m));
                     hi[h][0] = v.x; hi[h][1] = v.y; hi[h][2] = v.z; hi[h][3] = v.w;
                 }
             }

@@ -228,7 +228,7 @@ __device__ __forceinline__ void load_state(const Setup& s, const Args& a, int w,
         float v[16];
 #pragma unroll
         for (int i = 0; i < 16; i += 4) {
-            const float4 x = r.live ? __ldg(reinterpret_cast<const float4*>(src + cb + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 x = r.live ? ld_chain(reinterpret_cast<const float4*>(src + cb + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
             v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
         }
         tmem_st_words16(((uint32_t)(32 * w) << 16) + s.tmem + cb, reinterpret_cast<const uint32_t(&)[16]>(v));
@@ -632,7 +632,7 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
             float gsv[HC];
 #pragma unroll
             for (int i = 0; i < HC; i += 4) {
-                const float4 x = live ? __ldcs(reinterpret_cast<const float4*>(gsrc + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 x = live ? ld_chain<kLdOnce>(reinterpret_cast<const float4*>(gsrc + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 gsv[i] = x.x; gsv[i + 1] = x.y; gsv[i + 2] = x.z; gsv[i + 3] = x.w;
             }
             if (!(ok = wait_bar_warp(cx, bX, ph, 106))) break;
@@ -771,7 +771,7 @@ bwd_suffix_rows(const __grid_constant__ CUtensorMap map_do, const __grid_constan
 
 // dV [N/H, T, H, D] = sum over the bucket blocks of their shares [block][N, T, D], in block order; 8 values per thread
 __global__ void __launch_bounds__(256)
-bwd_dv_sum(const float* __restrict__ shares, __nv_bfloat16* __restrict__ dv, int64_t rows, int64_t T, int heads, int D,
+bwd_dv_sum(const float* shares, __nv_bfloat16* __restrict__ dv, int64_t rows, int64_t T, int heads, int D,
            int blocks) {
     chain_release();
     chain_wait();
@@ -783,7 +783,7 @@ bwd_dv_sum(const float* __restrict__ shares, __nv_bfloat16* __restrict__ dv, int
     float acc[8] = {};
     for (int b = 0; b < blocks; ++b) {
         const float4* p = reinterpret_cast<const float4*>(shares + (b * rows + r) * D + c);
-        const float4 x = __ldcs(p), y = __ldcs(p + 1);
+        const float4 x = ld_chain<kLdOnce>(p), y = ld_chain<kLdOnce>(p + 1);
         acc[0] += x.x; acc[1] += x.y; acc[2] += x.z; acc[3] += x.w;
         acc[4] += y.x; acc[5] += y.y; acc[6] += y.z; acc[7] += y.w;
     }

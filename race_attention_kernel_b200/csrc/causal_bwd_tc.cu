@@ -44,7 +44,7 @@ inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 // a chain of 512 tokens: 32 streams of 16384 tokens, 134 MB, took 39 us.)
 template <bool kChunks>
 __global__ void __launch_bounds__(kPwThreads)
-bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, float* __restrict__ chunk, int64_t T, int64_t nblk,
+bwd_block_sums(const float* x, float* __restrict__ sums, float* __restrict__ chunk, int64_t T, int64_t nblk,
                int64_t nchunk) {
     constexpr int kCh = kBlk / 64, kSums = kChunks ? kCh : 1, kWarps = kPwThreads / 32;
     __shared__ __align__(16) float red[kWarps][kSums][64];
@@ -65,7 +65,7 @@ bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, float* __r
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
             const int t = 64 * j + 16 * u + slot;
-            v[u] = t < len ? __ldg(p + t * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = t < len ? ld_chain(p + t * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -103,7 +103,7 @@ bwd_block_sums(const float* __restrict__ x, float* __restrict__ sums, float* __r
 // in-place exclusive scan over the blocks of a stream (reverse: suffix sums, last block first); carry is the A part
 // ([64] floats at offset S*D) of a packed state per stream or null; total (nullable) receives carry + everything
 __global__ void __launch_bounds__(64)
-bwd_block_scan(float* __restrict__ sums, const float* __restrict__ carry_state, float* __restrict__ total_state,
+bwd_block_scan(float* __restrict__ sums, const float* carry_state, float* __restrict__ total_state,
                int64_t nblk, int reverse) {
     chain_release();
     chain_wait();
@@ -137,7 +137,7 @@ bwd_block_scan(float* __restrict__ sums, const float* __restrict__ carry_state, 
 // flight; the sums of the threads behind it come through shared memory.  (One thread per block and column, 4 bytes and
 // four tokens at a time: 32 streams of 16384 tokens, 403 MB, took 103 us.)
 __global__ void __launch_bounds__(kPwThreads)
-bwd_pointwise_rev(const float* __restrict__ g, float* __restrict__ pdpk, const float* __restrict__ gsuffix, int64_t T,
+bwd_pointwise_rev(const float* g, float* __restrict__ pdpk, const float* gsuffix, int64_t T,
                   int64_t nblk) {
     constexpr int kOwn = 8, kSlots = kPwThreads / 16, kPiece = kOwn * kSlots;
     __shared__ float4 part[2][kSlots][16];
@@ -158,7 +158,7 @@ bwd_pointwise_rev(const float* __restrict__ g, float* __restrict__ pdpk, const f
 #pragma unroll
         for (int u = 0; u < kOwn; ++u) {
             const bool live = t + u < len;
-            gv[u] = live ? __ldcs(gp + (t + u) * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+            gv[u] = live ? ld_chain<kLdOnce>(gp + (t + u) * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
             pv[u] = live ? pp[(t + u) * 16] : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -184,7 +184,7 @@ bwd_pointwise_rev(const float* __restrict__ g, float* __restrict__ pdpk, const f
 
 // dst[n] = the state src[n] with its B part ([64][64]) transposed and its A part zeroed
 __global__ void __launch_bounds__(256)
-bwd_transpose_state(const float* __restrict__ src, float* __restrict__ dst) {
+bwd_transpose_state(const float* src, float* __restrict__ dst) {
     __shared__ float tile[64][65];
     chain_release();
     chain_wait();

@@ -145,7 +145,7 @@ constexpr int kScanShort = 16;   // tiles
 
 template <int V, int kInFlight>
 __global__ void __launch_bounds__(128)
-tile_scan(float* __restrict__ ws, const float* __restrict__ carry_in, float* __restrict__ state_out,
+tile_scan(float* ws, const float* carry_in, float* state_out,
           int64_t tiles, int state_floats, int write_prefix, int reverse) {
     using Vec = typename ScanVec<V>::T;
     chain_release();

@@ -238,9 +238,9 @@ struct Heads {   // head counts of the layouts [N/h, T, h, 64] of the four tenso
 };
 constexpr int kModeBucket = 0, kModeGlobal = 1, kModeRaw = 2, kModeRawX = 3;
 template <int kMode, bool kReverse = false, bool kProj = false, bool kWorkerK = kProj>
-__device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, const float* __restrict__ pq,
+__device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, const float* pq,
                                           const CUtensorMap* map_k, const CUtensorMap* map_v,
-                                          float* __restrict__ out, const float* __restrict__ slice, int64_t T,
+                                          float* __restrict__ out, const float* slice, int64_t T,
                                           const int64_t t_begin, const int64_t t_end, const int64_t n, float eps,
                                           const Heads hd, int withhold_chunk, const bool l2_last_use = false,
                                           const uint32_t* ptab = nullptr, const BwdX* bx = nullptr,
@@ -311,19 +311,25 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
 #pragma unroll
             for (int half = 0; half < 2; ++half) {
                 float xv[16], av[16];
+                float2 a2[4];   // A before the chunk: all requested before the first store
+#pragma unroll
+                for (int xx = 0; xx < 4; ++xx) {
+                    const int col = 8 * (4 * half + xx) + 2 * q;
+                    const float2 b2 = ld_chain(reinterpret_cast<const float2*>(ab + col));
+                    const float2 c2 = ld_chain(reinterpret_cast<const float2*>(ac + col));
+                    a2[xx] = make_float2(b2.x + c2.x, b2.y + c2.y);
+                }
                 tmem_ld32(lane_base + tmO(wg) + 32 * half, xv);
                 tmem_ld32(lane_base + tmAG(wg) + 32 * half, av);
 #pragma unroll
                 for (int xx = 0; xx < 4; ++xx) {
                     const int x = 4 * half + xx, col = 8 * x + 2 * q;
-                    const float2 b2 = __ldg(reinterpret_cast<const float2*>(ab + col));
-                    const float2 c2 = __ldg(reinterpret_cast<const float2*>(ac + col));
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         const int row = rbase + 8 * h;
                         if (row < valid) {
-                            const float a0 = (b2.x + c2.x) + av[4 * xx + 2 * h];
-                            const float a1 = (b2.y + c2.y) + av[4 * xx + 2 * h + 1];
+                            const float a0 = a2[xx].x + av[4 * xx + 2 * h];
+                            const float a1 = a2[xx].y + av[4 * xx + 2 * h + 1];
                             const float i0 = __fdividef(1.f, a0 + bx->eps), i1 = __fdividef(1.f, a1 + bx->eps);
                             const float2 pq2 = pqv[2 * x + h];
                             const float2 w2 = make_float2(pq2.x * i0, pq2.y * i1);
@@ -347,7 +353,7 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
                 const float* prow = bx->pq_true + (n * T + tok0 + row) * S + 2 * q;
 #pragma unroll
                 for (int x = 0; x < 8; ++x)
-                    pqv[2 * x + h] = row < valid ? __ldcs(reinterpret_cast<const float2*>(prow + 8 * x))
+                    pqv[2 * x + h] = row < valid ? ld_chain<kLdOnce>(reinterpret_cast<const float2*>(prow + 8 * x))
                                                  : make_float2(0.f, 0.f);
             }
         };
@@ -360,7 +366,7 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
                 const float* prow = pq_n + (tok0 + row) * pq_stride + 2 * q;
 #pragma unroll
                 for (int x = 0; x < 8; ++x)
-                    pqv[2 * x + h] = row < valid ? __ldcs(reinterpret_cast<const float2*>(prow + 8 * x))
+                    pqv[2 * x + h] = row < valid ? ld_chain<kLdOnce>(reinterpret_cast<const float2*>(prow + 8 * x))
                                                  : make_float2(0.f, 0.f);
             }
         };
@@ -551,7 +557,7 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
             for (int h = 0; h < 2; ++h) {
                 const int off = (rbase + 8 * h) * D + 8 * x + 2 * q;
                 const float2 b2 = carry_smem ? *reinterpret_cast<const float2*>(carry_smem + off)
-                                             : __ldcg(reinterpret_cast<const float2*>(slice + off));
+                                             : ld_chain<kLdL2>(reinterpret_cast<const float2*>(slice + off));
                 v[4 * x + 2 * h] = b2.x; v[4 * x + 2 * h + 1] = b2.y;
             }
         {   // tril[t][j] = (j <= t), exact in bf16, as an A operand in tensor memory
@@ -569,8 +575,8 @@ __device__ __forceinline__ void out_phase(const Ctx& cx, const uint32_t tmem, co
         tc_fence_before();
         if (warp == 8 && !carry_smem) {   // (folded: the A part is there already)
             float* ac = reinterpret_cast<float*>(cx.sm + oAcar);
-            ac[lane] = __ldcg(slice + S * D + lane);
-            ac[lane + 32] = __ldcg(slice + S * D + lane + 32);
+            ac[lane] = ld_chain<kLdL2>(slice + S * D + lane);
+            ac[lane + 32] = ld_chain<kLdL2>(slice + S * D + lane + 32);
         }
         __syncwarp();
         if (lane == 0) {
@@ -756,10 +762,10 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols) {
 // kProj: pq is Q, map_k covers K and `planes` [16][64] are the hyperplanes (out_phase).
 template <int kMode, bool kReverse, bool kProj>
 __global__ void __launch_bounds__(kThreads, 1)
-causal_out_tc(const float* __restrict__ pq, const __grid_constant__ CUtensorMap map_k,
+causal_out_tc(const float* pq, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, float* __restrict__ out,
-              const float* __restrict__ ws, int64_t T, int tile_tokens, float eps, const Heads hd, int* status,
-              long long wait_cycles, int withhold_chunk, const float* __restrict__ planes, const BwdX bwdx,
+              const float* ws, int64_t T, int tile_tokens, float eps, const Heads hd, int* status,
+              long long wait_cycles, int withhold_chunk, const float* planes, const BwdX bwdx,
               const CarryFold cf) {
     extern __shared__ uint8_t smem_raw[];
     Ctx cx;
@@ -1113,7 +1119,7 @@ template <bool kProj>
 __global__ void __launch_bounds__(TotalsLayoutOf<kProj>::kThreads, 1)
 tile_totals_tc(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                float* __restrict__ ws, int64_t T, int tile_tokens, const Heads hd, int* status,
-               const float* __restrict__ planes, int64_t tiles, int tile0) {
+               const float* planes, int64_t tiles, int tile0) {
     extern __shared__ uint8_t smem_raw[];
     Ctx cx;
     cx.sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);

@@ -106,7 +106,7 @@ template <int D, bool kGlobal>
 __global__ void __launch_bounds__(kThreads, 1)
 causal_out_tc_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
-                   const float* __restrict__ ws, int64_t T, int S, int G, int tile_tokens, float eps, int heads,
+                   const float* ws, int64_t T, int S, int G, int tile_tokens, float eps, int heads,
                    int* status, const CarryFold cf) {
     using Ly = Lay<D>;
     constexpr int DH = D / 64;   // 64-column halves of a [64][D] accumulator
@@ -781,7 +781,7 @@ enum BarW {
 __global__ void __launch_bounds__(kWThreads, 1)
 causal_out_wide_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                      const __grid_constant__ CUtensorMap map_vs, __nv_bfloat16* __restrict__ out,
-                     const float* __restrict__ ws, int64_t T, int S, int D, int G, int tile_tokens, float eps,
+                     const float* ws, int64_t T, int S, int D, int G, int tile_tokens, float eps,
                      int* status) {
     using Ly = LayW;
     extern __shared__ uint8_t smem_raw[];
@@ -1254,7 +1254,7 @@ template <int DSX, int NWG, int NST>
 __global__ void __launch_bounds__((LayW4<DSX, NWG, NST>::kThreads), 1)
 causal_out_wide4_bf16(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_vs, __nv_bfloat16* __restrict__ out,
-                      const float* __restrict__ ws, int64_t T, int S, int D, int G, int tile_tokens, float eps,
+                      const float* ws, int64_t T, int S, int D, int G, int tile_tokens, float eps,
                       int heads, int* status) {
     using Ly = LayW4<DSX, NWG, NST>;
     extern __shared__ uint8_t smem_raw[];

@@ -32,6 +32,25 @@ __host__ __device__ inline int state_floats_per_stream(int S, int D) { return S 
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Loads of a chained kernel.  What it reads may have been written while it was already resident, so it must not go through
+// the read-only path (__ldg, or a plain load of a const __restrict__ parameter: both promise that the data does not change
+// while the grid lives), and the compiler must not move it ahead of chain_wait.
+enum LdPolicy { kLdCached, kLdL2, kLdOnce };   // ld.global, .cg (L2 only), .cs (streamed)
+#define RACE_LD_CHAIN(T, SUFFIX, OUT, ...)                                                                             \
+    template <LdPolicy kPolicy = kLdCached>                                                                            \
+    __device__ __forceinline__ T ld_chain(const T* p) {                                                                \
+        T v;                                                                                                           \
+        if (kPolicy == kLdOnce) asm volatile("ld.global.cs." SUFFIX " " OUT ";" : __VA_ARGS__ : "l"(p) : "memory");    \
+        else if (kPolicy == kLdL2) asm volatile("ld.global.cg." SUFFIX " " OUT ";" : __VA_ARGS__ : "l"(p) : "memory"); \
+        else asm volatile("ld.global." SUFFIX " " OUT ";" : __VA_ARGS__ : "l"(p) : "memory");                          \
+        return v;                                                                                                      \
+    }
+RACE_LD_CHAIN(float, "f32", "%0, [%1]", "=f"(v))
+RACE_LD_CHAIN(float2, "v2.f32", "{%0, %1}, [%2]", "=f"(v.x), "=f"(v.y))
+RACE_LD_CHAIN(float4, "v4.f32", "{%0, %1, %2, %3}, [%4]", "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w))
+RACE_LD_CHAIN(uint4, "v4.u32", "{%0, %1, %2, %3}, [%4]", "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w))
+#undef RACE_LD_CHAIN
+
 // The state a tile starts from, formed by the output kernel itself (fold): carry_in + the totals of the tiles before it,
 // added tile by tile in the order tile_scan adds them, so both routes give the same bits.  Not folded: the slot of the
 // tile already holds that prefix (tile_scan).  The CTA of the last tile also writes the state after the sequence.
@@ -53,7 +72,7 @@ __device__ __forceinline__ void fold_prefix(const float* p, int64_t step, int cn
 #pragma unroll
         for (int u = 0; u < kCols; ++u) {
             const int i = base + 4 * NT * u;
-            run[u] = carry && i < state_floats ? __ldcg(reinterpret_cast<const float4*>(carry + i))
+            run[u] = carry && i < state_floats ? ld_chain<kLdL2>(reinterpret_cast<const float4*>(carry + i))
                                                : make_float4(0.f, 0.f, 0.f, 0.f);
         }
         for (int t = 0; t < cnt; t += kTiles) {
@@ -64,7 +83,7 @@ __device__ __forceinline__ void fold_prefix(const float* p, int64_t step, int cn
                 for (int u = 0; u < kCols; ++u) {
                     const int i = base + 4 * NT * u;
                     x[j][u] = t + j < cnt && i < state_floats
-                                  ? __ldcg(reinterpret_cast<const float4*>(p + (t + j) * step + i))
+                                  ? ld_chain<kLdL2>(reinterpret_cast<const float4*>(p + (t + j) * step + i))
                                   : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
@@ -81,7 +100,7 @@ __device__ __forceinline__ void fold_prefix(const float* p, int64_t step, int cn
             if (i >= state_floats) continue;
             *reinterpret_cast<float4*>(i < b_floats ? sb + i : sa + (i - b_floats)) = run[u];
             if (state_out) {
-                const float4 x = __ldcg(reinterpret_cast<const float4*>(p + cnt * step + i));
+                const float4 x = ld_chain<kLdL2>(reinterpret_cast<const float4*>(p + cnt * step + i));
                 *reinterpret_cast<float4*>(state_out + i) =
                     make_float4(run[u].x + x.x, run[u].y + x.y, run[u].z + x.z, run[u].w + x.w);
             }

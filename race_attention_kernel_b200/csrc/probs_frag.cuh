@@ -52,20 +52,20 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], const uint32_t (&a
 struct PlaneFrags {
     uint32_t hi[16], lo[16];
 };
-__device__ __forceinline__ void plane_frag(const float* __restrict__ planes, int f, int lane, uint32_t& hi,
+__device__ __forceinline__ void plane_frag(const float* planes, int f, int lane, uint32_t& hi,
                                            uint32_t& lo) {
     const int j = f >> 2, nt = (f >> 1) & 1, half = f & 1, g = lane >> 2, t = lane & 3;
-    const float2 p = __ldg(reinterpret_cast<const float2*>(planes + (8 * nt + g) * 64 + 16 * j + 8 * half + 2 * t));
+    const float2 p = ld_chain(reinterpret_cast<const float2*>(planes + (8 * nt + g) * 64 + 16 * j + 8 * half + 2 * t));
     split_pair(p.x, p.y, hi, lo);
 }
-__device__ __forceinline__ void load_plane_frags(const float* __restrict__ planes, int lane, PlaneFrags& pf) {
+__device__ __forceinline__ void load_plane_frags(const float* planes, int lane, PlaneFrags& pf) {
 #pragma unroll
     for (int f = 0; f < 16; ++f) plane_frag(planes, f, lane, pf.hi[f], pf.lo[f]);
 }
 // The same table in shared memory for kernels that cannot keep 32 registers for it: word (2 f + limb) * 32 + lane
 // (a warp reads 32 consecutive words: no bank conflicts).  Written by nthreads threads; the caller synchronises.
 constexpr int kPlaneTabWords = 16 * 2 * 32;
-__device__ __forceinline__ void build_plane_tab(const float* __restrict__ planes, uint32_t* tab, int tid,
+__device__ __forceinline__ void build_plane_tab(const float* planes, uint32_t* tab, int tid,
                                                 int nthreads) {
     for (int i = tid; i < 16 * 32; i += nthreads) {
         const int f = i >> 5, lane = i & 31;

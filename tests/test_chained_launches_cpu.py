@@ -40,6 +40,21 @@ def test_nothing_is_read_before_the_wait(file, name):
     """Not the hyperplanes either: the kernel before may be a caller's, and what it wrote is visible after the wait only."""
     text = next(t for f, n, t in WAITING if (f, n) == (file, name))
     before = text[text.index("{"):text.index("chain_wait();")]
-    assert not re.search(r"__ld(g|cg|cs)|build_plane_tab|load_plane_frags|fold_prefix|tma_load", before)
+    assert not re.search(r"__ld(g|cg|cs)|ld_chain|build_plane_tab|load_plane_frags|fold_prefix|tma_load", before)
     pointers = set(re.findall(r"\*\s*(?:__restrict__\s+)?(\w+)\s*[,)]", text[:text.index("{")]))
     assert not [p for p in pointers if re.search(rf"(?<![\w.]){p}\[|\*\s*{p}\b(?!\s*[*+-])", before)]
+
+
+CHAINED_FILES = ["causal_tc.cu", "causal_tc_bf16.cu", "causal_bwd_tc.cu", "causal_bwd_bf16_tc.cu", "bucket_probs_bwd.cu", "probs_frag.cuh"]
+
+
+@pytest.mark.parametrize("file", CHAINED_FILES)
+def test_helpers_of_chained_kernels_load_what_may_still_change(file):
+    assert "__ldg(" not in re.sub(r"//[^\n]*", "", open(os.path.join(CSRC, file)).read())
+
+
+@pytest.mark.parametrize("file,name", [(f, n) for f, n, t in WAITING if "__global__" in t])
+def test_no_input_of_a_chained_kernel_is_declared_constant_for_its_life(file, name):
+    text = next(t for f, n, t in WAITING if (f, n) == (file, name))
+    assert "__ldg(" not in text
+    assert not re.search(r"const \w+\s*\*\s*__restrict__", text)
