@@ -64,9 +64,9 @@ bool variant_supported(const Dims& dm, int dtype, int variant) {
 
 int chunk_of(int variant) { return family(variant) == RACE_VARIANT_TENSOR ? tensor_chunk_tokens() : kSimtChunk; }
 
-int pick_tile(const Dims& dm, int dtype, int variant) {
+int pick_tile(const Dims& dm, int variant) {
     if (is_single_pass(variant)) return tensor_single_pass_tile_tokens(dm, sm_count());
-    if (variant == RACE_VARIANT_TENSOR) return tensor_default_tile_tokens(dm, dtype, sm_count());
+    if (variant == RACE_VARIANT_TENSOR) return tensor_default_tile_tokens(dm, sm_count());
     return simt_default_tile_tokens(dm, sm_count());
 }
 
@@ -121,7 +121,7 @@ int race_b200_select_tile_tokens(const RaceShape* shape, int variant, int* tile_
     if (rc != RACE_OK) return rc;
     const int var = resolve_variant(dm, shape->dtype, variant);
     if (!variant_supported(dm, shape->dtype, var)) return RACE_ERR_VARIANT;
-    *tile_tokens = pick_tile(dm, shape->dtype, var);
+    *tile_tokens = pick_tile(dm, var);
     return RACE_OK;
 }
 
@@ -130,7 +130,7 @@ size_t race_b200_causal_workspace_bytes(const RaceShape* shape, int tile_tokens,
     if (check_shape(shape, &dm) != RACE_OK) return 0;
     const int var = resolve_variant(dm, shape->dtype, variant);
     if (!variant_supported(dm, shape->dtype, var)) return 0;
-    const int tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, shape->dtype, var);
+    const int tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, var);
     return workspace_bytes_for(dm, shape->dtype, var, tile);
 }
 
@@ -155,7 +155,8 @@ static int causal_entry(const void* probs_q, const void* probs_k, const void* v,
     if (global_norm && family(var) == RACE_VARIANT_TENSOR && shape->dtype != RACE_DTYPE_F32 && dm.S != 64)
         return RACE_ERR_VARIANT;
     if (tile_tokens < 0) return RACE_ERR_TILE;
-    const int tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, shape->dtype, var);
+    const bool bf16_only = shape->dtype == RACE_DTYPE_BF16 && var == RACE_VARIANT_TENSOR && phases == kPhaseAll && !state_out;
+    const int tile = tile_tokens > 0 ? tile_tokens : bf16_only ? tensor_bf16_tile_tokens(dm, sm_count()) : pick_tile(dm, var);
     if (tile % chunk_of(var) != 0) return RACE_ERR_TILE;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t sf = (size_t)dm.N * state_floats_per_stream(dm.S, dm.D);
@@ -199,7 +200,7 @@ int race_b200_causal_fwd(const void* probs_q, const void* probs_k, const void* v
 size_t race_b200_causal_heads_workspace_bytes(const RaceShape* shape) {
     Dims dm;
     if (check_shape(shape, &dm) != RACE_OK || !causal_heads_supported(dm, shape->dtype)) return 0;
-    return workspace_bytes_for(dm, shape->dtype, RACE_VARIANT_TENSOR, pick_tile(dm, shape->dtype, RACE_VARIANT_TENSOR));
+    return workspace_bytes_for(dm, shape->dtype, RACE_VARIANT_TENSOR, pick_tile(dm, RACE_VARIANT_TENSOR));
 }
 
 int race_b200_causal_fwd_heads(const void* probs_q, const void* probs_k, const void* v, void* out,
@@ -253,7 +254,7 @@ int race_b200_causal_fwd_qkv(const void* q, const void* k, const void* v, const 
     if (n_planes <= 0 || n_planes > 12 || shape->n_buckets != (1 << n_planes)) return RACE_ERR_SHAPE;
     if (!tensor_qkv_supported(dm, shape->dtype, shape->n_tables, shape->n_buckets)) return RACE_ERR_VARIANT;
     if (tile_tokens < 0) return RACE_ERR_TILE;
-    const int tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, shape->dtype, RACE_VARIANT_TENSOR);
+    const int tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, RACE_VARIANT_TENSOR);
     if (tile % tensor_chunk_tokens() != 0) return RACE_ERR_TILE;
     cudaStream_t st = (cudaStream_t)stream;
     const size_t sf = (size_t)dm.N * state_floats_per_stream(dm.S, dm.D);

@@ -233,7 +233,7 @@ bool causal_bwd_tensor_supported(const Dims& dm, int dtype) {
 }
 
 int causal_bwd_tensor_tile_tokens(const Dims& dm, int sm_count) {
-    return tensor_default_tile_tokens(dm, RACE_DTYPE_F32, sm_count);
+    return tensor_default_tile_tokens(dm, sm_count);
 }
 
 size_t causal_bwd_tensor_workspace_bytes(const Dims& dm, int tile_tokens) {

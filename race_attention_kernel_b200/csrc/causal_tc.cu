@@ -1433,34 +1433,46 @@ int tensor_single_pass_tile_tokens(const Dims& dm, int sm_count) {
     return (int)(tile < C ? C : (tile > 1024 ? 1024 : tile));
 }
 
-int tensor_default_tile_tokens(const Dims& dm, int dtype, int sm_count) {
-    // One CTA per SM at a time: the CTAs of the output pass run in waves of sm_count, so the tile length (a multiple of
-    // the chunk) is chosen to fill the last wave, against the totals pass, which covers every tile but the last of a
-    // stream: cost = waves x (tokens per tile + the set-up of a CTA, about one and a half chunks) + 0.4 x the totals'
-    // tokens per SM (a token costs the totals kernels 0.36 to 0.43 of what it costs the output kernels; they are bound by
-    // memory, not by waves).  So many short streams get one tile each and no totals at all.  At most 2048 tokens in
-    // fp32, where a longer tile would add more terms into one accumulator, and 4096 in bf16.
+int tensor_default_tile_tokens(const Dims& dm, int sm_count) {
+    // The CTAs run in waves of sm_count, so the tile length (a multiple of the chunk) is chosen to fill the last wave:
+    // cost = waves x (tokens per tile + the set-up of a CTA, about one and a half chunks), with a CTA per bucket group.
+    // An accumulator adds up a whole tile and rounds every addition down, so the error of its sums grows with the tile:
+    // what leaves in fp32 (fp32 results, states) has no longer tiles than these.  (64 streams of 8192 tokens in tiles of
+    // 960 / 2048: fp32 out 4.6e-6 / 5.9e-6 off the 64-bit result, B of the state 5.5e-6 / 8.3e-6; B of bf16 streams in
+    // tiles of 960 / 4096: 0.9e-6 / 4.5e-6.)
+    const int64_t groups = dm.S > 64 ? dm.S / 64 : 1;
+    const int64_t sms = sm_count > 0 ? sm_count : 148;
+    int best = 2048;
+    double best_cost = 1e300;
+    for (int tile = 2048; tile >= C; tile -= C) {
+        const int64_t ctas = dm.N * groups * ((dm.T + tile - 1) / tile);
+        const int64_t waves = (ctas + sms - 1) / sms;
+        const double cost = (double)waves * (tile + 96.0);
+        if (cost < best_cost * 0.999) { best_cost = cost; best = tile; }
+        if (ctas > 64 * sms) break;   // many waves already: shorter tiles only add state traffic
+    }
+    return best;
+}
+
+int tensor_bf16_tile_tokens(const Dims& dm, int sm_count) {
+    // bf16 outputs alone (their rounding is a hundred times the accumulators'): up to 4096 tokens, the waves of the output
+    // pass against the totals pass, which covers every tile but the last of a stream: + 0.4 x the totals' tokens per SM (a
+    // token costs the totals kernels 0.36 to 0.43 of what it costs the output kernels; they are bound by memory, not by
+    // waves).  So many short streams get one tile each and no totals at all.
     // CTAs of the output pass per (stream, tile): slices of the head dimension when there are several bucket groups
     const int64_t groups = dm.S > 128 ? dm.D / 64 : dm.S > 64 ? dm.D / 32 : 1;
     const int64_t sms = sm_count > 0 ? sm_count : 148;
-    const int longest = dtype == RACE_DTYPE_BF16 ? 4096 : 2048;
-    int best = 2048, waves_only = 2048;
-    double best_cost = 1e300, best_waves = 1e300;
-    for (int tile = longest; tile >= C; tile -= C) {
+    int best = 2048;
+    double best_cost = 1e300;
+    for (int tile = 4096; tile >= C; tile -= C) {
         const int64_t tiles = (dm.T + tile - 1) / tile, ctas = dm.N * groups * tiles;
         const int64_t waves = (ctas + sms - 1) / sms;
         const int64_t len = std::min<int64_t>(tile, (dm.T + C - 1) / C * C);
         const double cost = (double)waves * (len + 96.0) + 0.4 * (double)(dm.N * groups * (tiles - 1) * len) / sms;
         if (cost < best_cost * 0.999) { best_cost = cost; best = tile; }
-        if (tile <= 2048 && waves * (tile + 96.0) < best_waves * 0.999) {
-            best_waves = waves * (tile + 96.0);
-            waves_only = tile;
-        }
-        if (ctas > 64 * sms) break;   // many waves already: shorter tiles only add state traffic
+        if (ctas > 64 * sms) break;
     }
-    // not shorter than what the waves alone ask for: near a tie the totals' term would take up to 1.7 times the tiles,
-    // and the workspace (bounded in the allocation-free entry) with them, for a part in a thousand of the time
-    return std::max(best, waves_only);
+    return std::max(best, tensor_default_tile_tokens(dm, sm_count));   // never more workspace than the rule above asks for
 }
 
 // fp32 single-pass kernel: [totals of every tile | inclusive prefix of every tile | carry slot per CTA | flags, ticket]

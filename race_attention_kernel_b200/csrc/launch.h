@@ -129,7 +129,8 @@ cudaError_t decode_step_qkv_launch(const void* k, const void* v, const void* q, 
 // ---- tcgen05 tensor-core causal path (causal_tc.cu) ------------------------------------------
 bool tensor_supported(const Dims& dm, int dtype);
 int tensor_chunk_tokens();
-int tensor_default_tile_tokens(const Dims& dm, int dtype, int sm_count);
+int tensor_default_tile_tokens(const Dims& dm, int sm_count);
+int tensor_bf16_tile_tokens(const Dims& dm, int sm_count);   // bf16 without a state to return: at least as long
 size_t tensor_workspace_bytes(const Dims& dm, int dtype, int tile_tokens);
 // the single-pass form of the fp32 forward (one persistent kernel): its tile length and its workspace
 int tensor_single_pass_tile_tokens(const Dims& dm, int sm_count);

@@ -1,0 +1,27 @@
+"""Errors against 64 bits where a step for speed could cost some: sums of whole tiles, and gradients of fp32 tensors."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import race_oracle as ro
+
+pytestmark = pytest.mark.gpu
+
+
+# An accumulator rounds each of its additions down: of a tile of n tokens it takes n / 16 per limb product (three in fp32,
+# one in bf16), each half a unit of 2^-23 off on average, on a sum that has grown to two thirds of its end by then.  The
+# tile of 64 streams of 8192 tokens has at most 1024: 64 x 2^-24 x 2/3 = 2.5e-6 in bf16, three times that in fp32.
+@pytest.mark.parametrize("dt,bound", [(torch.bfloat16, 2.5e-6), (torch.float32, 7.6e-6)])
+def test_state_of_many_streams(dt, bound):
+    import race_attention_kernel_b200.ops as ops
+    N, T = 64, 8192
+    g = torch.Generator(device="cuda").manual_seed(0)
+    pq, pk = (torch.softmax(torch.randn(N, T, 4, 16, device="cuda", generator=g), -1).to(dt) for _ in range(2))
+    v = torch.randn(N, T, 64, device="cuda", generator=g).to(dt)
+    out, A, B = ops.race_causal_prefix(pq, pk, v, return_state=True)
+    p64, v64 = pk.flatten(2).double(), v.double()
+    assert ro.rel_l2(A.flatten(1), p64.sum(1)) <= 5e-7
+    assert ro.rel_l2(B.flatten(1, 2), p64.transpose(1, 2) @ v64) <= bound
+    if dt == torch.bfloat16:   # outputs alone take longer tiles: the same but for their rounding
+        assert ro.rel_l2(ops.race_causal_prefix(pq, pk, v), out) <= 1e-3
