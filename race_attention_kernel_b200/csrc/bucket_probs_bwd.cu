@@ -31,7 +31,7 @@ struct BwdProbs {
     static constexpr int NT = L * K / 8, NJ = D / 16, R = 1 << K, TPL = L / 4, NS = 2 * NT;   // NS plane slots per lane
     static constexpr int KS = NS / 4, NB = D / 8;                                            // second product
     static constexpr int kTab1 = NT * NJ * 32, kTab2 = NB * KS * 32;                         // 16-byte items
-    static constexpr int smem_bytes(bool x32) { return (kTab1 + kTab2) * 16 + (x32 ? kTab1 * 8 : 0); }
+    static constexpr int smem_bytes(bool x32) { return (kTab1 + kTab2) * (16 + (x32 ? 8 : 0)); }
     static constexpr int kCtas = D == 64 ? 5 : 3;   // resident CTAs per SM (registers)
     static_assert(D % 32 == 0 && L % 4 == 0 && (L * K) % 16 == 0, "geometry of the tensor-core producer");
     // plane of slot s of lane t of a quad
@@ -61,6 +61,23 @@ __device__ __forceinline__ void load_dp(const __nv_bfloat16* p, float (&v)[R]) {
     }
 }
 
+// c += a . b over one k-step with three limbs of both (b = {b0 hi, b1 hi, b0 lo, b1 lo}, r = the third limbs): an accumulator of
+// its own, small products first, added to c with rounding.  The tensor core rounds its additions down, and in one chain over
+// all k-steps that is a bias of the size of the projections (d_k = 128: 11): dK and dQ 4.3e-6 off the 64-bit result, where
+// fp32 FMAs are 1.3e-6 off.
+__device__ __forceinline__ void six_products(float (&c)[4], const uint32_t (&hi)[4], const uint32_t (&lo)[4],
+                                             const uint32_t (&rest)[4], const uint4& b, const uint2& r) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16_16816(s, rest, b.x, b.y);
+    mma_bf16_16816(s, lo, b.z, b.w);
+    mma_bf16_16816(s, hi, r.x, r.y);
+    mma_bf16_16816(s, lo, b.x, b.y);
+    mma_bf16_16816(s, hi, b.z, b.w);
+    mma_bf16_16816(s, hi, b.x, b.y);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] += s[i];
+}
+
 template <int D, int L, int K, typename Tx, typename Tp>
 __global__ void __launch_bounds__(kBwdThreads, BwdProbs<D, L, K>::kCtas)
 bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
@@ -75,7 +92,8 @@ bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
     extern __shared__ __align__(16) uint8_t bwd_smem[];
     uint4* tab1 = reinterpret_cast<uint4*>(bwd_smem);          // [(nt NJ + j) 32 + lane] = {b0 hi, b1 hi, b0 lo, b1 lo}
     uint4* tab2 = tab1 + W::kTab1;                             // [(nb KS + j) 32 + lane]
-    uint2* tab1r = reinterpret_cast<uint2*>(tab2 + W::kTab2);   // fp32 rows: third limbs {b0, b1} of tab1
+    uint2* tab1r = reinterpret_cast<uint2*>(tab2 + W::kTab2);   // fp32 rows: third limbs {b0, b1} of tab1 ...
+    uint2* tab2r = tab1r + W::kTab1;                            // ... and of tab2
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     chain_release();
     chain_wait();
@@ -101,6 +119,7 @@ bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
         split_pair(v[0], v[1], w.x, w.z);
         split_pair(v[2], v[3], w.y, w.w);
         tab2[i] = w;
+        if (kX32) tab2r[i] = make_uint2(rest_pair(v[0], v[1], w.x, w.z), rest_pair(v[2], v[3], w.y, w.w));
     }
     __syncthreads();
     const float inv_scale = rsqrtf((float)D);
@@ -164,13 +183,11 @@ bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
                     const uint4 b = tab1[(nt * NJ + j) * 32 + lane];
                     if constexpr (kX32) {
                         const uint2 r = tab1r[(nt * NJ + j) * 32 + lane];
-                        mma_bf16_16816(acc[nt], ar, b.x, b.y);
-                        mma_bf16_16816(acc[nt], alo, b.z, b.w);
-                        mma_bf16_16816(acc[nt], ahi, r.x, r.y);
-                        mma_bf16_16816(acc[nt], alo, b.x, b.y);
+                        six_products(acc[nt], ahi, alo, ar, b, r);
+                    } else {
+                        mma_bf16_16816(acc[nt], ahi, b.z, b.w);
+                        mma_bf16_16816(acc[nt], ahi, b.x, b.y);
                     }
-                    mma_bf16_16816(acc[nt], ahi, b.z, b.w);
-                    mma_bf16_16816(acc[nt], ahi, b.x, b.y);
                 }
             }
         }
@@ -222,13 +239,14 @@ bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
             }
         }
         // A fragments of the second product: slots 4 j .. 4 j + 3 of both rows
-        uint32_t ahi[KS][4], alo[KS][4];
+        uint32_t ahi[KS][4], alo[KS][4], ar[KS][4];
 #pragma unroll
         for (int j = 0; j < KS; ++j)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                split_pair(acc[2 * j][2 * h], acc[2 * j][2 * h + 1], ahi[j][h], alo[j][h]);
-                split_pair(acc[2 * j + 1][2 * h], acc[2 * j + 1][2 * h + 1], ahi[j][2 + h], alo[j][2 + h]);
+            for (int i = 0; i < 4; ++i) {
+                const int nt = 2 * j + (i >> 1), h = i & 1;
+                split_pair(acc[nt][2 * h], acc[nt][2 * h + 1], ahi[j][i], alo[j][i]);
+                if (kX32) ar[j][i] = rest_pair(acc[nt][2 * h], acc[nt][2 * h + 1], ahi[j][i], alo[j][i]);
             }
 #pragma unroll
         for (int m = 0; m < D / 32; ++m) {
@@ -240,9 +258,14 @@ bucket_probs_bwd_mma(const Tx* x0, const Tx* x1, const float* planes,
 #pragma unroll
                 for (int j = 0; j < KS; ++j) {
                     const uint4 b = tab2[((4 * m + i) * KS + j) * 32 + lane];
-                    mma_bf16_16816(o[i], ahi[j], b.z, b.w);
-                    mma_bf16_16816(o[i], alo[j], b.x, b.y);
-                    mma_bf16_16816(o[i], ahi[j], b.x, b.y);
+                    if constexpr (kX32) {
+                        const uint2 r = tab2r[((4 * m + i) * KS + j) * 32 + lane];
+                        six_products(o[i], ahi[j], alo[j], ar[j], b, r);
+                    } else {
+                        mma_bf16_16816(o[i], ahi[j], b.z, b.w);
+                        mma_bf16_16816(o[i], alo[j], b.x, b.y);
+                        mma_bf16_16816(o[i], ahi[j], b.x, b.y);
+                    }
                 }
             }
 #pragma unroll
