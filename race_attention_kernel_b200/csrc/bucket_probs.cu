@@ -285,6 +285,41 @@ __device__ __forceinline__ void pack8(const float* v, uint4& w) {
     w.z = *reinterpret_cast<uint32_t*>(&c); w.w = *reinterpret_cast<uint32_t*>(&d);
 }
 
+// Products of the planes' probabilities 1/2 -+ half, rounded once: the two halves of a bucket's bits as unevaluated sums
+// hi + lo, then one fused product per bucket.  Rounded at every factor they are 9e-8 off, which is more than a softmax in
+// fp32 (fp32, d_k = 128, K = 6: outputs 1.06e-7 against 0.69e-7 off the 64-bit result).
+template <int N>
+__device__ __forceinline__ void exact_half(const float* half, float (&hi)[1 << N], float (&lo)[1 << N]) {
+    hi[0] = 1.f;
+    lo[0] = 0.f;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const float p1 = 0.5f + half[k], p0 = 0.5f - half[k];
+        const float e1 = half[k] - (p1 - 0.5f), e0 = (0.5f - p0) - half[k];   // exact: what the sums lost
+#pragma unroll
+        for (int i = (1 << N) / 2 - 1; i >= 0; --i)
+            if (i < (1 << k)) {
+                const float h = hi[i], l = lo[i];
+                hi[2 * i] = h * p0;
+                lo[2 * i] = fmaf(h, p0, -hi[2 * i]) + fmaf(h, e0, l * p0);
+                hi[2 * i + 1] = h * p1;
+                lo[2 * i + 1] = fmaf(h, p1, -hi[2 * i + 1]) + fmaf(h, e1, l * p1);
+            }
+    }
+}
+template <int K>
+__device__ __forceinline__ void exact_products(const float (&half)[K], float (&vals)[1 << K]) {
+    constexpr int KB = K / 2, KA = K - KB;   // the first planes are the upper bits of a bucket
+    float ah[1 << KA], al[1 << KA], bh[1 << KB], bl[1 << KB];
+    exact_half<KA>(half, ah, al);
+    exact_half<KB>(half + KA, bh, bl);
+#pragma unroll
+    for (int i = 0; i < (1 << KA); ++i)
+#pragma unroll
+        for (int j = 0; j < (1 << KB); ++j)
+            vals[(i << KB) + j] = fmaf(ah[i], bh[j], fmaf(ah[i], bl[j], al[i] * bh[j]));
+}
+
 // kExact (fp32 rows): three limbs of rows and planes in six products, the accuracy of an fp32 product, for the forward
 // of a training step: the gradients of the probabilities nearly cancel over a table, which magnifies the 2^-17 of two.
 template <int D, int L, int K, typename Tx, typename Tp, bool kExact>
@@ -407,7 +442,7 @@ bucket_probs_mma_wide(const Tx* x0, const Tx* x1, const float* planes,
         for (int h = 0; h < 2; ++h) {
 #pragma unroll
             for (int tb = 0; tb < TPL; ++tb) {
-                float p0[K], p1[K];
+                float p0[K], p1[K], half_bit[K];
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
                     const int s = tb * K + k, nt = s >> 1, i = 2 * h + (s & 1);
@@ -420,18 +455,23 @@ bucket_probs_mma_wide(const Tx* x0, const Tx* x1, const float* planes,
                     const float half = 0.5f * th * poly;
                     p1[k] = 0.5f + half;
                     p0[k] = 0.5f - half;
+                    half_bit[k] = half;
                 }
                 float vals[R];
-                vals[0] = p0[0];
-                vals[1] = p1[0];
+                if constexpr (kExact) {
+                    exact_products<K>(half_bit, vals);
+                } else {
+                    vals[0] = p0[0];
+                    vals[1] = p1[0];
 #pragma unroll
-                for (int k = 1; k < K; ++k) {
+                    for (int k = 1; k < K; ++k) {
 #pragma unroll
-                    for (int i = R / 2 - 1; i >= 0; --i) {     // constant bounds: every index is known at compile time
-                        if (i < (1 << k)) {
-                            const float b = vals[i];
-                            vals[2 * i] = b * p0[k];
-                            vals[2 * i + 1] = b * p1[k];
+                        for (int i = R / 2 - 1; i >= 0; --i) {     // constant bounds: every index is known at compile time
+                            if (i < (1 << k)) {
+                                const float b = vals[i];
+                                vals[2 * i] = b * p0[k];
+                                vals[2 * i + 1] = b * p1[k];
+                            }
                         }
                     }
                 }

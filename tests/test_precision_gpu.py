@@ -52,3 +52,10 @@ def test_gradient_of_the_producer_in_fp32(dk, L, K):
     (ref,) = torch.autograd.grad(_probs64(x64, planes, L, K), x64, dp.double())
     assert ro.rel_l2(ops.bucket_probs_streams_bwd(x, planes, dp, L, K), ref) <= 10 * 2.0 ** -24
 
+
+@pytest.mark.parametrize("dk,L,K", [(64, 4, 4), (128, 8, 6)])
+def test_probabilities_of_a_training_step_in_fp32(dk, L, K):
+    """Rounded once: at most 2^-24, a little over half of that in the mean square, and 1e-8 from the projections."""
+    import race_attention_kernel_b200.ops as ops
+    x, planes, _ = _rows(dk, L, K)
+    assert ro.rel_l2(ops.bucket_probs_streams(x, planes, L, K, exact=True), _probs64(x.double(), planes, L, K)) <= 4.5e-8
