@@ -221,7 +221,9 @@ int race_b200_causal_fwd_heads(const void* probs_q, const void* probs_k, const v
 
 /*
  * race_b200_causal_bwd_carry with v, d_out and d_v in the operator's layout [n_streams/heads, seq_len, heads, d_k] when
- * shape->heads > 1 (fp32 with L*R = 64, d_k = 64; bf16 with L*R 64, 128, 256 or 512, d_k 64 or 128; race_b200_causal_bwd_workspace_bytes is 0 where it is not built).
+ * shape->heads > 1 (fp32 with L*R = 64, d_k = 64; bf16 with L*R 64, 128, 256 or 512, d_k 64 or 128;
+ * race_b200_causal_bwd_workspace_bytes is 0 where it is not built).  bf16 with heads > 1 forms d_carry_in on the tensor cores
+ * too, from two 16-bit limbs of its operands (8e-6 off); with heads <= 1 it has the precision of fp32 products.
  */
 int race_b200_causal_bwd_heads(const void* probs_q, const void* probs_k, const void* v, const void* d_out,
                                const float* carry_in, const float* d_state_out, void* d_probs_q, void* d_probs_k,

@@ -567,16 +567,23 @@ bool causal_bwd_supported(const Dims& dm, int dtype) {
                                   (dtype == RACE_DTYPE_BF16 && causal_bwd_bf16_supported(dm)));
 }
 
-int causal_bwd_tile_tokens(const Dims& dm, int dtype, int sm_count) {
-    if (dtype == RACE_DTYPE_BF16 && causal_bwd_bf16_supported(dm)) return causal_bwd_bf16_tile_tokens(dm, sm_count);
+// bf16 on the tensor cores, unless the gradient of a carried-in state is asked for: that is an fp32 tensor, and the two-limb
+// products there leave it 8e-6 (A part) and 7e-7 (B part) off the 64-bit result, where the fp32 products here are 2e-7 off.
+// (V, dO, dV with heads have the tensor kernels only.)
+static bool bwd_on_bf16_tensor(const Dims& dm, int dtype, bool grad_carry) {
+    return dtype == RACE_DTYPE_BF16 && causal_bwd_bf16_supported(dm) && !(grad_carry && dm.H == 1);
+}
+
+int causal_bwd_tile_tokens(const Dims& dm, int dtype, int sm_count, bool grad_carry) {
+    if (bwd_on_bf16_tensor(dm, dtype, grad_carry)) return causal_bwd_bf16_tile_tokens(dm, sm_count);
     if (causal_bwd_tensor_supported(dm, dtype)) return causal_bwd_tensor_tile_tokens(dm, sm_count);
     return simt_default_tile_tokens(dm, sm_count);
 }
 
 // [prefix tile states | suffix tile states | W | g], each part 256-byte aligned
-size_t causal_bwd_workspace_bytes(const Dims& dm, int dtype, int tile_tokens) {
+size_t causal_bwd_workspace_bytes(const Dims& dm, int dtype, int tile_tokens, bool grad_carry) {
     if (dm.N == 0 || dm.T == 0) return 0;
-    if (dtype == RACE_DTYPE_BF16 && causal_bwd_bf16_supported(dm)) return causal_bwd_bf16_workspace_bytes(dm, tile_tokens);
+    if (bwd_on_bf16_tensor(dm, dtype, grad_carry)) return causal_bwd_bf16_workspace_bytes(dm, tile_tokens);
     if (causal_bwd_tensor_supported(dm, dtype)) return causal_bwd_tensor_workspace_bytes(dm, tile_tokens);
     const int64_t tiles = (dm.T + tile_tokens - 1) / tile_tokens;
     const size_t states = align256((size_t)dm.N * tiles * state_floats_per_stream(dm.S, dm.D) * sizeof(float));
@@ -587,7 +594,7 @@ size_t causal_bwd_workspace_bytes(const Dims& dm, int dtype, int tile_tokens) {
 cudaError_t causal_bwd_simt(const void* pq, const void* pk, const void* v, const void* dout, const float* carry_in,
                             const float* d_state, void* dpq, void* dpk, void* dv, float* d_carry, void* ws,
                             const Dims& dm, int dtype, int tile_tokens, cudaStream_t stream, int* status) {
-    if (dtype == RACE_DTYPE_BF16 && causal_bwd_bf16_supported(dm))
+    if (bwd_on_bf16_tensor(dm, dtype, d_carry != nullptr))
         return causal_bwd_bf16(pq, pk, v, dout, carry_in, d_state, dpq, dpk, dv, d_carry, ws, dm, tile_tokens, stream, status);
     // fp32, S = 64, d_k = 64: the backward as passes of the tcgen05 forward kernels
     if (causal_bwd_tensor_supported(dm, dtype))

@@ -73,8 +73,9 @@ inline bool fold_carry(int64_t N, int64_t tiles, int64_t state_floats, const flo
 
 // ---- causal backward (causal_bwd_simt.cu): S <= 64, d_k <= 128 ---------------------------------
 bool causal_bwd_supported(const Dims& dm, int dtype);
-int causal_bwd_tile_tokens(const Dims& dm, int dtype, int sm_count);
-size_t causal_bwd_workspace_bytes(const Dims& dm, int dtype, int tile_tokens);
+// grad_carry: with the gradient of a carried-in state
+int causal_bwd_tile_tokens(const Dims& dm, int dtype, int sm_count, bool grad_carry);
+size_t causal_bwd_workspace_bytes(const Dims& dm, int dtype, int tile_tokens, bool grad_carry);
 // carry_in: state before the first token (nullable); d_state: gradient reaching the state after the last token
 // (nullable); d_carry: receives the gradient of carry_in (nullable)
 cudaError_t causal_bwd_simt(const void* pq, const void* pk, const void* v, const void* dout, const float* carry_in,

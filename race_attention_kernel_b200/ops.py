@@ -495,6 +495,13 @@ def race_causal_backward(probsQ, probsK, V, grad_out, eps: float = 1e-6, *, carr
     N, T, L, R, dk = _check_inputs(probsQ, probsK, V)
     if grad_out.shape != V.shape or not grad_out.is_cuda:
         raise RuntimeError("grad_out must be a CUDA tensor shaped like V")
+    if V.dim() == 5 and return_grad_carry and V.dtype == torch.bfloat16:
+        # the kernels that form this fp32 result with fp32 products take streams
+        M, B, _, H, _ = V.shape
+        V2, g2 = (t.permute(0, 1, 3, 2, 4).reshape(N, T, dk) for t in (V, grad_out))
+        dpq, dpk, dv, dcarry = race_causal_backward(probsQ, probsK, V2, g2, eps, carry_in=carry_in, grad_state=grad_state,
+                                                    return_grad_carry=True)
+        return dpq, dpk, dv.view(M, B, H, T, dk).permute(0, 1, 3, 2, 4).contiguous(), dcarry
     # autograd may hand over an expanded (stride-0) gradient: the kernels need dense rows
     grad_out = grad_out.to(V.dtype).contiguous()
     L_ = _lib.lib()

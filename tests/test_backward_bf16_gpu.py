@@ -4,6 +4,8 @@ from __future__ import annotations
 import pytest
 import torch
 
+from oracle import race_oracle as ro
+
 pytestmark = pytest.mark.gpu
 
 GEOMETRIES = [(L, R, dk) for L, R in ((4, 16), (2, 64), (4, 64), (8, 64)) for dk in (64, 128)]
@@ -52,4 +54,43 @@ def test_outputs_that_begin_between_two_sectors(L, R, dk):
                                          ctypes.byref(sh), ops._stream(), None)
     assert rc == 0
     for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
+def _reference(pq, pk, v, dO, A0, B0, d_state):
+    """Gradients in 64 bits of one chunk (src/race_baseline.py:45-51 with the state of the tokens before it)."""
+    q, k, x, a, b = (t.double().requires_grad_(True) for t in (pq.flatten(2), pk.flatten(2), v, A0.flatten(1), B0.flatten(1, 2)))
+    w = q / (a.unsqueeze(1) + k.cumsum(1) + 1e-6)
+    out = torch.tril(w @ k.transpose(1, 2)) @ x + w @ b
+    state = torch.cat([(b + k.transpose(1, 2) @ x).flatten(1), a + k.sum(1)], 1)
+    dq, dk, dx, da, db = torch.autograd.grad((out, state), (q, k, x, a, b), (dO.double(), d_state.double()))
+    return dq.view_as(pq), dk.view_as(pk), dx, torch.cat([db.flatten(1), da], 1)
+
+
+@pytest.mark.parametrize("L,R,dk", GEOMETRIES)
+@pytest.mark.parametrize("T", [1, 128, 129, 1500])
+def test_chunk_of_a_longer_sequence(L, R, dk, T):
+    import race_attention_kernel_b200.ops as ops
+    N, S = 4, L * R
+    pq, pk, v, dO = _inputs(N, T, L, R, dk, seed=T + S + dk)
+    g = torch.Generator(device="cuda").manual_seed(T)
+    A0 = torch.rand(N, L, R, device="cuda", generator=g) * 20 + 1
+    B0 = torch.randn(N, L, R, dk, device="cuda", generator=g) * 5
+    d_state = torch.randn(N, S * (dk + 1), device="cuda", generator=g)
+    kw = dict(carry_in=ops.pack_state(A0, B0), grad_state=d_state)
+    ref = _reference(pq, pk, v, dO, A0, B0, d_state)
+    for got in (ops.race_causal_backward(pq, pk, v, dO, **kw),
+                ops.race_causal_backward(pq, pk, v, dO, return_grad_carry=True, **kw)):
+        for a, b in zip(got[:3], ref):      # nothing but the results is rounded to bf16: 2^-9
+            assert ro.rel_l2(a, b) <= 4e-3
+    # the gradient of the carry is an fp32 tensor: fp32 products and sums of T terms
+    assert ro.rel_l2(got[3][:, S * dk:], ref[3][:, S * dk:]) <= 1e-6
+    assert ro.rel_l2(got[3][:, :S * dk], ref[3][:, :S * dk]) <= 1e-6
+    # V and the gradient in the operator's layout, as two heads
+
+    def operator_layout(x):
+        return x.view(1, 2, 2, T, dk).permute(0, 1, 3, 2, 4).contiguous()
+
+    heads = ops.race_causal_backward(pq, pk, operator_layout(v), operator_layout(dO), return_grad_carry=True, **kw)
+    for a, b in zip(heads, (got[0], got[1], operator_layout(got[2]), got[3])):
         assert torch.equal(a, b)
