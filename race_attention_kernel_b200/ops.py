@@ -540,10 +540,10 @@ class _RaceCausalChunk(torch.autograd.Function):
     def backward(ctx, grad_out, grad_state):
         probsQ, probsK, V, state = ctx.saved_tensors
         gs = None if grad_state is None else grad_state.float().contiguous()
-        dpq, dpk, dv, dcarry = race_causal_backward(probsQ, probsK, V, grad_out, ctx.eps, carry_in=state,
-                                                    grad_state=gs, return_grad_carry=True)
         g = ctx.needs_input_grad
-        return (dpq if g[0] else None, dpk if g[1] else None, dv if g[2] else None, dcarry if g[3] else None, None)
+        dpq, dpk, dv, *dcarry = race_causal_backward(probsQ, probsK, V, grad_out, ctx.eps, carry_in=state,
+                                                     grad_state=gs, return_grad_carry=g[3])
+        return (dpq if g[0] else None, dpk if g[1] else None, dv if g[2] else None, dcarry[0] if g[3] else None, None)
 
 
 def race_causal_chunk(probsQ, probsK, V, state, eps: float = 1e-6):
