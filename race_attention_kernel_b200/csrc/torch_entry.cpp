@@ -55,6 +55,12 @@ at::Tensor planes_rows(const at::Tensor& planes_T, const at::Tensor& ref) {
     return p.contiguous();
 }
 
+// The kernels want 16-byte boundaries.  A contiguous tensor off them is refused by the C entries, except where this package
+// has always copied it on the way: then it is copied here.
+at::Tensor on_boundary(const at::Tensor& t, bool copies) {
+    return copies && (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15) ? t.clone() : t;
+}
+
 struct Fail : std::exception {
     std::string msg;
     explicit Fail(std::string m) : msg(std::move(m)) {}
@@ -102,10 +108,10 @@ PyObject* step_impl(PyObject* const* args, Py_ssize_t nargs) {
         N == 0 || T == 0 || !race_b200_decode_qkv_is_supported(&sh, (int)P))
         return none();
     c10::cuda::CUDAGuard guard(k->device());
-    const at::Tensor planes = planes_rows(*pt, *k);
+    const at::Tensor planes = planes_rows(*pt, *k), va = on_boundary(*v, H > 1 && T > 1);
     at::Tensor out = at::empty(k->sizes(), k->options());
     float* state = st->data_ptr<float>();
-    check(race_b200_decode_step_qkv(k->const_data_ptr(), v->const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
+    check(race_b200_decode_step_qkv(k->const_data_ptr(), va.const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
                                     out.data_ptr(), state, state, &sh, (int)P, c10::cuda::getCurrentCUDAStream().stream()),
           "race_b200_decode_step_qkv");
     return THPVariable_Wrap(out);
@@ -146,11 +152,12 @@ PyObject* forward_impl(PyObject* const* args, Py_ssize_t nargs) {
               "race_b200_causal_fwd_qkv");
     } else {
         at::Tensor pk = at::empty({N, T, L, R}, k->options()), pq = at::empty({N, T, L, R}, k->options());
+        const at::Tensor va = on_boundary(*v, H > 1 && T > 1 && !race_b200_is_supported(&sh, RACE_VARIANT_AUTO));
         check(race_b200_bucket_probs_streams_pair(k->const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
                                                   pk.data_ptr(), pq.data_ptr(), MB, T, (int32_t)H, (int32_t)dk, (int32_t)L,
                                                   (int32_t)P, sh.dtype, 0, stream),
               "race_b200_bucket_probs_streams_pair");
-        check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), v->const_data_ptr(), out.data_ptr(), carry_p,
+        check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), va.const_data_ptr(), out.data_ptr(), carry_p,
                                          state_p, ws.data_ptr(), wb, &sh, stream, status),
               "race_b200_causal_fwd_heads");
     }
@@ -195,11 +202,13 @@ struct TrainOp : torch::autograd::Function<TrainOp> {
                          dtype_of(k), (float)eps, (int32_t)k.size(3)};
     }
 
-    static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& k, const at::Tensor& v,
-                              const at::Tensor& q, const at::Tensor& planes, int64_t L, int64_t P, double eps, int64_t status) {
-        c10::cuda::CUDAGuard guard(k.device());
+    static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& k_in, const at::Tensor& v_in,
+                              const at::Tensor& q_in, const at::Tensor& planes_in, int64_t L, int64_t P, double eps, int64_t status) {
+        c10::cuda::CUDAGuard guard(k_in.device());
         void* stream = c10::cuda::getCurrentCUDAStream().stream();
-        const RaceShape sh = shape(k, L, P, eps);
+        const RaceShape sh = shape(k_in, L, P, eps);
+        const at::Tensor k = on_boundary(k_in, true), q = on_boundary(q_in, true), planes = on_boundary(planes_in, true),
+                         v = on_boundary(v_in, sh.heads > 1 && sh.seq_len > 1);
         at::Tensor pk = at::empty({sh.n_streams, sh.seq_len, L, 1ll << P}, k.options()), pq = at::empty_like(pk);
         check(race_b200_bucket_probs_streams_pair(k.const_data_ptr(), q.const_data_ptr(), planes.const_data_ptr<float>(),
                                                   pk.data_ptr(), pq.data_ptr(), k.size(0) * k.size(1), sh.seq_len, sh.heads,
@@ -230,7 +239,7 @@ struct TrainOp : torch::autograd::Function<TrainOp> {
             c10::cuda::CUDAGuard guard(k.device());
             void* stream = c10::cuda::getCurrentCUDAStream().stream();
             const RaceShape sh = shape(k, L, P, ctx->saved_data["eps"].toDouble());
-            const at::Tensor g = grads[0].to(v.scalar_type()).contiguous();   // may come expanded (stride 0)
+            const at::Tensor g = on_boundary(grads[0].to(v.scalar_type()).contiguous(), true);   // may come expanded (stride 0)
             at::Tensor dpq = at::empty_like(pq), dpk = at::empty_like(pk), dv = at::empty(v.sizes(), v.options());
             const size_t wb = race_b200_causal_bwd_workspace_bytes(&sh);
             at::Tensor ws = bytes(wb, k);

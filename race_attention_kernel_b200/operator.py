@@ -33,9 +33,12 @@ class _CausalOperator(torch.autograd.Function):
     @staticmethod
     def forward(ctx, Khf, Vhf, Qhf, planes, L, K, eps):
         M, B, T, H, dk = Khf.shape
+        Khf, Qhf, planes = (_on_boundary(t) for t in (Khf, Qhf, planes))
         pK = ops.bucket_probs_streams(Khf, planes, L, K, exact=True)
         pQ = ops.bucket_probs_streams(Qhf, planes, L, K, exact=True)
         shape = (M * B * H, T, L, 1 << K, dk, Vhf.dtype)
+        if H > 1 and T > 1:
+            Vhf = _on_boundary(Vhf)
         V2 = None
         if ops.is_supported(*shape, "auto", heads=H):
             out = ops.race_causal_prefix(pQ, pK, Vhf, eps)
@@ -57,7 +60,7 @@ class _CausalOperator(torch.autograd.Function):
         want_k, want_v, want_q = ctx.needs_input_grad[:3]
         grad_out = grad_out.to(V.dtype)
         if ctx.bwd_heads:
-            dpq, dpk, dV = ops.race_causal_backward(pQ, pK, V, grad_out, ctx.eps)
+            dpq, dpk, dV = ops.race_causal_backward(pQ, pK, V, _on_boundary(grad_out.contiguous()), ctx.eps)
         else:
             V2 = V if V.dim() == 3 else _streams(V)
             dpq, dpk, dV = ops.race_causal_backward(pQ, pK, V2, _streams(grad_out), ctx.eps)
@@ -65,6 +68,11 @@ class _CausalOperator(torch.autograd.Function):
         dK = ops.bucket_probs_streams_bwd(Khf, planes, dpk, L, K) if want_k else None
         dQ = ops.bucket_probs_streams_bwd(Qhf, planes, dpq, L, K) if want_q else None
         return dK, dV if want_v else None, dQ, None, None, None, None
+
+
+def _on_boundary(x: torch.Tensor) -> torch.Tensor:
+    """The kernels want 16-byte boundaries; gradients are also given for rows that begin elsewhere."""
+    return x if x.data_ptr() % 16 == 0 else x.clone()
 
 
 def _streams(x: torch.Tensor) -> torch.Tensor:

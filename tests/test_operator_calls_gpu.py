@@ -62,3 +62,43 @@ def test_steps_of_different_lengths_from_two_threads():
     for t in threads:
         t.join()
     assert codes == {64: {0}, 20: {0}}
+
+
+def _off_boundary(x):
+    """The same values in a contiguous tensor that begins 4 bytes (bf16: 2) after a 16-byte boundary."""
+    y = torch.empty(x.numel() + 1, device=x.device, dtype=x.dtype)[1:].view_as(x).copy_(x)
+    assert y.is_contiguous() and y.data_ptr() % 16
+    return y
+
+
+@pytest.mark.parametrize("dk,K,L,dt", [(64, 4, 4, torch.float32), (64, 4, 4, torch.bfloat16), (128, 6, 8, torch.bfloat16),
+                                       (128, 6, 8, torch.float32)])
+def test_training_takes_rows_off_the_boundary(dk, K, L, dt):
+    ace, x = _ace(dk, K, L), _inputs(1, 150, 3, dk, dt, n=4)
+
+    def grads(inputs, g):
+        leaves = [t.requires_grad_(True) for t in inputs]
+        out = ace(*leaves)
+        return (out.detach(), *torch.autograd.grad(out, leaves, g))
+
+    want = grads([t.clone() for t in x[:3]], x[3])
+    for i in range(3):
+        got = grads([_off_boundary(t) if i == j else t.clone() for j, t in enumerate(x[:3])], x[3])
+        assert all(map(torch.equal, got, want))
+    assert all(map(torch.equal, grads([t.clone() for t in x[:3]], _off_boundary(x[3])), want))
+    ace.planes_T = _off_boundary(ace.planes_T.T.contiguous()).T
+    assert all(map(torch.equal, grads([t.clone() for t in x[:3]], x[3]), want))
+
+
+def test_v_off_the_boundary_where_it_was_always_copied():
+    ace, (k, v, q) = _ace(), _inputs(1, 150, 3, 64, torch.bfloat16)
+    with torch.no_grad():
+        assert torch.equal(ace(k, _off_boundary(v), q), ace(k, v, q))
+        with pytest.raises(RuntimeError, match="aligned"):
+            ace(_off_boundary(k), v, q)
+    states = [torch.zeros(3, 64 * 65, device="cuda") for _ in range(2)]
+    k, v, q = (t[:, :, :5].contiguous() for t in (k, v, q))
+    assert torch.equal(ace.step(k, _off_boundary(v), q, states[0]), ace.step(k, v, q, states[1]))
+    assert torch.equal(*states)
+    with pytest.raises(RuntimeError, match="aligned"):
+        ace.step(_off_boundary(k), v, q, states[0])
