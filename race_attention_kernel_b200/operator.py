@@ -18,6 +18,7 @@ the bucket probabilities with differentiable torch ops and run the prefix path t
 """
 from __future__ import annotations
 
+import functools
 import itertools
 
 import torch
@@ -70,6 +71,12 @@ class _CausalOperator(torch.autograd.Function):
         return dK, dV if want_v else None, dQ, None, None, None, None
 
 
+@functools.cache
+def _corners(K: int) -> torch.Tensor:
+    """[K, 2**K] (src/race_baseline.py:30-32), on the host; not to be written to."""
+    return torch.tensor(list(itertools.product([-1.0, 1.0], repeat=K)), dtype=torch.float64, device="cpu").T
+
+
 def _on_boundary(x: torch.Tensor) -> torch.Tensor:
     """The kernels want 16-byte boundaries; gradients are also given for rows that begin elsewhere."""
     return x if x.data_ptr() % 16 == 0 else x.clone()
@@ -95,8 +102,7 @@ class BatchedACE(nn.Module):
         # construction gives the same planes
         planes = torch.randn(L, K, d_k, device=device)
         self.register_buffer("planes_T", planes.view(L * K, d_k).T)
-        corners = torch.tensor(list(itertools.product([-1.0, 1.0], repeat=K)), device=device)
-        self.register_buffer("protos_T", corners.T)
+        self.register_buffer("protos_T", _corners(K).to(device, torch.get_default_dtype(), copy=True))
         self.eps = 1e-6
         self.variant = "auto"
         # form the bucket probabilities inside the prefix kernels where that path exists (fp32, d_k = 64, L = 4,
@@ -120,11 +126,32 @@ class BatchedACE(nn.Module):
         logits = proj.tanh().div(dk ** 0.5) @ protos_T
         return torch.softmax(logits, dim=-1).to(x2.dtype)
 
+    def _protos_are_corners(self) -> bool:
+        """Whether ``protos_T`` holds what the kernels are built on: training honours other prototypes, with torch ops.
+        Compared by value, which reads back from the GPU, when the buffer is another tensor than at the last comparison or
+        has been written to since (its version counter; writes through ``.data`` are not counted by torch)."""
+        p = self.protos_T
+        if p.requires_grad:
+            return False
+        seen = self.__dict__.get("_protos_seen")
+        if seen is None or p.is_inference() or seen[0] is not p or seen[1:3] != (p._version, p.data_ptr()):
+            same = torch.equal(p.detach().to("cpu", torch.float64), _corners(self.K))
+            if p.is_inference():
+                return same
+            seen = self.__dict__["_protos_seen"] = (p, p._version, p.data_ptr(), same)
+        return seen[3]
+
+    def _apply(self, fn, *args, **kwargs):
+        super()._apply(fn, *args, **kwargs)
+        if not self.protos_T.is_meta:
+            self._protos_are_corners()   # read back here, where tensors move anyway, and not in the first training step
+        return self
+
     def _forward_autograd(self, Khf, Vhf, Qhf):
         M, B, T, H, dk = Khf.shape
         dev = self.planes_T.device if self.planes_T.is_cuda else torch.device("cuda", torch.cuda.current_device())
         if (ops.bucket_probs_bwd_is_supported(dk, self.L, self.K, Khf.dtype)
-                and not (self.planes_T.requires_grad or self.protos_T.requires_grad)):
+                and not self.planes_T.requires_grad and self._protos_are_corners()):
             planes = self.planes_T.T.contiguous().float().to(dev)
             out = _CausalOperator.apply(*(t.to(dev).contiguous() for t in (Khf, Vhf, Qhf)), planes, self.L, self.K, self.eps)
             return out if Khf.is_cuda else out.cpu()
@@ -152,7 +179,7 @@ class BatchedACE(nn.Module):
             if carry_in is not None or return_state:
                 raise RuntimeError("carry_in / return_state are inference-only; chain ops.race_causal_chunk "
                                    "for differentiable chunked sequences")
-            if Khf.is_cuda and not self.protos_T.requires_grad:
+            if Khf.is_cuda and self._protos_are_corners():
                 out = _lib.native().train_forward(self.planes_T, Khf, Vhf, Qhf, self.L, self.K, self.eps,
                                                   ops._status_ptr(Khf.get_device()))
                 if out is not None:

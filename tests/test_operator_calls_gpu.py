@@ -102,3 +102,38 @@ def test_v_off_the_boundary_where_it_was_always_copied():
     assert torch.equal(*states)
     with pytest.raises(RuntimeError, match="aligned"):
         ace.step(_off_boundary(k), v, q, states[0])
+
+
+def test_training_honours_other_prototypes():
+    """Assigned, written in place or loaded; and the corners again, however they come back."""
+    import copy
+    ace, x = _ace(), _inputs(1, 70, 2, 64, torch.float32)
+
+    def out(module=ace):
+        return module(x[0].clone().requires_grad_(True), x[1], x[2]).detach()
+
+    def by_hand(protos):
+        p = [torch.softmax(((t.double().permute(0, 1, 3, 2, 4).reshape(2, 70, 64) @ ace.planes_T.double()).view(2, 70, 4, 4).tanh() / 8)
+                           @ protos.double(), -1).flatten(2) for t in (x[0], x[2])]
+        v = x[1].double().permute(0, 1, 3, 2, 4).reshape(2, 70, 64)
+        o = torch.tril((p[1] / (p[0].cumsum(1) + ace.eps)) @ p[0].transpose(1, 2)) @ v
+        return o.view(1, 1, 2, 70, 64).permute(0, 1, 3, 2, 4)
+
+    def close(a, b):
+        return float((a - b).norm() / b.norm()) < 3e-5
+
+    corners = ace.protos_T.clone()
+    other = corners * torch.linspace(8.0, 12.0, 16, device="cuda")
+    want, want_other = out(), by_hand(other)
+    assert close(want, by_hand(corners)) and not close(want, want_other)
+    ace.protos_T = other
+    assert close(out(), want_other)
+    ace.protos_T = corners.clone()
+    assert torch.equal(out(), want)
+    with torch.no_grad():
+        ace.protos_T.copy_(other)
+    assert close(out(), want_other) and close(out(copy.deepcopy(ace)), want_other)
+    ace.load_state_dict({**ace.state_dict(), "protos_T": corners})
+    assert torch.equal(out(), want) and torch.equal(out(copy.deepcopy(ace)), want)
+    ace.load_state_dict({**ace.state_dict(), "protos_T": other})
+    assert close(out(), want_other)
