@@ -84,6 +84,16 @@ void raise_on_wait(int* status, const char* what) {
 
 PyObject* none() { Py_RETURN_NONE; }
 
+// Other Python threads run while a call allocates and launches (a full launch queue, or the synchronisation with
+// RACE_B200_CHECK_STATUS=1, would hold them up), as they did when the calls went through ctypes.  No Python object may be
+// touched meanwhile; hooks and modes of torch take the lock for themselves.
+struct WithoutGil {
+    PyThreadState* state = PyEval_SaveThread();
+    WithoutGil() = default;
+    WithoutGil(const WithoutGil&) = delete;
+    ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 // out, or (out, A [N,L,R], B [N,L,R,d_k]) as views of the packed state
 PyObject* result(const at::Tensor& out, const at::Tensor& state, int64_t N, int64_t L, int64_t R, int64_t dk) {
     if (!state.defined()) return THPVariable_Wrap(out);
@@ -107,13 +117,17 @@ PyObject* step_impl(PyObject* const* args, Py_ssize_t nargs) {
     if (pt->dim() != 2 || pt->size(0) != dk || pt->size(1) != L * P || !state_ok(*st, *k, N * (L << P) * (dk + 1)) ||
         N == 0 || T == 0 || !race_b200_decode_qkv_is_supported(&sh, (int)P))
         return none();
-    c10::cuda::CUDAGuard guard(k->device());
-    const at::Tensor planes = planes_rows(*pt, *k), va = on_boundary(*v, H > 1 && T > 1);
-    at::Tensor out = at::empty(k->sizes(), k->options());
-    float* state = st->data_ptr<float>();
-    check(race_b200_decode_step_qkv(k->const_data_ptr(), va.const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
-                                    out.data_ptr(), state, state, &sh, (int)P, c10::cuda::getCurrentCUDAStream().stream()),
-          "race_b200_decode_step_qkv");
+    at::Tensor out;
+    {
+        WithoutGil unlocked;
+        c10::cuda::CUDAGuard guard(k->device());
+        const at::Tensor planes = planes_rows(*pt, *k), va = on_boundary(*v, H > 1 && T > 1);
+        out = at::empty(k->sizes(), k->options());
+        float* state = st->data_ptr<float>();
+        check(race_b200_decode_step_qkv(k->const_data_ptr(), va.const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
+                                        out.data_ptr(), state, state, &sh, (int)P, c10::cuda::getCurrentCUDAStream().stream()),
+              "race_b200_decode_step_qkv");
+    }
     return THPVariable_Wrap(out);
 }
 
@@ -138,30 +152,34 @@ PyObject* forward_impl(PyObject* const* args, Py_ssize_t nargs) {
                           : race_b200_causal_heads_workspace_bytes(&sh);
     if (!qkv && !wb) return none();
     int* status = (int*)PyLong_AsVoidPtr(args[10]);
-    c10::cuda::CUDAGuard guard(k->device());
-    void* stream = c10::cuda::getCurrentCUDAStream().stream();
-    const at::Tensor planes = planes_rows(*pt, *k);
-    at::Tensor out = at::empty(v->sizes(), v->options());
-    at::Tensor state = want_state ? floats({N, L * R * (dk + 1)}, *k) : at::Tensor();
-    const float* carry_p = carry ? carry->const_data_ptr<float>() : nullptr;
-    float* state_p = want_state ? state.data_ptr<float>() : nullptr;
-    at::Tensor ws = bytes(wb, *k);
-    if (qkv) {
-        check(race_b200_causal_fwd_qkv(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), planes.const_data_ptr<float>(),
-                                       out.data_ptr(), carry_p, state_p, ws.data_ptr(), wb, &sh, (int)P, 0, 0, stream, status),
-              "race_b200_causal_fwd_qkv");
-    } else {
-        at::Tensor pk = at::empty({N, T, L, R}, k->options()), pq = at::empty({N, T, L, R}, k->options());
-        const at::Tensor va = on_boundary(*v, H > 1 && T > 1 && !race_b200_is_supported(&sh, RACE_VARIANT_AUTO));
-        check(race_b200_bucket_probs_streams_pair(k->const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
-                                                  pk.data_ptr(), pq.data_ptr(), MB, T, (int32_t)H, (int32_t)dk, (int32_t)L,
-                                                  (int32_t)P, sh.dtype, 0, stream),
-              "race_b200_bucket_probs_streams_pair");
-        check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), va.const_data_ptr(), out.data_ptr(), carry_p,
-                                         state_p, ws.data_ptr(), wb, &sh, stream, status),
-              "race_b200_causal_fwd_heads");
+    at::Tensor out, state;
+    {
+        WithoutGil unlocked;
+        c10::cuda::CUDAGuard guard(k->device());
+        void* stream = c10::cuda::getCurrentCUDAStream().stream();
+        const at::Tensor planes = planes_rows(*pt, *k);
+        out = at::empty(v->sizes(), v->options());
+        if (want_state) state = floats({N, L * R * (dk + 1)}, *k);
+        const float* carry_p = carry ? carry->const_data_ptr<float>() : nullptr;
+        float* state_p = want_state ? state.data_ptr<float>() : nullptr;
+        at::Tensor ws = bytes(wb, *k);
+        if (qkv) {
+            check(race_b200_causal_fwd_qkv(q->const_data_ptr(), k->const_data_ptr(), v->const_data_ptr(), planes.const_data_ptr<float>(),
+                                           out.data_ptr(), carry_p, state_p, ws.data_ptr(), wb, &sh, (int)P, 0, 0, stream, status),
+                  "race_b200_causal_fwd_qkv");
+        } else {
+            at::Tensor pk = at::empty({N, T, L, R}, k->options()), pq = at::empty({N, T, L, R}, k->options());
+            const at::Tensor va = on_boundary(*v, H > 1 && T > 1 && !race_b200_is_supported(&sh, RACE_VARIANT_AUTO));
+            check(race_b200_bucket_probs_streams_pair(k->const_data_ptr(), q->const_data_ptr(), planes.const_data_ptr<float>(),
+                                                      pk.data_ptr(), pq.data_ptr(), MB, T, (int32_t)H, (int32_t)dk, (int32_t)L,
+                                                      (int32_t)P, sh.dtype, 0, stream),
+                  "race_b200_bucket_probs_streams_pair");
+            check(race_b200_causal_fwd_heads(pq.const_data_ptr(), pk.const_data_ptr(), va.const_data_ptr(), out.data_ptr(), carry_p,
+                                             state_p, ws.data_ptr(), wb, &sh, stream, status),
+                  "race_b200_causal_fwd_heads");
+        }
+        raise_on_wait(status, "BatchedACE.forward");
     }
-    raise_on_wait(status, "BatchedACE.forward");
     return result(out, state, N, L, R, dk);
 }
 
@@ -180,17 +198,21 @@ PyObject* prefix_impl(PyObject* const* args, Py_ssize_t nargs) {
     RaceShape sh{N, T, (int32_t)L, (int32_t)R, (int32_t)dk, dtype_of(*v), (float)PyFloat_AsDouble(args[3]), 0};
     if (!race_b200_is_supported(&sh, RACE_VARIANT_AUTO)) return none();
     int* status = (int*)PyLong_AsVoidPtr(args[6]);
-    c10::cuda::CUDAGuard guard(v->device());
-    at::Tensor out = at::empty(v->sizes(), v->options());
-    at::Tensor state = want_state ? floats({N, L * R * (dk + 1)}, *v) : at::Tensor();
-    const size_t wb = race_b200_causal_workspace_bytes(&sh, 0, RACE_VARIANT_AUTO);
-    at::Tensor ws = bytes(wb, *v);
-    check(race_b200_causal_fwd(pq->const_data_ptr(), pk->const_data_ptr(), v->const_data_ptr(), out.data_ptr(),
-                               carry ? carry->const_data_ptr<float>() : nullptr,
-                               want_state ? state.data_ptr<float>() : nullptr, ws.data_ptr(), wb, &sh, 0, RACE_VARIANT_AUTO,
-                               c10::cuda::getCurrentCUDAStream().stream(), status),
-          "race_b200_causal_fwd");
-    raise_on_wait(status, "race_b200_causal_fwd");
+    at::Tensor out, state;
+    {
+        WithoutGil unlocked;
+        c10::cuda::CUDAGuard guard(v->device());
+        out = at::empty(v->sizes(), v->options());
+        if (want_state) state = floats({N, L * R * (dk + 1)}, *v);
+        const size_t wb = race_b200_causal_workspace_bytes(&sh, 0, RACE_VARIANT_AUTO);
+        at::Tensor ws = bytes(wb, *v);
+        check(race_b200_causal_fwd(pq->const_data_ptr(), pk->const_data_ptr(), v->const_data_ptr(), out.data_ptr(),
+                                   carry ? carry->const_data_ptr<float>() : nullptr,
+                                   want_state ? state.data_ptr<float>() : nullptr, ws.data_ptr(), wb, &sh, 0, RACE_VARIANT_AUTO,
+                                   c10::cuda::getCurrentCUDAStream().stream(), status),
+              "race_b200_causal_fwd");
+        raise_on_wait(status, "race_b200_causal_fwd");
+    }
     return result(out, state, N, L, R, dk);
 }
 
@@ -296,7 +318,12 @@ PyObject* train_impl(PyObject* const* args, Py_ssize_t nargs) {
         !race_b200_causal_heads_workspace_bytes(&sh) || !race_b200_causal_bwd_workspace_bytes(&sh))
         return none();
     const int64_t status = (int64_t)PyLong_AsVoidPtr(args[7]);
-    return THPVariable_Wrap(TrainOp::apply(*k, *v, *q, planes_rows(*pt, *k), L, P, eps, status));
+    at::Tensor out;
+    {
+        WithoutGil unlocked;
+        out = TrainOp::apply(*k, *v, *q, planes_rows(*pt, *k), L, P, eps, status);
+    }
+    return THPVariable_Wrap(out);
 }
 
 template <PyObject* (*kImpl)(PyObject* const*, Py_ssize_t)>

@@ -137,3 +137,35 @@ def test_training_honours_other_prototypes():
     assert torch.equal(out(), want) and torch.equal(out(copy.deepcopy(ace)), want)
     ace.load_state_dict({**ace.state_dict(), "protos_T": other})
     assert close(out(), want_other)
+
+
+@pytest.mark.parametrize("kind", ["forward", "training", "prefix"])
+def test_other_threads_run_while_a_call_waits(kind, monkeypatch):
+    """The call synchronises here (RACE_B200_CHECK_STATUS=1) behind a kernel that keeps the GPU busy for half a second."""
+    import threading
+    import time
+
+    import race_attention_kernel_b200.ops as ops
+    monkeypatch.setenv("RACE_B200_CHECK_STATUS", "1")
+    ace, (k, v, q) = _ace(), _inputs(1, 64, 2, 64, torch.float32)
+    p = torch.softmax(torch.randn(2, 64, 4, 16, device="cuda"), -1)
+    call = {"forward": lambda: ace(k, v, q), "training": lambda: ace(k.requires_grad_(True), v, q),
+            "prefix": lambda: ops.race_causal_prefix(p, p, v[0, 0].permute(1, 0, 2).contiguous())}[kind]
+    call()
+    stamps, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            stamps.append(time.perf_counter())
+            time.sleep(0.005)
+
+    t = threading.Thread(target=tick)
+    t.start()
+    torch.cuda._sleep(int(1e9))
+    t0 = time.perf_counter()
+    call()
+    waited = time.perf_counter() - t0
+    stop.set()
+    t.join()
+    assert waited > 0.2
+    assert max(b - a for a, b in zip(stamps, stamps[1:])) < 0.5 * waited
