@@ -178,7 +178,9 @@ static int causal_entry(const void* probs_q, const void* probs_k, const void* v,
     if (!aligned16(probs_q) || !aligned16(probs_k) || !aligned16(v) || !aligned16(out) ||
         !aligned16(workspace) || !aligned16(carry_in) || !aligned16(state_out))
         return RACE_ERR_ALIGN;
-    if (workspace_bytes < workspace_bytes_for(dm, shape->dtype, var, tile, /*totals_or_resume=*/phases != kPhaseAll))
+    // what race_b200_causal_workspace_bytes says, also where a longer tile would do with less
+    const int asked_tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, var);
+    if (workspace_bytes < workspace_bytes_for(dm, shape->dtype, var, asked_tile, /*totals_or_resume=*/phases != kPhaseAll))
         return RACE_ERR_WORKSPACE;
     if (family(var) == RACE_VARIANT_TENSOR)
         return (int)causal_fwd_tensor(probs_q, probs_k, v, out, carry_in, state_out, workspace,
@@ -423,6 +425,7 @@ int race_b200_noncausal_fwd(const void* probs_q, const void* probs_k, const void
         !aligned16(totals) || !aligned16(workspace))
         return RACE_ERR_ALIGN;
     const int tile = noncausal_totals_tile(shape, dm);
+    if (workspace_bytes < race_b200_causal_workspace_bytes(shape, tile, RACE_VARIANT_AUTO)) return RACE_ERR_WORKSPACE;
     const bool direct = tile >= dm.T;   // one tile per stream: its totals are the state, no workspace between them
     rc = race_b200_tile_totals(probs_k, v, totals, direct ? (void*)totals : workspace,
                                direct ? sf * sizeof(float) : workspace_bytes, shape, tile, RACE_VARIANT_AUTO, stream, nullptr);
