@@ -36,12 +36,7 @@ int check_shape(const RaceShape* sh, Dims* dm) {
     return RACE_OK;
 }
 
-int sm_count() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess)
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 148;
-}
+int sm_count() { return device_sm_count(); }
 
 // the single-pass form exists for the fp32 tensor kernels; everything else about it is the TENSOR family
 inline bool is_single_pass(int variant) { return variant == RACE_VARIANT_TENSOR_SINGLE_PASS; }

@@ -12,8 +12,10 @@ namespace race {
 // launch with programmatic dependence on the kernel before (common.cuh); for kernels in which every thread calls chain_wait
 // before its first access to global memory, so that the launch means the same as a plain one
 // Only for calls of up to 2^17 stream-tokens of 64 buckets, whose kernels take microseconds: in longer ones a successor
-// with 200 KB of shared memory that is resident early takes the L1 from the streaming kernel still running (a training
-// step of 2^19 stream-tokens: 1.32 -> 1.56 ms with every launch chained).
+// with 200 KB of shared memory that is resident early takes the L1 from the streaming kernel still running.  Plain over
+// chained time of whole calls, eight heads, at 2^13 / 2^15 / 2^17 / 2^19: fp32 forward 1.25 / 1.12 / 1.03 / 1.01, training
+// 1.06 / 1.10 / 0.99 / 0.93; bf16 with S = 64 forward 1.10 / 1.16 / 1.01 / 0.93, training 1.03 / 1.03 / 0.93 / 0.90; bf16 with
+// S = 512 forward 1.24 / 1.12 / 1.06 / 1.04, training 1.04 / 1.04 / 1.06 / 0.97.
 inline bool chain_launches(int64_t stream_tokens, int buckets) { return stream_tokens * buckets <= (64ll << 17); }
 inline bool chain_launches(const Dims& dm) { return chain_launches(dm.N * dm.T, dm.S); }
 template <typename... P, typename... A>
@@ -30,6 +32,13 @@ cudaError_t launch_chain(bool chained, void (*kern)(P...), dim3 grid, dim3 block
     cfg.attrs = attr;
     cfg.numAttrs = chained ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
+}
+
+// SMs of the current device (148 where there is none)
+inline int device_sm_count() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 148;
 }
 
 // the driver's tensor-map encoder (causal_tc.cu); null if it cannot be looked up
@@ -58,17 +67,18 @@ cudaError_t causal_scan_tiles(float* ws, const float* carry_in, float* state_out
 constexpr int kPhaseTotals = 1, kPhaseOutput = 2, kPhaseAll = 3, kPhasePrefixOnly = 4;
 
 // Whether the output kernel forms the state before each tile itself (CarryFold) instead of a tile_scan launch between
-// the two.  A launch costs 3 to 5 us in the chain of a small call; folding reads every tile's predecessors again, about
-// tiles^2 / 2 states per stream, from lines of L2 that many CTAs ask for at once: fp32 with 8 streams, 13 tiles (777
-// tokens) 17.8 -> 16.1 us, 16 tiles (4096 tokens) equal,
-// and bf16 with 8 streams, 16 tiles (1000 tokens) 24.9 -> 22.1; hence the line at N tiles^2 = 14 per SM.  One or two
-// tiles: always less than the scan reads and writes (bf16, 48 streams of three tiles: 100 -> 93 us).
+// the two.  A launch costs 2 to 5 us in the chain of a small call; folding reads every tile's predecessors again, about
+// tiles^2 / 2 states per stream, from lines of L2 that many CTAs ask for at once.  Scan over fold time of 64-token tiles:
+// 1.10 wherever N tiles^2 is at most 2048 (1 to 64 streams, 2 to 32 tiles; at least 1.06 with d_k = 128, whose states are twice
+// as large); from 4096 on 0.99 to 1.02 with d_k = 64 and 0.94 to 0.97 with d_k = 128; at 8192 down to 0.96 and 0.78.  Hence
+// the line at N tiles^2 = 14 per SM.  One or two tiles: always less than the scan reads and writes (bf16, 48 streams of three
+// tiles: 100 -> 93 us).
 // A state written over the carry it came from would be read by other tiles' CTAs after the write: scan then.
 inline bool fold_carry(int64_t N, int64_t tiles, int64_t state_floats, const float* carry_in, const float* state_out) {
     if (tiles > 1 && carry_in && state_out && carry_in < state_out + N * state_floats &&
         state_out < carry_in + N * state_floats)
         return false;
-    return tiles <= 2 || (tiles <= 32 && N * tiles * tiles <= 14 * 148);
+    return tiles <= 2 || (tiles <= 32 && N * tiles * tiles <= 14 * (int64_t)device_sm_count());
 }
 
 // ---- causal backward (causal_bwd_simt.cu): S <= 64, d_k <= 128 ---------------------------------
