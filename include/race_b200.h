@@ -23,8 +23,9 @@
  * permuted view of the output (src/race_baseline.py:40,52) is needed; the probabilities stay
  * [N, T, L, R].  Supported by the tensor variant of race_b200_causal_fwd, race_b200_tile_totals and
  * race_b200_causal_fwd_resume for fp32 (S = 64, d_k = 64) and for bf16 with S = 256 or 512 (d_k = 64 or
- * 128); every other entry point, shape and variant rejects heads > 1 with RACE_ERR_SHAPE / reports
- * it as unsupported.
+ * 128), by race_b200_causal_fwd_heads also for bf16 with S = 64, by race_b200_causal_fwd_qkv,
+ * race_b200_decode_step_qkv and race_b200_causal_bwd_heads for the shapes they take; every other entry
+ * point, shape and variant rejects heads > 1 with RACE_ERR_SHAPE / reports it as unsupported.
  */
 #ifndef RACE_B200_H_
 #define RACE_B200_H_
@@ -188,7 +189,8 @@ int race_b200_causal_fwd_qkv(const void* q, const void* k, const void* v, const 
  *   dPK_j[s] = sum_{t>=j} g_t[s] + (sum_{t>=j} W_t[s] dO_t).V_j,  dV_j = sum_s pK_j[s] sum_{t>=j} W_t[s] dO_t.
  * Recomputes the forward's prefix states (nothing has to be saved by the forward).  fp32 with L*R = 64, d_k = 64
  * runs as three plain causal / anti-causal passes of the forward's tcgen05 kernels plus two streaming kernels;
- * every other shape (L*R <= 64 or a multiple of 64 up to 512, d_k <= 128, bf16) on CUDA-core kernels; heads <= 1.  workspace: 256-byte aligned, >= race_b200_causal_bwd_workspace_bytes()
+ * bf16 with L*R 64, 128, 256 or 512 and d_k 64 or 128 on tcgen05 kernels of its own; every other shape (L*R <= 64 or a
+ * multiple of 64 up to 512, d_k <= 128) on CUDA-core kernels; heads <= 1.  workspace: 256-byte aligned, >= race_b200_causal_bwd_workspace_bytes()
  * (two fp32 [N,T,L*R] scratch arrays plus tile states).  status: as in race_b200_causal_fwd (the prefix
  * states come from the forward's tile-totals kernel, whose waits are bounded).
  */

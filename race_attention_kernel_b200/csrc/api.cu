@@ -174,7 +174,7 @@ static int causal_entry(const void* probs_q, const void* probs_k, const void* v,
         !aligned16(workspace) || !aligned16(carry_in) || !aligned16(state_out))
         return RACE_ERR_ALIGN;
     // what race_b200_causal_workspace_bytes says, also where a longer tile would do with less
-    const int asked_tile = tile_tokens > 0 ? tile_tokens : pick_tile(dm, var);
+    const int asked_tile = tile_tokens == 0 && bf16_only ? pick_tile(dm, var) : tile;
     if (workspace_bytes < workspace_bytes_for(dm, shape->dtype, var, asked_tile, /*totals_or_resume=*/phases != kPhaseAll))
         return RACE_ERR_WORKSPACE;
     if (family(var) == RACE_VARIANT_TENSOR)

@@ -9,11 +9,13 @@
 // are taken first, so the common part of dP, which the softmax cancels, does not cost precision.
 //
 // A warp takes 16 rows at a time and nothing but x, dP and dx crosses memory.  Both contractions ([16 x D] . [D x L K]
-// and [16 x L K] . [L K x D]) run on mma.sync m16n8k16 with bf16 hi/lo limbs and fp32 accumulation (bf16 rows of x are
-// exact in one limb).  fp32 rows and their planes take a third limb in the first product: the factor 1 - th^2 =
-// 4 e^(-2 |proj|) / .. turns an absolute error of proj (3e-5 with two limbs) into twice that relative error of dx.  The index permutations of the forward kernel (bucket_probs_mma_wide) put the K planes of whole
-// tables into one lane of a quad, and the accumulators of the first product are, lane by lane, the A fragments of the
-// second; its columns are permuted so that a lane ends up with eight consecutive features of its two rows.
+// and [16 x L K] . [L K x D]) run on mma.sync m16n8k16 with bf16 limbs and fp32 accumulation: bf16 rows of x are exact in
+// one limb, against hi/lo limbs of the planes and of dproj; fp32 rows, their planes and dproj take three limbs and every
+// k-step an accumulator of its own (six_products), since nothing rounds the result afterwards and the factor 1 - th^2 =
+// 4 e^(-2 |proj|) / .. turns an absolute error of proj (3e-5 with two limbs) into twice that relative error of dx.  The
+// index permutations of the forward kernel (bucket_probs_mma_wide) put the K planes of whole tables into one lane of a quad,
+// and the accumulators of the first product are, lane by lane, the A fragments of the second; its columns are permuted so
+// that a lane ends up with eight consecutive features of its two rows.
 // Bound by memory (x, dP in, dx out) at d_k = 64, by the 240 mma.sync per 16 rows at d_k = 128, L = 8, K = 6.
 #include <algorithm>
 

@@ -7,6 +7,8 @@
 
 #include <cudaTypedefs.h>
 
+#include <atomic>
+
 namespace race {
 
 // launch with programmatic dependence on the kernel before (common.cuh); for kernels in which every thread calls chain_wait
@@ -34,11 +36,15 @@ cudaError_t launch_chain(bool chained, void (*kern)(P...), dim3 grid, dim3 block
     return cudaLaunchKernelEx(&cfg, kern, static_cast<A&&>(args)...);
 }
 
-// SMs of the current device (148 where there is none)
+// SMs of the current device (148 where there is none); asked for several times in a call, so the answer is kept per device
 inline int device_sm_count() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 148;
+    static std::atomic<int> known[64];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    if (dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
 }
 
 // the driver's tensor-map encoder (causal_tc.cu); null if it cannot be looked up

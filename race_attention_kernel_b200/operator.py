@@ -13,7 +13,7 @@ accepted and streamed through the device; there is no CPU compute path.
 Gradients: the reference module is differentiable through K, V and Q (plain autograd over
 src/race_baseline.py:41-51).  Here, when autograd is recording and an input requires a gradient,
 ``forward`` is one autograd node over the kernels: the producer, the prefix forward, and for the gradients
-the causal backward and the backward of the producer (in C++ where every kernel takes the operator's layout).  Geometries the producer's backward does not cover form
+the causal backward and the backward of the producer (in C++ where every kernel takes the operator's layout).  Geometries the producer's backward does not cover, planes with a gradient and other prototypes form
 the bucket probabilities with differentiable torch ops and run the prefix path through ``ops.race_causal``.
 """
 from __future__ import annotations
@@ -135,7 +135,7 @@ class BatchedACE(nn.Module):
             return False
         seen = self.__dict__.get("_protos_seen")
         if seen is None or p.is_inference() or seen[0] is not p or seen[1:3] != (p._version, p.data_ptr()):
-            same = torch.equal(p.detach().to("cpu", torch.float64), _corners(self.K))
+            same = torch.equal(p.detach().cpu().double(), _corners(self.K))
             if p.is_inference():
                 return same
             seen = self.__dict__["_protos_seen"] = (p, p._version, p.data_ptr(), same)
