@@ -18,7 +18,6 @@ the bucket probabilities with differentiable torch ops and run the prefix path t
 """
 from __future__ import annotations
 
-import functools
 import itertools
 
 import torch
@@ -71,12 +70,6 @@ class _CausalOperator(torch.autograd.Function):
         return dK, dV if want_v else None, dQ, None, None, None, None
 
 
-@functools.cache
-def _corners(K: int) -> torch.Tensor:
-    """[K, 2**K] (src/race_baseline.py:30-32), on the host; not to be written to."""
-    return torch.tensor(list(itertools.product([-1.0, 1.0], repeat=K)), dtype=torch.float64, device="cpu").T
-
-
 def _on_boundary(x: torch.Tensor) -> torch.Tensor:
     """The kernels want 16-byte boundaries; gradients are also given for rows that begin elsewhere."""
     return x if x.data_ptr() % 16 == 0 else x.clone()
@@ -102,7 +95,9 @@ class BatchedACE(nn.Module):
         # construction gives the same planes
         planes = torch.randn(L, K, d_k, device=device)
         self.register_buffer("planes_T", planes.view(L * K, d_k).T)
-        self.register_buffer("protos_T", _corners(K).to(device, torch.get_default_dtype(), copy=True))
+        corners = torch.tensor(list(itertools.product([-1.0, 1.0], repeat=K)), device=device)
+        self.register_buffer("protos_T", corners.T)
+        self._protos_hold_corners()
         self.eps = 1e-6
         self.variant = "auto"
         # form the bucket probabilities inside the prefix kernels where that path exists (fp32, d_k = 64, L = 4,
@@ -126,26 +121,40 @@ class BatchedACE(nn.Module):
         logits = proj.tanh().div(dk ** 0.5) @ protos_T
         return torch.softmax(logits, dim=-1).to(x2.dtype)
 
+    def _protos_unchanged(self, p) -> bool:
+        """The buffer is the tensor last found to hold the corners, and has not been written to since."""
+        seen = self.__dict__.get("_protos_seen")
+        return seen is not None and seen[0] is p and not p.is_inference() and seen[1:] == (p._version, p.data_ptr())
+
     def _protos_are_corners(self) -> bool:
         """Whether ``protos_T`` holds what the kernels are built on: training honours other prototypes, with torch ops.
         Compared by value, which reads back from the GPU, when the buffer is another tensor than at the last comparison or
         has been written to since (its version counter; writes through ``.data`` are not counted by torch)."""
         p = self.protos_T
-        if p.requires_grad:
-            return False
-        seen = self.__dict__.get("_protos_seen")
-        if seen is None or p.is_inference() or seen[0] is not p or seen[1:3] != (p._version, p.data_ptr()):
-            same = torch.equal(p.detach().cpu().double(), _corners(self.K))
-            if p.is_inference():
-                return same
-            seen = self.__dict__["_protos_seen"] = (p, p._version, p.data_ptr(), same)
-        return seen[3]
+        if self._protos_unchanged(p):
+            return not p.requires_grad
+        same = p.dim() == 2 and p.T.tolist() == [list(c) for c in itertools.product([-1.0, 1.0], repeat=self.K)]
+        if same:
+            self._protos_hold_corners()
+        return same and not p.requires_grad
 
-    def _apply(self, fn, *args, **kwargs):
-        super()._apply(fn, *args, **kwargs)
-        if not self.protos_T.is_meta:
-            self._protos_are_corners()   # read back here, where tensors move anyway, and not in the first training step
+    def _protos_hold_corners(self) -> None:
+        p = self.protos_T
+        if type(p) is torch.Tensor and not p.is_meta and not p.is_inference():
+            self.__dict__["_protos_seen"] = (p, p._version, p.data_ptr())
+
+    def _move(self, move, *args, **kwargs):
+        known = self._protos_unchanged(self.protos_T)
+        move(*args, **kwargs)
+        if known:   # the same values elsewhere: nothing to read back
+            self._protos_hold_corners()
         return self
+
+    def to(self, *args, **kwargs):
+        return self._move(super().to, *args, **kwargs)
+
+    def cuda(self, *args, **kwargs):
+        return self._move(super().cuda, *args, **kwargs)
 
     def _forward_autograd(self, Khf, Vhf, Qhf):
         M, B, T, H, dk = Khf.shape
