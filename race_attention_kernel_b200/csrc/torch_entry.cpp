@@ -47,8 +47,8 @@ at::Tensor bytes(size_t n, const at::Tensor& like) {
     return at::empty({(int64_t)(n < 256 ? 256 : n)}, like.options().dtype(at::kByte));
 }
 
-// planes_T [d_k, L K] (any strides) -> a tensor whose memory is fp32 [L K, d_k]; usually the buffer is the transposed view
-// of exactly that, and is returned as it is (a view of it would take a third of a microsecond of a step's six)
+// planes_T [d_k, L K] (any type, strides) -> the same in fp32 with the memory of rows, [L K, d_k]; usually the buffer is the
+// transposed view of exactly that, and is returned as it is (a view of it would take a third of a microsecond of a step's six)
 at::Tensor planes_rows(const at::Tensor& planes_T, const at::Tensor& ref) {
     if (planes_T.scalar_type() == at::kFloat && planes_T.device() == ref.device() && planes_T.layout() == at::kStrided &&
         planes_T.stride(0) == 1 && planes_T.stride(1) == planes_T.size(0))
@@ -56,7 +56,7 @@ at::Tensor planes_rows(const at::Tensor& planes_T, const at::Tensor& ref) {
     at::Tensor p = planes_T.t();
     if (p.device() != ref.device() || p.scalar_type() != at::kFloat)
         p = p.to(ref.options().dtype(at::kFloat));
-    return p.contiguous();
+    return p.contiguous().t();
 }
 
 // The kernels want 16-byte boundaries.  A contiguous tensor off them is refused by the C entries, except where this package
@@ -255,14 +255,17 @@ struct TrainOp : torch::autograd::Function<TrainOp> {
 
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
         const auto saved = ctx->get_saved_variables();
-        const at::Tensor &k = saved[0], &v = saved[1], &q = saved[2], &planes = saved[3], &pk = saved[4], &pq = saved[5];
         const auto dims = ctx->saved_data["dims"].toIntVector();
         const int64_t L = dims[0], P = dims[1];
         int* status = (int*)dims[2];
         torch::autograd::variable_list res(8);
         {
             at::AutoGradMode no_grad(false);
-            c10::cuda::CUDAGuard guard(k.device());
+            c10::cuda::CUDAGuard guard(saved[0].device());
+            // (hooks on saved tensors may hand back other memory: the kernels need dense rows)
+            auto dense = [](const at::Tensor& t) { return on_boundary(t.contiguous(), true); };
+            const at::Tensor k = dense(saved[0]), v = dense(saved[1]), q = dense(saved[2]), pk = dense(saved[4]), pq = dense(saved[5]);
+            const at::Tensor planes = on_boundary(planes_rows(saved[3], k), true);
             void* stream = c10::cuda::getCurrentCUDAStream().stream();
             const RaceShape sh = shape(k, L, P, ctx->saved_data["eps"].toDouble());
             const at::Tensor g = on_boundary(grads[0].to(v.scalar_type()).contiguous(), true);   // may come expanded (stride 0)

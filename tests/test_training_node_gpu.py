@@ -69,3 +69,28 @@ def test_fp32_with_wide_rows(B, T, H):
     ref = (o, *torch.autograd.grad(o, (k, v, q), x[3].double()))
     for a, b in zip(_call(ace, x[:3], x[3]), ref):
         assert ro.rel_l2(a, b) <= 20 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("dk,K,L,dt", GEOMETRIES)
+def test_saved_tensors_that_go_elsewhere(dk, K, L, dt):
+    """Hooks and dispatch modes around the node in C++: what comes back may lie in memory differently."""
+    from torch.autograd.graph import save_on_cpu, saved_tensors_hooks
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Through(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    ace, x = _setup(dk, K, L, dt)
+    want = _call(ace, x[:3], x[3])
+    strided = saved_tensors_hooks(lambda t: t.transpose(0, 1).contiguous(), lambda t: t.transpose(0, 1))
+    for context in (save_on_cpu(), save_on_cpu(pin_memory=True), strided, Through()):
+        with context:
+            got = _call(ace, x[:3], x[3])
+        assert all(map(torch.equal, got, want))
+    # planes that are stored the other way round, through the same hooks
+    ace.planes_T = ace.planes_T.contiguous()
+    for context in (save_on_cpu(pin_memory=True), strided):
+        with context:
+            got = _call(ace, x[:3], x[3])
+        assert all(map(torch.equal, got, want))
