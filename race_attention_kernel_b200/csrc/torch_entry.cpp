@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -342,6 +343,9 @@ PyObject* guarded(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
             return nullptr;
         }
         return r;
+    } catch (python_error& e) {   // raised by a hook or a mode in Python: on as it is (a checkpoint ends its second run so)
+        e.restore();
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, e.what());
     } catch (const c10::OutOfMemoryError& e) {
         PyObject* mod = PyImport_ImportModule("torch");   // raise the class torch's own allocations raise
         PyObject* cls = mod ? PyObject_GetAttrString(mod, "OutOfMemoryError") : nullptr;

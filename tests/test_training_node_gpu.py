@@ -73,8 +73,9 @@ def test_fp32_with_wide_rows(B, T, H):
 
 @pytest.mark.parametrize("dk,K,L,dt", GEOMETRIES)
 def test_saved_tensors_that_go_elsewhere(dk, K, L, dt):
-    """Hooks and dispatch modes around the node in C++: what comes back may lie in memory differently."""
+    """Hooks, checkpoints and dispatch modes around the node in C++: what comes back may lie in memory differently."""
     from torch.autograd.graph import save_on_cpu, saved_tensors_hooks
+    from torch.utils.checkpoint import checkpoint
     from torch.utils._python_dispatch import TorchDispatchMode
 
     class Through(TorchDispatchMode):
@@ -88,6 +89,10 @@ def test_saved_tensors_that_go_elsewhere(dk, K, L, dt):
         with context:
             got = _call(ace, x[:3], x[3])
         assert all(map(torch.equal, got, want))
+    leaves = [t.detach().requires_grad_(True) for t in x[:3]]
+    out = checkpoint(ace, *leaves, use_reentrant=False)
+    out.backward(x[3])
+    assert all(map(torch.equal, (out, *(t.grad for t in leaves)), want))
     # planes that are stored the other way round, through the same hooks
     ace.planes_T = ace.planes_T.contiguous()
     for context in (save_on_cpu(pin_memory=True), strided):
