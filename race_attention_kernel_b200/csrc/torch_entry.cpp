@@ -25,7 +25,8 @@
 
 namespace {
 
-const at::Tensor* tensor_of(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+// tensors and parameters; subclasses take the general path, which gives their type back
+const at::Tensor* tensor_of(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
 
 // a contiguous CUDA tensor of one of the two element types
 bool plain(const at::Tensor& t) {

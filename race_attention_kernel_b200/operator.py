@@ -159,7 +159,7 @@ class BatchedACE(nn.Module):
     def _forward_autograd(self, Khf, Vhf, Qhf):
         M, B, T, H, dk = Khf.shape
         dev = self.planes_T.device if self.planes_T.is_cuda else torch.device("cuda", torch.cuda.current_device())
-        if (ops.bucket_probs_bwd_is_supported(dk, self.L, self.K, Khf.dtype)
+        if (Khf.numel() and Khf.dtype == Vhf.dtype == Qhf.dtype and ops.bucket_probs_bwd_is_supported(dk, self.L, self.K, Khf.dtype)
                 and not self.planes_T.requires_grad and self._protos_are_corners()):
             planes = self.planes_T.T.contiguous().float().to(dev)
             out = _CausalOperator.apply(*(t.to(dev).contiguous() for t in (Khf, Vhf, Qhf)), planes, self.L, self.K, self.eps)

@@ -169,3 +169,29 @@ def test_other_threads_run_while_a_call_waits(kind, monkeypatch):
     t.join()
     assert waited > 0.2
     assert max(b - a for a, b in zip(stamps, stamps[1:])) < 0.5 * waited
+
+
+@pytest.mark.parametrize("shape", [(0, 5, 3), (2, 0, 3), (2, 5, 0)])
+def test_training_on_nothing(shape):
+    B, T, H = shape
+    x = [t.requires_grad_(True) for t in _inputs(B, T, H, 64, torch.float32)]
+    out = _ace()(*x)
+    assert out.shape == (1, B, T, H, 64)
+    for g, t in zip(torch.autograd.grad(out, x, torch.zeros_like(out)), x):
+        assert g.shape == t.shape
+
+
+def test_training_refuses_mixed_types_in_words():
+    k, v, q = _inputs(1, 5, 2, 64, torch.float32)
+    with pytest.raises(RuntimeError, match="dtype"):
+        _ace()(k.requires_grad_(True), v.double(), q)
+
+
+def test_a_tensor_subclass_gets_its_type_back():
+    class Tagged(torch.Tensor):
+        pass
+
+    ace, x = _ace(), _inputs(1, 70, 2, 64, torch.float32)
+    with torch.no_grad():
+        out = ace(*(t.as_subclass(Tagged) for t in x))
+        assert type(out) is Tagged and torch.equal(out.as_subclass(torch.Tensor), ace(*x))
